@@ -70,12 +70,6 @@ static PlainKernel pick_plain(int bits, bool sgn, int mode) {
   }
 }
 
-static uint32_t pow2_at_least(uint32_t x) {
-  uint32_t p = 1;
-  while (p < x) p <<= 1;
-  return p;
-}
-
 // P(Bin(n, f) >= r) in log space
 static double binom_tail(uint32_t n, double f, uint32_t r) {
   if (r == 0) return 1.0;
@@ -203,6 +197,7 @@ struct Engine {
 
   int plain_grid = 0, smem_optin = 0;
   size_t plain_smem = 0, final_smem = 0;
+  size_t tail_bytes = 0;  // of d_sample_keys: free once the thresholds are known (final_grid)
   // batched pass
   uint32_t* d_qtab = nullptr;     // [blocks][batch_qtab_words(cols)] words
   int batch_warps_n = 0, batch_grid = 0;
@@ -299,6 +294,9 @@ struct Engine {
               cudaStream_t s, bool pre = false);
   int enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score,
                     cudaStream_t s, bool pre = false);
+  // CTAs per query of k_final (FinalArgs::comp and done set in `scratch`, nq queries, where more
+  // than one)
+  uint32_t final_grid(uint32_t nq, void* scratch, size_t scratch_bytes, FinalArgs* fa) const;
   // the final Top-K ranks the candidates by integer score: no FP32 values or no FP32 queries
   bool int_final(const float* d_q) const { return !has_f32 || d_q == nullptr; }
   int repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cudaStream_t s,
@@ -613,11 +611,8 @@ int Engine::apply_config(const Config& c) {
   } else {
     d_qtab_tc = nullptr;
   }
-  {
-    uint32_t kp = 1;
-    while (kp < p.k_max) kp <<= 1;
-    final_smem = final_smem_bytes(cols, std::max(nslots, p.k_max), kp);
-  }
+  final_smem = final_smem_bytes(cols, std::max(nslots, p.k_max), p.k_max);
+  tail_bytes = maxB_blk * std::max<uint32_t>(n_sample_rows, 1) * 4;
   prm = p;
   cur = c;
   configured = true;
@@ -993,8 +988,6 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   sa.cand = d_cand;
   sa.cand_key = d_cand_key;
   sa.status = d_status;
-  k_select<false><<<dim3(split, nq), 512, 0, s>>>(sa);
-  AES_CK(cudaGetLastError());
   FinalArgs fa{};
   fa.csr_ptr = d_csr_ptr;
   fa.csr_col = d_csr_col;
@@ -1004,15 +997,33 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   fa.cols = cols;
   fa.cand = d_cand;
   fa.nslots = nslots;
-  fa.kp = pow2_at_least(k);
   fa.k = k;
   fa.out_idx = d_idx;
   fa.out_score = d_score;
   fa.status = d_status;
   fa.cand_key = int_final(d_q) ? d_cand_key : nullptr;
-  k_final<<<nq, kThreadsFinal, final_smem, s>>>(fa);
+  const uint32_t fg = final_grid(nq, d_sample_keys, tail_bytes, &fa);
+  sa.done = fa.done;
+  k_select<false><<<dim3(split, nq), 512, 0, s>>>(sa);
+  AES_CK(cudaGetLastError());
+  k_final<<<dim3(fg, nq), kThreadsFinal, final_smem, s>>>(fa);
   AES_CK(cudaGetLastError());
   return AES_OK;
+}
+
+// Rescoring is latency-bound (a row pointer, then the row's entries, from DRAM), so a few queries'
+// candidates are spread over CTAs of 64 rows each until there are two CTAs per SM; from twice the
+// SM count of queries on, one CTA per query fills the chip.  The composites pass between a query's
+// CTAs through the sample keys' memory, dead by then; where it is too small, one CTA per query.
+uint32_t Engine::final_grid(uint32_t nq, void* scratch, size_t scratch_bytes, FinalArgs* fa) const {
+  fa->comp = nullptr;
+  fa->done = nullptr;
+  constexpr uint32_t per = (kThreadsFinal / 32) * kFinalRows;
+  const uint32_t g = std::min((fa->nslots + per - 1) / per, 2u * (uint32_t)sm_count / nq);
+  if (fa->cand_key || g <= 1 || (size_t)nq * (fa->nslots * 8ull + 4) > scratch_bytes) return 1;
+  fa->comp = static_cast<uint64_t*>(scratch);
+  fa->done = reinterpret_cast<uint32_t*>(fa->comp + (size_t)nq * fa->nslots);
+  return g;
 }
 
 // Replays the launch sequence of enqueue() as one CUDA graph (captured on first use for these
@@ -1086,8 +1097,6 @@ int Engine::repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cud
     sa.cand = d_cand;
     sa.cand_key = d_cand_key;
     sa.status = d_status;
-    k_select<true><<<dim3(split, 1), 512, 0, s>>>(sa);
-    AES_CK(cudaGetLastError());
     FinalArgs fa{};
     fa.csr_ptr = d_csr_ptr;
     fa.csr_col = d_csr_col;
@@ -1097,13 +1106,16 @@ int Engine::repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cud
     fa.cols = cols;
     fa.cand = d_cand + (size_t)q * nslots;
     fa.nslots = nslots;
-    fa.kp = pow2_at_least(k);
     fa.k = k;
     fa.out_idx = d_idx + (size_t)q * k;
     fa.out_score = d_score + (size_t)q * k;
     fa.status = nullptr;
     fa.cand_key = last_int_final ? d_cand_key + (size_t)q * nslots : nullptr;
-    k_final<<<1, kThreadsFinal, final_smem, s>>>(fa);
+    const uint32_t fg = final_grid(1, d_sample_keys, tail_bytes, &fa);
+    sa.done = fa.done;
+    k_select<true><<<dim3(split, 1), 512, 0, s>>>(sa);
+    AES_CK(cudaGetLastError());
+    k_final<<<fg, kThreadsFinal, final_smem, s>>>(fa);
     AES_CK(cudaGetLastError());
   }
   if (nrep) {
@@ -1490,8 +1502,6 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
   if (!e.has_f32) return aes::fail(AES_ERR_STATE, "the matrix was created without FP32 values");
   if (!e.q32_given) return aes::fail(AES_ERR_STATE, "the loaded queries have no FP32 values");
   AES_CK(cudaSetDevice(e.device));
-  uint32_t kp = 1;
-  while (kp < k) kp <<= 1;
   // Filtered select: every S-th row key is a sample; its r-th largest key lies below the K-th
   // largest key of all rows except with probability 1e-12 (binomial tail), so only the rows at or
   // above it need the select.  S is the largest power of two whose expected survivors fit the
@@ -1524,13 +1534,14 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
   fa.cols = e.cols;
   fa.cand = e.d_exact_cand;
   fa.nslots = k;
-  fa.kp = kp;
   fa.k = k;
   fa.out_idx = e.d_out_idx;
   fa.out_score = e.d_out_score;
   fa.status = nullptr;
   fa.cand_key = nullptr;
+  const uint32_t fg = e.final_grid(1, e.d_sample_keys, e.tail_bytes, &fa);
   SelectArgs sa{};
+  sa.done = fa.done;
   sa.q0 = 0;
   sa.split = 1;
   sa.slice = e.rows;
@@ -1564,7 +1575,7 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
       k_select<true><<<dim3(1, 1), 512, 0, e.stream>>>(sa);
     }
     AES_CK(cudaGetLastError());
-    k_final<<<1, kThreadsFinal, e.final_smem, e.stream>>>(fa);
+    k_final<<<fg, kThreadsFinal, e.final_smem, e.stream>>>(fa);
     AES_CK(cudaGetLastError());
     AES_CK(cudaEventRecord(e.ev1, e.stream));
     AES_CK(cudaMemcpyAsync(e.h_status, e.d_status, 4, cudaMemcpyDeviceToHost, e.stream));
@@ -1577,7 +1588,7 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
       sa.allkeys = e.d_allkeys;
       k_select<true><<<dim3(1, 1), 512, 0, e.stream>>>(sa);
       AES_CK(cudaGetLastError());
-      k_final<<<1, kThreadsFinal, e.final_smem, e.stream>>>(fa);
+      k_final<<<fg, kThreadsFinal, e.final_smem, e.stream>>>(fa);
       AES_CK(cudaGetLastError());
       AES_CK(cudaEventRecord(e.ev1, e.stream));
       AES_CK(cudaStreamSynchronize(e.stream));
@@ -1785,8 +1796,6 @@ extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, 
   sa.cand = cand;
   sa.cand_key = cand_key;
   sa.status = status;
-  k_select<false><<<dim3(e.split, 1), 512, 0, s>>>(sa);
-  AES_CK(cudaGetLastError());
   FinalArgs fa{};
   fa.csr_ptr = e.d_csr_ptr;
   fa.csr_col = e.d_csr_col;
@@ -1796,13 +1805,16 @@ extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, 
   fa.cols = e.cols;
   fa.cand = cand;
   fa.nslots = e.nslots;
-  fa.kp = aes::pow2_at_least(k);
   fa.k = k;
   fa.out_idx = d_idx;
   fa.out_score = d_score;
   fa.status = status;
   fa.cand_key = e.has_f32 ? nullptr : cand_key;
-  k_final<<<1, kThreadsFinal, e.final_smem, s>>>(fa);
+  const uint32_t fg = e.final_grid(1, skeys, L.thr - L.skeys, &fa);
+  sa.done = fa.done;
+  k_select<false><<<dim3(e.split, 1), 512, 0, s>>>(sa);
+  AES_CK(cudaGetLastError());
+  k_final<<<fg, kThreadsFinal, e.final_smem, s>>>(fa);
   AES_CK(cudaGetLastError());
   // counted like aes_run_device's launches: quantise, sample pass, threshold, filter pass,
   // select, final
@@ -1824,7 +1836,7 @@ extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, 
     k_select<true><<<dim3(e.split, 1), 512, 0, s>>>(sa);
     AES_CK(cudaGetLastError());
     fa.status = nullptr;
-    k_final<<<1, kThreadsFinal, e.final_smem, s>>>(fa);
+    k_final<<<fg, kThreadsFinal, e.final_smem, s>>>(fa);
     AES_CK(cudaGetLastError());
     AES_CK(cudaStreamSynchronize(s));
   }

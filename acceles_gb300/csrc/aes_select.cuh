@@ -123,6 +123,53 @@ __device__ __forceinline__ void warp_find_suffix_bin(const uint32_t* hist, int n
   }
 }
 
+// The bin holding the need-th largest item of a kHistBins histogram (1 <= need <= its total):
+// {bin, items above it, items in it}.  Every thread of a THREADS-wide block calls it; sh holds
+// THREADS / 32 + 3 words.  Each thread sums its share of the bins, a warp scan and the warps'
+// totals give the items above it: two barriers, where one warp walking 64 bins per lane took 2 us.
+struct TopBin {
+  uint32_t bin, above, in;
+};
+template <int THREADS>
+__device__ __forceinline__ TopBin block_top_bin(const uint32_t* hist, uint32_t need, uint32_t* sh) {
+  constexpr int PER = kHistBins / THREADS, NW = THREADS / 32;
+  static_assert(PER == 2 || PER == 4 || PER == 8, "bins per thread");
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t h[PER], own = 0;
+#pragma unroll
+  for (int i = 0; i < PER; i++) {
+    h[i] = hist[threadIdx.x * PER + i];
+    own += h[i];
+  }
+  uint32_t incl = own;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t u = __shfl_down_sync(0xFFFFFFFFu, incl, d);
+    if (lane + d < 32) incl += u;
+  }
+  if (lane == 0) sh[warp] = incl;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < NW; w++) incl += w > (int)warp ? sh[w] : 0u;
+  uint32_t acc = incl - own;
+  if (acc < need && incl >= need) {
+    bool found = false;
+#pragma unroll
+    for (int i = PER - 1; i >= 0; i--) {
+      if (!found && acc + h[i] >= need) {
+        sh[NW] = threadIdx.x * PER + i;
+        sh[NW + 1] = acc;
+        sh[NW + 2] = h[i];
+        found = true;
+      }
+      acc += h[i];
+    }
+  }
+  __syncthreads();
+  const TopBin r{sh[NW], sh[NW + 1], sh[NW + 2]};
+  return r;
+}
+
 // ---------------------------------------------------------------------------------------------
 // k_threshold: per (query, partition), a lower bound L of the r-th largest sample key (exact
 // within 2^shift2), so that every row at or above the partition's Top-CK boundary has a key
@@ -358,6 +405,7 @@ struct SelectArgs {
   uint32_t* cand;           // [nq][split*ntop] rows, 0xFFFFFFFF = empty slot
   uint32_t* cand_key;       // [nq][split*ntop]
   uint32_t* status;         // [nq]
+  uint32_t* done;           // [nq] (implicit: [1]) or null: k_final's CTA counters, zeroed here
 };
 
 template <bool IMPLICIT>
@@ -372,6 +420,7 @@ __global__ void k_select(SelectArgs a) {
   const uint32_t need = min(a.ntop, prow);
   uint32_t* cr = a.cand + ((size_t)q * a.split + p) * a.ntop;
   uint32_t* ck = a.cand_key + ((size_t)q * a.split + p) * a.ntop;
+  if (a.done && p == 0 && threadIdx.x == 0) a.done[IMPLICIT ? 0u : q] = 0u;
   for (uint32_t i = threadIdx.x; i < a.ntop; i += blockDim.x) { cr[i] = 0xFFFFFFFFu; ck[i] = 0; }
   uint32_t n;
   if (IMPLICIT) {
@@ -418,11 +467,17 @@ __global__ void k_select(SelectArgs a) {
 // ---------------------------------------------------------------------------------------------
 // k_final: FP32 rescoring of every candidate (sequential over the row's entries in column
 // order, separately rounded multiply and add) and the final Top-K in sort_tuples order.
-// One CTA per query. Each warp rescores 32 slots at a time: it loads its rows' entries row by
-// row (lane = entry, coalesced, 8 rows in flight), stages the rounded products in shared memory
-// and each lane then sums its own row's products in entry order. The K largest (score, row)
-// composites are found by a block radix select, then only those are sorted by a bitonic network
-// in shared memory.
+//
+// Bound by latency: a candidate row is a dependent chain of the row pointer, then its entries,
+// from DRAM.  So the candidates of a few queries are spread over gridDim.x CTAs of 16 warps each,
+// and a warp takes 4 rows at a time: their entries are loaded row by row (lane = entry, coalesced;
+// up to 128 per row in one round trip), the rounded products staged in shared memory, and lane r
+// then sums row r's products in entry order.  The query's last CTA to finish selects the K best
+// (score, row) composites.  With several hundred queries gridDim.x is 1, the composites stay in
+// shared memory and, where there are rows for every warp, a warp takes 32 at a time, which costs
+// a quarter of the summing steps.
+// Selection: one 2048-bin histogram of the scores leaves K and a few more, which are ranked by
+// counting (or, past 256, sorted).
 // ---------------------------------------------------------------------------------------------
 struct FinalArgs {
   const uint32_t* csr_ptr;   // [rows+1]
@@ -431,7 +486,7 @@ struct FinalArgs {
   const float* q32;          // [nq][ld32]
   uint32_t ld32, cols;
   const uint32_t* cand;      // [nq][nslots]
-  uint32_t nslots, kp, k;    // kp: power of two >= k
+  uint32_t nslots, k;
   uint32_t* out_idx;         // [nq][k]
   float* out_score;          // [nq][k]
   const uint32_t* status;    // [nq]; queries with a set status are left to the repair path
@@ -439,112 +494,234 @@ struct FinalArgs {
   // integer candidate score (no FP32 rescoring: a pre-quantised matrix or query without FP32
   // values) and out_score holds that score
   const uint32_t* cand_key;
+  uint64_t* comp;            // gridDim.x > 1: [nq][nslots] composites between the CTAs of a query
+  uint32_t* done;            // gridDim.x > 1: [nq] CTAs finished, zero before the launch
 };
 
 constexpr int kThreadsFinal = 512;  // two CTAs per SM: a 256-query batch runs in one wave
-constexpr int kFinalStageLd = 33;   // staged products: 32 rows x 33 floats per warp
+constexpr int kFinalRows = 4;       // several CTAs per query: candidate rows a warp takes at a time
+constexpr int kFinalChunk = 128;    // and entries per row staged at a time
+constexpr int kFinalStage = 32 * 33;  // staged products per warp: 32 rows x 32 or 4 x 128, padded
+static_assert(kFinalRows * (kFinalChunk + 1) <= kFinalStage, "staging");
+constexpr uint32_t kFinalRankMax = 256;  // survivors of the histogram ranked by counting
 
+// slots of the selected composites: K and what shares the K-th one's histogram bin
+__host__ __device__ inline uint32_t final_list_slots(uint32_t k) {
+  uint32_t n = 512;
+  while (n < 2 * k) n <<= 1;
+  return n;
+}
 // dynamic shared memory of k_final: the query, the composites of all slots, then one region
-// holding first the per-warp product staging and afterwards the kp selected composites
-__host__ __device__ inline size_t final_smem_bytes(uint32_t cols, uint32_t nslots, uint32_t kp) {
-  const size_t stage = (size_t)(kThreadsFinal / 32) * 32 * kFinalStageLd * 4;
-  const size_t top = (size_t)kp * 8;
+// holding first the per-warp product staging and afterwards the selected composites
+__host__ __device__ inline size_t final_smem_bytes(uint32_t cols, uint32_t nslots, uint32_t k) {
+  const size_t stage = (size_t)(kThreadsFinal / 32) * kFinalStage * 4;
+  const size_t top = (size_t)final_list_slots(k) * 8;
   return (((size_t)cols * 4 + 15) & ~(size_t)15) + (size_t)nslots * 8 + (stage > top ? stage : top);
+}
+
+// FP32 scores of the candidate rows of one warp's group of ROWS: lane r < ROWS gets the score of
+// its row (s: its first entry, n: its entries; 0 for the other lanes).  CHUNK entries of every row
+// are staged at a time, the loads of several rows in flight.
+template <int ROWS, int CHUNK>
+__device__ __forceinline__ float rescore_rows(const FinalArgs& a, const float* qs, float* sp,
+                                              uint32_t s, uint32_t n) {
+  constexpr int U = CHUNK / 32, LD = CHUNK + 1;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t longest = __reduce_max_sync(0xFFFFFFFFu, n);
+  float acc = 0.0f;
+  for (uint32_t c = 0; c < longest; c += CHUNK) {
+    if (U == 1 || longest - c <= 32u) {
+#pragma unroll 8
+      for (int j = 0; j < ROWS; j++) {
+        const uint32_t sj = __shfl_sync(0xFFFFFFFFu, s, j), nj = __shfl_sync(0xFFFFFFFFu, n, j);
+        const uint32_t o = c + lane;
+        float p = 0.0f;
+        if (o < nj) p = __fmul_rn(__ldg(a.csr_val + sj + o), qs[__ldg(a.csr_col + sj + o)]);
+        sp[j * LD + lane] = p;
+      }
+    } else {
+      constexpr int J = ROWS < 4 ? ROWS : 4;  // rows in flight
+#pragma unroll 1
+      for (int j0 = 0; j0 < ROWS; j0 += J) {
+        float v[J][U];
+        uint32_t cc[J][U];
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+          const uint32_t sj = __shfl_sync(0xFFFFFFFFu, s, j0 + j), nj = __shfl_sync(0xFFFFFFFFu, n, j0 + j);
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            const uint32_t o = c + lane + 32u * u;
+            v[j][u] = o < nj ? __ldg(a.csr_val + sj + o) : 0.0f;
+            cc[j][u] = o < nj ? __ldg(a.csr_col + sj + o) : 0u;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < J; j++)
+#pragma unroll
+          for (int u = 0; u < U; u++)
+            sp[(j0 + j) * LD + lane + 32 * u] = __fmul_rn(v[j][u], qs[cc[j][u]]);
+      }
+    }
+    __syncwarp();
+    const uint32_t m = n > c ? min(n - c, (uint32_t)CHUNK) : 0u;
+    for (uint32_t e = 0; e < m; e++) acc = __fadd_rn(acc, sp[lane * LD + e]);
+    __syncwarp();
+  }
+  return acc;
 }
 
 __global__ void __launch_bounds__(kThreadsFinal, 2) k_final(FinalArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ uint32_t hist[256];
+  __shared__ __align__(16) uint32_t hist[kHistBins];
   __shared__ uint64_t sh64[72];
-  __shared__ uint32_t s_cnt;
+  __shared__ uint32_t sh[kThreadsFinal / 32 + 3], swmin[kThreadsFinal / 32], swmax[kThreadsFinal / 32],
+      swn[kThreadsFinal / 32];
+  __shared__ uint32_t s_cnt, s_last;
   float* qs = reinterpret_cast<float*>(smem);
   uint64_t* comp = reinterpret_cast<uint64_t*>(smem + ((a.cols * 4 + 15) & ~15u));
-  uint64_t* top = comp + a.nslots;  // after the rescoring; the product staging before it
-  const uint32_t q = blockIdx.x;
+  uint64_t* list = comp + a.nslots;  // after the rescoring; the product staging before it
+  const uint32_t q = blockIdx.y;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (a.status && a.status[q]) return;
-  if (!a.cand_key) {
-    const float* x = a.q32 + (size_t)q * a.ld32;
-    for (uint32_t j = threadIdx.x; j < a.cols; j += blockDim.x) qs[j] = x[j];
-  }
-  if (threadIdx.x == 0) s_cnt = 0;
-  __syncthreads();
   const uint32_t* cr = a.cand + (size_t)q * a.nslots;
-  if (a.cand_key) {  // integer ranking: the candidate keys themselves
+  if (threadIdx.x == 0) s_cnt = 0;
+  if (a.cand_key) {  // integer ranking: the candidate keys themselves (one CTA per query)
     const uint32_t* ck = a.cand_key + (size_t)q * a.nslots;
     for (uint32_t i = threadIdx.x; i < a.nslots; i += blockDim.x) {
       const uint32_t row = cr[i];
       comp[i] = row != 0xFFFFFFFFu ? ((uint64_t)ck[i] << 32) | row : 0ull;
     }
   } else {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    float* sp = reinterpret_cast<float*>(top) + warp * (32 * kFinalStageLd);
-    for (uint32_t g = warp * 32; g < a.nslots; g += nwarps * 32) {
+    const float* x = a.q32 + (size_t)q * a.ld32;
+    for (uint32_t j = threadIdx.x; j < a.cols; j += blockDim.x) qs[j] = x[j];
+    __syncthreads();
+    const bool many = gridDim.x > 1;
+    const bool few = many || a.nslots < 32u * (kThreadsFinal / 32);  // a group of 32 leaves warps idle
+    const uint32_t rows = few ? kFinalRows : 32u;
+    float* sp = reinterpret_cast<float*>(list) + warp * kFinalStage;
+    const uint32_t step = gridDim.x * (kThreadsFinal / 32) * rows;
+    for (uint32_t g = (blockIdx.x * (kThreadsFinal / 32) + warp) * rows; g < a.nslots; g += step) {
       const uint32_t i = g + lane;
-      const uint32_t row = i < a.nslots ? cr[i] : 0xFFFFFFFFu;
+      const bool mine = lane < rows && i < a.nslots;
+      const uint32_t row = mine ? cr[i] : 0xFFFFFFFFu;
       uint32_t s = 0, n = 0;
       if (row != 0xFFFFFFFFu) {
-        s = a.csr_ptr[row];
-        n = a.csr_ptr[row + 1] - s;
+        s = __ldg(a.csr_ptr + row);
+        n = __ldg(a.csr_ptr + row + 1) - s;
       }
-      const uint32_t rounds = (__reduce_max_sync(0xFFFFFFFFu, n) + 31) >> 5;
-      float acc = 0.0f;
-      for (uint32_t r = 0; r < rounds; r++) {
-        const uint32_t o = r * 32 + lane;
-#pragma unroll 8
-        for (int j = 0; j < 32; j++) {
-          const uint32_t sj = __shfl_sync(0xFFFFFFFFu, s, j), nj = __shfl_sync(0xFFFFFFFFu, n, j);
-          float p = 0.0f;
-          if (o < nj) p = __fmul_rn(__ldg(a.csr_val + sj + o), qs[__ldg(a.csr_col + sj + o)]);
-          sp[j * kFinalStageLd + lane] = p;
-        }
-        __syncwarp();
-        const uint32_t m = n > r * 32 ? min(n - r * 32, 32u) : 0u;
-        for (uint32_t e = 0; e < m; e++) acc = __fadd_rn(acc, sp[lane * kFinalStageLd + e]);
-        __syncwarp();
+      const float acc = few ? rescore_rows<kFinalRows, kFinalChunk>(a, qs, sp, s, n)
+                            : rescore_rows<32, 32>(a, qs, sp, s, n);
+      if (mine) {
+        const uint64_t c = row != 0xFFFFFFFFu ? ((uint64_t)key_f32(acc) << 32) | row : 0ull;
+        if (many) a.comp[(size_t)q * a.nslots + i] = c;
+        else comp[i] = c;
       }
-      if (i < a.nslots) comp[i] = row != 0xFFFFFFFFu ? ((uint64_t)key_f32(acc) << 32) | row : 0ull;
+    }
+    if (many) {  // the query's last CTA goes on with every CTA's composites
+      __threadfence();
+      __syncthreads();
+      if (threadIdx.x == 0) s_last = atomicAdd(a.done + q, 1u) == gridDim.x - 1;
+      __syncthreads();
+      if (!s_last) return;
+      __threadfence();
+      for (uint32_t i = threadIdx.x; i < a.nslots; i += blockDim.x)
+        comp[i] = __ldcg(reinterpret_cast<const unsigned long long*>(a.comp) + (size_t)q * a.nslots + i);
     }
   }
+  for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) hist[i] = 0;
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < a.kp; i += blockDim.x) top[i] = 0;
-  // composites of filled slots are unique (rows are); empty slots are 0 and never selected
-  const uint32_t need = min(a.k, a.nslots);
-  const uint64_t tau = block_select_tau([&](uint32_t i) -> uint64_t { return comp[i]; }, a.nslots,
-                                        need, hist, sh64);
+  // filled slots (composites of rows are unique and not 0; empty slots are 0), range of their keys
+  uint32_t mn = 0xFFFFFFFFu, mx = 0, nv = 0;
   for (uint32_t i = threadIdx.x; i < a.nslots; i += blockDim.x) {
     const uint64_t c = comp[i];
-    if (c != 0 && c >= tau) {
-      const uint32_t o = atomicAdd(&s_cnt, 1u);
-      if (o < a.kp) top[o] = c;
+    if (c != 0) {
+      mn = min(mn, (uint32_t)(c >> 32));
+      mx = max(mx, (uint32_t)(c >> 32));
+      nv++;
     }
+  }
+  mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+  mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+  nv = __reduce_add_sync(0xFFFFFFFFu, nv);
+  if (lane == 0) {
+    swmin[warp] = mn;
+    swmax[warp] = mx;
+    swn[warp] = nv;
   }
   __syncthreads();
-  // bitonic sort of the kp selected composites, descending
-  for (uint32_t kk = 2; kk <= a.kp; kk <<= 1) {
-    for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
-      for (uint32_t i = threadIdx.x; i < a.kp; i += blockDim.x) {
-        uint32_t l = i ^ j;
-        if (l > i) {
-          uint64_t ci = top[i], cl = top[l];
-          bool desc = ((i & kk) == 0);
-          if (desc ? (ci < cl) : (ci > cl)) { top[i] = cl; top[l] = ci; }
-        }
-      }
-      __syncthreads();
-    }
+  nv = 0;
+#pragma unroll
+  for (int w = 0; w < kThreadsFinal / 32; w++) {
+    mn = min(mn, swmin[w]);
+    mx = max(mx, swmax[w]);
+    nv += swn[w];
   }
-  for (uint32_t i = threadIdx.x; i < a.k; i += blockDim.x) {
-    uint64_t c = (i < a.kp) ? top[i] : 0;
-    uint32_t* oi = a.out_idx + (size_t)q * a.k;
-    float* os = a.out_score + (size_t)q * a.k;
-    if (c == 0) {
-      oi[i] = 0xFFFFFFFFu;
-      os[i] = -__int_as_float(0x7f800000);
-    } else {
-      oi[i] = (uint32_t)c;
-      const uint32_t key = (uint32_t)(c >> 32);
-      os[i] = a.cand_key ? (float)(int32_t)(key ^ 0x80000000u) : key_to_f32(key);
+  const uint32_t need = min(a.k, nv);
+  uint32_t m = 0;
+  if (need) {
+    const uint32_t span = mx - mn;
+    const int bl = span ? 32 - __clz(span) : 0;
+    const int shift = bl > 11 ? bl - 11 : 0;
+    for (uint32_t i = threadIdx.x; i < a.nslots; i += blockDim.x) {
+      const uint64_t c = comp[i];
+      if (c != 0) atomicAdd(&hist[((uint32_t)(c >> 32) - mn) >> shift], 1u);
     }
+    __syncthreads();
+    const TopBin t = block_top_bin<kThreadsFinal>(hist, need, sh);
+    const uint32_t slots = final_list_slots(a.k);
+    uint64_t tau = (uint64_t)(mn + (t.bin << shift)) << 32;
+    m = t.above + t.in;
+    if (m > slots) {  // many equal or nearly equal scores: the exact K-th composite
+      tau = block_select_tau([&](uint32_t i) -> uint64_t { return comp[i]; }, a.nslots, need, hist, sh64);
+      m = need;
+    }
+    for (uint32_t i = threadIdx.x; i < a.nslots; i += blockDim.x) {
+      const uint64_t c = comp[i];
+      if (c != 0 && c >= tau) list[atomicAdd(&s_cnt, 1u)] = c;
+    }
+    __syncthreads();
+  }
+  uint32_t* oi = a.out_idx + (size_t)q * a.k;
+  float* os = a.out_score + (size_t)q * a.k;
+  auto put = [&](uint32_t o, uint64_t c) {
+    oi[o] = (uint32_t)c;
+    const uint32_t key = (uint32_t)(c >> 32);
+    os[o] = a.cand_key ? (float)(int32_t)(key ^ 0x80000000u) : key_to_f32(key);
+  };
+  if (m <= kFinalRankMax) {
+    // a composite's place is the number of larger ones, counted by `per` threads of a warp
+    uint32_t per = 32;
+    while (per > 1 && m * per > kThreadsFinal) per >>= 1;
+    const uint32_t i = threadIdx.x / per, part = threadIdx.x % per;
+    const uint64_t c = i < m ? list[i] : 0ull;
+    uint32_t above = 0;
+    if (i < m)
+      for (uint32_t j = part; j < m; j += per) above += list[j] > c ? 1u : 0u;
+    for (uint32_t d = per >> 1; d > 0; d >>= 1) above += __shfl_xor_sync(0xFFFFFFFFu, above, d);
+    if (i < m && part == 0 && above < need) put(above, c);
+  } else {  // bitonic sort, descending
+    uint32_t np = 1;
+    while (np < m) np <<= 1;
+    for (uint32_t i = m + threadIdx.x; i < np; i += blockDim.x) list[i] = 0;
+    __syncthreads();
+    for (uint32_t kk = 2; kk <= np; kk <<= 1) {
+      for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
+        for (uint32_t i = threadIdx.x; i < np; i += blockDim.x) {
+          const uint32_t l = i ^ j;
+          if (l > i) {
+            const uint64_t ci = list[i], cl = list[l];
+            const bool desc = ((i & kk) == 0);
+            if (desc ? (ci < cl) : (ci > cl)) { list[i] = cl; list[l] = ci; }
+          }
+        }
+        __syncthreads();
+      }
+    }
+    for (uint32_t i = threadIdx.x; i < need; i += blockDim.x) put(i, list[i]);
+  }
+  for (uint32_t i = need + threadIdx.x; i < a.k; i += blockDim.x) {
+    oi[i] = 0xFFFFFFFFu;
+    os[i] = -__int_as_float(0x7f800000);
   }
 }
 
