@@ -136,6 +136,8 @@ struct Engine {
   uint32_t* d_part_sample_begin = nullptr;
   uint32_t* d_part_r = nullptr;
 
+  uint32_t part_samples = 0;  // most sample rows of a partition
+
   uint32_t split = 1, slice = 0, ntop = 0, nslots = 0, ck_eff = 0, cap = 0;
 
   uint32_t maxB = 1, ld32 = 0, ld8 = 0;
@@ -303,6 +305,8 @@ struct Engine {
              uint32_t* repaired);
   int run_plain(int mode, uint32_t q, cudaStream_t s, uint32_t nq_y = 1);
   int run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0 = 0, uint32_t nblk = 0);
+  int run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint32_t* cnt, cudaStream_t s);
+  int run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s);
   int run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair);
   int prof_open(cudaStream_t s);
   int prof_close(cudaStream_t s);
@@ -524,6 +528,9 @@ int Engine::apply_config(const Config& c) {
   ss = c.ss;
   n_sample_tiles = c.n_sample_tiles;
   n_sample_rows = c.n_sample_rows;
+  part_samples = 0;
+  for (uint32_t q = 0; q < split; q++)
+    part_samples = std::max(part_samples, c.part_begin[q + 1] - c.part_begin[q]);
   maxB = c.maxB;
   const aes_params& p = c.p;
 
@@ -913,6 +920,37 @@ int Engine::run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0, uint
   return AES_OK;
 }
 
+// Thresholds of every (query, partition) from the sample keys [nq][n_sample_rows]; resets cnt
+int Engine::run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint32_t* cnt,
+                          cudaStream_t s) {
+  if (part_samples <= kThrWarpKeys) {
+    const uint64_t pairs = (uint64_t)split * nq;  // (below 2^28: max_batch and ck bound both)
+    k_threshold_warp<<<(uint32_t)((pairs + kThrWarps - 1) / kThrWarps), kThrWarps * 32, 0, s>>>(
+        keys, n_sample_rows, d_part_sample_begin, split, (uint32_t)pairs, d_part_r, thr, cnt);
+  } else {
+    k_threshold<<<dim3(split, nq), kThreadsThr, 0, s>>>(keys, n_sample_rows, 0, d_part_sample_begin,
+                                                        split, d_part_r, thr, cnt);
+  }
+  AES_CK(cudaGetLastError());
+  return AES_OK;
+}
+
+// Top-ntop of every (query, partition) of an nq-query batch from the survivors.  A CTA per pair
+// while one wave of them holds every pair (four CTAs per SM), else, where partitions keep few
+// candidates, a warp per pair: 100 queries x 32 partitions 29 -> 15.5 us; 8 x 32 stay at 8 us (a
+// warp per pair 12 us: one pair past its registers holds the rest up).
+int Engine::run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s) {
+  sa.pairs = sa.split * nq;
+  if (sa.ntop <= kSelWarpTop && sa.pairs > 4u * (uint32_t)sm_count) {
+    constexpr uint32_t W = kSelWarpThreads / 32;
+    k_select_warp<<<(sa.pairs + W - 1) / W, kSelWarpThreads, 0, s>>>(sa);
+  } else {
+    k_select<false><<<dim3(sa.split, nq), kThreadsSel, 0, s>>>(sa);
+  }
+  AES_CK(cudaGetLastError());
+  return AES_OK;
+}
+
 int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score,
                     cudaStream_t s, bool pre) {
   AES_CK(cudaMemsetAsync(d_status, 0, nq * 4ull, s));
@@ -954,9 +992,8 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
     AES_CK(cudaGetLastError());
     n_launch++;
   }
-  k_threshold<<<dim3(split, nq), kThreadsThr, 0, s>>>(batched ? d_keys_t : d_sample_keys, n_sample_rows, 0,
-                                              d_part_sample_begin, split, d_part_r, d_thr, d_cnt);
-  AES_CK(cudaGetLastError());
+  int rct = run_threshold(batched ? d_keys_t : d_sample_keys, nq, d_thr, d_cnt, s);
+  if (rct) return rct;
   if (batched) {
     if (use_tc) {
       // two blocks per launch by CTA pairs where there are two; a last odd block alone
@@ -1004,8 +1041,7 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   fa.cand_key = int_final(d_q) ? d_cand_key : nullptr;
   const uint32_t fg = final_grid(nq, d_sample_keys, tail_bytes, &fa);
   sa.done = fa.done;
-  k_select<false><<<dim3(split, nq), 512, 0, s>>>(sa);
-  AES_CK(cudaGetLastError());
+  if ((rct = run_select(sa, nq, s))) return rct;
   k_final<<<dim3(fg, nq), kThreadsFinal, final_smem, s>>>(fa);
   AES_CK(cudaGetLastError());
   return AES_OK;
@@ -1113,7 +1149,7 @@ int Engine::repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cud
     fa.cand_key = last_int_final ? d_cand_key + (size_t)q * nslots : nullptr;
     const uint32_t fg = final_grid(1, d_sample_keys, tail_bytes, &fa);
     sa.done = fa.done;
-    k_select<true><<<dim3(split, 1), 512, 0, s>>>(sa);
+    k_select<true><<<dim3(split, 1), kThreadsSel, 0, s>>>(sa);
     AES_CK(cudaGetLastError());
     k_final<<<fg, kThreadsFinal, final_smem, s>>>(fa);
     AES_CK(cudaGetLastError());
@@ -1569,10 +1605,10 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
       sa.surv = e.d_surv;
       sa.cnt = e.d_cnt;
       sa.cap = e.cap;
-      k_select<false><<<dim3(1, 1), 512, 0, e.stream>>>(sa);
+      k_select<false><<<dim3(1, 1), kThreadsSel, 0, e.stream>>>(sa);
     } else {
       sa.allkeys = e.d_allkeys;
-      k_select<true><<<dim3(1, 1), 512, 0, e.stream>>>(sa);
+      k_select<true><<<dim3(1, 1), kThreadsSel, 0, e.stream>>>(sa);
     }
     AES_CK(cudaGetLastError());
     k_final<<<fg, kThreadsFinal, e.final_smem, e.stream>>>(fa);
@@ -1586,7 +1622,7 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     if (S && e.h_status[0]) {  // the sample bound missed or the buffer overflowed: every row
       AES_CK(cudaEventRecord(e.ev0, e.stream));
       sa.allkeys = e.d_allkeys;
-      k_select<true><<<dim3(1, 1), 512, 0, e.stream>>>(sa);
+      k_select<true><<<dim3(1, 1), kThreadsSel, 0, e.stream>>>(sa);
       AES_CK(cudaGetLastError());
       k_final<<<fg, kThreadsFinal, e.final_smem, e.stream>>>(fa);
       AES_CK(cudaGetLastError());
@@ -1781,9 +1817,7 @@ extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, 
     return AES_OK;
   };
   if ((rc = plain(MODE_SAMPLE, skeys))) return rc;
-  k_threshold<<<dim3(e.split, 1), kThreadsThr, 0, s>>>(skeys, e.n_sample_rows, 0, e.d_part_sample_begin,
-                                               e.split, e.d_part_r, thr, cnt);
-  AES_CK(cudaGetLastError());
+  if ((rc = e.run_threshold(skeys, 1, thr, cnt, s))) return rc;
   if ((rc = plain(MODE_FILTER, nullptr))) return rc;
   SelectArgs sa{};
   sa.surv = surv;
@@ -1812,8 +1846,7 @@ extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, 
   fa.cand_key = e.has_f32 ? nullptr : cand_key;
   const uint32_t fg = e.final_grid(1, skeys, L.thr - L.skeys, &fa);
   sa.done = fa.done;
-  k_select<false><<<dim3(e.split, 1), 512, 0, s>>>(sa);
-  AES_CK(cudaGetLastError());
+  if ((rc = e.run_select(sa, 1, s))) return rc;
   k_final<<<fg, kThreadsFinal, e.final_smem, s>>>(fa);
   AES_CK(cudaGetLastError());
   // counted like aes_run_device's launches: quantise, sample pass, threshold, filter pass,
@@ -1833,7 +1866,7 @@ extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, 
     if ((rc = plain(MODE_ALL, e.d_allkeys))) return rc;
     sa.allkeys = e.d_allkeys;
     sa.q0 = 0;
-    k_select<true><<<dim3(e.split, 1), 512, 0, s>>>(sa);
+    k_select<true><<<dim3(e.split, 1), kThreadsSel, 0, s>>>(sa);
     AES_CK(cudaGetLastError());
     fa.status = nullptr;
     k_final<<<fg, kThreadsFinal, e.final_smem, s>>>(fa);

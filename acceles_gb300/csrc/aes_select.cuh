@@ -82,46 +82,8 @@ __global__ void k_quantize(const float* __restrict__ q32, uint32_t cols, uint32_
 // block helpers
 // ---------------------------------------------------------------------------------------------
 constexpr int kHistBins = 2048;
-constexpr int kThrILP = 4;  // keys in flight per thread in the threshold passes
+constexpr int kThrILP = 12;  // keys in flight per thread in the threshold passes
 constexpr int kThreadsThr = 512;  // at most 64 registers: two CTAs per SM, a 256-query batch in one wave
-
-// Largest bin b with sum(hist[b..]) >= need; *above = sum(hist[b+1..]).  Executed by warp 0.
-__device__ __forceinline__ void warp_find_suffix_bin(const uint32_t* hist, int nbins,
-                                                     uint32_t need, int* bin_out,
-                                                     uint32_t* above_out) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const int per = nbins / 32;
-  // lane l owns bins [l*per, (l+1)*per); suffix sums from the top
-  uint32_t own = 0;
-  for (int i = 0; i < per; i++) own += hist[lane * per + i];
-  // exclusive suffix over lanes: sum of lanes > l
-  uint32_t incl = own;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    uint32_t u = __shfl_down_sync(0xFFFFFFFFu, incl, d);
-    if (lane + d < 32) incl += u;
-  }
-  uint32_t excl = incl - own;  // bins above this lane's chunk
-  // the chunk holding the boundary: excl < need <= incl
-  bool mine = (excl < need) && (incl >= need);
-  uint32_t msk = __ballot_sync(0xFFFFFFFFu, mine);
-  if (msk == 0) {  // need exceeds the total: take everything
-    if (lane == 0) { *bin_out = 0; *above_out = 0; }
-    return;
-  }
-  uint32_t owner = __ffs(msk) - 1;
-  if (lane == owner) {
-    uint32_t acc = excl;
-    int b = (int)(lane * per + per - 1);
-    for (; b >= (int)(lane * per); b--) {
-      uint32_t h = hist[b];
-      if (acc + h >= need) break;
-      acc += h;
-    }
-    *bin_out = b;
-    *above_out = acc;
-  }
-}
 
 // The bin holding the need-th largest item of a kHistBins histogram (1 <= need <= its total):
 // {bin, items above it, items in it}.  Every thread of a THREADS-wide block calls it; sh holds
@@ -170,23 +132,88 @@ __device__ __forceinline__ TopBin block_top_bin(const uint32_t* hist, uint32_t n
   return r;
 }
 
+// The r-th largest (1 <= r <= total) of the keys a warp holds, N per lane (lanes without a key
+// hold 0, which is below every real one or equal to it): the largest t with at least r keys >= t,
+// found bit by bit below the bits that the smallest and the largest key share.
+template <int N>
+__device__ __forceinline__ uint32_t warp_rth_key(const uint32_t (&k)[N], uint32_t mn, uint32_t mx,
+                                                 uint32_t r) {
+  const uint32_t diff = mn ^ mx;
+  if (diff == 0) return mn;
+  int bit = 31 - __clz(diff);
+  uint32_t t = bit == 31 ? 0u : mx & ~((2u << bit) - 1u);
+  for (; bit >= 0; bit--) {
+    const uint32_t c = t | (1u << bit);
+    uint32_t n = 0;
+#pragma unroll
+    for (int i = 0; i < N; i++) n += k[i] >= c ? 1u : 0u;
+    if (__reduce_add_sync(0xFFFFFFFFu, n) >= r) t = c;
+  }
+  return t;
+}
+
 // ---------------------------------------------------------------------------------------------
-// k_threshold: per (query, partition), a lower bound L of the r-th largest sample key (exact
+// k_threshold: per (query, partition), the r-th largest sample key (or a lower bound of it exact
 // within 2^shift2), so that every row at or above the partition's Top-CK boundary has a key
 // >= L with overwhelming probability; a miss is detected later (ST_MISS) and repaired.
 // Also resets the partition's survivor counter.
+//
+// Latency-bound: a few thousand keys from L2 per partition, and a select.  Two forms:
+// k_threshold_warp, one warp per (query, partition), where no partition has more than
+// kThrWarpKeys samples: the keys stay in registers (100 queries x 32 partitions of 195 samples:
+// 43 -> 6.7 us); k_threshold, one CTA each, for the rest.
 // ---------------------------------------------------------------------------------------------
+constexpr uint32_t kThrWarpKeys = 512;   // 16 per lane
+constexpr int kThrWarps = 4;             // (query, partition) pairs per CTA
+constexpr uint32_t kThrRankMax = 128;    // ranks up to which the CTA form selects by group maxima
+constexpr uint32_t kThrListMax = 1024;
+
+__global__ void __launch_bounds__(kThrWarps * 32) k_threshold_warp(
+    const uint32_t* __restrict__ keys_all, uint32_t ld_keys, const uint32_t* __restrict__ part_begin,
+    uint32_t split, uint32_t pairs, const uint32_t* __restrict__ r_part, uint32_t* __restrict__ thr,
+    uint32_t* __restrict__ cnt) {
+  constexpr int N = kThrWarpKeys / 32;
+  const uint32_t i = blockIdx.x * kThrWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  if (i >= pairs) return;
+  const uint32_t p = i % split, q = i / split;
+  const uint32_t a = __ldg(part_begin + p), n = __ldg(part_begin + p + 1) - a, r = __ldg(r_part + p);
+  const uint32_t* kb = keys_all + (size_t)q * ld_keys + a;
+  uint32_t k[N], mn = 0xFFFFFFFFu, mx = 0;
+#pragma unroll
+  for (int u = 0; u < N; u++) {
+    const uint32_t j = u * 32 + lane;
+    k[u] = j < n ? kb[j] : 0u;
+    if (j < n) {
+      mn = min(mn, k[u]);
+      mx = max(mx, k[u]);
+    }
+  }
+  mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+  mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+  // too few samples: keep every row of the partition
+  const uint32_t t = (n < r || r == 0) ? 0u : warp_rth_key<N>(k, mn, mx, r);
+  if (lane == 0) {
+    thr[i] = t;
+    cnt[i] = 0;
+  }
+}
+
 // Sample keys of query q: keys[base(q) + i * stride] with base(q) = q * ld_keys and stride 1
 // (one query per pass), or, when qblk > 0 (batched passes of qblk queries),
 // base(q) = (q / qblk) * qblk * ld_keys + q % qblk and stride qblk.
+//
+// Ranks up to kThrRankMax: every thread's largest key is found in one pass; the r-th largest of
+// those maxima (of 128 groups of four threads where r is small) is a bound that r keys reach and
+// few others do, so the few threads at or above it gather their keys of at least that bound, and
+// the r-th largest of the gathered keys is the answer.  One read of the keys, where two
+// histograms took three: 27 -> 12.8 us for 39k keys, r = 24.  Larger ranks: two histograms.
 __global__ void __launch_bounds__(kThreadsThr, 2) k_threshold(const uint32_t* __restrict__ keys_all, uint32_t ld_keys, uint32_t qblk,
                             const uint32_t* __restrict__ part_begin, uint32_t split,
                             const uint32_t* __restrict__ r_part, uint32_t* __restrict__ thr,
                             uint32_t* __restrict__ cnt) {
-  __shared__ uint32_t hist[kHistBins];
-  __shared__ uint32_t smin[32], smax[32];
-  __shared__ int s_bin;
-  __shared__ uint32_t s_above;
+  __shared__ __align__(16) uint32_t hist[kHistBins];
+  __shared__ uint32_t smin[kThreadsThr / 32], smax[kThreadsThr / 32], sh[kThreadsThr / 32 + 3];
+  __shared__ uint32_t s_bound, s_n;
   const uint32_t p = blockIdx.x, q = blockIdx.y;
   const uint32_t stride = qblk ? qblk : 1u;
   const uint32_t* kb = keys_all + (qblk ? (size_t)(q / qblk) * qblk * ld_keys + q % qblk
@@ -205,43 +232,96 @@ __global__ void __launch_bounds__(kThreadsThr, 2) k_threshold(const uint32_t* __
     if (threadIdx.x == 0) *T = 0;  // too few samples: keep every row of the partition
     return;
   }
-  // every pass reads kThrILP keys per thread before using them: the loops are bound by global
+  // every pass reads several keys per thread before using them: the loops are bound by global
   // load latency otherwise
   uint32_t mn = 0xFFFFFFFFu, mx = 0;
-  for (uint32_t i0 = a; i0 < b; i0 += blockDim.x * kThrILP) {
+  for (uint32_t i0 = a; i0 < b; i0 += kThreadsThr * kThrILP) {
     uint32_t v[kThrILP];
 #pragma unroll
     for (int u = 0; u < kThrILP; u++) {
-      const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
-      v[u] = i < b ? kk[i] : kk[a];
+      const uint32_t i = i0 + u * kThreadsThr + threadIdx.x;
+      v[u] = i < b ? kk[i] : 0u;
     }
 #pragma unroll
     for (int u = 0; u < kThrILP; u++) {
-      mn = min(mn, v[u]);
-      mx = max(mx, v[u]);
+      const uint32_t i = i0 + u * kThreadsThr + threadIdx.x;
+      if (i < b) {
+        mn = min(mn, v[u]);
+        mx = max(mx, v[u]);
+      }
     }
   }
+  if (r <= kThrRankMax && n >= (uint32_t)kThreadsThr) {
+    const uint32_t own = mx;
+    uint32_t* gm = hist;  // group maxima
+    uint32_t per = 1;     // threads per maximum: 128 groups are enough for r <= 32
+    uint32_t g = mx;
+    if (r <= 32u) {
+      per = 4;
+      g = max(g, __shfl_xor_sync(0xFFFFFFFFu, g, 1));
+      g = max(g, __shfl_xor_sync(0xFFFFFFFFu, g, 2));
+    }
+    const uint32_t ng = kThreadsThr / per, mine = threadIdx.x / per;
+    if (threadIdx.x % per == 0) gm[mine] = g;
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    uint32_t gt = 0, ge = 0;
+    for (uint32_t j = threadIdx.x % per; j < ng; j += per) {
+      gt += gm[j] > g ? 1u : 0u;
+      ge += gm[j] >= g ? 1u : 0u;
+    }
+    for (uint32_t d = per >> 1; d > 0; d >>= 1) {
+      gt += __shfl_xor_sync(0xFFFFFFFFu, gt, d);
+      ge += __shfl_xor_sync(0xFFFFFFFFu, ge, d);
+    }
+    if (gt < r && ge >= r) s_bound = g;  // (the same value from every thread that gets here)
+    __syncthreads();
+    const uint32_t bound = s_bound;
+    uint32_t* list = hist + kThreadsThr;  // kThrListMax keys
+    if (own >= bound) {
+      for (uint32_t i0 = a; i0 < b; i0 += kThreadsThr * kThrILP) {
+        uint32_t v[kThrILP];
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    mn = min(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, d));
-    mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, d));
+        for (int u = 0; u < kThrILP; u++) {
+          const uint32_t i = i0 + u * kThreadsThr + threadIdx.x;
+          v[u] = i < b ? kk[i] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < kThrILP; u++) {
+          const uint32_t i = i0 + u * kThreadsThr + threadIdx.x;
+          if (i < b && v[u] >= bound) {
+            const uint32_t o = atomicAdd(&s_n, 1u);
+            if (o < kThrListMax) list[o] = v[u];
+          }
+        }
+      }
+    }
+    __syncthreads();
+    const uint32_t m = s_n;  // >= r
+    if (m <= kThrListMax) {
+      for (uint32_t i = threadIdx.x; i < m; i += kThreadsThr) {
+        const uint32_t v = list[i];
+        uint32_t lgt = 0, lge = 0;
+        for (uint32_t j = 0; j < m; j++) {
+          lgt += list[j] > v ? 1u : 0u;
+          lge += list[j] >= v ? 1u : 0u;
+        }
+        if (lgt < r && lge >= r) *T = v;
+      }
+      return;
+    }
+    __syncthreads();  // many equal keys: the histograms below
   }
+  mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+  mx = __reduce_max_sync(0xFFFFFFFFu, mx);
   if ((threadIdx.x & 31) == 0) { smin[threadIdx.x >> 5] = mn; smax[threadIdx.x >> 5] = mx; }
+  for (int i = threadIdx.x; i < kHistBins; i += kThreadsThr) hist[i] = 0;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    uint32_t nw = (blockDim.x + 31) / 32;
-    mn = threadIdx.x < nw ? smin[threadIdx.x] : 0xFFFFFFFFu;
-    mx = threadIdx.x < nw ? smax[threadIdx.x] : 0u;
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      mn = min(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, d));
-      mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, d));
-    }
-    if (threadIdx.x == 0) { smin[0] = mn; smax[0] = mx; }
+  for (int w = 0; w < kThreadsThr / 32; w++) {
+    mn = min(mn, smin[w]);
+    mx = max(mx, smax[w]);
   }
-  __syncthreads();
-  mn = smin[0];
-  mx = smax[0];
   const uint32_t span = mx - mn;
   if (span == 0) {
     if (threadIdx.x == 0) *T = mn;
@@ -249,51 +329,45 @@ __global__ void __launch_bounds__(kThreadsThr, 2) k_threshold(const uint32_t* __
   }
   const int bl = 32 - __clz(span);           // bits of span
   const int sh1 = bl > 11 ? bl - 11 : 0;
-  for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) hist[i] = 0;
-  __syncthreads();
-  for (uint32_t i0 = a; i0 < b; i0 += blockDim.x * kThrILP) {
+  for (uint32_t i0 = a; i0 < b; i0 += kThreadsThr * kThrILP) {
     uint32_t v[kThrILP];
 #pragma unroll
     for (int u = 0; u < kThrILP; u++) {
-      const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
+      const uint32_t i = i0 + u * kThreadsThr + threadIdx.x;
       v[u] = i < b ? kk[i] : 0u;
     }
 #pragma unroll
     for (int u = 0; u < kThrILP; u++) {
-      const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
+      const uint32_t i = i0 + u * kThreadsThr + threadIdx.x;
       if (i < b) atomicAdd(&hist[(v[u] - mn) >> sh1], 1u);
     }
   }
   __syncthreads();
-  if (threadIdx.x < 32) warp_find_suffix_bin(hist, kHistBins, r, &s_bin, &s_above);
-  __syncthreads();
-  const uint32_t b1 = (uint32_t)s_bin, above1 = s_above;
+  const TopBin t1 = block_top_bin<kThreadsThr>(hist, r, sh);
   if (sh1 == 0) {
-    if (threadIdx.x == 0) *T = mn + b1;
+    if (threadIdx.x == 0) *T = mn + t1.bin;
     return;
   }
   const int sh2 = sh1 > 11 ? sh1 - 11 : 0;
+  for (int i = threadIdx.x; i < kHistBins; i += kThreadsThr) hist[i] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) hist[i] = 0;
-  __syncthreads();
-  for (uint32_t i0 = a; i0 < b; i0 += blockDim.x * kThrILP) {
+  for (uint32_t i0 = a; i0 < b; i0 += kThreadsThr * kThrILP) {
     uint32_t v[kThrILP];
 #pragma unroll
     for (int u = 0; u < kThrILP; u++) {
-      const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
+      const uint32_t i = i0 + u * kThreadsThr + threadIdx.x;
       v[u] = i < b ? kk[i] : 0u;
     }
 #pragma unroll
     for (int u = 0; u < kThrILP; u++) {
-      const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
-      if ((i < b) && (((v[u] - mn) >> sh1) == b1))
+      const uint32_t i = i0 + u * kThreadsThr + threadIdx.x;
+      if ((i < b) && (((v[u] - mn) >> sh1) == t1.bin))
         atomicAdd(&hist[((v[u] - mn) >> sh2) & ((1u << (sh1 - sh2)) - 1u)], 1u);
     }
   }
   __syncthreads();
-  if (threadIdx.x < 32) warp_find_suffix_bin(hist, kHistBins, r - above1, &s_bin, &s_above);
-  __syncthreads();
-  if (threadIdx.x == 0) *T = mn + (b1 << sh1) + ((uint32_t)s_bin << sh2);
+  const TopBin t2 = block_top_bin<kThreadsThr>(hist, r - t1.above, sh);
+  if (threadIdx.x == 0) *T = mn + (t1.bin << sh1) + (t2.bin << sh2);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -392,8 +466,15 @@ __device__ uint64_t block_select_tau(Get get, uint32_t n, uint32_t need, uint32_
 }
 
 // ---------------------------------------------------------------------------------------------
-// k_select: per (query, partition) exact Top-ntop of the survivors by (key desc, row desc).
-// implicit = true reads every row of the partition from a full key array (slow path).
+// k_select: per (query, partition) exact Top-ntop of the survivors by (key desc, row desc), in any
+// order.  implicit = true reads every row of the partition from a full key array (slow path).
+//
+// Latency-bound: some thousand survivors from L2 and a few block-wide steps.  One 2048-bin
+// histogram of the keys puts all but the boundary bin's survivors on one side; those few are ranked
+// by counting (6k survivors: 16 -> 8.4 us; the radix passes before took one 8-bit digit each).  Up
+// to 16 survivors per thread stay in registers between the steps.  Where
+// partitions keep few candidates each (k_select_warp), a warp per (query, partition) bounds the
+// boundary by the maxima of 64 groups of its survivors instead and ranks those above.
 // ---------------------------------------------------------------------------------------------
 struct SelectArgs {
   const uint2* surv;        // [nq][split][cap]
@@ -406,13 +487,120 @@ struct SelectArgs {
   uint32_t* cand_key;       // [nq][split*ntop]
   uint32_t* status;         // [nq]
   uint32_t* done;           // [nq] (implicit: [1]) or null: k_final's CTA counters, zeroed here
+  uint32_t pairs;           // k_select_warp: queries * split
 };
 
+constexpr int kThreadsSel = 512;
+constexpr int kSelKeys = 16;             // survivors per thread kept in registers
+constexpr uint32_t kSelListMax = 1024;   // survivors of the boundary bin ranked by counting
+
+// Block-wide select of the `need` (1 <= need <= n) largest composites of the items key(i), row(i),
+// i < n; each goes to put(slot, key, row), slots 0 .. need - 1 in any order.
+template <int THREADS>
+struct SelectShared {
+  __align__(16) uint32_t hist[kHistBins];
+  uint64_t sh64[72];
+  uint64_t list[kSelListMax];
+  uint32_t sh[THREADS / 32 + 3], wmin[THREADS / 32], wmax[THREADS / 32];
+  uint32_t n_out, n_list;
+};
+template <int THREADS, bool REGS, class Key, class Row, class Put>
+__device__ __forceinline__ void block_select(SelectShared<THREADS>& S, uint32_t n, uint32_t need,
+                                             const Key& key, const Row& row, const Put& put) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  uint32_t k[REGS ? kSelKeys : 1];
+  if constexpr (REGS) {
+#pragma unroll
+    for (int u = 0; u < kSelKeys; u++) k[u] = u * THREADS + tid < n ? key(u * THREADS + tid) : 0u;
+  }
+  // f(item, its key) for this thread's items; every thread of a warp makes the same calls, with
+  // item >= n for none
+  auto each = [&](auto&& f) {
+    if constexpr (REGS) {
+#pragma unroll
+      for (int u = 0; u < kSelKeys; u++)
+        if (u * THREADS < n) f((uint32_t)(u * THREADS) + tid, k[u]);
+    } else {
+      for (uint32_t i0 = 0; i0 < n; i0 += THREADS * 4) {
+        uint32_t v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const uint32_t i = i0 + u * THREADS + tid;
+          v[u] = i < n ? key(i) : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          if (i0 + u * THREADS < n) f(i0 + u * THREADS + tid, v[u]);
+      }
+    }
+  };
+  uint32_t mn = 0xFFFFFFFFu, mx = 0;
+  each([&](uint32_t i, uint32_t v) {
+    if (i < n) {
+      mn = min(mn, v);
+      mx = max(mx, v);
+    }
+  });
+  mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+  mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+  if (lane == 0) {
+    S.wmin[warp] = mn;
+    S.wmax[warp] = mx;
+  }
+  if (tid == 0) S.n_out = S.n_list = 0;
+  for (uint32_t i = tid; i < kHistBins; i += THREADS) S.hist[i] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < THREADS / 32; w++) {
+    mn = min(mn, S.wmin[w]);
+    mx = max(mx, S.wmax[w]);
+  }
+  const uint32_t span = mx - mn;
+  const int bl = span ? 32 - __clz(span) : 0;
+  const int shift = bl > 11 ? bl - 11 : 0;
+  each([&](uint32_t i, uint32_t v) {
+    if (i < n) atomicAdd(&S.hist[(v - mn) >> shift], 1u);
+  });
+  __syncthreads();
+  TopBin t = block_top_bin<THREADS>(S.hist, need, S.sh);
+  uint64_t tau = ~0ull;        // items of the boundary bin that are kept: composites >= tau
+  const bool big = t.in > kSelListMax;
+  if (big)                     // many equal or nearly equal keys: the exact boundary composite
+    tau = block_select_tau([&](uint32_t i) -> uint64_t { return ((uint64_t)key(i) << 32) | row(i); },
+                           n, need, S.hist, S.sh64);
+  each([&](uint32_t i, uint32_t v) {
+    const uint32_t bin = (v - mn) >> shift;
+    bool take = i < n && bin > t.bin;
+    uint32_t r = 0;
+    if (take) r = row(i);
+    if (i < n && bin == t.bin) {
+      r = row(i);
+      if (big) take = (((uint64_t)v << 32) | r) >= tau;
+      else S.list[atomicAdd(&S.n_list, 1u)] = ((uint64_t)v << 32) | r;
+    }
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, take);
+    if (m) {
+      uint32_t o = 0;
+      if (lane == 0) o = atomicAdd(&S.n_out, (uint32_t)__popc(m));
+      o = __shfl_sync(0xFFFFFFFFu, o, 0) + __popc(m & ((1u << lane) - 1u));
+      if (take) put(o, v, r);
+    }
+  });
+  __syncthreads();
+  if (!big) {
+    const uint32_t rest = need - t.above;  // of the boundary bin
+    for (uint32_t i = tid; i < t.in; i += THREADS) {
+      const uint64_t c = S.list[i];
+      uint32_t above = 0;
+      for (uint32_t j = 0; j < t.in; j++) above += S.list[j] > c ? 1u : 0u;
+      if (above < rest) put(t.above + above, (uint32_t)(c >> 32), (uint32_t)c);
+    }
+  }
+}
+
 template <bool IMPLICIT>
-__global__ void k_select(SelectArgs a) {
-  __shared__ uint32_t hist[256];
-  __shared__ uint64_t sh64[72];
-  __shared__ uint32_t s_out;
+__global__ void __launch_bounds__(kThreadsSel, 1) k_select(SelectArgs a) {
+  __shared__ SelectShared<kThreadsSel> S;
   const uint32_t p = blockIdx.x, q = IMPLICIT ? a.q0 : blockIdx.y;
   const uint32_t r0 = p * a.slice;
   const uint32_t r1 = (a.split <= 1 || p == a.split - 1) ? a.n_rows : (p + 1) * a.slice;
@@ -421,46 +609,127 @@ __global__ void k_select(SelectArgs a) {
   uint32_t* cr = a.cand + ((size_t)q * a.split + p) * a.ntop;
   uint32_t* ck = a.cand_key + ((size_t)q * a.split + p) * a.ntop;
   if (a.done && p == 0 && threadIdx.x == 0) a.done[IMPLICIT ? 0u : q] = 0u;
-  for (uint32_t i = threadIdx.x; i < a.ntop; i += blockDim.x) { cr[i] = 0xFFFFFFFFu; ck[i] = 0; }
-  uint32_t n;
-  if (IMPLICIT) {
-    n = (a.split <= 1) ? a.n_rows : prow;
-  } else {
-    n = a.cnt[(size_t)q * a.split + p];
-    if (n > a.cap) {
-      if (threadIdx.x == 0) atomicOr(a.status + q, ST_OVERFLOW);
-      return;
-    }
-    if (n < need) {
-      if (threadIdx.x == 0) atomicOr(a.status + q, ST_MISS);
-      return;
-    }
+  uint32_t n = IMPLICIT ? prow : a.cnt[(size_t)q * a.split + p];
+  const bool over = !IMPLICIT && n > a.cap, miss = !IMPLICIT && n < need;
+  for (uint32_t i = (over || miss ? 0u : need) + threadIdx.x; i < a.ntop; i += kThreadsSel) {
+    cr[i] = 0xFFFFFFFFu;
+    ck[i] = 0;
   }
-  const uint32_t base = (a.split <= 1) ? 0 : r0;
-  const uint2* sv = a.surv + ((size_t)q * a.split + p) * a.cap;
-  auto get = [&](uint32_t i) -> uint64_t {
-    if (IMPLICIT) {
-      uint32_t row = base + i;
-      return ((uint64_t)a.allkeys[row] << 32) | row;
-    } else {
-      uint2 v = sv[i];
-      return ((uint64_t)v.x << 32) | v.y;
-    }
-  };
-  __syncthreads();
+  if (over || miss) {
+    if (threadIdx.x == 0) atomicOr(a.status + q, over ? ST_OVERFLOW : ST_MISS);
+    return;
+  }
   if (need == 0) return;
-  const uint64_t tau = block_select_tau(get, n, need, hist, sh64);
-  if (threadIdx.x == 0) s_out = 0;
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    uint64_t c = get(i);
-    if (c >= tau) {
-      uint32_t o = atomicAdd(&s_out, 1u);
-      if (o < a.ntop) {
-        cr[o] = (uint32_t)c;
-        ck[o] = (uint32_t)(c >> 32);
+  auto put = [&](uint32_t o, uint32_t key, uint32_t row) {
+    cr[o] = row;
+    ck[o] = key;
+  };
+  if constexpr (IMPLICIT) {
+    const uint32_t base = (a.split <= 1) ? 0 : r0;
+    block_select<kThreadsSel, false>(S, n, need, [&](uint32_t i) { return a.allkeys[base + i]; },
+                                     [&](uint32_t i) { return base + i; }, put);
+  } else {
+    const uint2* sv = a.surv + ((size_t)q * a.split + p) * a.cap;
+    auto key = [&](uint32_t i) { return sv[i].x; };
+    auto row = [&](uint32_t i) { return sv[i].y; };
+    if (n <= (uint32_t)(kThreadsSel * kSelKeys)) block_select<kThreadsSel, true>(S, n, need, key, row, put);
+    else block_select<kThreadsSel, false>(S, n, need, key, row, put);
+  }
+}
+
+// One warp per (query, partition), for partitions that keep few candidates: up to kSelWarpKeys
+// survivors in registers, 32 per lane.  A pair with more, or with many keys at its boundary, is
+// selected by the whole CTA afterwards.
+constexpr uint32_t kSelWarpTop = 64;     // the most candidates per partition of this form
+constexpr uint32_t kSelWarpKeys = 1024;
+constexpr uint32_t kSelWarpList = 128;   // the most of them at or above the groups' bound
+constexpr int kSelWarpThreads = 256;
+
+__global__ void __launch_bounds__(kSelWarpThreads) k_select_warp(SelectArgs a) {
+  constexpr int N = kSelWarpKeys / 32, W = kSelWarpThreads / 32;
+  __shared__ SelectShared<kSelWarpThreads> S;
+  __shared__ uint64_t s_list[W][kSelWarpList];
+  __shared__ uint32_t s_big[W];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  auto need_of = [&](uint32_t p) {
+    const uint32_t r1 = (a.split <= 1 || p == a.split - 1) ? a.n_rows : (p + 1) * a.slice;
+    return min(a.ntop, a.split <= 1 ? a.n_rows : r1 - p * a.slice);
+  };
+  const uint32_t i0 = blockIdx.x * W, pair = i0 + warp;
+  bool big = false;
+  if (pair < a.pairs) {
+    const uint32_t p = pair % a.split, q = pair / a.split, need = need_of(p);
+    if (a.done && p == 0 && lane == 0) a.done[q] = 0u;
+    const uint32_t n = a.cnt[pair];
+    uint32_t* cr = a.cand + (size_t)pair * a.ntop;
+    uint32_t* ck = a.cand_key + (size_t)pair * a.ntop;
+    const bool over = n > a.cap, miss = n < need;
+    for (uint32_t i = (over || miss ? 0u : need) + lane; i < a.ntop; i += 32) {
+      cr[i] = 0xFFFFFFFFu;
+      ck[i] = 0;
+    }
+    if (over || miss) {
+      if (lane == 0) atomicOr(a.status + q, over ? ST_OVERFLOW : ST_MISS);
+    } else if (n > kSelWarpKeys) {
+      big = need != 0;
+    } else if (need) {
+      const uint2* sv = a.surv + (size_t)pair * a.cap;
+      uint32_t k[N], g[2] = {0u, 0u};  // the larger keys of two groups per lane
+#pragma unroll
+      for (int u = 0; u < N; u++) {
+        const uint32_t i = u * 32 + lane;
+        k[u] = i < n ? sv[i].x : 0u;
+        g[u & 1] = max(g[u & 1], k[u]);
+      }
+      // the need-th largest of the 64 groups' maxima: need keys reach it and few others do
+      const uint32_t mx = __reduce_max_sync(0xFFFFFFFFu, max(g[0], g[1]));
+      const uint32_t mn = __reduce_min_sync(0xFFFFFFFFu, min(g[0], g[1]));
+      const uint32_t t = warp_rth_key<2>(g, mn, mx, need);
+      uint32_t own = 0;
+#pragma unroll
+      for (int u = 0; u < N; u++) own += (uint32_t)(u * 32) + lane < n && k[u] >= t ? 1u : 0u;
+      const uint32_t incl = warp_incl_sum(own, lane);
+      const uint32_t m = __shfl_sync(0xFFFFFFFFu, incl, 31);
+      big = m > kSelWarpList;
+      if (!big) {  // gather their places, then the rows in one go, and rank them by counting
+        uint32_t o = incl - own;
+#pragma unroll
+        for (int u = 0; u < N; u++)
+          if ((uint32_t)(u * 32) + lane < n && k[u] >= t) s_list[warp][o++] = u * 32 + lane;
+        __syncwarp();
+        for (uint32_t i = lane; i < m; i += 32) {
+          const uint2 v = sv[s_list[warp][i]];
+          s_list[warp][i] = ((uint64_t)v.x << 32) | v.y;
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < m; i += 32) {
+          const uint64_t c = s_list[warp][i];
+          uint32_t x = 0;
+          for (uint32_t j = 0; j < m; j++) x += s_list[warp][j] > c ? 1u : 0u;
+          if (x < need) {
+            cr[x] = (uint32_t)c;
+            ck[x] = (uint32_t)(c >> 32);
+          }
+        }
       }
     }
+  }
+  if (lane == 0) s_big[warp] = big ? 1u : 0u;
+  __syncthreads();
+  for (int w = 0; w < W; w++) {
+    if (!s_big[w]) continue;
+    const uint32_t pr = i0 + w;
+    const uint2* sv = a.surv + (size_t)pr * a.cap;
+    uint32_t* cr = a.cand + (size_t)pr * a.ntop;
+    uint32_t* ck = a.cand_key + (size_t)pr * a.ntop;
+    block_select<kSelWarpThreads, false>(
+        S, a.cnt[pr], need_of(pr % a.split), [&](uint32_t i) { return sv[i].x; },
+        [&](uint32_t i) { return sv[i].y; },
+        [&](uint32_t o, uint32_t key, uint32_t row) {
+          cr[o] = row;
+          ck[o] = key;
+        });
+    __syncthreads();
   }
 }
 

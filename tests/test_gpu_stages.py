@@ -47,3 +47,46 @@ def test_final_forms(nq, ck, k, deg, ties):
     eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=8, split=1, ck=ck, k_max=k,
                  max_batch=nq)
     _check(m, eng, Q, 1, ck, k, every=max(1, nq // 4))
+
+
+@pytest.mark.parametrize("rows,split,ck,stride,nq,deg", [
+    (60000, 1, 512, 16, 2, 20),    # about 3.7k samples, rank up to 128: group maxima
+    (60000, 1, 64, 16, 2, 20),     # a small rank: 128 groups of four threads
+    (60000, 1, 2048, 4, 2, 20),    # a rank above 128: histograms
+    (20000, 1, 256, 1, 2, 20),     # every row sampled
+    (600, 1, 64, 1, 1, 20),        # a few more samples than a warp holds
+    (500, 1, 64, 1, 1, 20),        # and as many as it does
+    (60000, 32, 512, 4, 3, 20),    # a warp per (query, partition)
+    (60000, 32, 512, 64, 3, 20),   # few samples: many survivors, past a warp's registers
+    (60000, 7, 455, 16, 3, 20),    # 65 candidates per partition: a CTA each
+    (30000, 2, 128, 2, 40, 20),    # 64 of them, batched pass
+    (30000, 2, 128, 2, 400, 20),   # ... and a warp per pair for the select
+    (60000, 32, 512, 64, 40, 20),  # a warp per pair, some pairs past its registers
+    (30000, 1, 4096, 64, 2, 4),    # more survivors than the select keeps in registers
+])
+def test_threshold_and_select_forms(rows, split, ck, stride, nq, deg):
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, 512, max(1, deg // 2), deg, seed=rows + ck)
+    Q = (np.random.default_rng(stride).random((nq, 512)) * 2 - 1).astype(np.float32)
+    m = orc.Matrix(rows, 512, ptr, col, val, 8, 0)
+    eng = E.SpMV(rows, 512, ptr=ptr, col=col, val=val, bits=8, split=split, ck=ck, k_max=50,
+                 max_batch=nq, sample_stride=stride)
+    _check(m, eng, Q, split, ck, 50, every=max(1, nq // 5))
+
+
+@pytest.mark.parametrize("split,ck", [(1, 500), (1, 2000), (8, 400), (32, 512)])
+def test_select_ties(split, ck):
+    """Scores of a handful of values only: the boundary falls among thousands of equal keys and
+    the larger rows stay."""
+    rows, cols = 40000, 64
+    rng = np.random.default_rng(split + ck)
+    ptr = np.arange(rows + 1, dtype=np.uint64) * 2
+    col = np.sort(rng.integers(0, 8, (rows, 2)) * 8 + np.array([0, 1]), axis=1).astype(np.uint32).reshape(-1)
+    val = rng.integers(1, 3, 2 * rows).astype(np.float32)
+    Q = np.ones((2, cols), np.float32)
+    m = orc.Matrix(rows, cols, ptr, col, val, 6, 0)
+    eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=6, split=split, ck=ck, k_max=60, max_batch=2)
+    _check(m, eng, Q, split, ck, 60)
+    if split > 1:  # many pairs: a warp each
+        Q = np.repeat(Q[:1], 100, axis=0)
+        eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=6, split=split, ck=ck, k_max=60, max_batch=100)
+        _check(m, eng, Q, split, ck, 60, every=33)
