@@ -4,6 +4,8 @@
 // A run enqueues, on the handle's stream:
 //   k_quantize -> k_cand_plain(sample tiles) -> k_threshold -> k_cand_plain(all tiles, filter)
 //   -> k_select -> k_final
+// with the filter pass by fours of queries (k_cand_multi) for a few of them and by blocks of 128
+// (k_cand_batch, k_cand_tc; their own sample pass) for many.
 // and afterwards repairs, on the exact slow path, any query whose sample threshold missed or
 // whose survivor buffer overflowed (status bits).  Reference host API replaced:
 // struct SpMV, src/fpga/src/host_spmv_ucsr.cpp:134-829 (zhaijiaqi/AccelES).
@@ -24,6 +26,7 @@
 #include "aes_kernels.cuh"
 #include "aes_select.cuh"
 #include "aes_batch.cuh"
+#include "aes_multi.cuh"
 #include "aes_tc.cuh"
 
 namespace aes {
@@ -67,6 +70,20 @@ static PlainKernel pick_plain(int bits, bool sgn, int mode) {
     case 4: return sgn ? plain_kernel<4, true>(mode) : plain_kernel<4, false>(mode);
     case 6: return sgn ? plain_kernel<6, true>(mode) : plain_kernel<6, false>(mode);
     default: return sgn ? plain_kernel<8, true>(mode) : plain_kernel<8, false>(mode);
+  }
+}
+
+typedef void (*MultiKernel)(MultiArgs);
+template <int B>
+static MultiKernel multi_kernel(bool sgn, bool scaled) {
+  return sgn ? k_cand_multi<B, true, false>
+             : (scaled ? k_cand_multi<B, false, true> : k_cand_multi<B, false, false>);
+}
+static MultiKernel pick_multi(int bits, bool sgn, bool scaled) {
+  switch (bits) {
+    case 4: return multi_kernel<4>(sgn, scaled);
+    case 6: return multi_kernel<6>(sgn, scaled);
+    default: return multi_kernel<8>(sgn, scaled);
   }
 }
 
@@ -205,6 +222,7 @@ struct Engine {
   int batch_warps_n = 0, batch_grid = 0;
   size_t batch_smem = 0;
   uint32_t batch_mode = 0;        // 0 auto, 1 never, else always
+  uint32_t multi_max = 0;         // auto: the most queries that take the four-query pass
   bool use_tc = false;            // batched candidate pass on the tensor cores
   uint8_t* d_qtab_tc = nullptr;   // [blocks][tc_qtab_bytes(cols)] e4m3 query operands
   size_t tc_smem = 0;
@@ -305,6 +323,7 @@ struct Engine {
              uint32_t* repaired);
   int run_plain(int mode, uint32_t q, cudaStream_t s, uint32_t nq_y = 1);
   int run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0 = 0, uint32_t nblk = 0);
+  int run_multi(uint32_t nq, cudaStream_t s);
   int run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint32_t* cnt, cudaStream_t s);
   int run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s);
   int run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair);
@@ -579,6 +598,11 @@ int Engine::apply_config(const Config& c) {
   batch_warps_n = batch_warps((int)bits, cols, split);  // the most that fit
   if (p.batch_warps && (int)p.batch_warps < batch_warps_n) batch_warps_n = (int)p.batch_warps;
   if (batch_warps_n < 1) batch_mode = 1;  // query table does not fit: plain passes only
+  // Auto batches: up to this many queries the four-query pass, above it blocks of 128.  Whole calls,
+  // four-query pass against 128-query block: 8-bit, 40 queries 290 / 298 us (1M rows x 20 entries),
+  // 48 queries 730 / 829 us (4M); 6-bit, 64 queries 395 / 449 us (1M); 4-bit 428 / 459 us.  The
+  // tensor-core pass costs less per entry the larger the matrix: 24 queries 201 / 286 us (1M x 32).
+  multi_max = use_tc ? 24 : (bits == 8 ? 48 : 64);
   if (batch_mode != 1) {
     batch_smem = batch_smem_bytes((int)bits, cols, split, batch_warps_n);
     int occb = 0;
@@ -736,6 +760,7 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
     AES_CK(raise_smem((const void*)pick_plain((int)bits, sgn, mode)));
   for (int mode = 0; mode < 2; mode++)
     AES_CK(raise_smem((const void*)pick_batch((int)bits, sgn, mode)));
+  AES_CK(raise_smem((const void*)pick_multi((int)bits, sgn, d_rowscale != nullptr)));
   AES_CK(raise_smem((const void*)k_final));
   if (tc_ready) {
     AES_CK(raise_smem((const void*)k_cand_tc<2, false>));
@@ -920,6 +945,53 @@ int Engine::run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0, uint
   return AES_OK;
 }
 
+// The filter pass of an nq-query batch, four queries per matrix read
+int Engine::run_multi(uint32_t nq, cudaStream_t s) {
+  MultiArgs a{};
+  a.tiles = d_tiles;
+  a.tile_rowbase = d_tile_rowbase;
+  a.n_tiles = (uint32_t)tiles;
+  a.n_rows = rows;
+  a.cols = cols;
+  a.q8 = d_q8;
+  a.q8_ld = ld8;
+  a.nq = nq;
+  a.rowscale = d_rowscale;
+  a.split = split;
+  a.slice = slice;
+  a.thr = d_thr;
+  a.cnt = d_cnt;
+  a.surv = d_surv;
+  a.cap = cap;
+  // One CTA per SM holds the query table, so `waves` waves of CTAs share the groups of four
+  // queries.  Every warp pays for its table (about 1.5 tiles' time) and for the tile that closes
+  // its last row besides its own tiles, so few CTAs per group, all groups at once, beat a wave per
+  // group: 40 queries of a 400k x 500 matrix 300 -> 163 us, of 4M x 1024 670 -> 620 us.
+  const uint32_t groups = (nq + kMultiQ - 1) / kMultiQ;
+  uint32_t grid = 1;
+  double best = 1e300;
+  for (uint32_t waves = 1; waves <= groups; waves++) {
+    const uint32_t g = std::max<uint32_t>(
+        1, std::min<uint64_t>((uint64_t)sm_count * waves / groups, (uint64_t)sm_count));
+    const double cost = (double)((g * (uint64_t)groups + sm_count - 1) / sm_count) *
+                        (2.5 + (double)((tiles + (uint64_t)g * kMultiWarps - 1) / ((uint64_t)g * kMultiWarps)));
+    if (cost < best) {
+      best = cost;
+      grid = g;
+    }
+  }
+  const bool prof = (prm.flags & AES_FLAG_PROFILE) != 0;
+  int rc = prof ? prof_open(s) : AES_OK;
+  if (rc) return rc;
+  pick_multi((int)bits, sgn, d_rowscale != nullptr)
+      <<<dim3(grid, groups), kMultiThreads, multi_smem_bytes(cols, split), s>>>(a);
+  AES_CK(cudaGetLastError());
+  if (prof && (rc = prof_close(s))) return rc;
+  n_launch++;
+  n_cand++;
+  return AES_OK;
+}
+
 // Thresholds of every (query, partition) from the sample keys [nq][n_sample_rows]; resets cnt
 int Engine::run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint32_t* cnt,
                           cudaStream_t s) {
@@ -961,7 +1033,7 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
     n_launch++;
   }
   n_launch += 3;  // threshold, select, final
-  const bool batched = batch_mode != 1 && (batch_mode != 0 || nq >= 16);
+  const bool batched = batch_mode != 1 && (batch_mode != 0 || nq > multi_max);
   last_batched = batched;
   const uint32_t nblk = (nq + kBatchQ - 1) / kBatchQ;
   if (batched) {
@@ -1008,6 +1080,12 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
       int rc = run_batch(MODE_FILTER, nq, s);
       if (rc) return rc;
     }
+  } else if (batch_mode == 0) {
+    // four queries per matrix read; one left over takes the plain pass
+    const uint32_t alone = nq % kMultiQ == 1 ? 1u : 0u;
+    int rc = nq > alone ? run_multi(nq - alone, s) : AES_OK;
+    if (rc == AES_OK && alone) rc = run_plain(MODE_FILTER, nq - 1, s);
+    if (rc) return rc;
   } else {
     for (uint32_t q = 0; q < nq; q++) {
       int rc = run_plain(MODE_FILTER, q, s);

@@ -3,8 +3,8 @@
 Each matrix is resident once and has one or more batch slots: the engine handle that owns it and
 views of it (aes_create_view), each with its own CUDA stream and batch buffers, each served by
 one worker thread.  A request (matrix, FP32 query, K) is queued on its matrix; a free slot's
-worker takes every request waiting (up to max_batch), runs them as one batch (from 16 queries on,
-one matrix read scores 128 queries) and completes each request with its first K results.
+worker takes every request waiting (up to max_batch), runs them as one batch (one matrix read
+scores four queries, or 128 of a larger batch) and completes each request with its first K results.
 Requests that arrive while batches are on the GPU join the next batch as soon as a slot frees;
 batches of one matrix, and of different matrices, run on the GPU at the same time.
 

@@ -59,7 +59,8 @@ typedef struct aes_params {
   uint32_t max_batch;     /* most queries per aes_set_query / aes_run_device call */
   uint32_t pack_parts;    /* Ultra-CSR packing partitions (SPMV_PARTITIONS = 32) */
   uint32_t sample_stride; /* threshold sample: one 32-packet tile in this many (0 = auto) */
-  uint32_t batch_tile;    /* queries per matrix pass in the batched kernel (0 = auto) */
+  uint32_t batch_tile;    /* queries per matrix pass: 1 = one; 0 = auto: four for a few queries,
+                             blocks of 128 for more; else blocks of 128 */
   int32_t device;         /* CUDA device ordinal */
   uint32_t flags;         /* AES_FLAG_* bits */
   uint64_t seed;          /* seed of the empty-row rule (check_empty_rows is unseeded) */

@@ -90,3 +90,34 @@ def test_select_ties(split, ck):
         Q = np.repeat(Q[:1], 100, axis=0)
         eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=6, split=split, ck=ck, k_max=60, max_batch=100)
         _check(m, eng, Q, split, ck, 60, every=33)
+
+
+@pytest.mark.parametrize("bits,quant", [(4, 0), (4, 1), (4, 2), (6, 0), (6, 1), (6, 2), (8, 0), (8, 1), (8, 2)])
+@pytest.mark.parametrize("rows,cols,lo,hi,split,nq", [
+    (9, 40, 1, 6, 1, 2),            # less than a tile
+    (20000, 1024, 10, 30, 1, 4),    # one group of four
+    (30001, 777, 1, 4, 32, 7),      # several rows per span; two groups, the last short
+    (3000, 500, 150, 400, 5, 5),    # rows over several packets and tiles; one query alone
+    (20000, 333, 5, 12, 1500, 6),   # partitions of a few rows, thresholds in global memory
+    (20000, 96, 8, 20, 3, 17),      # groups share the SMs; one query alone
+])
+def test_four_query_pass(bits, quant, rows, cols, lo, hi, split, nq):
+    """A few queries per call (auto batch tile): four per matrix read, the last one alone where
+    one is left over.  One query is all zero, another has a single entry."""
+    ck = max(64, 2 * split) if split > 1 else 200
+    k = 30
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, lo, hi, seed=rows + bits)
+    if quant == 0:
+        val = val * np.where(np.random.default_rng(1).random(val.shape[0]) < 0.5, -1, 1).astype(np.float32)
+    rng = np.random.default_rng(nq)
+    Q = rng.random((nq, cols)).astype(np.float32)
+    if quant == 0:
+        Q = Q * 2 - 1
+    Q[1] = 0
+    if nq > 2:
+        Q[2] = 0
+        Q[2, cols // 2] = 1
+    m = orc.Matrix(rows, cols, ptr, col, val, bits, quant)
+    eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=bits, quant=quant, split=split, ck=ck,
+                 k_max=k, max_batch=nq)
+    _check(m, eng, Q, split, ck, k)
