@@ -87,19 +87,23 @@ static MultiKernel pick_multi(int bits, bool sgn, bool scaled) {
   }
 }
 
-// P(Bin(n, f) >= r) in log space
-static double binom_tail(uint32_t n, double f, uint32_t r) {
-  if (r == 0) return 1.0;
-  if (r > n) return 0.0;
-  if (f <= 0.0) return 0.0;
-  if (f >= 1.0) return 1.0;
-  double lf = std::log(f), l1f = std::log1p(-f), s = 0.0;
-  for (uint32_t k = r; k <= n; k++) {
-    double lt = std::lgamma((double)n + 1) - std::lgamma((double)k + 1) -
-                std::lgamma((double)(n - k) + 1) + k * lf + (n - k) * l1f;
-    s += std::exp(lt);
+// The smallest r >= floor(n f) with P(Bin(n, f) >= r) <= 1e-12, 0 < f < 1
+static uint32_t binom_rank(uint32_t n, double f) {
+  const uint32_t r0 = (uint32_t)std::floor(n * f);
+  std::vector<double> pmf;  // of r0, r0 + 1, ... until it is negligible
+  double x = std::exp(std::lgamma((double)n + 1) - std::lgamma((double)r0 + 1) -
+                      std::lgamma((double)(n - r0) + 1) + r0 * std::log(f) +
+                      (n - r0) * std::log1p(-f));
+  for (uint32_t k = r0; k <= n; k++) {
+    pmf.push_back(x);
+    if (x < 1e-30 && k > n * f) break;
+    x *= (double)(n - k) / (double)(k + 1) * (f / (1.0 - f));
   }
-  return s;
+  double tail = 0.0;
+  size_t i = pmf.size();
+  while (i > 0 && tail + pmf[i - 1] <= 1e-12) tail += pmf[--i];
+  const uint32_t r = r0 + (uint32_t)i;
+  return r ? r : 1;
 }
 
 // Device arrays of a resident matrix (Ultra-CSR tiles, row bases, row scales, FP32 CSR,
@@ -163,6 +167,7 @@ struct Engine {
   uint32_t* d_sample_keys = nullptr;
   uint32_t* d_keys_t = nullptr;   // batched sample keys moved to [query][sample rows]
   uint32_t* d_exact_aux = nullptr;  // FP32-only pass: sample range {0, n} and rank r
+  uint32_t exact_k = 0, exact_S = 0, exact_r = 0;  // the K d_exact_aux is for (0: none), its plan
   uint32_t* d_thr = nullptr;
   uint32_t* d_cnt = nullptr;
   uint2* d_surv = nullptr;
@@ -267,6 +272,7 @@ struct Engine {
     bytes -= cfg_bytes;
     cfg_bytes = 0;
     configured = false;
+    exact_k = 0;
     nq_loaded = 0;
     ran = false;
     last_from_device = false;
@@ -504,11 +510,7 @@ int Engine::plan_config(const aes_params& p, Config* c) const {
     uint32_t n1 = c->ntop ? c->ntop - 1 : 0;
     uint32_t r = 1;
     if (f >= 1.0) r = std::max<uint32_t>(c->ntop, 1);
-    else {
-      r = (uint32_t)std::floor(n1 * f);
-      while (r <= n1 && binom_tail(n1, f, r) > 1e-12) r++;
-      r = std::max<uint32_t>(r, 1);
-    }
+    else if (f > 0.0) r = binom_rank(n1, f);
     c->part_r[q] = r;
     double expect = f > 0 ? (double)r / f : (double)prow[q];
     size_t cc = (size_t)std::min<double>((double)prow[q], 4.0 * expect + 4.0 * c->ntop + 1024.0);
@@ -762,6 +764,7 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
     AES_CK(raise_smem((const void*)pick_batch((int)bits, sgn, mode)));
   AES_CK(raise_smem((const void*)pick_multi((int)bits, sgn, d_rowscale != nullptr)));
   AES_CK(raise_smem((const void*)k_final));
+  AES_CK(raise_smem((const void*)k_exact_multi<8>));
   if (tc_ready) {
     AES_CK(raise_smem((const void*)k_cand_tc<2, false>));
     AES_CK(raise_smem((const void*)k_cand_tc<3, false>));
@@ -1607,7 +1610,8 @@ int aes_get_stats(aes_handle* h, aes_stats* st, int reset) {
   return AES_OK;
 }
 
-int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score, uint64_t* ns) {
+int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score,
+                  uint64_t* ns_out) {
   using namespace aes::dev;
   if (!h || !out_idx || !out_score) return aes::fail(AES_ERR_INVALID, "NULL argument");
   Engine& e = h->e;
@@ -1616,105 +1620,160 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
   if (!e.has_f32) return aes::fail(AES_ERR_STATE, "the matrix was created without FP32 values");
   if (!e.q32_given) return aes::fail(AES_ERR_STATE, "the loaded queries have no FP32 values");
   AES_CK(cudaSetDevice(e.device));
+  const uint32_t nq = e.nq_loaded;
+  cudaStream_t s = e.stream;
   // Filtered select: every S-th row key is a sample; its r-th largest key lies below the K-th
   // largest key of all rows except with probability 1e-12 (binomial tail), so only the rows at or
   // above it need the select.  S is the largest power of two whose expected survivors fit the
   // survivor buffer; a miss or an overflow is detected by the select and falls back to the
   // select over every row, so the result is exact either way.
-  uint32_t S = 0, r = 0;
-  for (uint32_t cs = 1024; cs >= 2 && e.rows >= 4u * k; cs >>= 1) {
-    const uint32_t nsm = (e.rows + cs - 1) / cs;
-    const double f = 1.0 / cs;
-    const uint32_t n1 = k - 1;
-    uint32_t rr = (uint32_t)std::floor(n1 * f);
-    while (rr <= n1 && aes::binom_tail(n1, f, rr) > 1e-12) rr++;
-    rr = std::max<uint32_t>(rr, 1);
-    if (rr > nsm) continue;
-    if (2.0 * rr / f + k + 64.0 <= (double)e.cap) {
-      S = cs;
-      r = rr;
-      break;
+  if (e.exact_k != k) {
+    e.exact_k = k;
+    e.exact_S = e.exact_r = 0;
+    for (uint32_t cs = 1024; cs >= 2 && e.rows >= 4u * k; cs >>= 1) {
+      const uint32_t rr = aes::binom_rank(k - 1, 1.0 / cs);
+      if (rr > (e.rows + cs - 1) / cs) continue;
+      if (2.0 * rr * cs + k + 64.0 <= (double)e.cap) {
+        e.exact_S = cs;
+        e.exact_r = rr;
+        break;
+      }
+    }
+    if (e.exact_S) {
+      const uint32_t aux[3] = {0u, (e.rows + e.exact_S - 1) / e.exact_S, e.exact_r};
+      cudaError_t ce = cudaMemcpyAsync(e.d_exact_aux, aux, sizeof(aux), cudaMemcpyHostToDevice, s);
+      if (ce != cudaSuccess) e.exact_k = 0;
+      AES_CK(ce);
     }
   }
-  if (S) {
-    const uint32_t aux[3] = {0u, (e.rows + S - 1) / S, r};
-    AES_CK(cudaMemcpy(e.d_exact_aux, aux, sizeof(aux), cudaMemcpyHostToDevice));
-  }
+  const uint32_t S = e.exact_S;
   FinalArgs fa{};
   fa.csr_ptr = e.d_csr_ptr;
   fa.csr_col = e.d_csr_col;
   fa.csr_val = e.d_csr_val;
   fa.ld32 = e.ld32;
   fa.cols = e.cols;
-  fa.cand = e.d_exact_cand;
   fa.nslots = k;
   fa.k = k;
-  fa.out_idx = e.d_out_idx;
-  fa.out_score = e.d_out_score;
   fa.status = nullptr;
-  fa.cand_key = nullptr;
-  const uint32_t fg = e.final_grid(1, e.d_sample_keys, e.tail_bytes, &fa);
+  fa.key_f32 = 1u;  // the selected keys are those of the exact FP32 scores
   SelectArgs sa{};
-  sa.done = fa.done;
-  sa.q0 = 0;
   sa.split = 1;
   sa.slice = e.rows;
   sa.n_rows = e.rows;
   sa.ntop = k;
-  sa.cand = e.d_exact_cand;
-  sa.cand_key = e.d_exact_key;
   sa.status = e.d_status;
-  float total_ms = 0.0f;
-  for (uint32_t q = 0; q < e.nq_loaded; q++) {
-    fa.q32 = e.d_q32 + (size_t)q * e.ld32;
-    AES_CK(cudaMemsetAsync(e.d_status, 0, 4, e.stream));
-    AES_CK(cudaEventRecord(e.ev0, e.stream));
-    k_exact_all<<<e.sm_count * 8, kExactWarps * 32, exact_all_smem_bytes(e.cols), e.stream>>>(
+  // every row of query q: keys, the select over all of them
+  auto all_rows = [&](uint32_t q) -> int {
+    k_exact_all<false><<<e.sm_count * 8, kExactWarps * 32, exact_all_smem_bytes(e.cols), s>>>(
         e.d_csr_ptr, e.d_csr_col, e.d_csr_val, e.d_q32 + (size_t)q * e.ld32, e.cols, e.rows,
-        e.d_allkeys);
+        e.d_allkeys, nullptr, nullptr, nullptr, 0u);
     AES_CK(cudaGetLastError());
-    if (S) {
-      k_threshold<<<dim3(1, 1), kThreadsThr, 0, e.stream>>>(e.d_allkeys, 0, S, e.d_exact_aux, 1,
-                                                           e.d_exact_aux + 2, e.d_thr, e.d_cnt);
-      AES_CK(cudaGetLastError());
-      k_filter_keys<<<e.sm_count * 4, 256, 0, e.stream>>>(e.d_allkeys, e.rows, e.d_thr, e.d_cnt,
-                                                         e.d_surv, e.cap);
-      AES_CK(cudaGetLastError());
-      sa.surv = e.d_surv;
-      sa.cnt = e.d_cnt;
-      sa.cap = e.cap;
-      k_select<false><<<dim3(1, 1), kThreadsSel, 0, e.stream>>>(sa);
-    } else {
-      sa.allkeys = e.d_allkeys;
-      k_select<true><<<dim3(1, 1), kThreadsSel, 0, e.stream>>>(sa);
+    sa.q0 = 0;
+    sa.allkeys = e.d_allkeys;
+    sa.cand = e.d_exact_cand;
+    sa.cand_key = e.d_exact_key;
+    k_select<true><<<dim3(1, 1), kThreadsSel, 0, s>>>(sa);
+    AES_CK(cudaGetLastError());
+    fa.cand = e.d_exact_cand;
+    fa.cand_key = e.d_exact_key;
+    fa.out_idx = e.d_out_idx + (size_t)q * k;
+    fa.out_score = e.d_out_score + (size_t)q * k;
+    k_final<<<1, kThreadsFinal, e.final_smem, s>>>(fa);
+    AES_CK(cudaGetLastError());
+    return AES_OK;
+  };
+  // the sampled rows' keys live in the key array (S queries' samples fit in it), the selected
+  // candidates in the sample keys' memory of the low-bit pass, else one query at a time
+  const uint32_t ns = S ? (e.rows + S - 1) / S : 0;
+  uint32_t chunk = S ? (uint32_t)std::min<uint64_t>({e.rows / ns, e.tail_bytes / (k * 8ull), nq}) : 0;
+  chunk = std::max<uint32_t>(chunk, 1);
+  AES_CK(cudaMemsetAsync(e.d_status, 0, nq * 4ull, s));
+  AES_CK(cudaEventRecord(e.ev0, s));
+  for (uint32_t q0 = 0; q0 < nq; q0 += chunk) {
+    if (!S) {
+      int rc = all_rows(q0);  // (chunk is 1)
+      if (rc) return rc;
+      continue;
     }
+    const uint32_t n = std::min(chunk, nq - q0);
+    const float* q32 = e.d_q32 + (size_t)q0 * e.ld32;
+    fa.q32 = q32;
+    const uint32_t groups = (ns + kExSampleRows - 1) / kExSampleRows;
+    k_exact_sample<<<dim3(groups, n), kThreadsExSample, exact_sample_smem_bytes(e.cols), s>>>(
+        fa, S, ns, e.d_allkeys);
     AES_CK(cudaGetLastError());
-    k_final<<<fg, kThreadsFinal, e.final_smem, e.stream>>>(fa);
+    k_threshold<<<dim3(1, n), kThreadsThr, 0, s>>>(e.d_allkeys, ns, 0, e.d_exact_aux, 1,
+                                                   e.d_exact_aux + 2, e.d_thr, e.d_cnt);
     AES_CK(cudaGetLastError());
-    AES_CK(cudaEventRecord(e.ev1, e.stream));
-    AES_CK(cudaMemcpyAsync(e.h_status, e.d_status, 4, cudaMemcpyDeviceToHost, e.stream));
-    AES_CK(cudaStreamSynchronize(e.stream));
+    for (uint32_t i = 0; i < n;) {  // groups of eight queries, then four, a last one alone
+      ExactArgs x{};
+      x.ptr = e.d_csr_ptr;
+      x.col = e.d_csr_col;
+      x.val = e.d_csr_val;
+      x.q = q32 + (size_t)i * e.ld32;
+      x.ld = e.ld32;
+      x.cols = e.cols;
+      x.rows = e.rows;
+      x.thr = e.d_thr + i;
+      x.cnt = e.d_cnt + i;
+      x.surv = e.d_surv + (size_t)i * e.cap;
+      x.cap = e.cap;
+      const uint32_t left = n - i;
+      if (left > 4) {
+        const uint32_t g = left >= 8 ? left / 8 : 1;
+        x.nq = std::min(left, 8 * g);
+        k_exact_multi<8><<<dim3((4 * e.sm_count + g - 1) / g, g), kExactWarps * 32,
+                           exact_multi_smem_bytes<8>(e.cols), s>>>(x);
+      } else if (left > 1) {
+        x.nq = left;
+        k_exact_multi<4><<<4 * e.sm_count, kExactWarps * 32, exact_multi_smem_bytes<4>(e.cols), s>>>(x);
+      } else {
+        x.nq = 1;
+        k_exact_all<true><<<e.sm_count * 8, kExactWarps * 32, exact_all_smem_bytes(e.cols), s>>>(
+            x.ptr, x.col, x.val, x.q, x.cols, x.rows, nullptr, x.thr, x.cnt, x.surv, x.cap);
+      }
+      AES_CK(cudaGetLastError());
+      i += x.nq;
+    }
+    sa.allkeys = nullptr;
+    sa.surv = e.d_surv;
+    sa.cnt = e.d_cnt;
+    sa.cap = e.cap;
+    sa.status = e.d_status + q0;
+    sa.cand = n > 1 ? e.d_sample_keys : e.d_exact_cand;
+    sa.cand_key = n > 1 ? e.d_sample_keys + (size_t)n * k : e.d_exact_key;
+    k_select<false><<<dim3(1, n), kThreadsSel, 0, s>>>(sa);
+    AES_CK(cudaGetLastError());
+    fa.cand = sa.cand;
+    fa.cand_key = sa.cand_key;
+    fa.out_idx = e.d_out_idx + (size_t)q0 * k;
+    fa.out_score = e.d_out_score + (size_t)q0 * k;
+    k_final<<<dim3(1, n), kThreadsFinal, e.final_smem, s>>>(fa);
+    AES_CK(cudaGetLastError());
+  }
+  AES_CK(cudaEventRecord(e.ev1, s));
+  AES_CK(cudaMemcpyAsync(e.h_status, e.d_status, nq * 4ull, cudaMemcpyDeviceToHost, s));
+  AES_CK(cudaStreamSynchronize(s));
+  float total_ms = 0.0f;
+  AES_CK(cudaEventElapsedTime(&total_ms, e.ev0, e.ev1));
+  sa.status = e.d_status;
+  for (uint32_t q = 0; S && q < nq; q++) {  // the sample bound missed or the buffer overflowed
+    if (!e.h_status[q]) continue;
+    AES_CK(cudaEventRecord(e.ev0, s));
+    int rc = all_rows(q);
+    if (rc) return rc;
+    AES_CK(cudaEventRecord(e.ev1, s));
+    AES_CK(cudaStreamSynchronize(s));
     float ms = 0.0f;
     AES_CK(cudaEventElapsedTime(&ms, e.ev0, e.ev1));
     total_ms += ms;
-    if (S && e.h_status[0]) {  // the sample bound missed or the buffer overflowed: every row
-      AES_CK(cudaEventRecord(e.ev0, e.stream));
-      sa.allkeys = e.d_allkeys;
-      k_select<true><<<dim3(1, 1), kThreadsSel, 0, e.stream>>>(sa);
-      AES_CK(cudaGetLastError());
-      k_final<<<fg, kThreadsFinal, e.final_smem, e.stream>>>(fa);
-      AES_CK(cudaGetLastError());
-      AES_CK(cudaEventRecord(e.ev1, e.stream));
-      AES_CK(cudaStreamSynchronize(e.stream));
-      AES_CK(cudaEventElapsedTime(&ms, e.ev0, e.ev1));
-      total_ms += ms;
-      e.n_repaired++;
-    }
-    AES_CK(cudaMemcpyAsync(out_idx + (size_t)q * k, e.d_out_idx, k * 4ull, cudaMemcpyDeviceToHost, e.stream));
-    AES_CK(cudaMemcpyAsync(out_score + (size_t)q * k, e.d_out_score, k * 4ull, cudaMemcpyDeviceToHost, e.stream));
-    AES_CK(cudaStreamSynchronize(e.stream));
+    e.n_repaired++;
   }
-  if (ns) *ns = (uint64_t)((double)total_ms * 1e6);
+  AES_CK(cudaMemcpyAsync(out_idx, e.d_out_idx, (size_t)nq * k * 4ull, cudaMemcpyDeviceToHost, s));
+  AES_CK(cudaMemcpyAsync(out_score, e.d_out_score, (size_t)nq * k * 4ull, cudaMemcpyDeviceToHost, s));
+  AES_CK(cudaStreamSynchronize(s));
+  if (ns_out) *ns_out = (uint64_t)((double)total_ms * 1e6);
   return AES_OK;
 }
 

@@ -7,7 +7,7 @@
 //                     (split_approximate, quantify_util.py:173-196; sort_tuples order)
 //   k_final           FP32 rescoring of the candidates (quantify_util.py:354-356 in FP32;
 //                     gold_algorithms.hpp:211-239 summation order) and the final Top-K
-//   k_exact_all, k_filter_keys   the FP32-only Top-K of every row
+//   k_exact_sample, k_exact_all, k_exact_multi   the FP32-only Top-K of every row
 #pragma once
 
 #include "aes_kernels.cuh"
@@ -761,8 +761,10 @@ struct FinalArgs {
   const uint32_t* status;    // [nq]; queries with a set status are left to the repair path
   // [nq][nslots] candidate keys, or null.  Given: the final Top-K ranks the candidates by their
   // integer candidate score (no FP32 rescoring: a pre-quantised matrix or query without FP32
-  // values) and out_score holds that score
+  // values) and out_score holds that score; with key_f32 they are the keys of FP32 scores that are
+  // already exact
   const uint32_t* cand_key;
+  uint32_t key_f32;
   uint64_t* comp;            // gridDim.x > 1: [nq][nslots] composites between the CTAs of a query
   uint32_t* done;            // gridDim.x > 1: [nq] CTAs finished, zero before the launch
 };
@@ -955,7 +957,7 @@ __global__ void __launch_bounds__(kThreadsFinal, 2) k_final(FinalArgs a) {
   auto put = [&](uint32_t o, uint64_t c) {
     oi[o] = (uint32_t)c;
     const uint32_t key = (uint32_t)(c >> 32);
-    os[o] = a.cand_key ? (float)(int32_t)(key ^ 0x80000000u) : key_to_f32(key);
+    os[o] = a.cand_key && !a.key_f32 ? (float)(int32_t)(key ^ 0x80000000u) : key_to_f32(key);
   };
   if (m <= kFinalRankMax) {
     // a composite's place is the number of larger ones, counted by `per` threads of a warp
@@ -1013,15 +1015,20 @@ __host__ inline size_t exact_all_smem_bytes(uint32_t cols) {
   return (size_t)cols * 4 + (size_t)kExactWarps * kExactChunk * 4;
 }
 
+// FILTER: no keys array; rows at or above the threshold go to the survivors (the count goes on past
+// cap, so that the select can tell an overflow).
+template <bool FILTER>
 __global__ void __launch_bounds__(kExactWarps * 32) k_exact_all(
     const uint32_t* __restrict__ ptr, const uint16_t* __restrict__ col,
     const float* __restrict__ val, const float* __restrict__ q, uint32_t cols, uint32_t rows,
-    uint32_t* __restrict__ keys) {
+    uint32_t* __restrict__ keys, const uint32_t* __restrict__ thr, uint32_t* __restrict__ cnt,
+    uint2* __restrict__ surv, uint32_t cap) {
   extern __shared__ __align__(16) unsigned char xsm[];
   float* qs = reinterpret_cast<float*>(xsm);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   float* sp = reinterpret_cast<float*>(xsm + (size_t)cols * 4) + warp * kExactChunk;
   for (uint32_t j = threadIdx.x; j < cols; j += blockDim.x) qs[j] = q[j];
+  const uint32_t th = FILTER ? *thr : 0u;
   __syncthreads();
   const uint32_t nblk = (rows + 31) / 32;
   for (uint32_t blk = blockIdx.x * kExactWarps + warp; blk < nblk; blk += gridDim.x * kExactWarps) {
@@ -1047,44 +1054,145 @@ __global__ void __launch_bounds__(kExactWarps * 32) k_exact_all(
       for (uint32_t i = a; i < b; i++) acc = __fadd_rn(acc, sp[i - c]);
       __syncwarp();
     }
-    if (r < rows) keys[r] = key_f32(acc);
+    if (r < rows) {
+      const uint32_t key = key_f32(acc);
+      if constexpr (FILTER) {
+        if (key >= th) {
+          const uint32_t i = atomicAdd(cnt, 1u);
+          if (i < cap) surv[i] = make_uint2(key, r);
+        }
+      } else {
+        keys[r] = key;
+      }
+    }
   }
 }
 
-// Rows whose key is at least *thr, appended as (key, row) to surv (warp-aggregated counter; the
-// count goes on past cap so the select can tell an overflow).  Used by the FP32-only pass after
-// a sample threshold, so that the select reads a few survivors instead of every row.
-__global__ void k_filter_keys(const uint32_t* __restrict__ keys, uint32_t rows,
-                              const uint32_t* __restrict__ thr, uint32_t* __restrict__ cnt,
-                              uint2* __restrict__ surv, uint32_t cap) {
-  const uint32_t th = *thr, lane = threadIdx.x & 31u;
-  const uint32_t stride = gridDim.x * blockDim.x;
-  const uint32_t n4 = (rows + 3) / 4;                    // groups of four keys (16-byte loads)
-  const uint32_t n_iter = (n4 + stride - 1) / stride;    // the same for every lane of a warp
-  for (uint32_t it = 0; it < n_iter; it++) {
-    const uint32_t g = it * stride + blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t k4[4] = {0u, 0u, 0u, 0u};
-    if (g * 4 + 3 < rows) {
-      const uint4 v = __ldcs(reinterpret_cast<const uint4*>(keys) + g);
-      k4[0] = v.x; k4[1] = v.y; k4[2] = v.z; k4[3] = v.w;
-    } else if (g < n4) {
-      for (uint32_t t = 0; t < 4 && g * 4 + t < rows; t++) k4[t] = keys[g * 4 + t];
-    }
+// FP32-only pass with a bound: rows whose key is at least their query's threshold are appended to
+// its survivors; nothing is written for the others.  T queries per matrix read.
+struct ExactArgs {
+  const uint32_t* ptr;
+  const uint16_t* col;
+  const float* val;
+  const float* q;       // [nq][ld], the launch's first query
+  uint32_t ld, cols, rows, nq;
+  const uint32_t* thr;  // [nq]
+  uint32_t* cnt;        // [nq]; counts on past cap, so that the select can tell an overflow
+  uint2* surv;          // [nq][cap]
+  uint32_t cap;
+};
+
+__device__ __forceinline__ void exact_emit(const ExactArgs& a, uint32_t q, uint32_t row, float score,
+                                           uint32_t th) {
+  const uint32_t key = key_f32(score);
+  if (key >= th) {
+    const uint32_t i = atomicAdd(a.cnt + q, 1u);
+    if (i < a.cap) a.surv[(size_t)q * a.cap + i] = make_uint2(key, row);
+  }
+}
+
+// Bound by shared memory: a lane walks its row's entries in column order (values and columns
+// staged from the CSR, 32 rows' entries being contiguous) and gathers the T queries' values of a
+// column with 16-byte loads, about 11 wavefronts each over random columns against 6.5 for the
+// entry itself; so eight queries per walk, or four for a last few.  1M rows x 20 entries: 43 us
+// for a query alone (and a key array to filter), 102 us for eight.  blockIdx.y: the group of T queries.
+template <int T>
+__host__ inline size_t exact_multi_smem_bytes(uint32_t cols) {
+  return (size_t)cols * T * 4 + (size_t)kExactWarps * kExactChunk * 6;
+}
+template <int T>
+__global__ void __launch_bounds__(kExactWarps * 32) k_exact_multi(ExactArgs a) {
+  static_assert(T == 4 || T == 8, "queries per walk");
+  extern __shared__ __align__(16) unsigned char xsm[];
+  float4* qs = reinterpret_cast<float4*>(xsm);  // [T / 4][cols]
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  float* sv = reinterpret_cast<float*>(xsm + (size_t)a.cols * T * 4) + warp * kExactChunk;
+  uint16_t* sc = reinterpret_cast<uint16_t*>(xsm + (size_t)a.cols * T * 4 +
+                                             (size_t)kExactWarps * kExactChunk * 4) + warp * kExactChunk;
+  const uint32_t q0 = blockIdx.y * T, nq = min((uint32_t)T, a.nq - q0);
+  uint32_t th[T];
 #pragma unroll
-    for (uint32_t t = 0; t < 4; t++) {
-      const uint32_t r = g * 4 + t;
-      const bool hit = r < rows && k4[t] >= th;
-      const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit);
-      if (m) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(cnt, (uint32_t)__popc(m));
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (hit) {
-          const uint32_t i = base + __popc(m & ((1u << lane) - 1u));
-          if (i < cap) surv[i] = make_uint2(k4[t], r);
+  for (int t = 0; t < T; t++) {
+    th[t] = (uint32_t)t < nq ? a.thr[q0 + t] : 0xFFFFFFFFu;
+    const float* x = a.q + (size_t)(q0 + ((uint32_t)t < nq ? t : 0u)) * a.ld;
+    for (uint32_t j = threadIdx.x; j < a.cols; j += blockDim.x)
+      reinterpret_cast<float*>(qs)[((size_t)(t / 4) * a.cols + j) * 4 + t % 4] = x[j];
+  }
+  __syncthreads();
+  const uint32_t nblk = (a.rows + 31) / 32;
+  for (uint32_t blk = blockIdx.x * kExactWarps + warp; blk < nblk; blk += gridDim.x * kExactWarps) {
+    const uint32_t r0 = blk * 32, r = r0 + lane;
+    const uint32_t rend = min(r0 + 32u, a.rows);
+    const uint32_t E0 = a.ptr[r0], E1 = a.ptr[rend];
+    const uint32_t s = r < a.rows ? a.ptr[r] : E1, e = r < a.rows ? a.ptr[r + 1] : E1;
+    float acc[T];
+#pragma unroll
+    for (int t = 0; t < T; t++) acc[t] = 0.0f;
+    for (uint32_t c = E0; c < E1; c += kExactChunk) {
+      const uint32_t n = min(kExactChunk, E1 - c);
+      float lv[kExactChunk / 32];
+      uint16_t lc[kExactChunk / 32];
+#pragma unroll
+      for (uint32_t u = 0; u < kExactChunk / 32; u++) {
+        const uint32_t i = u * 32 + lane;
+        lv[u] = i < n ? __ldg(a.val + c + i) : 0.0f;
+        lc[u] = i < n ? __ldg(a.col + c + i) : (uint16_t)0;
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < kExactChunk / 32; u++) {
+        sv[u * 32 + lane] = lv[u];
+        sc[u * 32 + lane] = lc[u];
+      }
+      __syncwarp();
+      const uint32_t b = max(s, c), d = min(e, c + n);
+      for (uint32_t i = b; i < d; i++) {
+        const float v = sv[i - c];
+        const uint32_t j = sc[i - c];
+#pragma unroll
+        for (int g = 0; g < T / 4; g++) {
+          const float4 x = qs[(size_t)g * a.cols + j];
+          acc[4 * g + 0] = __fadd_rn(acc[4 * g + 0], __fmul_rn(v, x.x));
+          acc[4 * g + 1] = __fadd_rn(acc[4 * g + 1], __fmul_rn(v, x.y));
+          acc[4 * g + 2] = __fadd_rn(acc[4 * g + 2], __fmul_rn(v, x.z));
+          acc[4 * g + 3] = __fadd_rn(acc[4 * g + 3], __fmul_rn(v, x.w));
         }
       }
+      __syncwarp();
     }
+    if (r < a.rows) {
+#pragma unroll
+      for (int t = 0; t < T; t++)
+        if ((uint32_t)t < nq) exact_emit(a, q0 + t, r, acc[t], th[t]);
+    }
+  }
+}
+
+// FP32 keys of rows 0, S, 2 S, ... (ns of them) per query (blockIdx.y): keys[nq][ns].  A warp takes
+// 8 sampled rows: latency-bound, their entries in one round trip.
+constexpr int kThreadsExSample = 256;
+constexpr uint32_t kExSampleRows = kThreadsExSample / 32 * 8;  // per CTA
+__host__ inline size_t exact_sample_smem_bytes(uint32_t cols) {
+  return (((size_t)cols * 4 + 15) & ~(size_t)15) + (size_t)(kThreadsExSample / 32) * kFinalStage * 4;
+}
+__global__ void __launch_bounds__(kThreadsExSample) k_exact_sample(FinalArgs a, uint32_t S, uint32_t ns,
+                                                                   uint32_t* __restrict__ keys) {
+  extern __shared__ __align__(16) unsigned char xsm[];
+  float* qs = reinterpret_cast<float*>(xsm);
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  float* sp = reinterpret_cast<float*>(xsm + ((a.cols * 4 + 15) & ~15u)) + warp * kFinalStage;
+  const float* x = a.q32 + (size_t)blockIdx.y * a.ld32;
+  for (uint32_t j = threadIdx.x; j < a.cols; j += blockDim.x) qs[j] = x[j];
+  __syncthreads();
+  for (uint32_t g = (blockIdx.x * (kThreadsExSample / 32) + warp) * 8; g < ns;
+       g += gridDim.x * kExSampleRows) {
+    const uint32_t i = lane < 8 ? g + lane : ns;
+    uint32_t s = 0, n = 0;
+    if (i < ns) {
+      s = __ldg(a.csr_ptr + (size_t)i * S);
+      n = __ldg(a.csr_ptr + (size_t)i * S + 1) - s;
+    }
+    const float acc = rescore_rows<8, 32>(a, qs, sp, s, n);
+    if (i < ns) keys[(size_t)blockIdx.y * ns + i] = key_f32(acc);
   }
 }
 

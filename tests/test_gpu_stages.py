@@ -121,3 +121,31 @@ def test_four_query_pass(bits, quant, rows, cols, lo, hi, split, nq):
     eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=bits, quant=quant, split=split, ck=ck,
                  k_max=k, max_batch=nq)
     _check(m, eng, Q, split, ck, k)
+
+
+@pytest.mark.parametrize("rows,cols,kind,p0,p1,nq,k,ck,stride", [
+    (30000, 1024, E.GEN_UNIFORM_DEG, 10, 30, 1, 100, 512, 0),   # one query: rows filtered as scored
+    (30001, 1024, E.GEN_UNIFORM_DEG, 0, 30, 17, 100, 512, 0),   # two groups of eight and one; empty rows
+    (30000, 333, E.GEN_UNIFORM_DEG, 10, 30, 12, 7, 512, 0),     # eight and four
+    (29999, 777, E.GEN_UNIFORM_DEG, 1, 3, 6, 33, 512, 0),       # six in a group of eight
+    (6000, 1024, E.GEN_GAMMA_DEG, 200, 1024, 11, 20, 512, 0),   # rows longer than a staged chunk's share
+    (31, 64, E.GEN_UNIFORM_DEG, 1, 9, 3, 40, 64, 0),            # fewer rows than results: no sample
+    (30000, 256, E.GEN_UNIFORM_DEG, 4, 9, 70, 100, 128, 256),   # more queries than one chunk takes
+])
+def test_fp32_only_batches(rows, cols, kind, p0, p1, nq, k, ck, stride):
+    ptr, col, val = E.gen_matrix(kind, rows, cols, p0, p1, seed=rows + nq)
+    val = val - np.float32(0.4)
+    eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=8, split=1, ck=ck, k_max=k, max_batch=nq,
+                 sample_stride=stride)
+    Q = (np.random.default_rng(nq).random((nq, cols)) * 2 - 1).astype(np.float32)
+    allrows = np.arange(rows, dtype=np.uint32)
+    eng.Q_reset(Q)
+    for kk in (k, max(1, k // 2)):  # a second K re-plans the sample
+        idx, sc, ns = eng.run_exact(k=kk)
+        assert ns > 0
+        for i in range(0, nq, max(1, nq // 6)):
+            s = orc.rescore_f32(ptr, col, val, Q[i], allrows)
+            ri, rs = orc.sort_tuples_f32(allrows, s)
+            n = min(kk, rows)
+            assert np.array_equal(idx[i, :n], ri[:n]) and np.array_equal(sc[i, :n], rs[:n]), i
+            assert np.all(idx[i, n:] == 0xFFFFFFFF)
