@@ -390,6 +390,9 @@ int Engine::run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair) {
   a.surv = d_surv;
   a.cap = cap;
   a.status = d_status;
+  // the hit queues take the sample keys' memory, dead once the thresholds are known
+  a.queue = reinterpret_cast<uint2*>(d_sample_keys);
+  a.queue_cap = (uint32_t)std::min<size_t>(kTcQueueMax, tail_bytes / (8ull * kTcQueues * (pair ? tc_grid2 : tc_grid)));
   a.mma_idle = (prm.flags & AES_FLAG_TEST_IDLE_MMA) ? 1u : 0u;
   const bool prof = (prm.flags & AES_FLAG_PROFILE) != 0;
   int rc = prof ? prof_open(s) : AES_OK;

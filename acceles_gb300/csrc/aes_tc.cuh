@@ -16,10 +16,11 @@
 //   - one thread issues the chunk's tcgen05.mma (kind::f8f6f4, M = 128, N = 128, K = 32 each)
 //     into one of four 128-column FP32 accumulators in tensor memory; tcgen05.commit signals
 //     mbarriers when a chunk buffer is read and when a tile's accumulator is complete;
-//   - epilogue warps read a complete accumulator with tcgen05.ld while the next tiles' MMAs run:
-//     every (row, query) score becomes the same candidate key as in the other passes and is
-//     compared with the query's threshold; hits are appended exactly as the dp4a pass appends
-//     them.
+//   - epilogue warps read a complete accumulator with tcgen05.ld while the next tiles' MMAs run and
+//     compare every (row, query) score with the query's threshold; a hit goes into the CTA's queue
+//     (device memory, in practice L2);
+//   - one warp drains the queue, appending the hits to the queries' survivors as the same candidate
+//     keys as in the other passes, so that no epilogue warp waits on an atomic's round trip.
 // Two blocks of 128 queries run together on CTA pairs (cta_group::2, M = 256 over the pair's two
 // row tiles, N = 256 queries): the same roles in each CTA, the even CTA's thread issuing the MMAs
 // (see k_cand_tc).
@@ -38,13 +39,14 @@ namespace dev {
 // Warp roles: warps 0-7 stage the chunks (producers), warps 8-15 read the accumulators (warp w
 // may only read tensor-memory lanes 32 (w % 4) .. + 31; warps 8-11 take the first half of the
 // queries, warps 12-15 the second), warp 16 allocates tensor memory and its lane 0 issues the
-// MMAs (on a pair: the even CTA's; lanes 0 and 1 of the odd CTA's forward barrier phases).
-// They hand work over through mbarriers only.
+// MMAs (on a pair: the even CTA's; lanes 0 and 1 of the odd CTA's forward barrier phases), warp 17
+// appends the hits.  They hand work over through mbarriers only.
 constexpr int kTcProducers = 256;
 constexpr int kTcEpiWarp = 8;
 constexpr int kTcEpilogue = 256;
 constexpr int kTcMmaWarp = 16;
-constexpr int kTcThreads = 17 * 32;
+constexpr int kTcDrainWarp = 17;
+constexpr int kTcThreads = 18 * 32;
 constexpr uint32_t kTcTmemCols = 512;  // all of tensor memory, in FP32 accumulators
 // Queries per launch and accumulators.  One CTA: 128 queries (N = 128, M = 128), four
 // accumulators of 128 columns.  A CTA pair (cta_group::2): 256 queries (N = 256, each CTA
@@ -57,16 +59,21 @@ struct TcShape {
 };
 // mbarriers of a kernel with nb chunk buffers and acc accumulators: staged[nb] (producers ->
 // MMA), done[nb] (MMA -> producers), full[acc] (MMA -> epilogue), empty[acc] (epilogue -> MMA),
-// drain (the MMA thread's own MMAs complete); then the tensor-memory address and the give-up
-// flag
-__host__ __device__ constexpr uint32_t tc_nbars(uint32_t nb, uint32_t acc) { return 2 * nb + 2 * acc + 1; }
+// drain (the MMA thread's own MMAs complete), queued[kTcQueues] (epilogue -> drain warp),
+// drained[kTcQueues] (drain warp -> epilogue); then the tensor-memory address, the give-up flag
+// and the counts of the hit queues
+constexpr uint32_t kTcQueues = 4;       // units whose hits may wait (a long row hits for most queries)
+__host__ __device__ constexpr uint32_t tc_nbars(uint32_t nb, uint32_t acc) {
+  return 2 * nb + 2 * acc + 1 + 2 * kTcQueues;
+}
+constexpr uint32_t kTcQueueMax = 4096;  // hits of a unit that its queue holds at most
 
 // shared memory of one CTA of the pass with nb chunk buffers (2 or 3)
 __host__ inline size_t tc_smem_bytes(uint32_t cols, uint32_t split, uint32_t nb, bool pair) {
   const uint32_t S = split <= 1 ? 1 : split;
   const uint32_t q = pair ? 2 * kTcQ : kTcQ;
   return tc_qtab_bytes(cols) + nb * (size_t)kTcChunkBytes + (size_t)S * q * 4 +
-         ((tc_nbars(nb, kTcTmemCols / q) * 8 + 8 + 15) & ~15u);
+         ((tc_nbars(nb, kTcTmemCols / q) * 8 + 8 + kTcQueues * 4 + 15) & ~15u);
 }
 // chunk buffers for a configuration: three where they fit next to the query operand and the
 // thresholds (the producers then run two chunks ahead of the MMAs), else two
@@ -98,6 +105,8 @@ struct TcArgs {
   uint2* surv;           // [nq_total][split][cap]
   uint32_t cap;
   uint32_t* status;      // [nq_total]
+  uint2* queue;          // [gridDim.x][kTcQueues][queue_cap] hit queues of successive units
+  uint32_t queue_cap;
   uint32_t mma_idle;     // failure-path test: the MMA role issues nothing, so every hand-over
                          // wait of the other roles runs out and the CTA gives up
 };
@@ -248,69 +257,126 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Epilogue warps: reads accumulator `dbuf` of row tile T (thread = row, half the queries) and
-// appends every (row, query) key at or above the query's threshold.  thf holds the thresholds as
-// FP32 bounds on rs * score: rs is the row's scale, or 1 without row scales (the score is an
-// exact integer in FP32, and times 1 it stays itself).
-// A block of 32 queries is compared without branches into a bit mask of hits.  The hits of a
-// thread then take their survivor slots with atomics issued back to back (none waits for
-// another's result) before any survivor is written, so a block costs one atomic round trip
-// however many of its queries hit; the eight epilogue warps all work on the same tile, so a
-// round trip per hit would leave nothing to hide it behind.
+// N scores of a row (FP32 bits) for consecutive queries that passed the epilogue's bound where
+// `hit` has a bit: appended to the query's survivors if they pass the threshold itself.  qp: query
+// and partition of the first; rs: the row's scale, negative without row scales.  The loads and the
+// atomics of all N are in flight together.
+template <int N>
+__device__ __forceinline__ void tc_append(const TcArgs& a, uint32_t S, size_t qp, uint32_t row,
+                                          const uint32_t* score, uint32_t hit, float rs) {
+  uint32_t key[N], th[N], ix[N];
+#pragma unroll
+  for (int j = 0; j < N; j++) th[j] = (hit >> j) & 1u ? __ldg(a.thr + qp + (size_t)j * S) : 0xFFFFFFFFu;
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    const float f = __uint_as_float(score[j]);
+    key[j] = rs >= 0.0f ? key_f32(__fmul_rn(f, rs)) : key_i32(__float2int_rn(f));
+    if (key[j] < th[j]) hit &= ~(1u << j);
+  }
+#pragma unroll
+  for (int j = 0; j < N; j++)
+    if ((hit >> j) & 1u) ix[j] = atomicAdd(a.cnt + qp + (size_t)j * S, 1u);
+#pragma unroll
+  for (int j = 0; j < N; j++)
+    if (((hit >> j) & 1u) && ix[j] < a.cap)
+      a.surv[(qp + (size_t)j * S) * a.cap + ix[j]] = make_uint2(key[j], row);
+}
+// The hit queue of a unit: entries (query | row in tile << 8, score as FP32 bits); a group of hits
+// that passes its end is appended by the epilogue thread itself, the slots it had taken marked
+constexpr uint32_t kTcNoHit = 0xFFFFFFFFu;
+struct TcQueue {
+  uint2* e;
+  uint32_t* n;    // entries taken (may pass cap)
+  uint32_t cap;
+};
 // The thread's row of tile T, and its row scale (loaded before the accumulator wait, so that the
 // load's latency passes while the MMAs finish)
 __device__ __forceinline__ uint32_t tc_epi_row(uint32_t T) {
   return T * kTcRows + ((threadIdx.x >> 5) & 3u) * 32u + (threadIdx.x & 31u);
 }
-// The accumulator goes back to the MMA role (an arrive on `empty`) as soon as the thread's last
-// load from it has completed, so the compares of the last block overlap the next MMAs.
+// two FP32 fused multiply-adds per instruction
+__device__ __forceinline__ void tc_fma2(float& x0, float& x1, float a0, float a1, float b, float c0,
+                                        float c1) {
+  asm("{\n .reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %4};\n"
+      " mov.b64 c, {%5, %6};\n fma.rn.f32x2 d, a, b, c;\n mov.b64 {%0, %1}, d;\n}\n"
+      : "=f"(x0), "=f"(x1) : "f"(a0), "f"(a1), "f"(b), "f"(c0), "f"(c1));
+}
+// x[j] = score j times rs minus its bound (nthf: negated bounds, the same for every lane: 16-byte
+// broadcasts)
+__device__ __forceinline__ void tc_margin8(float (&x)[8], const uint32_t* v, float rs, const float* nthf) {
+  const float4 t0 = reinterpret_cast<const float4*>(nthf)[0];
+  const float4 t1 = reinterpret_cast<const float4*>(nthf)[1];
+  tc_fma2(x[0], x[1], __uint_as_float(v[0]), __uint_as_float(v[1]), rs, t0.x, t0.y);
+  tc_fma2(x[2], x[3], __uint_as_float(v[2]), __uint_as_float(v[3]), rs, t0.z, t0.w);
+  tc_fma2(x[4], x[5], __uint_as_float(v[4]), __uint_as_float(v[5]), rs, t1.x, t1.y);
+  tc_fma2(x[6], x[7], __uint_as_float(v[6]), __uint_as_float(v[7]), rs, t1.z, t1.w);
+}
+// Epilogue warps: reads accumulator `dbuf` of row tile T (thread = row, half the queries) and
+// queues every (row, query) score at or above the query's bound.  nthf holds the negated bounds on
+// rs * score (rs is the row's scale, or 1 without row scales, where the score is an exact integer),
+// so a score passes where fma(score, rs, -bound) >= 0.  A block of 32 queries costs a fused
+// multiply-add per two scores and the maximum of each group of eight (three-operand maxima); only
+// groups that reach 0 are looked at again, and take their queue slots with one atomic per block.  The accumulator goes back to the MMA role (an
+// arrive on `empty`) as soon as the thread's last load from it has completed.
+// The epilogue was the pass's longest stage: a block with a hit waited for the survivor counter's
+// atomic in device memory (over 1500 cycles; hits come in bursts, a long row passing for most of the
+// queries), and each score took three instructions.  With the queues and the fused compares
+// 2M rows x 1024, 64M entries: 748 -> 395 us for 256 queries, 375 -> 291 us for 128.
 template <bool PAIR>
 __device__ __forceinline__ void tc_epilogue(const TcArgs& a, uint32_t T, uint32_t tmem,
-                                            uint32_t dbuf, const float* thf_all, uint32_t S,
-                                            float rs, uint32_t empty) {
+                                            uint32_t dbuf, const float* nthf_all, uint32_t S,
+                                            float rs, uint32_t empty, const TcQueue& hq) {
   constexpr uint32_t Q = TcShape<PAIR>::Q, HALF = Q / 2;
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t g = warp & 3u, h = (warp - kTcEpiWarp) >> 2;
   const uint32_t row = tc_epi_row(T);
   const bool valid = row < a.n_rows;
   const uint32_t p = valid ? part_of(row, S, a.slice) : 0u;
-  const float* thf = thf_all + p * Q;
+  const float* nthf = nthf_all + p * Q;
 #pragma unroll 1
   for (uint32_t col0 = h * HALF; col0 < h * HALF + HALF; col0 += 32u) {
     uint32_t v[32];
+    __syncwarp();  // tcgen05.ld needs the warp together again after a block with hits
     tc_ld32(tmem + dbuf * Q + col0 + ((g * 32u) << 16), v);
     if (col0 + 32u == h * HALF + HALF) {  // the last load of this unit has completed
       tc_fence_before();
       tc_arrive(empty);
     }
-    uint32_t hit = 0;
+    if (col0 >= a.nq) continue;
+    float m[4];
 #pragma unroll
-    for (int j4 = 0; j4 < 8; j4++) {  // the same 32 thresholds for every lane: 16-byte broadcasts
-      const float4 x = reinterpret_cast<const float4*>(thf + col0)[j4];
-      const float tj[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const float f = __uint_as_float(v[4 * j4 + u]);
-        hit |= (__fmul_rn(f, rs) >= tj[u] ? 1u : 0u) << (4 * j4 + u);
-      }
+    for (int j8 = 0; j8 < 4; j8++) {
+      float x[8];
+      tc_margin8(x, v + 8 * j8, rs, nthf + col0 + 8 * j8);
+      const float m0 = fmaxf(fmaxf(x[0], x[1]), x[2]), m1 = fmaxf(fmaxf(x[3], x[4]), x[5]);
+      m[j8] = fmaxf(fmaxf(m0, m1), fmaxf(x[6], x[7]));
     }
-    if (!valid || col0 >= a.nq) hit = 0;
-    else if (a.nq - col0 < 32u) hit &= (1u << (a.nq - col0)) - 1u;
-    const size_t qp0 = (size_t)(a.q0 + col0) * S + p;
+    if (fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])) >= 0.0f && valid) {
+      uint32_t hit = 0;
 #pragma unroll
-    for (int j0 = 0; j0 < 32; j0 += 16) {  // 16 slots at a time keeps the slot indices in registers
-      if (!((hit >> j0) & 0xFFFFu)) continue;
-      uint32_t ix[16];
+      for (int j8 = 0; j8 < 4; j8++) {
+        if (m[j8] >= 0.0f) {
+          float x[8];
+          tc_margin8(x, v + 8 * j8, rs, nthf + col0 + 8 * j8);
 #pragma unroll
-      for (int j = j0; j < j0 + 16; j++)
-        if ((hit >> j) & 1u) ix[j - j0] = atomicAdd(a.cnt + qp0 + (size_t)j * S, 1u);
-#pragma unroll
-      for (int j = j0; j < j0 + 16; j++) {
-        if (((hit >> j) & 1u) && ix[j - j0] < a.cap) {
-          const float f = __uint_as_float(v[j]);
-          const uint32_t key = a.rowscale ? key_f32(__fmul_rn(f, rs)) : key_i32(__float2int_rn(f));
-          a.surv[(qp0 + (size_t)j * S) * a.cap + ix[j - j0]] = make_uint2(key, row);
+          for (int j = 0; j < 8; j++) hit |= (x[j] >= 0.0f ? 1u : 0u) << (8 * j8 + j);
         }
+      }
+      const uint32_t nh = __popc(hit);
+      uint32_t i = atomicAdd(hq.n, nh);
+      if (i + nh <= hq.cap) {
+        const uint32_t meta = col0 | (row % kTcRows) << 8;
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+          if ((hit >> j) & 1u) hq.e[i++] = make_uint2(meta + j, v[j]);
+      } else {
+        for (; i < hq.cap; i++) hq.e[i] = make_uint2(kTcNoHit, 0u);
+        const size_t qp = (size_t)(a.q0 + col0) * S + p;
+#pragma unroll
+        for (int j8 = 0; j8 < 4; j8++)
+          if ((hit >> (8 * j8)) & 255u)
+            tc_append<8>(a, S, qp + (size_t)(8 * j8) * S, row, v + 8 * j8, hit >> (8 * j8),
+                         a.rowscale ? rs : -1.0f);
       }
     }
   }
@@ -371,7 +437,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
   static_assert(NB == 2 || NB == 3, "two or three chunk buffers");
   constexpr uint32_t Q = TcShape<PAIR>::Q, ACC = TcShape<PAIR>::ACC;
   constexpr uint32_t kDone = NB, kFull = 2 * NB, kEmpty = 2 * NB + ACC;
-  constexpr uint32_t kDrain = kEmpty + ACC, kBars = tc_nbars(NB, ACC);
+  constexpr uint32_t kDrain = kEmpty + ACC, kQueued = kDrain + 1, kDrained = kQueued + kTcQueues;
+  constexpr uint32_t kBars = tc_nbars(NB, ACC);
   constexpr uint32_t R = NB + 2;  // producer ring: the chunks of every buffer and two ahead
   extern __shared__ __align__(16) unsigned char smem[];
   const uint32_t qbytes = (a.kpad / 16u) * 2048u;
@@ -382,6 +449,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(thf + S * Q);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + kBars);
   volatile uint32_t* gave_up = tslot + 1;
+  uint32_t* hq_n = tslot + 2;  // [kTcQueues]
+  uint2* hq_e = a.queue + (size_t)blockIdx.x * kTcQueues * a.queue_cap;
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
   uint32_t rank = 0;  // the CTA's rank in its pair
   if constexpr (PAIR) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -395,20 +464,24 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
     for (uint32_t i = tid; i < qbytes / 16u; i += blockDim.x) dst[i] = src[i];
     uint4* z = reinterpret_cast<uint4*>(sa);
     for (uint32_t i = tid; i < NB * kTcChunkBytes / 16u; i += blockDim.x) z[i] = make_uint4(0, 0, 0, 0);
-    // thresholds as FP32 bounds on the score (int keys) or on rowscale * score:
-    // key >= th  <=>  x >= bound for every x the pass produces
+    // thresholds as negated FP32 bounds on the score (int keys) or on rowscale * score: every
+    // x with key(x) >= th has x >= bound.  With row scales the product is rounded before it becomes
+    // a key, and may round up to the threshold, so the bound is the float below it; the exact
+    // comparison is made where a hit is appended.
     for (uint32_t i = tid; i < S * Q; i += blockDim.x) {
       const uint32_t p = i / Q, q = i % Q;
       const uint32_t th = q < a.nq ? a.thr[(size_t)(a.q0 + q) * S + p] : 0xFFFFFFFFu;
       float fb;
       if (a.rowscale) {  // x >= +0, key(x) = bits(x) | 2^31; NaN bits: never
-        fb = th <= 0x80000000u ? -__int_as_float(0x7f800000) : __uint_as_float(th & 0x7FFFFFFFu);
+        fb = th <= 0x80000000u ? -__int_as_float(0x7f800000)
+                               : (th > 0xFF800000u ? __int_as_float(0x7f800000)
+                                                   : __uint_as_float((th & 0x7FFFFFFFu) - 1u));
       } else {           // |score| < 2^24, exact in FP32
         const int32_t b = (int32_t)(th ^ 0x80000000u);
         fb = b > (1 << 24) ? __int_as_float(0x7f800000)
                            : (b < -(1 << 24) ? -__int_as_float(0x7f800000) : __int2float_rn(b));
       }
-      thf[i] = fb;
+      thf[i] = -fb;
     }
   }
   if (tid == 0) {
@@ -419,10 +492,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
       // it stays off the producers' and the epilogue's paths)
       const uint32_t fwd = (PAIR && rank == 0) ? 1u : 0u;
       const uint32_t cnt = (b < kDone) ? (uint32_t)kTcProducers + fwd
-                                       : ((b >= kEmpty && b < kDrain) ? (uint32_t)kTcEpilogue + fwd : 1u);
+                           : ((b >= kEmpty && b < kDrain) ? (uint32_t)kTcEpilogue + fwd
+                           : ((b >= kQueued && b < kDrained) ? (uint32_t)kTcEpilogue : 1u));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(tc_smem_u32(bars + b)), "r"(cnt));
     }
     *gave_up = 0u;
+    for (uint32_t b = 0; b < kTcQueues; b++) hq_n[b] = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kTcMmaWarp) tc_alloc<PAIR>(tc_smem_u32(tslot));
@@ -434,6 +509,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
   const uint32_t tmem = *tslot;
   const uint32_t b_staged = tc_smem_u32(bars), b_done = tc_smem_u32(bars + kDone);
   const uint32_t b_full = tc_smem_u32(bars + kFull), b_empty = tc_smem_u32(bars + kEmpty);
+  const uint32_t b_queued = tc_smem_u32(bars + kQueued), b_drained = tc_smem_u32(bars + kDrained);
   const uint32_t ntl = n_units > unit ? (n_units - unit + units - 1) / units : 0u;
   const uint32_t total = ntl * a.nch;  // chunks of this CTA (PAIR: the same in both CTAs)
   bool ok = true;
@@ -503,19 +579,70 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
     for (uint32_t tl = 0; tl < ntl; tl++) {
       const uint32_t d = tl % ACC;
       const uint32_t T = tile_of(unit + tl * units), row = tc_epi_row(T);
+      // this unit's hit queue is drained of the unit kTcQueues back
+      const uint32_t hb = tl % kTcQueues;
+      if (tl >= kTcQueues) ok &= tc_wait(b_drained + 8u * hb, (tl / kTcQueues - 1u) & 1u, gave_up);
       // without row scales rs = 1: f * 1 is f exactly, so every score takes one path
       const float rs = a.rowscale ? (row < a.n_rows ? __ldg(a.rowscale + row) : 0.0f) : 1.0f;
-      ok &= tc_wait<PAIR>(b_full + 8u * d, (tl / ACC) & 1u, gave_up);
+      if (ok) ok &= tc_wait<PAIR>(b_full + 8u * d, (tl / ACC) & 1u, gave_up);
       ok = __all_sync(0xFFFFFFFFu, ok);  // tcgen05.ld needs the whole warp
       if (!ok) break;
       tc_fence_after();
-      tc_epilogue<PAIR>(a, T, tmem, d, thf, S, rs, b_empty + 8u * d);
+      tc_epilogue<PAIR>(a, T, tmem, d, thf, S, rs, b_empty + 8u * d,
+                        TcQueue{hq_e + (size_t)hb * a.queue_cap, hq_n + hb, a.queue_cap});
+      tc_arrive(b_queued + 8u * hb);
+    }
+  } else if (warp == kTcDrainWarp) {
+    // ---- drain: appends each unit's queued hits, four per lane at a time ------------------------
+    const uint32_t lane = tid & 31u;
+    for (uint32_t tl = 0; tl < ntl; tl++) {
+      const uint32_t b = tl % kTcQueues, T = tile_of(unit + tl * units);
+      ok = tc_wait(b_queued + 8u * b, (tl / kTcQueues) & 1u, gave_up);
+      if (!__all_sync(0xFFFFFFFFu, ok)) break;
+      const uint32_t n = min(*reinterpret_cast<volatile uint32_t*>(hq_n + b), a.queue_cap);
+      const volatile uint2* hq = hq_e + (size_t)b * a.queue_cap;
+      for (uint32_t i0 = 0; i0 < n; i0 += 128u) {
+        uint32_t meta[4], score[4], key[4], th[4], ix[4];
+        size_t qp[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const uint32_t i = i0 + u * 32u + lane;
+          meta[u] = i < n ? hq[i].x : kTcNoHit;
+          score[u] = i < n ? hq[i].y : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          th[u] = 0xFFFFFFFFu;
+          key[u] = 0u;
+          if (meta[u] != kTcNoHit) {
+            const uint32_t row = T * kTcRows + (meta[u] >> 8);
+            qp[u] = (size_t)(a.q0 + (meta[u] & 255u)) * S + part_of(row, S, a.slice);
+            th[u] = __ldg(a.thr + qp[u]);
+            const float f = __uint_as_float(score[u]);
+            key[u] = a.rowscale ? key_f32(__fmul_rn(f, __ldg(a.rowscale + row)))
+                                : key_i32(__float2int_rn(f));
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          if (meta[u] != kTcNoHit && key[u] >= th[u]) ix[u] = atomicAdd(a.cnt + qp[u], 1u);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          if (meta[u] != kTcNoHit && key[u] >= th[u] && ix[u] < a.cap)
+            a.surv[qp[u] * a.cap + ix[u]] = make_uint2(key[u], T * kTcRows + (meta[u] >> 8));
+      }
+      __syncwarp();
+      if (lane == 0) {
+        hq_n[b] = 0u;
+        tc_arrive(b_drained + 8u * b);
+      }
     }
   } else if ((tid & 31u) == 0 && rank == 0) {
     // ---- MMA issue (one thread; PAIR: of the even CTA) ----------------------------------------
-    // instruction descriptor: FP32 accumulator, e4m3 x e4m3, both K-major, N = Q, M = 128 (256
-    // over a pair)
-    const uint32_t idesc = (1u << 4) | ((Q >> 3) << 17) | (((PAIR ? 2u : 1u) * kTcRows >> 4) << 24);
+    // instruction descriptor: FP32 accumulator, e4m3 x e4m3, both K-major, N = Q (one CTA: no more
+    // than the queries need), M = 128 (256 over a pair)
+    const uint32_t n = PAIR ? Q : (min(a.nq, Q) + 15u) & ~15u;
+    const uint32_t idesc = (1u << 4) | ((n >> 3) << 17) | (((PAIR ? 2u : 1u) * kTcRows >> 4) << 24);
     const uint32_t sq_addr = tc_smem_u32(sq), sa_addr = tc_smem_u32(sa);
     uint32_t tl = 0, c = 0, issued = 0;
     for (uint32_t i = 0; i < total && !a.mma_idle; i++) {

@@ -149,3 +149,28 @@ def test_fp32_only_batches(rows, cols, kind, p0, p1, nq, k, ck, stride):
             n = min(kk, rows)
             assert np.array_equal(idx[i, :n], ri[:n]) and np.array_equal(sc[i, :n], rs[:n]), i
             assert np.all(idx[i, n:] == 0xFFFFFFFF)
+
+
+@pytest.mark.parametrize("rows,cols,quant,split,nq,ck,hot", [
+    (4000, 1024, 0, 1, 200, 4000, 0),   # every score passes: the hit queues overflow
+    (90000, 256, 0, 1, 130, 64, 300),   # rows that pass for every query, in one tile
+    (90000, 256, 1, 4, 256, 64, 300),   # with row scales and partitions
+    (3000, 96, 1, 1, 25, 100, 40),      # one block of few queries
+])
+def test_tensor_hit_queues(rows, cols, quant, split, nq, ck, hot):
+    """Hits of the tensor-core pass go through per-CTA queues: units with none, with bursts of one
+    row for every query and with more hits than a queue holds give the oracle's candidates."""
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 4, 12, seed=rows)
+    if hot:  # consecutive rows of many large entries
+        d = np.diff(ptr).astype(np.int64)
+        d[rows // 2:rows // 2 + hot] = cols // 2
+        ptr = np.concatenate([[0], np.cumsum(d)]).astype(np.uint64)
+        rng = np.random.default_rng(3)
+        col = np.concatenate([np.sort(rng.choice(cols, n, replace=False)) for n in d]).astype(np.uint32)
+        val = rng.random(int(ptr[-1])).astype(np.float32)
+    m = orc.Matrix(rows, cols, ptr, col, val, 4, quant)
+    eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=4, quant=quant, split=split, ck=ck,
+                 k_max=20, max_batch=nq, batch_tile=128, flags=E.FLAG_TENSOR)
+    assert eng.info()["tensor_tiles"] == 1
+    Q = np.random.default_rng(nq).random((nq, cols)).astype(np.float32)
+    _check(m, eng, Q, split, ck, 20, every=max(1, nq // 6))
