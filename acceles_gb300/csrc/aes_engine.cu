@@ -73,17 +73,19 @@ static PlainKernel pick_plain(int bits, bool sgn, int mode) {
   }
 }
 
+constexpr uint64_t kMultiSampleMax = 16 * 1024;  // sample tiles x groups of four queries
+
 typedef void (*MultiKernel)(MultiArgs);
-template <int B>
+template <int B, bool SAMPLE>
 static MultiKernel multi_kernel(bool sgn, bool scaled) {
-  return sgn ? k_cand_multi<B, true, false>
-             : (scaled ? k_cand_multi<B, false, true> : k_cand_multi<B, false, false>);
+  return sgn ? k_cand_multi<B, true, false, SAMPLE>
+             : (scaled ? k_cand_multi<B, false, true, SAMPLE> : k_cand_multi<B, false, false, SAMPLE>);
 }
-static MultiKernel pick_multi(int bits, bool sgn, bool scaled) {
+static MultiKernel pick_multi(int bits, bool sgn, bool scaled, bool sample) {
   switch (bits) {
-    case 4: return multi_kernel<4>(sgn, scaled);
-    case 6: return multi_kernel<6>(sgn, scaled);
-    default: return multi_kernel<8>(sgn, scaled);
+    case 4: return sample ? multi_kernel<4, true>(sgn, scaled) : multi_kernel<4, false>(sgn, scaled);
+    case 6: return sample ? multi_kernel<6, true>(sgn, scaled) : multi_kernel<6, false>(sgn, scaled);
+    default: return sample ? multi_kernel<8, true>(sgn, scaled) : multi_kernel<8, false>(sgn, scaled);
   }
 }
 
@@ -329,7 +331,7 @@ struct Engine {
              uint32_t* repaired);
   int run_plain(int mode, uint32_t q, cudaStream_t s, uint32_t nq_y = 1);
   int run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0 = 0, uint32_t nblk = 0);
-  int run_multi(uint32_t nq, cudaStream_t s);
+  int run_multi(uint32_t nq, cudaStream_t s, bool sample = false);
   int run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint32_t* cnt, cudaStream_t s);
   int run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s);
   int run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair);
@@ -765,7 +767,8 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
     AES_CK(raise_smem((const void*)pick_plain((int)bits, sgn, mode)));
   for (int mode = 0; mode < 2; mode++)
     AES_CK(raise_smem((const void*)pick_batch((int)bits, sgn, mode)));
-  AES_CK(raise_smem((const void*)pick_multi((int)bits, sgn, d_rowscale != nullptr)));
+  for (int sample = 0; sample < 2; sample++)
+    AES_CK(raise_smem((const void*)pick_multi((int)bits, sgn, d_rowscale != nullptr, sample)));
   AES_CK(raise_smem((const void*)k_final));
   AES_CK(raise_smem((const void*)k_exact_multi<8>));
   if (tc_ready) {
@@ -951,8 +954,8 @@ int Engine::run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0, uint
   return AES_OK;
 }
 
-// The filter pass of an nq-query batch, four queries per matrix read
-int Engine::run_multi(uint32_t nq, cudaStream_t s) {
+// The filter (or sample) pass of an nq-query batch, four queries per matrix read
+int Engine::run_multi(uint32_t nq, cudaStream_t s, bool sample) {
   MultiArgs a{};
   a.tiles = d_tiles;
   a.tile_rowbase = d_tile_rowbase;
@@ -969,6 +972,11 @@ int Engine::run_multi(uint32_t nq, cudaStream_t s) {
   a.cnt = d_cnt;
   a.surv = d_surv;
   a.cap = cap;
+  a.keys_out = d_sample_keys;
+  a.keys_ld = n_sample_rows;
+  a.sample_first = d_sample_first;
+  a.sample_stride = ss;
+  a.n_sample_tiles = n_sample_tiles;
   // One CTA per SM holds the query table, so `waves` waves of CTAs share the groups of four
   // queries.  Every warp pays for its table (about 1.5 tiles' time) and for the tile that closes
   // its last row besides its own tiles, so few CTAs per group, all groups at once, beat a wave per
@@ -976,25 +984,26 @@ int Engine::run_multi(uint32_t nq, cudaStream_t s) {
   const uint32_t groups = (nq + kMultiQ - 1) / kMultiQ;
   uint32_t grid = 1;
   double best = 1e300;
+  const uint64_t work = sample ? 2ull * n_sample_tiles : tiles;  // a sample tile and the one closing it
   for (uint32_t waves = 1; waves <= groups; waves++) {
     const uint32_t g = std::max<uint32_t>(
         1, std::min<uint64_t>((uint64_t)sm_count * waves / groups, (uint64_t)sm_count));
     const double cost = (double)((g * (uint64_t)groups + sm_count - 1) / sm_count) *
-                        (2.5 + (double)((tiles + (uint64_t)g * kMultiWarps - 1) / ((uint64_t)g * kMultiWarps)));
+                        (2.5 + (double)((work + (uint64_t)g * kMultiWarps - 1) / ((uint64_t)g * kMultiWarps)));
     if (cost < best) {
       best = cost;
       grid = g;
     }
   }
-  const bool prof = (prm.flags & AES_FLAG_PROFILE) != 0;
+  const bool prof = (prm.flags & AES_FLAG_PROFILE) && !sample;
   int rc = prof ? prof_open(s) : AES_OK;
   if (rc) return rc;
-  pick_multi((int)bits, sgn, d_rowscale != nullptr)
+  pick_multi((int)bits, sgn, d_rowscale != nullptr, sample)
       <<<dim3(grid, groups), kMultiThreads, multi_smem_bytes(cols, split), s>>>(a);
   AES_CK(cudaGetLastError());
   if (prof && (rc = prof_close(s))) return rc;
   n_launch++;
-  n_cand++;
+  if (!sample) n_cand++;
   return AES_OK;
 }
 
@@ -1042,21 +1051,38 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   const bool batched = batch_mode != 1 && (batch_mode != 0 || nq > multi_max);
   last_batched = batched;
   const uint32_t nblk = (nq + kBatchQ - 1) / kBatchQ;
-  if (batched) {
+  // The sample pass.  By fours of queries (query-major keys) up to about nine tiles of every warp of
+  // the chip; past that by blocks of 128, one read of the few sample tiles for all of a block, and a
+  // transpose of the keys.  By blocks and by fours: 100 queries of 400k x 500 35 / 9 us, 256 of
+  // 2M x 1024 46 / 35 us (14.7k tiles x groups), 512 of 4M x 1024 43 / 63 us (47k).
+  const uint64_t sample_work = (uint64_t)n_sample_tiles * ((nq + kMultiQ - 1) / kMultiQ);
+  const bool sample_blocks = batched && sample_work > kMultiSampleMax;
+  if (batched && (!use_tc || sample_blocks)) {
     k_qtable<<<(uint32_t)((nblk * batch_qtab_words(cols) + 255) / 256), 256, 0, s>>>(
         d_q8, ld8, cols, nq, d_qtab);
     AES_CK(cudaGetLastError());
     n_launch++;
-    if (use_tc) {
-      for (uint32_t b = 0; b < nblk; b++) {
-        const uint32_t nb = std::min<uint32_t>(kBatchQ, nq - b * kBatchQ);
-        k_qtable_tc<<<(kTcQ * tc_kpad(cols) + 255) / 256, 256, 0, s>>>(
-            d_q8, ld8, cols, b * kTcQ, nb, d_qtab_tc + (size_t)b * tc_qtab_bytes(cols));
-        AES_CK(cudaGetLastError());
-        n_launch++;
-      }
+  }
+  if (batched && use_tc) {
+    for (uint32_t b = 0; b < nblk; b++) {
+      const uint32_t nb = std::min<uint32_t>(kBatchQ, nq - b * kBatchQ);
+      k_qtable_tc<<<(kTcQ * tc_kpad(cols) + 255) / 256, 256, 0, s>>>(
+          d_q8, ld8, cols, b * kTcQ, nb, d_qtab_tc + (size_t)b * tc_qtab_bytes(cols));
+      AES_CK(cudaGetLastError());
+      n_launch++;
     }
+  }
+  if (sample_blocks) {
     int rc = run_batch(MODE_SAMPLE, nq, s);
+    if (rc) return rc;
+    if (n_sample_rows) {  // the threshold pass reads each query's keys contiguously
+      k_keys_transpose<<<dim3((n_sample_rows + kTransposeRows - 1) / kTransposeRows, nblk), 256, 0, s>>>(
+          d_sample_keys, n_sample_rows, nq, d_keys_t);
+      AES_CK(cudaGetLastError());
+      n_launch++;
+    }
+  } else if (batch_mode != 1 && nq > 1) {
+    int rc = run_multi(nq, s, true);
     if (rc) return rc;
   } else {
     for (uint32_t q0 = 0; q0 < nq; q0 += 65535u) {  // every query's sample pass in one launch
@@ -1064,13 +1090,7 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
       if (rc) return rc;
     }
   }
-  if (batched && n_sample_rows) {  // the threshold pass reads each query's keys contiguously
-    k_keys_transpose<<<dim3((n_sample_rows + kTransposeRows - 1) / kTransposeRows, nblk), 256, 0, s>>>(
-        d_sample_keys, n_sample_rows, nq, d_keys_t);
-    AES_CK(cudaGetLastError());
-    n_launch++;
-  }
-  int rct = run_threshold(batched ? d_keys_t : d_sample_keys, nq, d_thr, d_cnt, s);
+  int rct = run_threshold(sample_blocks ? d_keys_t : d_sample_keys, nq, d_thr, d_cnt, s);
   if (rct) return rct;
   if (batched) {
     if (use_tc) {

@@ -32,6 +32,10 @@ struct MultiArgs {
   uint32_t* cnt;                // [nq][split]
   uint2* surv;                  // [nq][split][cap]
   uint32_t cap;
+  uint32_t* keys_out;           // sample pass: [nq][keys_ld]
+  uint32_t keys_ld;
+  const uint32_t* sample_first; // owned-row offset per sample tile
+  uint32_t sample_stride, n_sample_tiles;
 };
 
 __host__ inline size_t multi_smem_bytes(uint32_t cols, uint32_t split) {
@@ -94,6 +98,29 @@ struct MultiEmit {
           if (i < a.cap) a.surv[qp * a.cap + i] = make_uint2(key, row);
         }
       }
+    }
+  }
+};
+
+// The sample pass: every row's key, query-major
+template <int SHIFT, bool SCALED>
+struct MultiSampleEmit {
+  const MultiArgs& a;
+  uint32_t q0, nq;
+  uint32_t base;  // first owned row of the tile minus its key index
+  __device__ __forceinline__ void bounds(uint32_t, uint32_t, int32_t (&b)[kMultiQ]) const {
+#pragma unroll
+    for (int t = 0; t < kMultiQ; t++) b[t] = 0;
+  }
+  __device__ __forceinline__ void operator()(bool valid, uint32_t row, const uint32_t (&sum)[kMultiQ],
+                                             const int32_t (&)[kMultiQ]) const {
+    if (!valid) return;
+    const float rs = SCALED ? __ldg(a.rowscale + row) : 0.0f;
+#pragma unroll
+    for (int t = 0; t < kMultiQ; t++) {
+      const int32_t sc = (int32_t)sum[t] >> SHIFT;
+      const uint32_t key = SCALED ? key_f32(__fmul_rn(__int2float_rn(sc), rs)) : key_i32(sc);
+      if ((uint32_t)t < nq) a.keys_out[(size_t)(q0 + t) * a.keys_ld + (row - base)] = key;
     }
   }
 };
@@ -347,7 +374,7 @@ __device__ void multi_range(const MultiArgs& a, uint32_t tb, uint32_t te, const 
   }
 }
 
-template <int B, bool SGN, bool SCALED>
+template <int B, bool SGN, bool SCALED, bool SAMPLE>
 __global__ void __launch_bounds__(kMultiThreads, 1) k_cand_multi(MultiArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);
@@ -373,6 +400,17 @@ __global__ void __launch_bounds__(kMultiThreads, 1) k_cand_multi(MultiArgs a) {
       qt[i] = make_uint4(v, v, v, v);
     }
   }
+  const uint32_t gw = blockIdx.x * kMultiWarps + warp, nw = gridDim.x * kMultiWarps;
+  constexpr int SHIFT = SCALED ? 0 : PacketSpans<B, SGN>::kScoreShift;
+  if constexpr (SAMPLE) {
+    __syncthreads();
+    for (uint32_t i = gw; i < a.n_sample_tiles; i += nw) {
+      const uint32_t t = i * a.sample_stride;
+      const MultiSampleEmit<SHIFT, SCALED> em{a, q0, nq, __ldg(a.sample_first + i)};
+      multi_range<B, SGN, SCALED>(a, t, t + 1, em, qtb, stg);
+    }
+    return;
+  }
   const bool in_smem = a.split > 1 && a.split <= kThrSmemMax;
   if (in_smem)
     for (uint32_t i = threadIdx.x; i < a.split * kMultiQ; i += kMultiThreads) {
@@ -380,11 +418,9 @@ __global__ void __launch_bounds__(kMultiThreads, 1) k_cand_multi(MultiArgs a) {
       thr_s[i] = t < nq ? a.thr[(size_t)(q0 + t) * a.split + p] : 0xFFFFFFFFu;
     }
   __syncthreads();
-  const uint32_t gw = blockIdx.x * kMultiWarps + warp, nw = gridDim.x * kMultiWarps;
   const uint64_t n = a.n_tiles;
   const uint32_t tb = (uint32_t)((n * gw) / nw), te = (uint32_t)((n * (gw + 1)) / nw);
-  const MultiEmit<SCALED ? 0 : PacketSpans<B, SGN>::kScoreShift, SCALED> em{
-      a, in_smem ? thr_s : nullptr, q0, nq};
+  const MultiEmit<SHIFT, SCALED> em{a, in_smem ? thr_s : nullptr, q0, nq};
   multi_range<B, SGN, SCALED>(a, tb, te, em, qtb, stg);
 }
 

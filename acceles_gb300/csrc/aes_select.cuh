@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kThrWarps * 32) k_threshold_warp(
 // base(q) = (q / qblk) * qblk * ld_keys + q % qblk and stride qblk.
 //
 // Ranks up to kThrRankMax: every thread's largest key is found in one pass; the r-th largest of
-// those maxima (of 128 groups of four threads where r is small) is a bound that r keys reach and
+// those maxima (of groups of two or four threads where r is small) is a bound that r keys reach and
 // few others do, so the few threads at or above it gather their keys of at least that bound, and
 // the r-th largest of the gathered keys is the answer.  One read of the keys, where two
 // histograms took three: 27 -> 12.8 us for 39k keys, r = 24.  Larger ranks: two histograms.
@@ -254,11 +254,14 @@ __global__ void __launch_bounds__(kThreadsThr, 2) k_threshold(const uint32_t* __
   if (r <= kThrRankMax && n >= (uint32_t)kThreadsThr) {
     const uint32_t own = mx;
     uint32_t* gm = hist;  // group maxima
-    uint32_t per = 1;     // threads per maximum: 128 groups are enough for r <= 32
+    uint32_t per = 1;     // threads per maximum: 128 groups are enough for r <= 32, 256 for 64
     uint32_t g = mx;
+    if (r <= 64u) {
+      per = 2;
+      g = max(g, __shfl_xor_sync(0xFFFFFFFFu, g, 1));
+    }
     if (r <= 32u) {
       per = 4;
-      g = max(g, __shfl_xor_sync(0xFFFFFFFFu, g, 1));
       g = max(g, __shfl_xor_sync(0xFFFFFFFFu, g, 2));
     }
     const uint32_t ng = kThreadsThr / per, mine = threadIdx.x / per;

@@ -174,3 +174,17 @@ def test_tensor_hit_queues(rows, cols, quant, split, nq, ck, hot):
     assert eng.info()["tensor_tiles"] == 1
     Q = np.random.default_rng(nq).random((nq, cols)).astype(np.float32)
     _check(m, eng, Q, split, ck, 20, every=max(1, nq // 6))
+
+
+@pytest.mark.parametrize("rows,stride,nq,bits,quant", [
+    (60000, 1, 40, 8, 0),     # every tile sampled, by fours of queries
+    (90000, 1, 200, 6, 0),    # ... by blocks of 128 (tiles x groups above the rule's line)
+    (40000, 8, 131, 4, 1),    # row scales; the last group of three
+])
+def test_sample_pass_forms(rows, stride, nq, bits, quant):
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, 600, 6, 18, seed=rows)
+    m = orc.Matrix(rows, 600, ptr, col, val, bits, quant)
+    eng = E.SpMV(rows, 600, ptr=ptr, col=col, val=val, bits=bits, quant=quant, split=1, ck=200, k_max=30,
+                 max_batch=nq, batch_tile=128, sample_stride=stride)
+    Q = np.random.default_rng(nq).random((nq, 600)).astype(np.float32)
+    _check(m, eng, Q, 1, 200, 30, every=max(1, nq // 6))
