@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -28,6 +29,7 @@
 #include "aes_batch.cuh"
 #include "aes_multi.cuh"
 #include "aes_tc.cuh"
+#include "aes_tf.cuh"
 
 namespace aes {
 const char* last_error_cstr();
@@ -138,6 +140,14 @@ struct Engine {
   uint32_t* d_tc_ent = nullptr;
   uint32_t tc_nch = 0, tc_rtiles = 0;
   bool tc_ready = false;
+  // the tensor-core pass as a filter (aes_tf.cuh): quantised rows, row sums, layout
+  uint32_t* d_tf_q = nullptr;
+  uint2* d_tf_rowstat = nullptr;
+  uint32_t *d_tf_ptr = nullptr, *d_tf_ent = nullptr;
+  bool tf_ready = false;
+  uint2* d_tf_list = nullptr;  // of the configuration: the filter's lists
+  uint32_t* d_tf_list_n = nullptr;
+  uint32_t tf_list_cap = 0;
   uint32_t* d_csr_ptr = nullptr;
   uint16_t* d_csr_col = nullptr;
   float* d_csr_val = nullptr;
@@ -210,9 +220,13 @@ struct Engine {
              std::tie(o.q, o.nq, o.k, o.idx, o.score, o.s, o.pre);
     }
   };
-  std::map<GraphKey, cudaGraphExec_t> graphs;
+  struct Graph {
+    cudaGraphExec_t ex;
+    uint64_t launches, cands;  // kernels inside
+    bool batched, tf;          // the forms it runs
+  };
+  std::map<GraphKey, Graph> graphs;
   uint64_t n_graph_launch = 0;
-  uint64_t graph_launches = 0, graph_cands = 0;  // kernels inside the last captured graph
 
   // profiling / counters
   uint64_t n_launch = 0, n_cand = 0, n_repaired = 0;
@@ -231,6 +245,8 @@ struct Engine {
   uint32_t batch_mode = 0;        // 0 auto, 1 never, else always
   uint32_t multi_max = 0;         // auto: the most queries that take the four-query pass
   bool use_tc = false;            // batched candidate pass on the tensor cores
+  bool use_tf = false;            // ... as a filter with an exact check
+  bool last_tf = false, last_pre = false;  // of the last run
   uint8_t* d_qtab_tc = nullptr;   // [blocks][tc_qtab_bytes(cols)] e4m3 query operands
   size_t tc_smem = 0;
   int tc_grid = 0;
@@ -250,7 +266,7 @@ struct Engine {
   ~Engine() { release(); }
 
   void drop_graphs() {
-    for (auto& g : graphs) cudaGraphExecDestroy(g.second);
+    for (auto& g : graphs) cudaGraphExecDestroy(g.second.ex);
     graphs.clear();
   }
 
@@ -334,16 +350,31 @@ struct Engine {
   int run_multi(uint32_t nq, cudaStream_t s, bool sample = false);
   int run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint32_t* cnt, cudaStream_t s);
   int run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s);
+  int run_check(uint32_t q0, uint32_t n, cudaStream_t s, uint32_t ctas);
   int run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair);
   int prof_open(cudaStream_t s);
   int prof_close(cudaStream_t s);
   int collect_profile();
   // the tensor-core pass serves a configuration: 4-bit layout built, flag set, thresholds of
   // every partition in shared memory, batched passes allowed
-  bool tc_usable(const aes_params& p, uint32_t S) const {
-    return tc_ready && (p.flags & AES_FLAG_TENSOR) && S <= kTcMaxSplit && p.batch_tile != 1 &&
-           tc_smem_bytes(cols, S, 2, false) <= (size_t)smem_optin;
+  bool tc_fits(const aes_params& p, uint32_t S) const {
+    return S <= kTcMaxSplit && p.batch_tile != 1 && tc_smem_bytes(cols, S, 2, false) <= (size_t)smem_optin;
   }
+  bool tc_usable(const aes_params& p, uint32_t S) const {
+    return tc_ready && (p.flags & AES_FLAG_TENSOR) && tc_fits(p, S);
+  }
+  // ... as a filter (build_tf has the reasons)
+  bool tf_usable(const aes_params& p, uint32_t S) const {
+    return tf_ready && p.max_batch > 64 && !p.mem_limit && tc_fits(p, S);
+  }
+  // entries of a filter CTA's list per block of 32 queries: twice its share of what the survivor
+  // buffers of 32 queries hold, or every row it can meet
+  uint32_t tf_list_entries(uint32_t c, uint32_t S) const {
+    const uint64_t share = 2ull * 32 * S * c / (uint32_t)sm_count + 512;
+    const uint64_t all = ((uint64_t)tc_rtiles / std::max(1, sm_count - 1) + 2) * kTcRows;
+    return (uint32_t)std::min(share, all);
+  }
+  int build_tf(const HostCSR& m, const aes_params& p, float gmax, size_t planned, size_t config);
 };
 
 // CUDA events around one full candidate-pass launch (AES_FLAG_PROFILE)
@@ -375,8 +406,10 @@ int Engine::prof_close(cudaStream_t s) {
 static_assert(kTcQ == kBatchQ, "tensor-core and dp4a passes use the same query blocks");
 int Engine::run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair) {
   TcArgs a{};
-  a.ent = d_tc_ent;
-  a.ptr = d_tc_ptr;
+  a.ent = use_tf ? d_tf_ent : d_tc_ent;
+  a.ptr = use_tf ? d_tf_ptr : d_tc_ptr;
+  a.rowstat = use_tf ? d_tf_rowstat : nullptr;
+  a.qstat = d_exact_aux + 4;
   a.n_rtiles = tc_rtiles;
   a.nch = tc_nch;
   a.kpad = tc_kpad(cols);
@@ -392,9 +425,13 @@ int Engine::run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair) {
   a.surv = d_surv;
   a.cap = cap;
   a.status = d_status;
-  // the hit queues take the sample keys' memory, dead once the thresholds are known
-  a.queue = reinterpret_cast<uint2*>(d_sample_keys);
-  a.queue_cap = (uint32_t)std::min<size_t>(kTcQueueMax, tail_bytes / (8ull * kTcQueues * (pair ? tc_grid2 : tc_grid)));
+  // the hit queues take the sample keys' memory, dead once the thresholds are known; a filter
+  // launch's lists their own
+  const uint32_t ctas = (uint32_t)(pair ? tc_grid2 : tc_grid);
+  a.queue = use_tf ? d_tf_list : reinterpret_cast<uint2*>(d_sample_keys);
+  a.queue_cap = use_tf ? tf_list_cap
+                       : (uint32_t)std::min<size_t>(kTcQueueMax, tail_bytes / (8ull * kTcQueues * ctas));
+  a.list_n = d_tf_list_n;
   a.mma_idle = (prm.flags & AES_FLAG_TEST_IDLE_MMA) ? 1u : 0u;
   const bool prof = (prm.flags & AES_FLAG_PROFILE) != 0;
   int rc = prof ? prof_open(s) : AES_OK;
@@ -423,6 +460,37 @@ int Engine::run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair) {
   if (prof && (rc = prof_close(s))) return rc;
   n_launch++;
   n_cand++;
+  return AES_OK;
+}
+
+// The exact check of what a filter launch of `ctas` CTAs let through for queries q0 .. q0 + n - 1
+int Engine::run_check(uint32_t q0, uint32_t n, cudaStream_t s, uint32_t ctas) {
+  TfCheck c{};
+  c.ptr = d_csr_ptr;
+  c.q = reinterpret_cast<const uint4*>(d_tf_q);
+  c.cols = cols;
+  c.seed = prm.seed;
+  c.q8 = d_q8;
+  c.ld8 = ld8;
+  c.sgn = sgn ? 1u : 0u;
+  c.q0 = q0;
+  c.nq = n;
+  c.list = d_tf_list;
+  c.list_n = d_tf_list_n;
+  c.list_cap = tf_list_cap;
+  c.ctas = ctas;
+  c.rowscale = d_rowscale;
+  c.thr = d_thr;
+  c.split = split;
+  c.slice = slice;
+  c.cap = cap;
+  c.status = d_status;
+  c.cnt = d_cnt;
+  c.surv = d_surv;
+  const uint32_t blocks = (n + 31) / 32;  // (six CTAs fit on an SM)
+  k_recheck<<<dim3(blocks, std::max(1u, 6u * (uint32_t)sm_count / blocks)), kThreadsCheck, check_smem_bytes(ld8), s>>>(c);
+  AES_CK(cudaGetLastError());
+  n_launch++;
   return AES_OK;
 }
 
@@ -467,12 +535,23 @@ int Engine::plan_config(const aes_params& p, Config* c) const {
   }
 
   // sample tiles: every ss-th tile, with the rows each one owns
-  // auto: every tile of a tiny matrix, else one tile in 64; one in 256 for a large matrix with
-  // one partition.  Several partitions keep Top-(CK/split) each: the bound of so few candidates
-  // from a sparse sample sits far below the boundary and lets many rows through to the survivor
-  // buffers (10M x 1024, 8-bit, 32 partitions: 99 us per pass at one tile in 256, 85 us at 64)
+  // auto: every tile of a tiny matrix, else one tile in 64, or in 256 of a large matrix with one
+  // partition (a 512-query batch of 95k tiles: 1.92 ms at 256, 2.02 at 128).  Several partitions keep Top-(CK/split) each: the bound of so few candidates from a
+  // sparse sample sits far below the boundary and lets many rows through to the survivor buffers
+  // (10M x 1024, 8-bit, 32 partitions: 99 us per pass at one tile in 256, 85 us at 64), so partitions
+  // of fewer rows are sampled up to one tile in 16, for some 780 rows each (100 queries of
+  // 400k x 500, 6-bit, 32 partitions: 278 us per call at 64, 223 us at 16).
+  // Under a memory limit the sparser rule, whose buffers are smaller: one in 64 and, above 16384
+  // tiles with one partition, 256.
   if (p.sample_stride) c->ss = p.sample_stride;
-  else c->ss = tiles <= 64 ? 1 : ((tiles <= 16384 || S > 1) ? 64 : 256);
+  else if (tiles <= 64) c->ss = 1;
+  else if (p.mem_limit) c->ss = (tiles <= 16384 || S > 1) ? 64 : 256;
+  else if (S > 1) {
+    c->ss = 64;
+    while (c->ss > 16 && c->slice / c->ss < 780) c->ss /= 2;
+  } else {
+    c->ss = tiles <= 65536 ? 64 : 256;
+  }
   const uint32_t ss_ = c->ss;
   c->n_sample_tiles = (uint32_t)((tiles + ss_ - 1) / ss_);
   auto owned_begin = [&](uint64_t t) -> uint64_t {
@@ -533,7 +612,8 @@ int Engine::plan_config(const aes_params& p, Config* c) const {
   plan += maxB * (ld32 * 4ull + ld8 + S * 8ull + (size_t)S * c->cap * 8 + c->nslots * 8ull + 4 +
                   p.k_max * 8ull);
   plan += nblk * batch_qtab_words(cols) * 4;
-  if (tc_usable(p, S)) plan += nblk * tc_qtab_bytes(cols);
+  if (tc_usable(p, S) || tf_usable(p, S)) plan += nblk * tc_qtab_bytes(cols);
+  if (!tc_usable(p, S) && tf_usable(p, S)) plan += (size_t)sm_count * kTcLists * (tf_list_entries(c->cap, S) * 8ull + 4);
   plan += p.k_max * 8ull;
   c->plan = plan;
 
@@ -581,10 +661,16 @@ int Engine::apply_config(const Config& c) {
   AES_AL(d_out_score, (size_t)maxB * std::max<uint32_t>(p.k_max, 1));
   AES_AL(d_qtab, (size_t)((maxB + kBatchQ - 1) / kBatchQ) * batch_qtab_words(cols));
   use_tc = tc_usable(p, split);
-  if (use_tc) AES_AL(d_qtab_tc, (size_t)((maxB + kTcQ - 1) / kTcQ) * tc_qtab_bytes(cols));
+  use_tf = !use_tc && tf_usable(p, split);
+  if (use_tf) {
+    tf_list_cap = tf_list_entries(cap, split);
+    AES_AL(d_tf_list, (size_t)sm_count * kTcLists * tf_list_cap);
+    AES_AL(d_tf_list_n, (size_t)sm_count * kTcLists);
+  }
+  if (use_tc || use_tf) AES_AL(d_qtab_tc, (size_t)((maxB + kTcQ - 1) / kTcQ) * tc_qtab_bytes(cols));
   AES_AL(d_exact_cand, std::max<uint32_t>(p.k_max, 1));
   AES_AL(d_exact_key, std::max<uint32_t>(p.k_max, 1));
-  AES_AL(d_exact_aux, 4);
+  AES_AL(d_exact_aux, 4 + kTfStats);  // and a filter launch's query statistics
 #undef AES_AL
   AES_CK(cudaMallocHost(&h_q32, (size_t)maxB * ld32 * sizeof(float)));
   AES_CK(cudaMallocHost(&h_q8, (size_t)maxB * ld8));
@@ -609,7 +695,9 @@ int Engine::apply_config(const Config& c) {
   // four-query pass against 128-query block: 8-bit, 40 queries 290 / 298 us (1M rows x 20 entries),
   // 48 queries 730 / 829 us (4M); 6-bit, 64 queries 395 / 449 us (1M); 4-bit 428 / 459 us.  The
   // tensor-core pass costs less per entry the larger the matrix: 24 queries 201 / 286 us (1M x 32).
-  multi_max = use_tc ? 24 : (bits == 8 ? 48 : 64);
+  // The filter form: 48 queries 301 / 303 us (6-bit, 1M), 709 / 708 us (8-bit, 4M), 164 / 142 us
+  // (400k x 500); 4-bit 32 queries 241 / 245 us.
+  multi_max = use_tc ? 24 : (use_tf ? (bits == 4 ? 32 : 44) : (bits == 8 ? 48 : 64));
   if (batch_mode != 1) {
     batch_smem = batch_smem_bytes((int)bits, cols, split, batch_warps_n);
     int occb = 0;
@@ -617,7 +705,7 @@ int Engine::apply_config(const Config& c) {
         &occb, (const void*)pick_batch((int)bits, sgn, MODE_FILTER), batch_warps_n * 32, batch_smem));
     batch_grid = std::max(1, occb) * sm_count;
   }
-  if (use_tc) {  // one CTA per SM (its shared memory), persistent over the 128-row tiles
+  if (use_tc || use_tf) {  // one CTA per SM (its shared memory), persistent over the 128-row tiles
     tc_nb = tc_bufs(cols, split, (size_t)smem_optin, false);
     tc_smem = tc_smem_bytes(cols, split, tc_nb, false);
     tc_grid = (int)std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)sm_count, tc_rtiles));
@@ -694,7 +782,7 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
   if (tiles >= 0xFFFFFFFFull) return fail(AES_ERR_UNSUPPORTED, "matrix too large");
   h_tile_rowbase = pm.tile_rowbase;
   tc_ready = !pm.tc_ptr.empty();
-  tc_nch = pm.tc_nch;
+  tc_nch = tc_nchunks(cols);
   tc_rtiles = (uint32_t)((rows + kTcRows - 1) / kTcRows);
   const size_t tc_bytes = tc_ready ? (pm.tc_ptr.size() + pm.tc_ent.size()) * 4 : 0;
 
@@ -754,6 +842,9 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
       AES_CK(cudaMemcpy(d_tc_ent, pm.tc_ent.data(), pm.tc_ent.size() * 4, cudaMemcpyHostToDevice));
   }
 
+  if ((rc = build_tf(m, p, pm.gmax, plan, c.plan))) return rc;
+  if (tf_ready && (rc = plan_config(p, &c))) return rc;  // (with the filter's lists)
+
   // the shared-memory limit is an attribute of the kernel, shared by every handle: raise it to
   // the device maximum (less the kernel's static shared memory) once, not to this handle's size
   auto raise_smem = [&](const void* f) -> cudaError_t {
@@ -771,7 +862,7 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
     AES_CK(raise_smem((const void*)pick_multi((int)bits, sgn, d_rowscale != nullptr, sample)));
   AES_CK(raise_smem((const void*)k_final));
   AES_CK(raise_smem((const void*)k_exact_multi<8>));
-  if (tc_ready) {
+  if (tc_ready || tf_ready) {
     AES_CK(raise_smem((const void*)k_cand_tc<2, false>));
     AES_CK(raise_smem((const void*)k_cand_tc<3, false>));
     AES_CK(raise_smem((const void*)k_cand_tc<2, true>));
@@ -786,6 +877,56 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
   rc = apply_config(c);
   if (rc) return rc;
   AES_CK(cudaDeviceSynchronize());
+  return AES_OK;
+}
+
+// The tensor-core layout and exact values behind the filter form of the batched pass (8 bytes per
+// entry and 24 per row), made on the device from the FP32 CSR: for handles whose batches can reach
+// it (above 64 queries), without a memory limit, and only where a quarter of the memory left over
+// holds it.  Not for pre-quantised matrices, nor where a row repeats a column (the dense tile
+// would keep one of the values).
+int Engine::build_tf(const HostCSR& m, const aes_params& p, float gmax, size_t planned, size_t config) {
+  if (p.max_batch <= 64 || p.mem_limit || !has_f32 || m.prequantized || tc_ready || nnz == 0 ||
+      p.batch_tile == 1)
+    return AES_OK;
+  const size_t need = nnz * 4 + tf_row_words(nnz, rows) * 4 + rows * 8ull + ((size_t)tc_rtiles * tc_nch + 1) * 4 + config;
+  size_t freeb = 0, totalb = 0;
+  AES_CK(cudaMemGetInfo(&freeb, &totalb));  // (the matrix arrays are allocated, the batch buffers not)
+  const size_t kept = planned + (64ull << 20);
+  if (freeb < kept || need > (freeb - kept) / 4) return AES_OK;
+  std::atomic<bool> dup{false};
+  parallel_for(rows, 1 << 16, [&](uint64_t b, uint64_t e) {
+    bool d = false;
+    for (uint64_t r = b; r < e; r++)
+      for (uint64_t i = m.ptr[r]; i + 1 < m.ptr[r + 1]; i++) d |= m.col[i] == m.col[i + 1];
+    if (d) dup = true;
+  });
+  if (dup) return AES_OK;
+  int rc = AES_OK;
+  if ((rc = dalloc(&d_tf_q, tf_row_words(nnz, rows))) || (rc = dalloc(&d_tf_rowstat, rows)) ||
+      (rc = dalloc(&d_tf_ent, nnz)) || (rc = dalloc(&d_tf_ptr, (size_t)tc_rtiles * tc_nch + 1)))
+    return rc;
+  TfMatrix a{};
+  a.ptr = d_csr_ptr;
+  a.col = d_csr_col;
+  a.val = d_csr_val;
+  a.rows = rows;
+  a.cols = cols;
+  a.nch = tc_nch;
+  a.bits = (int)bits;
+  a.quant = (int)quant;
+  a.gmax = gmax;
+  a.q = d_tf_q;
+  a.rowstat = d_tf_rowstat;
+  a.ent = d_tf_ent;
+  a.tptr = d_tf_ptr;
+  // (the default stream: after the uploads)
+  AES_CK(cudaMemsetAsync(d_tf_q, 0, tf_row_words(nnz, rows) * 4, 0));
+  k_tf_rows<<<std::min<uint32_t>((rows + 7) / 8, 16u * (uint32_t)sm_count), 256>>>(a);
+  AES_CK(cudaGetLastError());
+  k_tf_tiles<<<std::min<uint32_t>(tc_rtiles, 8u * (uint32_t)sm_count), 256>>>(a);
+  AES_CK(cudaGetLastError());
+  tf_ready = true;
   return AES_OK;
 }
 
@@ -809,6 +950,8 @@ int Engine::build_view(const Engine& b, const aes_params& p) {
   d_tiles = b.d_tiles; d_tile_rowbase = b.d_tile_rowbase; d_rowscale = b.d_rowscale;
   d_tc_ptr = b.d_tc_ptr; d_tc_ent = b.d_tc_ent; tc_nch = b.tc_nch; tc_rtiles = b.tc_rtiles;
   tc_ready = b.tc_ready;
+  d_tf_q = b.d_tf_q; d_tf_rowstat = b.d_tf_rowstat; d_tf_ptr = b.d_tf_ptr; d_tf_ent = b.d_tf_ent;
+  tf_ready = b.tf_ready;
   d_csr_ptr = b.d_csr_ptr; d_csr_col = b.d_csr_col; d_csr_val = b.d_csr_val;
   has_f32 = b.has_f32;
   ld32 = b.ld32; ld8 = b.ld8;
@@ -1012,8 +1155,11 @@ int Engine::run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint
                           cudaStream_t s) {
   if (part_samples <= kThrWarpKeys) {
     const uint64_t pairs = (uint64_t)split * nq;  // (below 2^28: max_batch and ck bound both)
-    k_threshold_warp<<<(uint32_t)((pairs + kThrWarps - 1) / kThrWarps), kThrWarps * 32, 0, s>>>(
-        keys, n_sample_rows, d_part_sample_begin, split, (uint32_t)pairs, d_part_r, thr, cnt);
+    const uint32_t g = (uint32_t)((pairs + kThrWarps - 1) / kThrWarps);
+    auto k = part_samples <= kThrWarpKeys / 2 ? k_threshold_warp<kThrWarpKeys / 64>
+                                              : k_threshold_warp<kThrWarpKeys / 32>;
+    k<<<g, kThrWarps * 32, 0, s>>>(keys, n_sample_rows, d_part_sample_begin, split, (uint32_t)pairs,
+                                   d_part_r, thr, cnt);
   } else {
     k_threshold<<<dim3(split, nq), kThreadsThr, 0, s>>>(keys, n_sample_rows, 0, d_part_sample_begin,
                                                         split, d_part_r, thr, cnt);
@@ -1050,6 +1196,9 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   n_launch += 3;  // threshold, select, final
   const bool batched = batch_mode != 1 && (batch_mode != 0 || nq > multi_max);
   last_batched = batched;
+  const bool tc = batched && (use_tc || use_tf), tf = batched && use_tf;
+  last_tf = tf;
+  last_pre = pre;
   const uint32_t nblk = (nq + kBatchQ - 1) / kBatchQ;
   // The sample pass.  By fours of queries (query-major keys) up to about nine tiles of every warp of
   // the chip; past that by blocks of 128, one read of the few sample tiles for all of a block, and a
@@ -1057,13 +1206,22 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   // 2M x 1024 46 / 35 us (14.7k tiles x groups), 512 of 4M x 1024 43 / 63 us (47k).
   const uint64_t sample_work = (uint64_t)n_sample_tiles * ((nq + kMultiQ - 1) / kMultiQ);
   const bool sample_blocks = batched && sample_work > kMultiSampleMax;
-  if (batched && (!use_tc || sample_blocks)) {
+  if (batched && (!tc || sample_blocks)) {
     k_qtable<<<(uint32_t)((nblk * batch_qtab_words(cols) + 255) / 256), 256, 0, s>>>(
         d_q8, ld8, cols, nq, d_qtab);
     AES_CK(cudaGetLastError());
     n_launch++;
   }
-  if (batched && use_tc) {
+  if (tf) {
+    uint32_t* st = d_exact_aux + 4;
+    AES_CK(cudaMemsetAsync(st, 0, kTfStats * 4, s));
+    k_tf_qstats<<<nq, 256, 0, s>>>(d_q8, ld8, cols, sgn ? 1u : 0u, st);
+    AES_CK(cudaGetLastError());
+    k_tf_qtable<<<(nblk * kTcQ * (tc_kpad(cols) / 16) + 255) / 256, 256, 0, s>>>(
+        d_q8, ld8, cols, nq, nblk, sgn ? 1u : 0u, st, d_qtab_tc);
+    AES_CK(cudaGetLastError());
+    n_launch += 2;
+  } else if (tc) {
     for (uint32_t b = 0; b < nblk; b++) {
       const uint32_t nb = std::min<uint32_t>(kBatchQ, nq - b * kBatchQ);
       k_qtable_tc<<<(kTcQ * tc_kpad(cols) + 255) / 256, 256, 0, s>>>(
@@ -1093,12 +1251,13 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   int rct = run_threshold(sample_blocks ? d_keys_t : d_sample_keys, nq, d_thr, d_cnt, s);
   if (rct) return rct;
   if (batched) {
-    if (use_tc) {
+    if (tc) {
       // two blocks per launch by CTA pairs where there are two; a last odd block alone
       for (uint32_t b = 0; b < nblk;) {
         const bool pair = tc_pair && b + 1 < nblk;
         const uint32_t nb = std::min<uint32_t>((pair ? 2u : 1u) * kBatchQ, nq - b * kBatchQ);
         int rc = run_tc(b, nb, s, pair);
+        if (rc == AES_OK && tf) rc = run_check(b * kBatchQ, nb, s, (uint32_t)(pair ? tc_grid2 : tc_grid));
         if (rc) return rc;
         b += pair ? 2u : 1u;
       }
@@ -1173,10 +1332,7 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
   GraphKey key{d_q, nq, k, d_idx, d_score, s, pre};
   auto it = graphs.find(key);
   if (it == graphs.end()) {
-    if (graphs.size() >= 64) {
-      for (auto& g : graphs) cudaGraphExecDestroy(g.second);
-      graphs.clear();
-    }
+    if (graphs.size() >= 64) drop_graphs();
     const uint32_t saved_flags = prm.flags;
     prm.flags &= ~AES_FLAG_PROFILE;
     const uint64_t saved_launch = n_launch, saved_cand = n_cand;
@@ -1194,15 +1350,17 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
     ce = cudaGraphInstantiate(&ex, graph, 0);
     cudaGraphDestroy(graph);
     if (ce != cudaSuccess) return ::aes::fail(AES_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ce));
-    it = graphs.emplace(key, ex).first;
-    graph_launches = n_launch - saved_launch;
-    graph_cands = n_cand - saved_cand;
+    it = graphs.emplace(key, Graph{ex, n_launch - saved_launch, n_cand - saved_cand, last_batched,
+                                   last_tf}).first;
     n_launch = saved_launch;
     n_cand = saved_cand;
   }
-  AES_CK(cudaGraphLaunch(it->second, s));
-  n_launch += graph_launches;
-  n_cand += graph_cands;
+  AES_CK(cudaGraphLaunch(it->second.ex, s));
+  n_launch += it->second.launches;
+  n_cand += it->second.cands;
+  last_batched = it->second.batched;
+  last_tf = it->second.tf;
+  last_pre = pre;
   n_graph_launch++;
   return AES_OK;
 }
@@ -1219,6 +1377,21 @@ int Engine::repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cud
                                                " has negative entries under an unsigned quantiser");
     if (h_status[q] & ST_DEVICE)
       return fail(AES_ERR_CUDA, "tensor-core candidate pass: a bounded wait gave up");
+  }
+  // The filter lets through more rows than reach the thresholds; where that overflows the survivor
+  // buffers of more than a few queries, its bounds are too wide for this data: the batch is run
+  // again, and later ones are run, with the dp4a pass.
+  if (last_tf) {
+    uint32_t over = 0;
+    for (uint32_t q = 0; q < nq; q++) over += (h_status[q] & ST_OVERFLOW) ? 1u : 0u;
+    if (over * 16 > nq) {
+      use_tf = false;
+      drop_graphs();
+      int rc = enqueue(last_q32, nq, k, d_idx, d_score, s, last_pre);
+      if (rc) return rc;
+      AES_CK(cudaMemcpyAsync(h_status, d_status, nq * 4ull, cudaMemcpyDeviceToHost, s));
+      AES_CK(cudaStreamSynchronize(s));
+    }
   }
   for (uint32_t q = 0; q < nq; q++) {
     if (!(h_status[q] & (ST_OVERFLOW | ST_MISS))) continue;

@@ -278,6 +278,7 @@ int quantize_and_pack(const HostCSR& m, const aes_params& p, PackedMatrix* out) 
       negative |= (neg[t] != 0);
     }
   }
+  out->gmax = (float)gmax;  // (an FP32 value)
   if (p.quant != AES_QUANT_SYM_GLOBAL && negative)
     return fail(AES_ERR_INVALID, "unsigned quantiser needs non-negative matrix values");
 

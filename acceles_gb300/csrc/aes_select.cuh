@@ -163,16 +163,16 @@ __device__ __forceinline__ uint32_t warp_rth_key(const uint32_t (&k)[N], uint32_
 // kThrWarpKeys samples: the keys stay in registers (100 queries x 32 partitions of 195 samples:
 // 43 -> 6.7 us); k_threshold, one CTA each, for the rest.
 // ---------------------------------------------------------------------------------------------
-constexpr uint32_t kThrWarpKeys = 512;   // 16 per lane
+constexpr uint32_t kThrWarpKeys = 1024;  // 32 per lane (16 for half as many)
 constexpr int kThrWarps = 4;             // (query, partition) pairs per CTA
 constexpr uint32_t kThrRankMax = 128;    // ranks up to which the CTA form selects by group maxima
 constexpr uint32_t kThrListMax = 1024;
 
+template <int N>
 __global__ void __launch_bounds__(kThrWarps * 32) k_threshold_warp(
     const uint32_t* __restrict__ keys_all, uint32_t ld_keys, const uint32_t* __restrict__ part_begin,
     uint32_t split, uint32_t pairs, const uint32_t* __restrict__ r_part, uint32_t* __restrict__ thr,
     uint32_t* __restrict__ cnt) {
-  constexpr int N = kThrWarpKeys / 32;
   const uint32_t i = blockIdx.x * kThrWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
   if (i >= pairs) return;
   const uint32_t p = i % split, q = i / split;

@@ -19,8 +19,8 @@
 //   - epilogue warps read a complete accumulator with tcgen05.ld while the next tiles' MMAs run and
 //     compare every (row, query) score with the query's threshold; a hit goes into the CTA's queue
 //     (device memory, in practice L2);
-//   - one warp drains the queue, appending the hits to the queries' survivors as the same candidate
-//     keys as in the other passes, so that no epilogue warp waits on an atomic's round trip.
+//   - three warps drain the queues, appending the hits to the queries' survivors as the same
+//     candidate keys as in the other passes, so that no epilogue warp waits on an atomic's round trip.
 // Two blocks of 128 queries run together on CTA pairs (cta_group::2, M = 256 over the pair's two
 // row tiles, N = 256 queries): the same roles in each CTA, the even CTA's thread issuing the MMAs
 // (see k_cand_tc).
@@ -39,14 +39,15 @@ namespace dev {
 // Warp roles: warps 0-7 stage the chunks (producers), warps 8-15 read the accumulators (warp w
 // may only read tensor-memory lanes 32 (w % 4) .. + 31; warps 8-11 take the first half of the
 // queries, warps 12-15 the second), warp 16 allocates tensor memory and its lane 0 issues the
-// MMAs (on a pair: the even CTA's; lanes 0 and 1 of the odd CTA's forward barrier phases), warp 17
-// appends the hits.  They hand work over through mbarriers only.
+// MMAs (on a pair: the even CTA's; lanes 0 and 1 of the odd CTA's forward barrier phases), warps
+// 17 to 19 append the hits.  They hand work over through mbarriers only.
 constexpr int kTcProducers = 256;
 constexpr int kTcEpiWarp = 8;
 constexpr int kTcEpilogue = 256;
 constexpr int kTcMmaWarp = 16;
-constexpr int kTcDrainWarp = 17;
-constexpr int kTcThreads = 18 * 32;
+constexpr int kTcDrainWarp = 17;  // and the two after it: unit t's hits are appended by 17 + t % 3
+constexpr uint32_t kTcDrains = 3;
+constexpr int kTcThreads = (17 + kTcDrains) * 32;
 constexpr uint32_t kTcTmemCols = 512;  // all of tensor memory, in FP32 accumulators
 // Queries per launch and accumulators.  One CTA: 128 queries (N = 128, M = 128), four
 // accumulators of 128 columns.  A CTA pair (cta_group::2): 256 queries (N = 256, each CTA
@@ -62,7 +63,9 @@ struct TcShape {
 // drain (the MMA thread's own MMAs complete), queued[kTcQueues] (epilogue -> drain warp),
 // drained[kTcQueues] (drain warp -> epilogue); then the tensor-memory address, the give-up flag
 // and the counts of the hit queues
-constexpr uint32_t kTcQueues = 4;       // units whose hits may wait (a long row hits for most queries)
+constexpr uint32_t kTcQueues = 6;       // units whose hits may wait (a long row hits for most queries)
+constexpr uint32_t kTcLists = 2 * kTcQ / 32;
+static_assert(kTcLists >= kTcQueues, "counts of queues and lists share their place");
 __host__ __device__ constexpr uint32_t tc_nbars(uint32_t nb, uint32_t acc) {
   return 2 * nb + 2 * acc + 1 + 2 * kTcQueues;
 }
@@ -73,7 +76,7 @@ __host__ inline size_t tc_smem_bytes(uint32_t cols, uint32_t split, uint32_t nb,
   const uint32_t S = split <= 1 ? 1 : split;
   const uint32_t q = pair ? 2 * kTcQ : kTcQ;
   return tc_qtab_bytes(cols) + nb * (size_t)kTcChunkBytes + (size_t)S * q * 4 +
-         ((tc_nbars(nb, kTcTmemCols / q) * 8 + 8 + kTcQueues * 4 + 15) & ~15u);
+         ((tc_nbars(nb, kTcTmemCols / q) * 8 + 8 + kTcLists * 4 + 15) & ~15u);
 }
 // chunk buffers for a configuration: three where they fit next to the query operand and the
 // thresholds (the producers then run two chunks ahead of the MMAs), else two
@@ -99,13 +102,21 @@ struct TcArgs {
   const uint8_t* qt;     // e4m3 query operand of this launch, tc_qtab_bytes(cols)
   uint32_t q0, nq;       // this launch scores queries q0 .. q0 + nq - 1 (nq <= 128)
   const float* rowscale;
+  // filter of approximate scores (aes_tf.cuh), or null: per row {sum |v'| << 13 | ceil(sum |d| / 2),
+  // sum v}, and the launch's query statistics
+  const uint2* rowstat;
+  const uint32_t* qstat;
   uint32_t split, slice; // split >= 1
   const uint32_t* thr;   // [nq_total][split]
   uint32_t* cnt;         // [nq_total][split]
   uint2* surv;           // [nq_total][split][cap]
   uint32_t cap;
   uint32_t* status;      // [nq_total]
-  uint2* queue;          // [gridDim.x][kTcQueues][queue_cap] hit queues of successive units
+  // [gridDim.x][kTcQueues][queue_cap] hit queues of successive units; a filter's lists of the rows it
+  // lets through, [gridDim.x][kTcLists][queue_cap] {row, mask of queries} per block of 32 queries,
+  // and their counts
+  uint2* queue;
+  uint32_t* list_n;      // [gridDim.x][kTcLists]
   uint32_t queue_cap;
   uint32_t mma_idle;     // failure-path test: the MMA role issues nothing, so every hand-over
                          // wait of the other roles runs out and the CTA gives up
@@ -281,8 +292,9 @@ __device__ __forceinline__ void tc_append(const TcArgs& a, uint32_t S, size_t qp
     if (((hit >> j) & 1u) && ix[j] < a.cap)
       a.surv[(qp + (size_t)j * S) * a.cap + ix[j]] = make_uint2(key[j], row);
 }
-// The hit queue of a unit: entries (query | row in tile << 8, score as FP32 bits); a group of hits
-// that passes its end is appended by the epilogue thread itself, the slots it had taken marked
+// The hit queue of a unit: entries (query | row in tile << 8, score as FP32 bits); hits past its end
+// are appended by the epilogue thread itself, the slots it had taken marked.  A filter: the CTA's
+// lists
 constexpr uint32_t kTcNoHit = 0xFFFFFFFFu;
 struct TcQueue {
   uint2* e;
@@ -311,10 +323,26 @@ __device__ __forceinline__ void tc_margin8(float (&x)[8], const uint32_t* v, flo
   tc_fma2(x[4], x[5], __uint_as_float(v[4]), __uint_as_float(v[5]), rs, t1.x, t1.y);
   tc_fma2(x[6], x[7], __uint_as_float(v[6]), __uint_as_float(v[7]), rs, t1.z, t1.w);
 }
+// Query statistics of a filter launch: the centre c of the values (aes_tf.cuh: 512 + max, 512 - min)
+__device__ __forceinline__ int tc_centre(const uint32_t* st) {
+  const int hi = (int)st[0] - 512, lo = 512 - (int)st[1];
+  return max(hi, -lo) <= 16 ? 0 : (hi + lo) / 2;
+}
+// Filter of approximate scores: minus what rs times the score may exceed rs times the approximate
+// one by, rounded away from zero: c sum v + E sum |v'| + Q sum |d|, and for the FP32 arithmetic
+// (the accumulator's, this one's and the compare's) 2^-12 of what the products can add up to.
+__device__ __forceinline__ float tc_limit(uint2 st, int centre, float E, float Q, float rs) {
+  const float r1 = (float)(st.x >> 13), r2 = 2.0f * (float)(st.x & 0x1FFFu);
+  const float c = __fmul_ru((float)centre, __int2float_ru((int)st.y));
+  float b = __fadd_ru(__fmul_ru(E, r1), __fmul_ru(Q, r2));
+  b = __fadd_ru(b, 0.000244140625f * (Q * r1 + fabsf(c)));
+  return -__fmul_ru(__fadd_ru(b, c), rs);
+}
 // Epilogue warps: reads accumulator `dbuf` of row tile T (thread = row, half the queries) and
 // queues every (row, query) score at or above the query's bound.  nthf holds the negated bounds on
 // rs * score (rs is the row's scale, or 1 without row scales, where the score is an exact integer),
-// so a score passes where fma(score, rs, -bound) >= 0.  A block of 32 queries costs a fused
+// so a score passes where fma(score, rs, -bound) >= lim (0, or what an approximate score of the row
+// may fall short by).  A block of 32 queries costs a fused
 // multiply-add per two scores and the maximum of each group of eight (three-operand maxima); only
 // groups that reach 0 are looked at again, and take their queue slots with one atomic per block.  The accumulator goes back to the MMA role (an
 // arrive on `empty`) as soon as the thread's last load from it has completed.
@@ -325,7 +353,8 @@ __device__ __forceinline__ void tc_margin8(float (&x)[8], const uint32_t* v, flo
 template <bool PAIR>
 __device__ __forceinline__ void tc_epilogue(const TcArgs& a, uint32_t T, uint32_t tmem,
                                             uint32_t dbuf, const float* nthf_all, uint32_t S,
-                                            float rs, uint32_t empty, const TcQueue& hq) {
+                                            float rs, float lim, uint32_t empty,
+                                            const TcQueue& hq) {
   constexpr uint32_t Q = TcShape<PAIR>::Q, HALF = Q / 2;
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t g = warp & 3u, h = (warp - kTcEpiWarp) >> 2;
@@ -351,21 +380,26 @@ __device__ __forceinline__ void tc_epilogue(const TcArgs& a, uint32_t T, uint32_
       const float m0 = fmaxf(fmaxf(x[0], x[1]), x[2]), m1 = fmaxf(fmaxf(x[3], x[4]), x[5]);
       m[j8] = fmaxf(fmaxf(m0, m1), fmaxf(x[6], x[7]));
     }
-    if (fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])) >= 0.0f && valid) {
+    if (fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])) >= lim && valid) {
       uint32_t hit = 0;
 #pragma unroll
       for (int j8 = 0; j8 < 4; j8++) {
-        if (m[j8] >= 0.0f) {
+        if (m[j8] >= lim) {
           float x[8];
           tc_margin8(x, v + 8 * j8, rs, nthf + col0 + 8 * j8);
 #pragma unroll
-          for (int j = 0; j < 8; j++) hit |= (x[j] >= 0.0f ? 1u : 0u) << (8 * j8 + j);
+          for (int j = 0; j < 8; j++) hit |= (x[j] >= lim ? 1u : 0u) << (8 * j8 + j);
         }
+      }
+      if (a.rowstat) {
+        const uint32_t l = col0 / 32u, k = atomicAdd(hq.n + l, 1u);
+        if (k < hq.cap) hq.e[(size_t)l * hq.cap + k] = make_uint2(row, hit);
+        continue;
       }
       const uint32_t nh = __popc(hit);
       uint32_t i = atomicAdd(hq.n, nh);
+      const uint32_t meta = col0 | (row % kTcRows) << 8;
       if (i + nh <= hq.cap) {
-        const uint32_t meta = col0 | (row % kTcRows) << 8;
 #pragma unroll
         for (int j = 0; j < 32; j++)
           if ((hit >> j) & 1u) hq.e[i++] = make_uint2(meta + j, v[j]);
@@ -423,8 +457,42 @@ __device__ __forceinline__ bool tc_producers_any(bool fail) {
 }
 
 
+// A drain warp: appends n queued scores of row tile T, four per lane in flight
+__device__ __forceinline__ void tc_drain_scores(const TcArgs& a, uint32_t S, const volatile uint2* hq,
+                                                uint32_t n, uint32_t T) {
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t i0 = 0; i0 < n; i0 += 128u) {
+    uint32_t meta[4], score[4], key[4], th[4], ix[4];
+    size_t qp[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const uint32_t i = i0 + u * 32u + lane;
+      meta[u] = i < n ? hq[i].x : kTcNoHit;
+      score[u] = i < n ? hq[i].y : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      th[u] = 0xFFFFFFFFu;
+      key[u] = 0u;
+      if (meta[u] != kTcNoHit) {
+        const uint32_t row = T * kTcRows + (meta[u] >> 8);
+        qp[u] = (size_t)(a.q0 + (meta[u] & 255u)) * S + part_of(row, S, a.slice);
+        th[u] = __ldg(a.thr + qp[u]);
+        const float f = __uint_as_float(score[u]);
+        key[u] = a.rowscale ? key_f32(__fmul_rn(f, __ldg(a.rowscale + row))) : key_i32(__float2int_rn(f));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (meta[u] != kTcNoHit && key[u] >= th[u]) ix[u] = atomicAdd(a.cnt + qp[u], 1u);
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (meta[u] != kTcNoHit && key[u] >= th[u] && ix[u] < a.cap)
+        a.surv[qp[u] * a.cap + ix[u]] = make_uint2(key[u], T * kTcRows + (meta[u] >> 8));
+  }
+}
 // One CTA per SM (PAIR: one CTA pair, a cluster of two, per two SMs), persistent over units of
-// work U = unit, unit + units, ...: a 128-row tile (one CTA), or two consecutive tiles, 2U for
+// work U: a 128-row tile (one CTA), or two consecutive tiles, 2U for
 // the even CTA and 2U + 1 for the odd one (PAIR).  Chunk i of the CTA is chunk i % nch of its
 // unit i / nch; chunk buffer i % NB; accumulator (unit t) t % ACC.
 // PAIR: the even CTA's MMA thread issues cta_group::2 MMAs with M = 256 (the two CTAs' row tiles
@@ -449,14 +517,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(thf + S * Q);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + kBars);
   volatile uint32_t* gave_up = tslot + 1;
-  uint32_t* hq_n = tslot + 2;  // [kTcQueues]
-  uint2* hq_e = a.queue + (size_t)blockIdx.x * kTcQueues * a.queue_cap;
+  uint32_t* hq_n = tslot + 2;  // [kTcLists]
+  uint2* hq_e = a.queue + (size_t)blockIdx.x * (a.rowstat ? kTcLists : kTcQueues) * a.queue_cap;
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
   uint32_t rank = 0;  // the CTA's rank in its pair
   if constexpr (PAIR) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  const uint32_t unit = PAIR ? (blockIdx.x >> 1) : blockIdx.x;
-  const uint32_t units = PAIR ? (gridDim.x >> 1) : gridDim.x;
   const uint32_t n_units = PAIR ? (a.n_rtiles + 1u) / 2u : a.n_rtiles;
+  // units unit, unit + 1, ... of the CTA (pair): consecutive, so that its hits fall into few partitions
+  uint32_t unit, ntl;
+  {
+    const uint32_t me = PAIR ? (blockIdx.x >> 1) : blockIdx.x, all = PAIR ? (gridDim.x >> 1) : gridDim.x;
+    unit = (uint32_t)((uint64_t)n_units * me / all);
+    ntl = (uint32_t)((uint64_t)n_units * (me + 1u) / all) - unit;
+  }
   auto tile_of = [&](uint32_t u) { return PAIR ? 2u * u + rank : u; };  // this CTA's row tile
   {
     const uint4* src = reinterpret_cast<const uint4*>(a.qt + (PAIR ? rank * qbytes : 0u));
@@ -477,9 +550,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
                                : (th > 0xFF800000u ? __int_as_float(0x7f800000)
                                                    : __uint_as_float((th & 0x7FFFFFFFu) - 1u));
       } else {           // |score| < 2^24, exact in FP32
-        const int32_t b = (int32_t)(th ^ 0x80000000u);
-        fb = b > (1 << 24) ? __int_as_float(0x7f800000)
-                           : (b < -(1 << 24) ? -__int_as_float(0x7f800000) : __int2float_rn(b));
+        const int32_t b = (int32_t)(th ^ 0x80000000u);  // (8-bit filter: below 2^26, rounded down)
+        fb = b > (1 << 26) ? __int_as_float(0x7f800000)
+                           : (b < -(1 << 26) ? -__int_as_float(0x7f800000) : __int2float_rd(b));
       }
       thf[i] = -fb;
     }
@@ -497,7 +570,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(tc_smem_u32(bars + b)), "r"(cnt));
     }
     *gave_up = 0u;
-    for (uint32_t b = 0; b < kTcQueues; b++) hq_n[b] = 0u;
+    for (uint32_t b = 0; b < kTcLists; b++) hq_n[b] = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kTcMmaWarp) tc_alloc<PAIR>(tc_smem_u32(tslot));
@@ -510,7 +583,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
   const uint32_t b_staged = tc_smem_u32(bars), b_done = tc_smem_u32(bars + kDone);
   const uint32_t b_full = tc_smem_u32(bars + kFull), b_empty = tc_smem_u32(bars + kEmpty);
   const uint32_t b_queued = tc_smem_u32(bars + kQueued), b_drained = tc_smem_u32(bars + kDrained);
-  const uint32_t ntl = n_units > unit ? (n_units - unit + units - 1) / units : 0u;
   const uint32_t total = ntl * a.nch;  // chunks of this CTA (PAIR: the same in both CTAs)
   bool ok = true;
 
@@ -533,7 +605,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
       la_i++;
       if (++la_c == a.nch) {
         la_c = 0;
-        la_t += (PAIR ? 2u : 1u) * units;
+        la_t += PAIR ? 2u : 1u;
       }
     };
     TcEnt E[R];
@@ -576,61 +648,37 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
     }
   } else if (warp < kTcEpiWarp + kTcEpilogue / 32) {
     // ---- epilogue -----------------------------------------------------------------------------
+    const int centre = a.rowstat ? tc_centre(a.qstat) : 0;
+    const float qE = a.rowstat ? (float)a.qstat[2] : 0.0f, qQ = a.rowstat ? (float)a.qstat[3] : 0.0f;
     for (uint32_t tl = 0; tl < ntl; tl++) {
       const uint32_t d = tl % ACC;
-      const uint32_t T = tile_of(unit + tl * units), row = tc_epi_row(T);
+      const uint32_t T = tile_of(unit + tl), row = tc_epi_row(T);
       // this unit's hit queue is drained of the unit kTcQueues back
       const uint32_t hb = tl % kTcQueues;
-      if (tl >= kTcQueues) ok &= tc_wait(b_drained + 8u * hb, (tl / kTcQueues - 1u) & 1u, gave_up);
+      if (tl >= kTcQueues && !a.rowstat) ok &= tc_wait(b_drained + 8u * hb, (tl / kTcQueues - 1u) & 1u, gave_up);
       // without row scales rs = 1: f * 1 is f exactly, so every score takes one path
       const float rs = a.rowscale ? (row < a.n_rows ? __ldg(a.rowscale + row) : 0.0f) : 1.0f;
+      const uint2 st = a.rowstat && row < a.n_rows ? __ldg(a.rowstat + row) : make_uint2(0u, 0u);
+      const float lim = a.rowstat ? tc_limit(st, centre, qE, qQ, rs) : 0.0f;
       if (ok) ok &= tc_wait<PAIR>(b_full + 8u * d, (tl / ACC) & 1u, gave_up);
       ok = __all_sync(0xFFFFFFFFu, ok);  // tcgen05.ld needs the whole warp
       if (!ok) break;
       tc_fence_after();
-      tc_epilogue<PAIR>(a, T, tmem, d, thf, S, rs, b_empty + 8u * d,
-                        TcQueue{hq_e + (size_t)hb * a.queue_cap, hq_n + hb, a.queue_cap});
-      tc_arrive(b_queued + 8u * hb);
+      tc_epilogue<PAIR>(a, T, tmem, d, thf, S, rs, lim, b_empty + 8u * d,
+                        a.rowstat ? TcQueue{hq_e, hq_n, a.queue_cap}
+                                  : TcQueue{hq_e + (size_t)hb * a.queue_cap, hq_n + hb, a.queue_cap});
+      if (!a.rowstat) tc_arrive(b_queued + 8u * hb);
     }
-  } else if (warp == kTcDrainWarp) {
-    // ---- drain: appends each unit's queued hits, four per lane at a time ------------------------
+  } else if (warp >= kTcDrainWarp) {
+    // ---- drain: appends the queued hits of every third unit, four per lane at a time -----------
     const uint32_t lane = tid & 31u;
-    for (uint32_t tl = 0; tl < ntl; tl++) {
-      const uint32_t b = tl % kTcQueues, T = tile_of(unit + tl * units);
+    for (uint32_t tl = warp - kTcDrainWarp; tl < ntl && !a.rowstat; tl += kTcDrains) {
+      const uint32_t b = tl % kTcQueues, T = tile_of(unit + tl);
       ok = tc_wait(b_queued + 8u * b, (tl / kTcQueues) & 1u, gave_up);
       if (!__all_sync(0xFFFFFFFFu, ok)) break;
       const uint32_t n = min(*reinterpret_cast<volatile uint32_t*>(hq_n + b), a.queue_cap);
       const volatile uint2* hq = hq_e + (size_t)b * a.queue_cap;
-      for (uint32_t i0 = 0; i0 < n; i0 += 128u) {
-        uint32_t meta[4], score[4], key[4], th[4], ix[4];
-        size_t qp[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const uint32_t i = i0 + u * 32u + lane;
-          meta[u] = i < n ? hq[i].x : kTcNoHit;
-          score[u] = i < n ? hq[i].y : 0u;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          th[u] = 0xFFFFFFFFu;
-          key[u] = 0u;
-          if (meta[u] != kTcNoHit) {
-            const uint32_t row = T * kTcRows + (meta[u] >> 8);
-            qp[u] = (size_t)(a.q0 + (meta[u] & 255u)) * S + part_of(row, S, a.slice);
-            th[u] = __ldg(a.thr + qp[u]);
-            const float f = __uint_as_float(score[u]);
-            key[u] = a.rowscale ? key_f32(__fmul_rn(f, __ldg(a.rowscale + row)))
-                                : key_i32(__float2int_rn(f));
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-          if (meta[u] != kTcNoHit && key[u] >= th[u]) ix[u] = atomicAdd(a.cnt + qp[u], 1u);
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-          if (meta[u] != kTcNoHit && key[u] >= th[u] && ix[u] < a.cap)
-            a.surv[qp[u] * a.cap + ix[u]] = make_uint2(key[u], T * kTcRows + (meta[u] >> 8));
-      }
+      tc_drain_scores(a, S, hq, n, T);
       __syncwarp();
       if (lane == 0) {
         hq_n[b] = 0u;
@@ -713,6 +761,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
     tc_fence_after();
     tc_dealloc<PAIR>(tmem);
   }
+  if (a.rowstat && tid < kTcLists) a.list_n[blockIdx.x * kTcLists + tid] = hq_n[tid];
   if (*gave_up && tid == 0) {
     for (uint32_t q = 0; q < a.nq; q++) atomicOr(a.status + a.q0 + q, ST_DEVICE);
   }

@@ -188,3 +188,98 @@ def test_sample_pass_forms(rows, stride, nq, bits, quant):
                  max_batch=nq, batch_tile=128, sample_stride=stride)
     Q = np.random.default_rng(nq).random((nq, 600)).astype(np.float32)
     _check(m, eng, Q, 1, 200, 30, every=max(1, nq // 6))
+
+
+def _filter_case(rows, cols, lo, hi, bits, quant, seed, signed):
+    """A CSR with an empty row, a row of zeros and a row quantised to nothing, and its queries."""
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, lo, hi, seed=seed)
+    d = np.diff(ptr).astype(np.int64)
+    keep = np.ones(len(val), bool)
+    e = rows // 3
+    keep[int(ptr[e]):int(ptr[e + 1])] = False
+    d[e] = 0
+    col, val = col[keep], val[keep]
+    ptr = np.concatenate([[0], np.cumsum(d)]).astype(np.uint64)
+    val[int(ptr[5]):int(ptr[6])] = 0
+    val[int(ptr[7]):int(ptr[8])] *= np.float32(1e-5)
+    if signed:
+        val = val * np.where(np.random.default_rng(seed).random(len(val)) < 0.5, -1, 1).astype(np.float32)
+    return ptr, col, val
+
+
+@pytest.mark.parametrize("bits,quant", [(4, 0), (4, 1), (4, 2), (6, 0), (6, 1), (6, 2), (8, 0), (8, 1), (8, 2)])
+@pytest.mark.parametrize("rows,cols,lo,hi,split,nq,kind", [
+    (40000, 1024, 10, 30, 1, 65, "dense"),    # one CTA's launch, the last block of one query
+    (40001, 500, 5, 25, 32, 150, "dense"),    # a CTA pair; partitions
+    (9000, 333, 100, 300, 3, 300, "mixed"),   # a pair and a single launch; rows of many pieces
+    (130, 40, 2, 8, 1, 129, "mixed"),         # two row tiles
+])
+def test_filter_pass(bits, quant, rows, cols, lo, hi, split, nq, kind):
+    """Batches above 64 queries of a handle without a memory limit: approximate FP8 scores filter
+    the rows and an exact integer check follows; with a memory limit the dp4a pass runs.  Both give
+    the oracle's candidates and Top-K."""
+    ck, k = max(96, 3 * split), 25
+    ptr, col, val = _filter_case(rows, cols, lo, hi, bits, quant, rows + bits, quant == 0)
+    rng = np.random.default_rng(nq)
+    Q = rng.random((nq, cols)).astype(np.float32)
+    if quant == 0:
+        Q = Q * 2 - 1
+    if kind == "mixed":  # a zero query, one-sided ones and sparse ones beside the rest
+        Q[1] = 0
+        Q[2::3] = np.abs(Q[2::3])
+        Q[3::5] *= rng.random((len(Q[3::5]), cols)) < 0.1
+    m = orc.Matrix(rows, cols, ptr, col, val, bits, quant)
+    kw = dict(ptr=ptr, col=col, val=val, bits=bits, quant=quant, split=split, ck=ck, k_max=k,
+              max_batch=nq, batch_tile=128)
+    eng = E.SpMV(rows, cols, **kw)
+    lim = E.SpMV(rows, cols, mem_limit=1 << 40, **kw)
+    assert eng.info()["device_bytes"] > lim.info()["device_bytes"]
+    for e in (eng, lim):
+        _check(m, e, Q, split, ck, k, every=max(1, nq // 7))
+        for i in (1, 2, 3):
+            assert set(e.read_candidates(i)[0].tolist()) == set(m.two_stage(Q[i], split, ck, k)[2].tolist())
+        # (only the zero query, whose rows all tie, may overflow its survivors)
+        assert e.stats()["repaired"] <= (1 if kind == "mixed" else 0)
+    # a view runs the same pass; a graph replays it
+    v = eng.view(flags=E.FLAG_GRAPHS)
+    for _ in range(2):
+        _check(m, v, Q, split, ck, k, every=max(1, nq // 2))
+
+
+def test_filter_pass_bounds_too_wide():
+    """Scores closer together than the filter's bounds: nearly every row passes, the lists overflow,
+    and the batch is run again (and later batches are run) with the dp4a pass; no query needs the
+    slow path."""
+    rows, cols, deg, nq, ck, k = 150_000, 512, 120, 70, 8, 8
+    rng = np.random.default_rng(5)
+    ptr = (np.arange(rows + 1) * deg).astype(np.uint64)
+    start = rng.integers(0, cols - deg, rows)
+    col = (start[:, None] + np.arange(deg)[None, :]).astype(np.uint32).reshape(-1)
+    val = (115 + rng.integers(-1, 2, rows * deg)).astype(np.float32)
+    val[0] = 127
+    Q = (115 + rng.integers(-1, 2, (nq, cols))).astype(np.float32)
+    Q[:, 0] = 127
+    m = orc.Matrix(rows, cols, ptr, col, val, 8, 0)
+    eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=8, split=1, ck=ck, k_max=k, max_batch=nq,
+                 batch_tile=128, sample_stride=4, flags=E.FLAG_GRAPHS)
+    for _ in range(2):
+        _check(m, eng, Q, 1, ck, k, every=30)
+    assert eng.stats()["repaired"] == 0
+
+
+def test_filter_pass_not_for_repeated_columns():
+    """A row holding a column twice would lose one value in the dense tile: the dp4a pass runs."""
+    rows, cols, nq = 3000, 64, 70
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 3, 6, seed=2)
+    r = np.repeat(np.arange(rows, dtype=np.uint32), np.diff(ptr).astype(np.int64))
+    r = np.concatenate([r, np.array([9], np.uint32)])
+    c = np.concatenate([col, col[int(ptr[9]):int(ptr[9]) + 1]])
+    v = np.concatenate([val, np.array([0.9], np.float32)])
+    kw = dict(row=r, col=c, val=v, bits=8, split=1, ck=64, k_max=10, max_batch=nq, batch_tile=128)
+    eng, lim = E.SpMV(rows, cols, **kw), E.SpMV(rows, cols, mem_limit=1 << 40, **kw)
+    Q = np.random.default_rng(1).random((nq, cols)).astype(np.float32)
+    for e in (eng, lim):
+        e.Q_reset(Q)
+        e(k=10)
+    assert np.array_equal(eng.read_topk()[0], lim.read_topk()[0])
+    assert np.array_equal(eng.read_topk()[1], lim.read_topk()[1])
