@@ -361,6 +361,7 @@ __device__ void batch_range(const BatchArgs& a, uint32_t tb, uint32_t te,
 
 template <int B, bool SGN, int MODE>
 __global__ void __launch_bounds__(kWarpsBatchMax * 32, 1) k_cand_batch(BatchArgs a) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char smem[];
   uint8_t* qtb = smem;                                           // [cols][33] words
   const size_t qtab_bytes = batch_qtab_words(a.cols) * 4;
@@ -448,6 +449,8 @@ constexpr uint32_t kTransposeRows = 32;
 __global__ void __launch_bounds__(256) k_keys_transpose(const uint32_t* __restrict__ in,
                                                         uint32_t n_rows, uint32_t nq,
                                                         uint32_t* __restrict__ out) {
+  grid_wait();
+  grid_next();
   __shared__ uint32_t t[kTransposeRows][kBatchQ + 1];
   const uint32_t blk = blockIdx.y;
   const uint32_t nb = min((uint32_t)kBatchQ, nq - blk * kBatchQ);
@@ -470,6 +473,8 @@ __global__ void __launch_bounds__(256) k_keys_transpose(const uint32_t* __restri
 // block of the batch in one launch.
 __global__ void k_qtable(const int8_t* __restrict__ q8, uint32_t ld8, uint32_t cols, uint32_t nq,
                          uint32_t* __restrict__ qtab) {
+  grid_wait();
+  grid_next();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t nblk = (nq + kBatchQ - 1) / kBatchQ;
   const uint64_t per = batch_qtab_words(cols);

@@ -327,6 +327,24 @@ struct Engine {
     return AES_OK;
   }
 
+  // Launches a kernel as a programmatic dependent of the kernel before it in the stream (grid_wait).
+  // Not inside a captured graph, whose kernels follow one another closely as it is: programmatic
+  // edges made its replays slower (40 queries of 2M x 1024: 338 -> 348 us).
+  template <class... P, class... A>
+  cudaError_t chain(void (*k)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A... a) const {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = capturing ? 0 : 1;
+    return cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
+  }
+  bool capturing = false;
   int build(const HostCSR& m, const aes_params& p);
   int build_view(const Engine& base, const aes_params& p);
   int plan_config(const aes_params& p, Config* c) const;
@@ -345,9 +363,9 @@ struct Engine {
   bool int_final(const float* d_q) const { return !has_f32 || d_q == nullptr; }
   int repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cudaStream_t s,
              uint32_t* repaired);
-  int run_plain(int mode, uint32_t q, cudaStream_t s, uint32_t nq_y = 1);
+  int run_plain(int mode, uint32_t q, cudaStream_t s, uint32_t nq_y = 1, bool first = false);
   int run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0 = 0, uint32_t nblk = 0);
-  int run_multi(uint32_t nq, cudaStream_t s, bool sample = false);
+  int run_multi(uint32_t nq, cudaStream_t s, bool sample = false, bool first = false);
   int run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint32_t* cnt, cudaStream_t s);
   int run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s);
   int run_check(uint32_t q0, uint32_t n, cudaStream_t s, uint32_t ctas);
@@ -442,19 +460,21 @@ int Engine::run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair) {
     cfg.blockDim = dim3(kTcThreads);
     cfg.dynamicSmemBytes = tc_smem2;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = capturing ? 1 : 2;
     AES_CK(tc_nb2 == 3 ? cudaLaunchKernelEx(&cfg, k_cand_tc<3, true>, a)
                        : cudaLaunchKernelEx(&cfg, k_cand_tc<2, true>, a));
   } else if (tc_nb == 3) {
-    k_cand_tc<3, false><<<tc_grid, kTcThreads, tc_smem, s>>>(a);
+    AES_CK(chain(k_cand_tc<3, false>, tc_grid, kTcThreads, tc_smem, s, a));
   } else {
-    k_cand_tc<2, false><<<tc_grid, kTcThreads, tc_smem, s>>>(a);
+    AES_CK(chain(k_cand_tc<2, false>, tc_grid, kTcThreads, tc_smem, s, a));
   }
   AES_CK(cudaGetLastError());
   if (prof && (rc = prof_close(s))) return rc;
@@ -488,8 +508,8 @@ int Engine::run_check(uint32_t q0, uint32_t n, cudaStream_t s, uint32_t ctas) {
   c.cnt = d_cnt;
   c.surv = d_surv;
   const uint32_t blocks = (n + 31) / 32;  // (six CTAs fit on an SM)
-  k_recheck<<<dim3(blocks, std::max(1u, 6u * (uint32_t)sm_count / blocks)), kThreadsCheck, check_smem_bytes(ld8), s>>>(c);
-  AES_CK(cudaGetLastError());
+  AES_CK(chain(k_recheck, dim3(blocks, std::max(1u, 6u * (uint32_t)sm_count / blocks)), kThreadsCheck,
+               check_smem_bytes(ld8), s, c));
   n_launch++;
   return AES_OK;
 }
@@ -1014,7 +1034,7 @@ int Engine::retune(const aes_params& p) {
 }
 
 // mode's pass for query q (MODE_SAMPLE: for queries q .. q + nq_y - 1 in one launch)
-int Engine::run_plain(int mode, uint32_t q, cudaStream_t s, uint32_t nq_y) {
+int Engine::run_plain(int mode, uint32_t q, cudaStream_t s, uint32_t nq_y, bool first) {
   PlainArgs a{};
   a.tiles = d_tiles;
   a.tile_rowbase = d_tile_rowbase;
@@ -1049,8 +1069,12 @@ int Engine::run_plain(int mode, uint32_t q, cudaStream_t s, uint32_t nq_y) {
   const bool prof = (prm.flags & AES_FLAG_PROFILE) && mode != MODE_SAMPLE;
   int rc = prof ? prof_open(s) : AES_OK;
   if (rc) return rc;
-  pick_plain((int)bits, sgn, mode)<<<dim3(grid, nq_y), plain_threads((int)bits), plain_smem, s>>>(a);
-  AES_CK(cudaGetLastError());
+  if (mode == MODE_ALL || first) {  // (what comes before it in the stream may be a copy)
+    pick_plain((int)bits, sgn, mode)<<<dim3(grid, nq_y), plain_threads((int)bits), plain_smem, s>>>(a);
+    AES_CK(cudaGetLastError());
+  } else {
+    AES_CK(chain(pick_plain((int)bits, sgn, mode), dim3(grid, nq_y), plain_threads((int)bits), plain_smem, s, a));
+  }
   if (prof && (rc = prof_close(s))) return rc;
   n_launch++;
   if (mode != MODE_SAMPLE) n_cand++;
@@ -1089,8 +1113,7 @@ int Engine::run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0, uint
   const bool prof = (prm.flags & AES_FLAG_PROFILE) && mode != MODE_SAMPLE;
   int rc = prof ? prof_open(s) : AES_OK;
   if (rc) return rc;
-  pick_batch((int)bits, sgn, mode)<<<dim3(grid, nblk), batch_warps_n * 32, batch_smem, s>>>(a);
-  AES_CK(cudaGetLastError());
+  AES_CK(chain(pick_batch((int)bits, sgn, mode), dim3(grid, nblk), batch_warps_n * 32, batch_smem, s, a));
   if (prof && (rc = prof_close(s))) return rc;
   n_launch++;
   if (mode != MODE_SAMPLE) n_cand++;
@@ -1098,7 +1121,7 @@ int Engine::run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0, uint
 }
 
 // The filter (or sample) pass of an nq-query batch, four queries per matrix read
-int Engine::run_multi(uint32_t nq, cudaStream_t s, bool sample) {
+int Engine::run_multi(uint32_t nq, cudaStream_t s, bool sample, bool first) {
   MultiArgs a{};
   a.tiles = d_tiles;
   a.tile_rowbase = d_tile_rowbase;
@@ -1141,9 +1164,13 @@ int Engine::run_multi(uint32_t nq, cudaStream_t s, bool sample) {
   const bool prof = (prm.flags & AES_FLAG_PROFILE) && !sample;
   int rc = prof ? prof_open(s) : AES_OK;
   if (rc) return rc;
-  pick_multi((int)bits, sgn, d_rowscale != nullptr, sample)
-      <<<dim3(grid, groups), kMultiThreads, multi_smem_bytes(cols, split), s>>>(a);
-  AES_CK(cudaGetLastError());
+  const MultiKernel k = pick_multi((int)bits, sgn, d_rowscale != nullptr, sample);
+  if (first) {
+    k<<<dim3(grid, groups), kMultiThreads, multi_smem_bytes(cols, split), s>>>(a);
+    AES_CK(cudaGetLastError());
+  } else {
+    AES_CK(chain(k, dim3(grid, groups), kMultiThreads, multi_smem_bytes(cols, split), s, a));
+  }
   if (prof && (rc = prof_close(s))) return rc;
   n_launch++;
   if (!sample) n_cand++;
@@ -1158,13 +1185,12 @@ int Engine::run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint
     const uint32_t g = (uint32_t)((pairs + kThrWarps - 1) / kThrWarps);
     auto k = part_samples <= kThrWarpKeys / 2 ? k_threshold_warp<kThrWarpKeys / 64>
                                               : k_threshold_warp<kThrWarpKeys / 32>;
-    k<<<g, kThrWarps * 32, 0, s>>>(keys, n_sample_rows, d_part_sample_begin, split, (uint32_t)pairs,
-                                   d_part_r, thr, cnt);
+    AES_CK(chain(k, g, kThrWarps * 32, 0, s, keys, n_sample_rows, d_part_sample_begin, split,
+                 (uint32_t)pairs, d_part_r, thr, cnt));
   } else {
-    k_threshold<<<dim3(split, nq), kThreadsThr, 0, s>>>(keys, n_sample_rows, 0, d_part_sample_begin,
-                                                        split, d_part_r, thr, cnt);
+    AES_CK(chain(k_threshold, dim3(split, nq), kThreadsThr, 0, s, keys, n_sample_rows, 0,
+                 d_part_sample_begin, split, d_part_r, thr, cnt));
   }
-  AES_CK(cudaGetLastError());
   return AES_OK;
 }
 
@@ -1176,29 +1202,32 @@ int Engine::run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s) {
   sa.pairs = sa.split * nq;
   if (sa.ntop <= kSelWarpTop && sa.pairs > 4u * (uint32_t)sm_count) {
     constexpr uint32_t W = kSelWarpThreads / 32;
-    k_select_warp<<<(sa.pairs + W - 1) / W, kSelWarpThreads, 0, s>>>(sa);
+    AES_CK(chain(k_select_warp, (sa.pairs + W - 1) / W, kSelWarpThreads, 0, s, sa));
   } else {
-    k_select<false><<<dim3(sa.split, nq), kThreadsSel, 0, s>>>(sa);
+    AES_CK(chain(k_select<false>, dim3(sa.split, nq), kThreadsSel, 0, s, sa));
   }
-  AES_CK(cudaGetLastError());
   return AES_OK;
 }
 
 int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score,
                     cudaStream_t s, bool pre) {
-  AES_CK(cudaMemsetAsync(d_status, 0, nq * 4ull, s));
-  if (!pre) {
-    k_quantize<<<nq, 256, 0, s>>>(d_q, cols, ld32, (int)bits, (int)quant,
-                                  (int)prm.query_quant, d_q8, ld8, d_status);
-    AES_CK(cudaGetLastError());
-    n_launch++;
-  }
-  n_launch += 3;  // threshold, select, final
   const bool batched = batch_mode != 1 && (batch_mode != 0 || nq > multi_max);
   last_batched = batched;
   const bool tc = batched && (use_tc || use_tf), tf = batched && use_tf;
   last_tf = tf;
   last_pre = pre;
+  // memsets first: the kernels that follow start one out of the other (chain)
+  if (tf) AES_CK(cudaMemsetAsync(d_exact_aux + 4, 0, kTfStats * 4, s));
+  if (pre) {
+    AES_CK(cudaMemsetAsync(d_status, 0, nq * 4ull, s));
+  } else {  // (sets the status words)
+    k_quantize<<<nq, quantize_threads(nq), 0, s>>>(d_q, cols, ld32, (int)bits, (int)quant,
+                                                   (int)prm.query_quant, d_q8, ld8, d_status);
+    AES_CK(cudaGetLastError());
+    n_launch++;
+  }
+  bool first = pre;  // the next kernel has no kernel of this batch before it
+  n_launch += 3;  // threshold, select, final
   const uint32_t nblk = (nq + kBatchQ - 1) / kBatchQ;
   // The sample pass.  By fours of queries (query-major keys) up to about nine tiles of every warp of
   // the chip; past that by blocks of 128, one read of the few sample tiles for all of a block, and a
@@ -1207,26 +1236,31 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   const uint64_t sample_work = (uint64_t)n_sample_tiles * ((nq + kMultiQ - 1) / kMultiQ);
   const bool sample_blocks = batched && sample_work > kMultiSampleMax;
   if (batched && (!tc || sample_blocks)) {
-    k_qtable<<<(uint32_t)((nblk * batch_qtab_words(cols) + 255) / 256), 256, 0, s>>>(
-        d_q8, ld8, cols, nq, d_qtab);
+    const uint32_t g = (uint32_t)((nblk * batch_qtab_words(cols) + 255) / 256);
+    if (first) k_qtable<<<g, 256, 0, s>>>(d_q8, ld8, cols, nq, d_qtab);
+    else AES_CK(chain(k_qtable, g, 256, 0, s, d_q8, ld8, cols, nq, d_qtab));
     AES_CK(cudaGetLastError());
+    first = false;
     n_launch++;
   }
   if (tf) {
     uint32_t* st = d_exact_aux + 4;
-    AES_CK(cudaMemsetAsync(st, 0, kTfStats * 4, s));
-    k_tf_qstats<<<nq, 256, 0, s>>>(d_q8, ld8, cols, sgn ? 1u : 0u, st);
+    if (first) k_tf_qstats<<<nq, 256, 0, s>>>(d_q8, ld8, cols, sgn ? 1u : 0u, st);
+    else AES_CK(chain(k_tf_qstats, nq, 256, 0, s, d_q8, ld8, cols, sgn ? 1u : 0u, st));
     AES_CK(cudaGetLastError());
-    k_tf_qtable<<<(nblk * kTcQ * (tc_kpad(cols) / 16) + 255) / 256, 256, 0, s>>>(
-        d_q8, ld8, cols, nq, nblk, sgn ? 1u : 0u, st, d_qtab_tc);
-    AES_CK(cudaGetLastError());
+    first = false;
+    AES_CK(chain(k_tf_qtable, (nblk * kTcQ * (tc_kpad(cols) / 16) + 255) / 256, 256, 0, s, d_q8, ld8, cols,
+                 nq, nblk, sgn ? 1u : 0u, st, d_qtab_tc));
     n_launch += 2;
   } else if (tc) {
     for (uint32_t b = 0; b < nblk; b++) {
       const uint32_t nb = std::min<uint32_t>(kBatchQ, nq - b * kBatchQ);
-      k_qtable_tc<<<(kTcQ * tc_kpad(cols) + 255) / 256, 256, 0, s>>>(
-          d_q8, ld8, cols, b * kTcQ, nb, d_qtab_tc + (size_t)b * tc_qtab_bytes(cols));
+      const uint32_t g = (kTcQ * tc_kpad(cols) + 255) / 256;
+      uint8_t* qt = d_qtab_tc + (size_t)b * tc_qtab_bytes(cols);
+      if (first) k_qtable_tc<<<g, 256, 0, s>>>(d_q8, ld8, cols, b * kTcQ, nb, qt);
+      else AES_CK(chain(k_qtable_tc, g, 256, 0, s, d_q8, ld8, cols, b * kTcQ, nb, qt));
       AES_CK(cudaGetLastError());
+      first = false;
       n_launch++;
     }
   }
@@ -1234,17 +1268,16 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
     int rc = run_batch(MODE_SAMPLE, nq, s);
     if (rc) return rc;
     if (n_sample_rows) {  // the threshold pass reads each query's keys contiguously
-      k_keys_transpose<<<dim3((n_sample_rows + kTransposeRows - 1) / kTransposeRows, nblk), 256, 0, s>>>(
-          d_sample_keys, n_sample_rows, nq, d_keys_t);
-      AES_CK(cudaGetLastError());
+      AES_CK(chain(k_keys_transpose, dim3((n_sample_rows + kTransposeRows - 1) / kTransposeRows, nblk), 256,
+                   0, s, d_sample_keys, n_sample_rows, nq, d_keys_t));
       n_launch++;
     }
   } else if (batch_mode != 1 && nq > 1) {
-    int rc = run_multi(nq, s, true);
+    int rc = run_multi(nq, s, true, first);
     if (rc) return rc;
   } else {
     for (uint32_t q0 = 0; q0 < nq; q0 += 65535u) {  // every query's sample pass in one launch
-      int rc = run_plain(MODE_SAMPLE, q0, s, std::min<uint32_t>(65535u, nq - q0));
+      int rc = run_plain(MODE_SAMPLE, q0, s, std::min<uint32_t>(65535u, nq - q0), first && q0 == 0);
       if (rc) return rc;
     }
   }
@@ -1305,8 +1338,7 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   const uint32_t fg = final_grid(nq, d_sample_keys, tail_bytes, &fa);
   sa.done = fa.done;
   if ((rct = run_select(sa, nq, s))) return rct;
-  k_final<<<dim3(fg, nq), kThreadsFinal, final_smem, s>>>(fa);
-  AES_CK(cudaGetLastError());
+  AES_CK(chain(k_final, dim3(fg, nq), kThreadsFinal, final_smem, s, fa));
   return AES_OK;
 }
 
@@ -1337,7 +1369,9 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
     prm.flags &= ~AES_FLAG_PROFILE;
     const uint64_t saved_launch = n_launch, saved_cand = n_cand;
     AES_CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    capturing = true;
     int rc = enqueue(d_q, nq, k, d_idx, d_score, s, pre);
+    capturing = false;
     cudaGraph_t graph = nullptr;
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
     prm.flags = saved_flags;
@@ -1899,9 +1933,8 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     k_exact_sample<<<dim3(groups, n), kThreadsExSample, exact_sample_smem_bytes(e.cols), s>>>(
         fa, S, ns, e.d_allkeys);
     AES_CK(cudaGetLastError());
-    k_threshold<<<dim3(1, n), kThreadsThr, 0, s>>>(e.d_allkeys, ns, 0, e.d_exact_aux, 1,
-                                                   e.d_exact_aux + 2, e.d_thr, e.d_cnt);
-    AES_CK(cudaGetLastError());
+    AES_CK(e.chain(k_threshold, dim3(1, n), kThreadsThr, 0, s, e.d_allkeys, ns, 0, e.d_exact_aux, 1,
+                      e.d_exact_aux + 2, e.d_thr, e.d_cnt));
     for (uint32_t i = 0; i < n;) {  // groups of eight queries, then four, a last one alone
       ExactArgs x{};
       x.ptr = e.d_csr_ptr;
@@ -1919,17 +1952,17 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
       if (left > 4) {
         const uint32_t g = left >= 8 ? left / 8 : 1;
         x.nq = std::min(left, 8 * g);
-        k_exact_multi<8><<<dim3((4 * e.sm_count + g - 1) / g, g), kExactWarps * 32,
-                           exact_multi_smem_bytes<8>(e.cols), s>>>(x);
+        AES_CK(e.chain(k_exact_multi<8>, dim3((4 * e.sm_count + g - 1) / g, g), kExactWarps * 32,
+                          exact_multi_smem_bytes<8>(e.cols), s, x));
       } else if (left > 1) {
         x.nq = left;
-        k_exact_multi<4><<<4 * e.sm_count, kExactWarps * 32, exact_multi_smem_bytes<4>(e.cols), s>>>(x);
+        AES_CK(e.chain(k_exact_multi<4>, 4 * e.sm_count, kExactWarps * 32,
+                          exact_multi_smem_bytes<4>(e.cols), s, x));
       } else {
         x.nq = 1;
-        k_exact_all<true><<<e.sm_count * 8, kExactWarps * 32, exact_all_smem_bytes(e.cols), s>>>(
-            x.ptr, x.col, x.val, x.q, x.cols, x.rows, nullptr, x.thr, x.cnt, x.surv, x.cap);
+        AES_CK(e.chain(k_exact_all<true>, e.sm_count * 8, kExactWarps * 32, exact_all_smem_bytes(e.cols), s,
+                          x.ptr, x.col, x.val, x.q, x.cols, x.rows, nullptr, x.thr, x.cnt, x.surv, x.cap));
       }
-      AES_CK(cudaGetLastError());
       i += x.nq;
     }
     sa.allkeys = nullptr;
@@ -1939,14 +1972,12 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     sa.status = e.d_status + q0;
     sa.cand = n > 1 ? e.d_sample_keys : e.d_exact_cand;
     sa.cand_key = n > 1 ? e.d_sample_keys + (size_t)n * k : e.d_exact_key;
-    k_select<false><<<dim3(1, n), kThreadsSel, 0, s>>>(sa);
-    AES_CK(cudaGetLastError());
+    AES_CK(e.chain(k_select<false>, dim3(1, n), kThreadsSel, 0, s, sa));
     fa.cand = sa.cand;
     fa.cand_key = sa.cand_key;
     fa.out_idx = e.d_out_idx + (size_t)q0 * k;
     fa.out_score = e.d_out_score + (size_t)q0 * k;
-    k_final<<<dim3(1, n), kThreadsFinal, e.final_smem, s>>>(fa);
-    AES_CK(cudaGetLastError());
+    AES_CK(e.chain(k_final, dim3(1, n), kThreadsFinal, e.final_smem, s, fa));
   }
   AES_CK(cudaEventRecord(e.ev1, s));
   AES_CK(cudaMemcpyAsync(e.h_status, e.d_status, nq * 4ull, cudaMemcpyDeviceToHost, s));
@@ -1980,8 +2011,7 @@ int aes_score_all(aes_handle* h, const float* q, uint32_t* keys) {
   cudaSetDevice(e.device);
   std::memcpy(e.h_q32, q, e.cols * 4ull);
   AES_CK(cudaMemcpyAsync(e.d_q32, e.h_q32, e.ld32 * 4ull, cudaMemcpyHostToDevice, e.stream));
-  AES_CK(cudaMemsetAsync(e.d_status, 0, 4, e.stream));
-  aes::dev::k_quantize<<<1, 256, 0, e.stream>>>(e.d_q32, e.cols, e.ld32, (int)e.bits, (int)e.quant,
+  aes::dev::k_quantize<<<1, aes::dev::quantize_threads(1), 0, e.stream>>>(e.d_q32, e.cols, e.ld32, (int)e.bits, (int)e.quant,
                                                 (int)e.prm.query_quant, e.d_q8, e.ld8, e.d_status);
   AES_CK(cudaGetLastError());
   int rc = e.run_plain(aes::dev::MODE_ALL, 0, e.stream);
@@ -2115,10 +2145,9 @@ extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, 
   uint32_t* cand_key = reinterpret_cast<uint32_t*>(base + L.cand_key);
   uint32_t* status = reinterpret_cast<uint32_t*>(base + L.status);
 
-  // the array keeps the previous call's contents: the status word starts at zero, the survivor
+  // the array keeps the previous call's contents: the status word is set by k_quantize, the survivor
   // counters are zeroed by k_threshold, every other region is fully written before it is read
-  AES_CK(cudaMemsetAsync(status, 0, 4, s));
-  k_quantize<<<1, 256, 0, s>>>(d_query, e.cols, e.ld32, (int)e.bits, (int)e.quant,
+  k_quantize<<<1, quantize_threads(1), 0, s>>>(d_query, e.cols, e.ld32, (int)e.bits, (int)e.quant,
                                (int)e.prm.query_quant, q8, e.ld8, status);
   AES_CK(cudaGetLastError());
   auto plain = [&](int mode, uint32_t* keys_out) -> int {
@@ -2145,8 +2174,13 @@ extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, 
       grid = std::min<int>(grid, (int)((e.n_sample_tiles + plain_warps((int)e.bits) - 1) /
                                        plain_warps((int)e.bits)));
     grid = std::max(grid, 1);
-    aes::pick_plain((int)e.bits, e.sgn, mode)<<<grid, plain_threads((int)e.bits), e.plain_smem, s>>>(a);
-    AES_CK(cudaGetLastError());
+    if (mode == MODE_ALL) {  // (after the status word's copy)
+      aes::pick_plain((int)e.bits, e.sgn, mode)<<<grid, plain_threads((int)e.bits), e.plain_smem, s>>>(a);
+      AES_CK(cudaGetLastError());
+    } else {
+      AES_CK(e.chain(aes::pick_plain((int)e.bits, e.sgn, mode), grid, plain_threads((int)e.bits),
+                        e.plain_smem, s, a));
+    }
     return AES_OK;
   };
   if ((rc = plain(MODE_SAMPLE, skeys))) return rc;

@@ -23,6 +23,18 @@ namespace dev {
 __host__ __device__ constexpr int plain_warps(int) { return 32; }
 __host__ __device__ constexpr int plain_threads(int B) { return plain_warps(B) * 32; }
 
+// Programmatic dependent launch: a kernel launched as a dependent (Engine::chain) starts while its
+// predecessor drains; it touches nothing that other kernels write before grid_wait(), which returns
+// once the predecessor is complete and its writes are visible.  grid_next() lets the next kernel start
+// in turn.  Kernels call it at their top after the wait, so what lies two kernels back is complete when
+// a kernel starts at all.  It hides the launch and drain between the short kernels around the
+// candidate pass, some 2 us each (one query of a small matrix 87 -> 75 us per call).  The long passes
+// over a whole batch leave it out: the next kernel then starts at their end.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 enum Mode : int { MODE_FILTER = 0, MODE_SAMPLE = 1, MODE_ALL = 2 };
 
 // status bits per query
@@ -559,6 +571,11 @@ __global__ void __launch_bounds__(plain_threads(B), 1) k_cand_plain(PlainArgs a)
   unsigned char* after = smem + (size_t)a.cols * kPlainTableBytesPerCol;
   uint4* stg = reinterpret_cast<uint4*>(after) + (size_t)warp * (kPlainTileBuf / 16);
   uint32_t* thr_s = reinterpret_cast<uint32_t*>(after + W * kPlainTileBuf);
+  // the filter's query was quantised before the sample pass, so its table is filled before the wait
+  if constexpr (MODE != MODE_FILTER) {
+    grid_wait();
+    grid_next();
+  }
   // replicate the query once per lane; the bytes are staged through the (not yet used) area
   // after the table so the fill needs one global round trip
   int8_t* qstage = reinterpret_cast<int8_t*>(after);
@@ -575,6 +592,8 @@ __global__ void __launch_bounds__(plain_threads(B), 1) k_cand_plain(PlainArgs a)
   __syncthreads();
   uint32_t thr0 = 0;
   if constexpr (MODE == MODE_FILTER) {
+    grid_wait();
+    grid_next();
     if (a.split > 1 && a.split <= kThrSmemMax)
       for (uint32_t i = threadIdx.x; i < a.split; i += blockDim.x) thr_s[i] = a.thr[i];
     thr0 = a.thr[0];

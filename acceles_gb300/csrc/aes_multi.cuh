@@ -383,6 +383,10 @@ __global__ void __launch_bounds__(kMultiThreads, 1) k_cand_multi(MultiArgs a) {
   uint4* stg = reinterpret_cast<uint4*>(after) + (size_t)warp * (kPlainTileBuf / 16);
   uint32_t* thr_s = reinterpret_cast<uint32_t*>(after + kMultiWarps * kPlainTileBuf);
   const uint32_t q0 = blockIdx.y * kMultiQ, nq = min((uint32_t)kMultiQ, a.nq - q0);
+  if constexpr (SAMPLE) {  // (the filter's queries were quantised before the sample pass)
+    grid_wait();
+    grid_next();
+  }
   {  // the columns' words through the tile buffers' area (4 KB), then one copy per lane
     uint32_t* qstage = reinterpret_cast<uint32_t*>(after);
     const int8_t* q8 = a.q8 + (size_t)q0 * a.q8_ld;
@@ -411,6 +415,7 @@ __global__ void __launch_bounds__(kMultiThreads, 1) k_cand_multi(MultiArgs a) {
     }
     return;
   }
+  grid_wait();
   const bool in_smem = a.split > 1 && a.split <= kThrSmemMax;
   if (in_smem)
     for (uint32_t i = threadIdx.x; i < a.split * kMultiQ; i += kMultiThreads) {

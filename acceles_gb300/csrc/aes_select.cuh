@@ -22,13 +22,19 @@ namespace dev {
 // integer arithmetic (aes_qexact.hpp), so no FP64 runs on the GPU.
 // quant: 0 symmetric, 1/2 unsigned (per query); qq: 0 numpy, 1 quantize_vec truncation.
 // ---------------------------------------------------------------------------------------------
-__global__ void k_quantize(const float* __restrict__ q32, uint32_t cols, uint32_t ld32, int bits,
+// threads per query: the rounding is a long chain of 64-bit divisions, so a few queries spread their
+// columns wide (1024 columns: 7.6 us with 256 threads, {QT} with 1024)
+__host__ inline unsigned quantize_threads(uint32_t nq) { return nq <= 64 ? 1024u : 256u; }
+__global__ void __launch_bounds__(1024) k_quantize(const float* __restrict__ q32, uint32_t cols, uint32_t ld32, int bits,
                            int quant, int qq, int8_t* __restrict__ q8, uint32_t ld8,
                            uint32_t* __restrict__ status) {
+  grid_wait();
+  grid_next();
   __shared__ float red[32];
   __shared__ int negs;
   const float* x = q32 + (size_t)blockIdx.x * ld32;
   int8_t* o = q8 + (size_t)blockIdx.x * ld8;
+  if (threadIdx.x == 0) status[blockIdx.x] = 0;
   if (qq == 1) {  // quantize_utils.hpp:8-18 (ap_fixed<32,B,AP_TRN_ZERO>, to_int, ap_int<B>)
     const int F = 32 - bits;
     for (uint32_t j = threadIdx.x; j < cols; j += blockDim.x) {
@@ -62,7 +68,7 @@ __global__ void k_quantize(const float* __restrict__ q32, uint32_t cols, uint32_
   __syncthreads();
   const float mm = red[0];  // max |x| (or max x)
   if (quant != 0 && negs) {
-    if (threadIdx.x == 0) atomicOr(status + blockIdx.x, ST_QUERY);
+    if (threadIdx.x == 0) status[blockIdx.x] = ST_QUERY;
     for (uint32_t j = threadIdx.x; j < cols; j += blockDim.x) o[j] = 0;
     return;
   }
@@ -173,6 +179,8 @@ __global__ void __launch_bounds__(kThrWarps * 32) k_threshold_warp(
     const uint32_t* __restrict__ keys_all, uint32_t ld_keys, const uint32_t* __restrict__ part_begin,
     uint32_t split, uint32_t pairs, const uint32_t* __restrict__ r_part, uint32_t* __restrict__ thr,
     uint32_t* __restrict__ cnt) {
+  grid_wait();
+  grid_next();
   const uint32_t i = blockIdx.x * kThrWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
   if (i >= pairs) return;
   const uint32_t p = i % split, q = i / split;
@@ -211,6 +219,8 @@ __global__ void __launch_bounds__(kThreadsThr, 2) k_threshold(const uint32_t* __
                             const uint32_t* __restrict__ part_begin, uint32_t split,
                             const uint32_t* __restrict__ r_part, uint32_t* __restrict__ thr,
                             uint32_t* __restrict__ cnt) {
+  grid_wait();
+  grid_next();
   __shared__ __align__(16) uint32_t hist[kHistBins];
   __shared__ uint32_t smin[kThreadsThr / 32], smax[kThreadsThr / 32], sh[kThreadsThr / 32 + 3];
   __shared__ uint32_t s_bound, s_n;
@@ -603,6 +613,8 @@ __device__ __forceinline__ void block_select(SelectShared<THREADS>& S, uint32_t 
 
 template <bool IMPLICIT>
 __global__ void __launch_bounds__(kThreadsSel, 1) k_select(SelectArgs a) {
+  grid_wait();
+  grid_next();
   __shared__ SelectShared<kThreadsSel> S;
   const uint32_t p = blockIdx.x, q = IMPLICIT ? a.q0 : blockIdx.y;
   const uint32_t r0 = p * a.slice;
@@ -649,6 +661,8 @@ constexpr uint32_t kSelWarpList = 128;   // the most of them at or above the gro
 constexpr int kSelWarpThreads = 256;
 
 __global__ void __launch_bounds__(kSelWarpThreads) k_select_warp(SelectArgs a) {
+  grid_wait();
+  grid_next();
   constexpr int N = kSelWarpKeys / 32, W = kSelWarpThreads / 32;
   __shared__ SelectShared<kSelWarpThreads> S;
   __shared__ uint64_t s_list[W][kSelWarpList];
@@ -845,6 +859,8 @@ __device__ __forceinline__ float rescore_rows(const FinalArgs& a, const float* q
 }
 
 __global__ void __launch_bounds__(kThreadsFinal, 2) k_final(FinalArgs a) {
+  grid_wait();
+  grid_next();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ __align__(16) uint32_t hist[kHistBins];
   __shared__ uint64_t sh64[72];
@@ -1026,6 +1042,7 @@ __global__ void __launch_bounds__(kExactWarps * 32) k_exact_all(
     const float* __restrict__ val, const float* __restrict__ q, uint32_t cols, uint32_t rows,
     uint32_t* __restrict__ keys, const uint32_t* __restrict__ thr, uint32_t* __restrict__ cnt,
     uint2* __restrict__ surv, uint32_t cap) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char xsm[];
   float* qs = reinterpret_cast<float*>(xsm);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -1105,6 +1122,7 @@ __host__ inline size_t exact_multi_smem_bytes(uint32_t cols) {
 }
 template <int T>
 __global__ void __launch_bounds__(kExactWarps * 32) k_exact_multi(ExactArgs a) {
+  grid_wait();
   static_assert(T == 4 || T == 8, "queries per walk");
   extern __shared__ __align__(16) unsigned char xsm[];
   float4* qs = reinterpret_cast<float4*>(xsm);  // [T / 4][cols]
@@ -1179,6 +1197,8 @@ __host__ inline size_t exact_sample_smem_bytes(uint32_t cols) {
 }
 __global__ void __launch_bounds__(kThreadsExSample) k_exact_sample(FinalArgs a, uint32_t S, uint32_t ns,
                                                                    uint32_t* __restrict__ keys) {
+  grid_wait();
+  grid_next();
   extern __shared__ __align__(16) unsigned char xsm[];
   float* qs = reinterpret_cast<float*>(xsm);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;

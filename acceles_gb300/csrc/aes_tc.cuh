@@ -87,6 +87,8 @@ __host__ inline uint32_t tc_bufs(uint32_t cols, uint32_t split, size_t smem_limi
 // e4m3 query operand of queries q0 .. q0 + nq - 1 (zero past nq and past cols)
 __global__ void k_qtable_tc(const int8_t* __restrict__ q8, uint32_t ld8, uint32_t cols, uint32_t q0,
                             uint32_t nq, uint8_t* __restrict__ qt) {
+  grid_wait();
+  grid_next();
   const uint32_t kp = tc_kpad(cols);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kTcQ * kp) return;
@@ -502,6 +504,7 @@ __device__ __forceinline__ void tc_drain_scores(const TcArgs& a, uint32_t S, con
 // layouts, since an operand descriptor addresses the same offset in both.
 template <uint32_t NB, bool PAIR>
 __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
+  grid_wait();
   static_assert(NB == 2 || NB == 3, "two or three chunk buffers");
   constexpr uint32_t Q = TcShape<PAIR>::Q, ACC = TcShape<PAIR>::ACC;
   constexpr uint32_t kDone = NB, kFull = 2 * NB, kEmpty = 2 * NB + ACC;

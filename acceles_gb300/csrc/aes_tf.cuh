@@ -174,6 +174,8 @@ constexpr uint32_t kTfStats = 4;
 
 __global__ void __launch_bounds__(256) k_tf_qstats(const int8_t* __restrict__ q8, uint32_t ld8,
                                                    uint32_t cols, uint32_t sgn, uint32_t* st) {
+  grid_wait();
+  grid_next();
   uint32_t hi = 0, lo = 0;
   for (uint32_t c = threadIdx.x; c < cols; c += 256) {
     const int8_t b = q8[(size_t)blockIdx.x * ld8 + c];
@@ -195,6 +197,8 @@ __global__ void __launch_bounds__(256) k_tf_qstats(const int8_t* __restrict__ q8
 __global__ void __launch_bounds__(256) k_tf_qtable(const int8_t* __restrict__ q8, uint32_t ld8,
                                                    uint32_t cols, uint32_t nq, uint32_t nblk, uint32_t sgn,
                                                    uint32_t* st, uint8_t* __restrict__ qt) {
+  grid_wait();
+  grid_next();
   const uint32_t per = tc_kpad(cols) / 16u;
   const int centre = tc_centre(st);
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
@@ -262,6 +266,7 @@ __host__ inline size_t check_smem_bytes(uint32_t ld8) { return (size_t)check_ld(
 // so a warp reads eight rows' 64-byte pieces per load and an entry costs four instructions, among
 // them the gather of the query's byte.
 __global__ void __launch_bounds__(kThreadsCheck) k_recheck(TfCheck a) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char csm[];
   __shared__ uint32_t s_most;  // entries of the longest list
   const int8_t* qs = reinterpret_cast<const int8_t*>(csm);
