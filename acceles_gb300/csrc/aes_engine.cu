@@ -186,13 +186,14 @@ struct Engine {
   uint32_t* d_cand = nullptr;
   uint32_t* d_cand_key = nullptr;
   uint32_t* d_status = nullptr;
-  uint32_t* d_out_idx = nullptr;
-  float* d_out_score = nullptr;
   uint32_t* d_allkeys = nullptr;
   uint32_t* d_exact_cand = nullptr;  // [k_max] candidates of the FP32-only pass
   uint32_t* d_exact_key = nullptr;
 
-  float* h_q32 = nullptr;         // pinned staging of queries
+  float* h_q32 = nullptr;         // queries in pinned memory: aes_run's kernels read them there
+  bool q32_on_device = false;     // ... and d_q32 holds a copy
+  uint32_t* h_out_idx = nullptr;  // pinned: aes_run's kernels write their results here
+  float* h_out_score = nullptr;
   int8_t* h_q8 = nullptr;         // pinned staging of pre-quantised queries
   uint32_t* h_status = nullptr;   // pinned
   uint32_t nq_loaded = 0;
@@ -214,10 +215,10 @@ struct Engine {
     uint32_t* idx;
     float* score;
     cudaStream_t s;
-    bool pre;
+    bool pre, host_q;
     bool operator<(const GraphKey& o) const {
-      return std::tie(q, nq, k, idx, score, s, pre) <
-             std::tie(o.q, o.nq, o.k, o.idx, o.score, o.s, o.pre);
+      return std::tie(q, nq, k, idx, score, s, pre, host_q) <
+             std::tie(o.q, o.nq, o.k, o.idx, o.score, o.s, o.pre, o.host_q);
     }
   };
   struct Graph {
@@ -276,6 +277,10 @@ struct Engine {
     cfg_allocs.clear();
     if (h_q32) cudaFreeHost(h_q32);
     if (h_q8) cudaFreeHost(h_q8);
+    if (h_out_idx) cudaFreeHost(h_out_idx);
+    if (h_out_score) cudaFreeHost(h_out_score);
+    h_out_idx = nullptr;
+    h_out_score = nullptr;
     if (h_status) cudaFreeHost(h_status);
     h_q32 = nullptr;
     h_q8 = nullptr;
@@ -283,9 +288,8 @@ struct Engine {
     d_sample_first = d_part_sample_begin = d_part_r = nullptr;
     d_q32 = nullptr;
     d_q8 = nullptr;
-    d_sample_keys = d_keys_t = d_thr = d_cnt = d_cand = d_cand_key = d_status = d_out_idx = nullptr;
+    d_sample_keys = d_keys_t = d_thr = d_cnt = d_cand = d_cand_key = d_status = nullptr;
     d_surv = nullptr;
-    d_out_score = nullptr;
     d_exact_cand = d_exact_key = d_qtab = d_exact_aux = nullptr;
     bytes -= cfg_bytes;
     cfg_bytes = 0;
@@ -352,10 +356,11 @@ struct Engine {
   int retune(const aes_params& p);
   // d_q: the FP32 queries, or null when there are none (pre-quantised queries alone); pre: the
   // quantised queries are already in d_q8
+  // host_q: the queries are still in h_q32 only (d_q == d_q32 is filled on the way)
   int enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score,
-              cudaStream_t s, bool pre = false);
+              cudaStream_t s, bool pre = false, bool host_q = false);
   int enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score,
-                    cudaStream_t s, bool pre = false);
+                    cudaStream_t s, bool pre = false, bool host_q = false);
   // CTAs per query of k_final (FinalArgs::comp and done set in `scratch`, nq queries, where more
   // than one)
   uint32_t final_grid(uint32_t nq, void* scratch, size_t scratch_bytes, FinalArgs* fa) const;
@@ -629,8 +634,7 @@ int Engine::plan_config(const aes_params& p, Config* c) const {
   size_t plan = (c->n_sample_tiles + 2ull * S + 2) * 4;
   plan += nblk * kBatchQ * (size_t)c->n_sample_rows * 4;
   plan += maxB * (size_t)c->n_sample_rows * 4;  // the same keys, query-major
-  plan += maxB * (ld32 * 4ull + ld8 + S * 8ull + (size_t)S * c->cap * 8 + c->nslots * 8ull + 4 +
-                  p.k_max * 8ull);
+  plan += maxB * (ld32 * 4ull + ld8 + S * 8ull + (size_t)S * c->cap * 8 + c->nslots * 8ull + 4);
   plan += nblk * batch_qtab_words(cols) * 4;
   if (tc_usable(p, S) || tf_usable(p, S)) plan += nblk * tc_qtab_bytes(cols);
   if (!tc_usable(p, S) && tf_usable(p, S)) plan += (size_t)sm_count * kTcLists * (tf_list_entries(c->cap, S) * 8ull + 4);
@@ -677,8 +681,6 @@ int Engine::apply_config(const Config& c) {
   AES_AL(d_cand, (size_t)maxB * std::max<uint32_t>(nslots, 1));
   AES_AL(d_cand_key, (size_t)maxB * std::max<uint32_t>(nslots, 1));
   AES_AL(d_status, maxB);
-  AES_AL(d_out_idx, (size_t)maxB * std::max<uint32_t>(p.k_max, 1));
-  AES_AL(d_out_score, (size_t)maxB * std::max<uint32_t>(p.k_max, 1));
   AES_AL(d_qtab, (size_t)((maxB + kBatchQ - 1) / kBatchQ) * batch_qtab_words(cols));
   use_tc = tc_usable(p, split);
   use_tf = !use_tc && tf_usable(p, split);
@@ -695,6 +697,8 @@ int Engine::apply_config(const Config& c) {
   AES_CK(cudaMallocHost(&h_q32, (size_t)maxB * ld32 * sizeof(float)));
   AES_CK(cudaMallocHost(&h_q8, (size_t)maxB * ld8));
   AES_CK(cudaMallocHost(&h_status, (size_t)maxB * sizeof(uint32_t)));
+  AES_CK(cudaMallocHost(&h_out_idx, (size_t)maxB * std::max<uint32_t>(p.k_max, 1) * sizeof(uint32_t)));
+  AES_CK(cudaMallocHost(&h_out_score, (size_t)maxB * std::max<uint32_t>(p.k_max, 1) * sizeof(float)));
   if (n_sample_tiles)
     AES_CK(cudaMemcpy(d_sample_first, c.sample_first.data(), n_sample_tiles * 4ull, cudaMemcpyHostToDevice));
   AES_CK(cudaMemcpy(d_part_sample_begin, c.part_begin.data(), (split + 1) * 4ull, cudaMemcpyHostToDevice));
@@ -1210,7 +1214,7 @@ int Engine::run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s) {
 }
 
 int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score,
-                    cudaStream_t s, bool pre) {
+                    cudaStream_t s, bool pre, bool host_q) {
   const bool batched = batch_mode != 1 && (batch_mode != 0 || nq > multi_max);
   last_batched = batched;
   const bool tc = batched && (use_tc || use_tf), tf = batched && use_tf;
@@ -1221,8 +1225,9 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   if (pre) {
     AES_CK(cudaMemsetAsync(d_status, 0, nq * 4ull, s));
   } else {  // (sets the status words)
-    k_quantize<<<nq, quantize_threads(nq), 0, s>>>(d_q, cols, ld32, (int)bits, (int)quant,
-                                                   (int)prm.query_quant, d_q8, ld8, d_status);
+    k_quantize<<<nq, quantize_threads(nq), 0, s>>>(host_q ? h_q32 : d_q, cols, ld32, (int)bits, (int)quant,
+                                                   (int)prm.query_quant, d_q8, ld8, d_status,
+                                                   host_q ? d_q32 : nullptr);
     AES_CK(cudaGetLastError());
     n_launch++;
   }
@@ -1334,6 +1339,7 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   fa.out_idx = d_idx;
   fa.out_score = d_score;
   fa.status = d_status;
+  fa.status_out = h_status;
   fa.cand_key = int_final(d_q) ? d_cand_key : nullptr;
   const uint32_t fg = final_grid(nq, d_sample_keys, tail_bytes, &fa);
   sa.done = fa.done;
@@ -1360,8 +1366,8 @@ uint32_t Engine::final_grid(uint32_t nq, void* scratch, size_t scratch_bytes, Fi
 // Replays the launch sequence of enqueue() as one CUDA graph (captured on first use for these
 // arguments).  Profiling events are not recorded inside graphs.
 int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx,
-                          float* d_score, cudaStream_t s, bool pre) {
-  GraphKey key{d_q, nq, k, d_idx, d_score, s, pre};
+                          float* d_score, cudaStream_t s, bool pre, bool host_q) {
+  GraphKey key{d_q, nq, k, d_idx, d_score, s, pre, host_q};
   auto it = graphs.find(key);
   if (it == graphs.end()) {
     if (graphs.size() >= 64) drop_graphs();
@@ -1370,7 +1376,7 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
     const uint64_t saved_launch = n_launch, saved_cand = n_cand;
     AES_CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     capturing = true;
-    int rc = enqueue(d_q, nq, k, d_idx, d_score, s, pre);
+    int rc = enqueue(d_q, nq, k, d_idx, d_score, s, pre, host_q);
     capturing = false;
     cudaGraph_t graph = nullptr;
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
@@ -1403,8 +1409,7 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
 // every row, select each partition's Top-CK from the full key array, rescore.
 int Engine::repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cudaStream_t s,
                    uint32_t* repaired) {
-  AES_CK(cudaMemcpyAsync(h_status, d_status, nq * 4ull, cudaMemcpyDeviceToHost, s));
-  AES_CK(cudaStreamSynchronize(s));
+  AES_CK(cudaStreamSynchronize(s));  // (k_final has written the status words to h_status)
   uint32_t nrep = 0;
   for (uint32_t q = 0; q < nq; q++) {
     if (h_status[q] & ST_QUERY) return fail(AES_ERR_QUERY, "query " + std::to_string(q) +
@@ -1423,7 +1428,6 @@ int Engine::repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cud
       drop_graphs();
       int rc = enqueue(last_q32, nq, k, d_idx, d_score, s, last_pre);
       if (rc) return rc;
-      AES_CK(cudaMemcpyAsync(h_status, d_status, nq * 4ull, cudaMemcpyDeviceToHost, s));
       AES_CK(cudaStreamSynchronize(s));
     }
   }
@@ -1711,8 +1715,11 @@ int aes_set_query(aes_handle* h, const float* q, uint32_t nq) {
   if (!e.configured) return aes::fail(AES_ERR_STATE, kUnconfigured);
   if (nq == 0 || nq > e.maxB) return aes::fail(AES_ERR_INVALID, "nq must be in [1, max_batch]");
   cudaSetDevice(e.device);
-  for (uint32_t i = 0; i < nq; i++) std::memcpy(e.h_q32 + (size_t)i * e.ld32, q + (size_t)i * e.cols, e.cols * 4ull);
-  AES_CK(cudaMemcpyAsync(e.d_q32, e.h_q32, (size_t)nq * e.ld32 * 4, cudaMemcpyHostToDevice, e.stream));
+  if (e.ld32 == e.cols) std::memcpy(e.h_q32, q, (size_t)nq * e.cols * 4ull);
+  else
+    for (uint32_t i = 0; i < nq; i++)
+      std::memcpy(e.h_q32 + (size_t)i * e.ld32, q + (size_t)i * e.cols, e.cols * 4ull);
+  e.q32_on_device = false;
   e.nq_loaded = nq;
   e.q_pre = false;
   e.q32_given = true;
@@ -1742,6 +1749,7 @@ int aes_set_query_quantized(aes_handle* h, const int8_t* q, const float* q_f32, 
       std::memcpy(e.h_q32 + (size_t)i * e.ld32, q_f32 + (size_t)i * e.cols, e.cols * 4ull);
     AES_CK(cudaMemcpyAsync(e.d_q32, e.h_q32, (size_t)nq * e.ld32 * 4, cudaMemcpyHostToDevice, e.stream));
   }
+  e.q32_on_device = true;
   e.nq_loaded = nq;
   e.q_pre = true;
   e.q32_given = q_f32 != nullptr;
@@ -1756,20 +1764,21 @@ int aes_run(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score, uint
   cudaSetDevice(e.device);
   const uint32_t nq = e.nq_loaded;
   const float* dq = e.q32_given ? e.d_q32 : nullptr;
+  const bool host_q = !e.q_pre && !e.q32_on_device;
   e.last_q32 = dq;
   e.last_int_final = e.int_final(dq);
   AES_CK(cudaEventRecord(e.ev0, e.stream));
   int rc = (e.prm.flags & AES_FLAG_GRAPHS)
-               ? e.enqueue_graph(dq, nq, k, e.d_out_idx, e.d_out_score, e.stream, e.q_pre)
-               : e.enqueue(dq, nq, k, e.d_out_idx, e.d_out_score, e.stream, e.q_pre);
+               ? e.enqueue_graph(dq, nq, k, e.h_out_idx, e.h_out_score, e.stream, e.q_pre, host_q)
+               : e.enqueue(dq, nq, k, e.h_out_idx, e.h_out_score, e.stream, e.q_pre, host_q);
   if (rc) return rc;
   AES_CK(cudaEventRecord(e.ev1, e.stream));
   uint32_t rep = 0;
-  rc = e.repair(nq, k, e.d_out_idx, e.d_out_score, e.stream, &rep);
+  rc = e.repair(nq, k, e.h_out_idx, e.h_out_score, e.stream, &rep);  // waits
   if (rc) return rc;
-  AES_CK(cudaMemcpyAsync(out_idx, e.d_out_idx, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, e.stream));
-  AES_CK(cudaMemcpyAsync(out_score, e.d_out_score, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, e.stream));
-  AES_CK(cudaStreamSynchronize(e.stream));
+  // (a fresh query stays in h_q32: the next run of it takes the same graph)
+  std::memcpy(out_idx, e.h_out_idx, (size_t)nq * k * 4);
+  std::memcpy(out_score, e.h_out_score, (size_t)nq * k * 4);
   if (ns) {
     float ms = 0.0f;
     AES_CK(cudaEventElapsedTime(&ms, e.ev0, e.ev1));
@@ -1795,6 +1804,7 @@ int aes_run_device(aes_handle* h, const float* d_queries, uint32_t nq, uint32_t 
     AES_CK(cudaMemcpy2DAsync(e.d_q32, e.ld32 * 4ull, d_queries, e.cols * 4ull, e.cols * 4ull, nq,
                              cudaMemcpyDeviceToDevice, s));
     d_queries = e.d_q32;
+    if (!e.q_pre) e.q32_on_device = false;  // (aes_set_query's queries are in h_q32)
   }
   e.last_q32 = d_queries;
   e.last_int_final = e.int_final(d_queries);
@@ -1852,6 +1862,10 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
   AES_CK(cudaSetDevice(e.device));
   const uint32_t nq = e.nq_loaded;
   cudaStream_t s = e.stream;
+  if (!e.q32_on_device) {
+    AES_CK(cudaMemcpyAsync(e.d_q32, e.h_q32, (size_t)nq * e.ld32 * 4, cudaMemcpyHostToDevice, s));
+    e.q32_on_device = true;
+  }
   // Filtered select: every S-th row key is a sample; its r-th largest key lies below the K-th
   // largest key of all rows except with probability 1e-12 (binomial tail), so only the rows at or
   // above it need the select.  S is the largest power of two whose expected survivors fit the
@@ -1907,8 +1921,9 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     AES_CK(cudaGetLastError());
     fa.cand = e.d_exact_cand;
     fa.cand_key = e.d_exact_key;
-    fa.out_idx = e.d_out_idx + (size_t)q * k;
-    fa.out_score = e.d_out_score + (size_t)q * k;
+    fa.out_idx = e.h_out_idx + (size_t)q * k;
+    fa.out_score = e.h_out_score + (size_t)q * k;
+    fa.status = fa.status_out = nullptr;
     k_final<<<1, kThreadsFinal, e.final_smem, s>>>(fa);
     AES_CK(cudaGetLastError());
     return AES_OK;
@@ -1975,12 +1990,13 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     AES_CK(e.chain(k_select<false>, dim3(1, n), kThreadsSel, 0, s, sa));
     fa.cand = sa.cand;
     fa.cand_key = sa.cand_key;
-    fa.out_idx = e.d_out_idx + (size_t)q0 * k;
-    fa.out_score = e.d_out_score + (size_t)q0 * k;
+    fa.out_idx = e.h_out_idx + (size_t)q0 * k;
+    fa.out_score = e.h_out_score + (size_t)q0 * k;
+    fa.status = e.d_status + q0;
+    fa.status_out = e.h_status + q0;
     AES_CK(e.chain(k_final, dim3(1, n), kThreadsFinal, e.final_smem, s, fa));
   }
   AES_CK(cudaEventRecord(e.ev1, s));
-  AES_CK(cudaMemcpyAsync(e.h_status, e.d_status, nq * 4ull, cudaMemcpyDeviceToHost, s));
   AES_CK(cudaStreamSynchronize(s));
   float total_ms = 0.0f;
   AES_CK(cudaEventElapsedTime(&total_ms, e.ev0, e.ev1));
@@ -1997,9 +2013,8 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     total_ms += ms;
     e.n_repaired++;
   }
-  AES_CK(cudaMemcpyAsync(out_idx, e.d_out_idx, (size_t)nq * k * 4ull, cudaMemcpyDeviceToHost, s));
-  AES_CK(cudaMemcpyAsync(out_score, e.d_out_score, (size_t)nq * k * 4ull, cudaMemcpyDeviceToHost, s));
-  AES_CK(cudaStreamSynchronize(s));
+  std::memcpy(out_idx, e.h_out_idx, (size_t)nq * k * 4ull);
+  std::memcpy(out_score, e.h_out_score, (size_t)nq * k * 4ull);
   if (ns_out) *ns_out = (uint64_t)((double)total_ms * 1e6);
   return AES_OK;
 }
@@ -2012,7 +2027,7 @@ int aes_score_all(aes_handle* h, const float* q, uint32_t* keys) {
   std::memcpy(e.h_q32, q, e.cols * 4ull);
   AES_CK(cudaMemcpyAsync(e.d_q32, e.h_q32, e.ld32 * 4ull, cudaMemcpyHostToDevice, e.stream));
   aes::dev::k_quantize<<<1, aes::dev::quantize_threads(1), 0, e.stream>>>(e.d_q32, e.cols, e.ld32, (int)e.bits, (int)e.quant,
-                                                (int)e.prm.query_quant, e.d_q8, e.ld8, e.d_status);
+                                                (int)e.prm.query_quant, e.d_q8, e.ld8, e.d_status, nullptr);
   AES_CK(cudaGetLastError());
   int rc = e.run_plain(aes::dev::MODE_ALL, 0, e.stream);
   if (rc) return rc;
@@ -2148,7 +2163,7 @@ extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, 
   // the array keeps the previous call's contents: the status word is set by k_quantize, the survivor
   // counters are zeroed by k_threshold, every other region is fully written before it is read
   k_quantize<<<1, quantize_threads(1), 0, s>>>(d_query, e.cols, e.ld32, (int)e.bits, (int)e.quant,
-                               (int)e.prm.query_quant, q8, e.ld8, status);
+                               (int)e.prm.query_quant, q8, e.ld8, status, nullptr);
   AES_CK(cudaGetLastError());
   auto plain = [&](int mode, uint32_t* keys_out) -> int {
     PlainArgs a{};

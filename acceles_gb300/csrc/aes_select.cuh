@@ -27,7 +27,7 @@ namespace dev {
 __host__ inline unsigned quantize_threads(uint32_t nq) { return nq <= 64 ? 1024u : 256u; }
 __global__ void __launch_bounds__(1024) k_quantize(const float* __restrict__ q32, uint32_t cols, uint32_t ld32, int bits,
                            int quant, int qq, int8_t* __restrict__ q8, uint32_t ld8,
-                           uint32_t* __restrict__ status) {
+                           uint32_t* __restrict__ status, float* __restrict__ copy) {
   grid_wait();
   grid_next();
   __shared__ float red[32];
@@ -35,6 +35,12 @@ __global__ void __launch_bounds__(1024) k_quantize(const float* __restrict__ q32
   const float* x = q32 + (size_t)blockIdx.x * ld32;
   int8_t* o = q8 + (size_t)blockIdx.x * ld8;
   if (threadIdx.x == 0) status[blockIdx.x] = 0;
+  if (copy) {  // the queries are in pinned host memory: the later stages read them from here
+    float* d = copy + (size_t)blockIdx.x * ld32;
+    for (uint32_t j = threadIdx.x; j < cols; j += blockDim.x) d[j] = x[j];
+    x = d;
+    __syncthreads();
+  }
   if (qq == 1) {  // quantize_utils.hpp:8-18 (ap_fixed<32,B,AP_TRN_ZERO>, to_int, ap_int<B>)
     const int F = 32 - bits;
     for (uint32_t j = threadIdx.x; j < cols; j += blockDim.x) {
@@ -782,6 +788,7 @@ struct FinalArgs {
   // already exact
   const uint32_t* cand_key;
   uint32_t key_f32;
+  uint32_t* status_out;      // [nq] or null: the status words, to pinned host memory
   uint64_t* comp;            // gridDim.x > 1: [nq][nslots] composites between the CTAs of a query
   uint32_t* done;            // gridDim.x > 1: [nq] CTAs finished, zero before the launch
 };
@@ -872,7 +879,11 @@ __global__ void __launch_bounds__(kThreadsFinal, 2) k_final(FinalArgs a) {
   uint64_t* list = comp + a.nslots;  // after the rescoring; the product staging before it
   const uint32_t q = blockIdx.y;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (a.status && a.status[q]) return;
+  if (a.status) {
+    const uint32_t st = a.status[q];
+    if (a.status_out && blockIdx.x == 0 && threadIdx.x == 0) a.status_out[q] = st;
+    if (st) return;
+  }
   const uint32_t* cr = a.cand + (size_t)q * a.nslots;
   if (threadIdx.x == 0) s_cnt = 0;
   if (a.cand_key) {  // integer ranking: the candidate keys themselves (one CTA per query)
