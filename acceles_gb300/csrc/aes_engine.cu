@@ -333,7 +333,10 @@ struct Engine {
 
   // Launches a kernel as a programmatic dependent of the kernel before it in the stream (grid_wait).
   // Not inside a captured graph, whose kernels follow one another closely as it is: programmatic
-  // edges made its replays slower (40 queries of 2M x 1024: 338 -> 348 us).
+  // edges made its replays slower (40 queries of 2M x 1024: 338 -> 348 us).  And only short kernels,
+  // or those of one CTA per SM: an early CTA is placed in the shared-memory split that the kernel
+  // before it has set up, so a kernel that wants several large CTAs on an SM may get one (16 queries
+  // of aes_run_exact: 254 us, or 417 on some runs).
   template <class... P, class... A>
   cudaError_t chain(void (*k)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A... a) const {
     cudaLaunchConfig_t cfg{};
@@ -513,8 +516,9 @@ int Engine::run_check(uint32_t q0, uint32_t n, cudaStream_t s, uint32_t ctas) {
   c.cnt = d_cnt;
   c.surv = d_surv;
   const uint32_t blocks = (n + 31) / 32;  // (six CTAs fit on an SM)
-  AES_CK(chain(k_recheck, dim3(blocks, std::max(1u, 6u * (uint32_t)sm_count / blocks)), kThreadsCheck,
-               check_smem_bytes(ld8), s, c));
+  k_recheck<<<dim3(blocks, std::max(1u, 6u * (uint32_t)sm_count / blocks)), kThreadsCheck,
+              check_smem_bytes(ld8), s>>>(c);
+  AES_CK(cudaGetLastError());
   n_launch++;
   return AES_OK;
 }
@@ -1344,7 +1348,12 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   const uint32_t fg = final_grid(nq, d_sample_keys, tail_bytes, &fa);
   sa.done = fa.done;
   if ((rct = run_select(sa, nq, s))) return rct;
-  AES_CK(chain(k_final, dim3(fg, nq), kThreadsFinal, final_smem, s, fa));
+  if (fg * nq <= (uint32_t)sm_count) {
+    AES_CK(chain(k_final, dim3(fg, nq), kThreadsFinal, final_smem, s, fa));
+  } else {  // two CTAs per SM
+    k_final<<<dim3(fg, nq), kThreadsFinal, final_smem, s>>>(fa);
+    AES_CK(cudaGetLastError());
+  }
   return AES_OK;
 }
 
@@ -1967,17 +1976,17 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
       if (left > 4) {
         const uint32_t g = left >= 8 ? left / 8 : 1;
         x.nq = std::min(left, 8 * g);
-        AES_CK(e.chain(k_exact_multi<8>, dim3((4 * e.sm_count + g - 1) / g, g), kExactWarps * 32,
-                          exact_multi_smem_bytes<8>(e.cols), s, x));
+        k_exact_multi<8><<<dim3((4 * e.sm_count + g - 1) / g, g), kExactWarps * 32,
+                           exact_multi_smem_bytes<8>(e.cols), s>>>(x);
       } else if (left > 1) {
         x.nq = left;
-        AES_CK(e.chain(k_exact_multi<4>, 4 * e.sm_count, kExactWarps * 32,
-                          exact_multi_smem_bytes<4>(e.cols), s, x));
+        k_exact_multi<4><<<4 * e.sm_count, kExactWarps * 32, exact_multi_smem_bytes<4>(e.cols), s>>>(x);
       } else {
         x.nq = 1;
-        AES_CK(e.chain(k_exact_all<true>, e.sm_count * 8, kExactWarps * 32, exact_all_smem_bytes(e.cols), s,
-                          x.ptr, x.col, x.val, x.q, x.cols, x.rows, nullptr, x.thr, x.cnt, x.surv, x.cap));
+        k_exact_all<true><<<e.sm_count * 8, kExactWarps * 32, exact_all_smem_bytes(e.cols), s>>>(
+            x.ptr, x.col, x.val, x.q, x.cols, x.rows, nullptr, x.thr, x.cnt, x.surv, x.cap);
       }
+      AES_CK(cudaGetLastError());
       i += x.nq;
     }
     sa.allkeys = nullptr;
