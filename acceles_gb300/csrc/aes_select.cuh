@@ -23,7 +23,7 @@ namespace dev {
 // quant: 0 symmetric, 1/2 unsigned (per query); qq: 0 numpy, 1 quantize_vec truncation.
 // ---------------------------------------------------------------------------------------------
 // threads per query: the rounding is a long chain of 64-bit divisions, so a few queries spread their
-// columns wide (1024 columns: 7.6 us with 256 threads, {QT} with 1024)
+// columns wide (1024 columns: 7.6 us with 256 threads, 5.5 with 1024)
 __host__ inline unsigned quantize_threads(uint32_t nq) { return nq <= 64 ? 1024u : 256u; }
 __global__ void __launch_bounds__(1024) k_quantize(const float* __restrict__ q32, uint32_t cols, uint32_t ld32, int bits,
                            int quant, int qq, int8_t* __restrict__ q8, uint32_t ld8,

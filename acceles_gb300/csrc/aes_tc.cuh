@@ -39,8 +39,7 @@ namespace dev {
 // Warp roles: warps 0-7 stage the chunks (producers), warps 8-15 read the accumulators (warp w
 // may only read tensor-memory lanes 32 (w % 4) .. + 31; warps 8-11 take the first half of the
 // queries, warps 12-15 the second), warp 16 allocates tensor memory and its lane 0 issues the
-// MMAs (on a pair: the even CTA's; lanes 0 and 1 of the odd CTA's forward barrier phases), warps
-// 17 to 19 append the hits.  They hand work over through mbarriers only.
+// MMAs (on a pair: the even CTA's), warps 17 to 19 append the hits.  They hand work over through mbarriers only.
 constexpr int kTcProducers = 256;
 constexpr int kTcEpiWarp = 8;
 constexpr int kTcEpilogue = 256;
@@ -137,30 +136,19 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {
 // Waits for the phase of the given parity to complete, for about a second at most, whether or
 // not another role has given up: the MMA thread's wait for its own MMAs in flight before the CTA
 // frees its tensor memory and leaves.
-// CL: acquire at cluster scope (a barrier that the peer CTA of a pair arrives on, or whose
-// phase orders work of the peer).
-template <bool CL>
 __device__ __forceinline__ uint32_t tc_try(uint32_t bar, uint32_t parity) {
   uint32_t done;
-  if constexpr (CL) {
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  } else {
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  }
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done;
 }
-template <bool CL = false>
 __device__ __forceinline__ bool tc_wait_own(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();
   uint32_t done = 0;
   while (!done) {
-    done = tc_try<CL>(bar, parity);
+    done = tc_try(bar, parity);
     if (!done && clock64() - t0 > (1ll << 31)) return false;
   }
   return true;
@@ -168,12 +156,11 @@ __device__ __forceinline__ bool tc_wait_own(uint32_t bar, uint32_t parity) {
 // Waits for the phase of the given parity to complete.  Gives up after about a second, or as
 // soon as another thread of the CTA has given up (*gave_up set), so that every role leaves its
 // loop instead of waiting on a partner that has left.
-template <bool CL = false>
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up) {
   const long long t0 = clock64();
   uint32_t done = 0;
   while (!done) {
-    done = tc_try<CL>(bar, parity);
+    done = tc_try(bar, parity);
     if (done) break;
     if (*gave_up) return false;
     if (clock64() - t0 > (1ll << 31)) {
@@ -192,16 +179,24 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// Arrives on a barrier of the pair's even CTA (the one whose thread issues the MMAs): through
-// its shared::cluster address, with release at cluster scope.  One CTA: a local arrive.
+// A warp's arrival, once for its 32 threads, on a barrier of the pair's even CTA (the one whose
+// thread issues the MMAs), through its shared::cluster address; one CTA: a local arrive.  The
+// default scope: what the arrival orders is shared memory that each CTA wrote itself and handed to
+// the async proxy (fence.proxy.async) or tensor memory that it has read (tcgen05 fence).  A release
+// at cluster scope waits for the thread's global accesses in flight, about 900 cycles, and had to be
+// kept off these paths by threads that forwarded each phase: 2M rows x 1024, 64M entries, 256
+// queries: 395 us so, 331 now.
 template <bool PAIR>
-__device__ __forceinline__ void tc_arrive_leader(uint32_t bar) {
-  if constexpr (PAIR) {
-    uint32_t ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(ra) : "r"(bar));
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(ra) : "memory");
-  } else {
-    tc_arrive(bar);
+__device__ __forceinline__ void tc_arrive_warp(uint32_t bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31u) == 0) {
+    if constexpr (PAIR) {
+      uint32_t ra;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(ra) : "r"(bar));
+      asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(ra) : "memory");
+    } else {
+      tc_arrive(bar);
+    }
   }
 }
 template <bool PAIR>
@@ -351,7 +346,7 @@ __device__ __forceinline__ float tc_limit(uint2 st, int centre, float E, float Q
 // The epilogue was the pass's longest stage: a block with a hit waited for the survivor counter's
 // atomic in device memory (over 1500 cycles; hits come in bursts, a long row passing for most of the
 // queries), and each score took three instructions.  With the queues and the fused compares
-// 2M rows x 1024, 64M entries: 748 -> 395 us for 256 queries, 375 -> 291 us for 128.
+// 2M rows x 1024, 64M entries, 256 queries: 748 -> 395 us (331 with tc_arrive_warp).
 template <bool PAIR>
 __device__ __forceinline__ void tc_epilogue(const TcArgs& a, uint32_t T, uint32_t tmem,
                                             uint32_t dbuf, const float* nthf_all, uint32_t S,
@@ -371,7 +366,7 @@ __device__ __forceinline__ void tc_epilogue(const TcArgs& a, uint32_t T, uint32_
     tc_ld32(tmem + dbuf * Q + col0 + ((g * 32u) << 16), v);
     if (col0 + 32u == h * HALF + HALF) {  // the last load of this unit has completed
       tc_fence_before();
-      tc_arrive(empty);
+      tc_arrive_warp<PAIR>(empty);
     }
     if (col0 >= a.nq) continue;
     float m[4];
@@ -562,14 +557,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
   }
   if (tid == 0) {
     for (uint32_t b = 0; b < kBars; b++) {
-      // The roles arrive on their own CTA's staged and empty barriers.  PAIR: a thread of the
-      // odd CTA forwards each completed phase of those to the even CTA's, which therefore take
-      // one arrival more (a release at cluster scope costs about a thousand cycles: forwarded,
-      // it stays off the producers' and the epilogue's paths)
-      const uint32_t fwd = (PAIR && rank == 0) ? 1u : 0u;
-      const uint32_t cnt = (b < kDone) ? (uint32_t)kTcProducers + fwd
-                           : ((b >= kEmpty && b < kDrain) ? (uint32_t)kTcEpilogue + fwd
-                           : ((b >= kQueued && b < kDrained) ? (uint32_t)kTcEpilogue : 1u));
+      // one arrival per warp; PAIR: both CTAs' producers and epilogues arrive on the even CTA's
+      // staged and empty barriers
+      const uint32_t both = PAIR ? 2u : 1u;
+      const uint32_t cnt = (b < kDone) ? both * kTcProducers / 32
+                           : ((b >= kEmpty && b < kDrain) ? both * kTcEpilogue / 32
+                           : ((b >= kQueued && b < kDrained) ? (uint32_t)kTcEpilogue / 32 : 1u));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(tc_smem_u32(bars + b)), "r"(cnt));
     }
     *gave_up = 0u;
@@ -626,7 +619,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
     auto step = [&](uint32_t i, TcEnt& cur, TcEnt& old, uint32_t& pb, uint32_t& pe) -> bool {
       unsigned char* ab = sa + buf * kTcChunkBytes;
       if (i >= NB) {  // the MMAs of chunk i - NB have read this buffer: clear its entries
-        ok &= tc_wait<PAIR>(b_done + 8u * buf, ((i - NB) / NB) & 1u, gave_up);
+        ok &= tc_wait(b_done + 8u * buf, ((i - NB) / NB) & 1u, gave_up);
         if (ok) old.stage(ab, a.ent, tid, true);
       }
       // every clear lands before any write of this chunk (they may share a byte); the
@@ -636,7 +629,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
       ptr_next(pb, pe);                   // chunk i + R + 2
       cur.stage(ab, a.ent, tid, false);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      tc_arrive(b_staged + 8u * buf);
+      tc_arrive_warp<PAIR>(b_staged + 8u * buf);
       buf = buf + 1 == NB ? 0u : buf + 1;
       return true;
     };
@@ -648,6 +641,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
         go = step(i0 + k, E[k], E[(k + 2) % R], Pb[(k + 2) % R], Pe[(k + 2) % R]);
         if (!go) break;
       }
+    }
+    // the odd CTA: before it leaves, the even CTA's commits for its last chunk buffers have landed
+    // (those before them were waited for above, those of the accumulators by the epilogue)
+    if (PAIR && rank == 1 && tid == 0 && go) {
+      bool landed = true;
+      for (uint32_t j = min(NB, total); j >= 1 && landed && !*gave_up; j--)
+        landed = tc_wait_own(b_done + 8u * ((total - j) % NB), ((total - j) / NB) & 1u);
+      if (!landed) *gave_up = 1u;
     }
   } else if (warp < kTcEpiWarp + kTcEpilogue / 32) {
     // ---- epilogue -----------------------------------------------------------------------------
@@ -663,14 +664,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
       const float rs = a.rowscale ? (row < a.n_rows ? __ldg(a.rowscale + row) : 0.0f) : 1.0f;
       const uint2 st = a.rowstat && row < a.n_rows ? __ldg(a.rowstat + row) : make_uint2(0u, 0u);
       const float lim = a.rowstat ? tc_limit(st, centre, qE, qQ, rs) : 0.0f;
-      if (ok) ok &= tc_wait<PAIR>(b_full + 8u * d, (tl / ACC) & 1u, gave_up);
+      if (ok) ok &= tc_wait(b_full + 8u * d, (tl / ACC) & 1u, gave_up);
       ok = __all_sync(0xFFFFFFFFu, ok);  // tcgen05.ld needs the whole warp
       if (!ok) break;
       tc_fence_after();
       tc_epilogue<PAIR>(a, T, tmem, d, thf, S, rs, lim, b_empty + 8u * d,
                         a.rowstat ? TcQueue{hq_e, hq_n, a.queue_cap}
                                   : TcQueue{hq_e + (size_t)hb * a.queue_cap, hq_n + hb, a.queue_cap});
-      if (!a.rowstat) tc_arrive(b_queued + 8u * hb);
+      if (!a.rowstat) tc_arrive_warp<false>(b_queued + 8u * hb);
     }
   } else if (warp >= kTcDrainWarp) {
     // ---- drain: appends the queued hits of every third unit, four per lane at a time -----------
@@ -698,8 +699,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
     uint32_t tl = 0, c = 0, issued = 0;
     for (uint32_t i = 0; i < total && !a.mma_idle; i++) {
       const uint32_t buf = i % NB, d = tl % ACC;
-      if (c == 0 && tl >= ACC) ok &= tc_wait<PAIR>(b_empty + 8u * d, ((tl - ACC) / ACC) & 1u, gave_up);
-      if (ok) ok &= tc_wait<PAIR>(b_staged + 8u * buf, (i / NB) & 1u, gave_up);
+      if (c == 0 && tl >= ACC) ok &= tc_wait(b_empty + 8u * d, ((tl - ACC) / ACC) & 1u, gave_up);
+      if (ok) ok &= tc_wait(b_staged + 8u * buf, (i / NB) & 1u, gave_up);
       if (!ok) break;
       tc_fence_after();
       const uint32_t nk = min(kTcChunkK, a.kpad - c * kTcChunkK) / 32u;
@@ -721,38 +722,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
     if (issued >= 1) {
       bool drained = true;
       for (uint32_t j = 1; j <= NB && j <= issued; j++)  // the last use of each chunk buffer
-        drained &= tc_wait_own<PAIR>(b_done + 8u * ((issued - j) % NB), ((issued - j) / NB) & 1u);
+        drained &= tc_wait_own(b_done + 8u * ((issued - j) % NB), ((issued - j) / NB) & 1u);
       const uint32_t tiles_full = issued / a.nch;  // units whose accumulator commit was issued
       for (uint32_t j = 1; j <= ACC && j <= tiles_full; j++)  // the last use of each accumulator
-        drained &= tc_wait_own<PAIR>(b_full + 8u * ((tiles_full - j) % ACC), ((tiles_full - j) / ACC) & 1u);
+        drained &= tc_wait_own(b_full + 8u * ((tiles_full - j) % ACC), ((tiles_full - j) / ACC) & 1u);
       tc_commit<PAIR>(tc_smem_u32(bars + kDrain), 1);
-      drained &= tc_wait_own<PAIR>(tc_smem_u32(bars + kDrain), 0u);
+      drained &= tc_wait_own(tc_smem_u32(bars + kDrain), 0u);
       if (!drained) *gave_up = 1u;
     }
-  } else if (PAIR && rank == 1 && (tid & 31u) == 1) {
-    // ---- the odd CTA: forwards each completed phase of its empty barriers (its epilogue has
-    // read the accumulator) to the even CTA's
-    for (uint32_t tl = 0; tl < ntl; tl++) {
-      const uint32_t d = tl % ACC;
-      if (!tc_wait(b_empty + 8u * d, (tl / ACC) & 1u, gave_up)) break;
-      tc_arrive_leader<PAIR>(b_empty + 8u * d);
-    }
-  } else if (PAIR && rank == 1 && (tid & 31u) == 0) {
-    // ---- the odd CTA: forwards each completed phase of its staged barriers (its producers have
-    // staged the chunk) to the even CTA's
-    for (uint32_t i = 0; i < total; i++) {
-      const uint32_t buf = i % NB;
-      if (!tc_wait(b_staged + 8u * buf, (i / NB) & 1u, gave_up)) break;
-      tc_arrive_leader<PAIR>(b_staged + 8u * buf);
-    }
-    // before the CTA leaves, the even CTA's commits to its barriers have landed (the last use of
-    // each chunk buffer and accumulator; skipped once it gave up)
-    bool drained = true;
-    for (uint32_t j = 1; j <= NB && j <= total && drained && !*gave_up; j++)
-      drained = tc_wait_own<PAIR>(b_done + 8u * ((total - j) % NB), ((total - j) / NB) & 1u);
-    for (uint32_t j = 1; j <= ACC && j <= ntl && drained && !*gave_up; j++)
-      drained = tc_wait_own<PAIR>(b_full + 8u * ((ntl - j) % ACC), ((ntl - j) / ACC) & 1u);
-    if (!drained) *gave_up = 1u;
   }
   tc_fence_before();
   __syncthreads();
