@@ -465,7 +465,7 @@ int Engine::run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair) {
   if (pair) {  // clusters of two CTAs: a pair per two SMs
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)tc_grid2);
-    cfg.blockDim = dim3(kTcThreads);
+    cfg.blockDim = dim3(TcShape<true>::THREADS);
     cfg.dynamicSmemBytes = tc_smem2;
     cfg.stream = s;
     cudaLaunchAttribute at[2];
@@ -480,9 +480,9 @@ int Engine::run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair) {
     AES_CK(tc_nb2 == 3 ? cudaLaunchKernelEx(&cfg, k_cand_tc<3, true>, a)
                        : cudaLaunchKernelEx(&cfg, k_cand_tc<2, true>, a));
   } else if (tc_nb == 3) {
-    AES_CK(chain(k_cand_tc<3, false>, tc_grid, kTcThreads, tc_smem, s, a));
+    AES_CK(chain(k_cand_tc<3, false>, tc_grid, TcShape<false>::THREADS, tc_smem, s, a));
   } else {
-    AES_CK(chain(k_cand_tc<2, false>, tc_grid, kTcThreads, tc_smem, s, a));
+    AES_CK(chain(k_cand_tc<2, false>, tc_grid, TcShape<false>::THREADS, tc_smem, s, a));
   }
   AES_CK(cudaGetLastError());
   if (prof && (rc = prof_close(s))) return rc;
@@ -746,7 +746,7 @@ int Engine::apply_config(const Config& c) {
       tc_grid2 = 2 * (int)pairs;
       cudaLaunchConfig_t cfg{};
       cfg.gridDim = dim3((unsigned)tc_grid2);
-      cfg.blockDim = dim3(kTcThreads);
+      cfg.blockDim = dim3(TcShape<true>::THREADS);
       cfg.dynamicSmemBytes = tc_smem2;
       cudaLaunchAttribute at[1];
       at[0].id = cudaLaunchAttributeClusterDimension;

@@ -19,7 +19,7 @@
 //   - epilogue warps read a complete accumulator with tcgen05.ld while the next tiles' MMAs run and
 //     compare every (row, query) score with the query's threshold; a hit goes into the CTA's queue
 //     (device memory, in practice L2);
-//   - three warps drain the queues, appending the hits to the queries' survivors as the same
+//   - two warps drain the queues, appending the hits to the queries' survivors as the same
 //     candidate keys as in the other passes, so that no epilogue warp waits on an atomic's round trip.
 // Two blocks of 128 queries run together on CTA pairs (cta_group::2, M = 256 over the pair's two
 // row tiles, N = 256 queries): the same roles in each CTA, the even CTA's thread issuing the MMAs
@@ -36,17 +36,17 @@
 namespace aes {
 namespace dev {
 
-// Warp roles: warps 0-7 stage the chunks (producers), warps 8-15 read the accumulators (warp w
-// may only read tensor-memory lanes 32 (w % 4) .. + 31; warps 8-11 take the first half of the
-// queries, warps 12-15 the second), warp 16 allocates tensor memory and its lane 0 issues the
-// MMAs (on a pair: the even CTA's), warps 17 to 19 append the hits.  They hand work over through mbarriers only.
-constexpr int kTcProducers = 256;
-constexpr int kTcEpiWarp = 8;
-constexpr int kTcEpilogue = 256;
-constexpr int kTcMmaWarp = 16;
-constexpr int kTcDrainWarp = 17;  // and the two after it: unit t's hits are appended by 17 + t % 3
-constexpr uint32_t kTcDrains = 3;
-constexpr int kTcThreads = (17 + kTcDrains) * 32;
+// Warp roles: warps 0-8 stage the chunks (producers, a group of three or four warps per chunk
+// buffer), one thread of warp 9 issues the MMAs (on a pair: the even CTA's; the warp also allocates
+// tensor memory), warps 10 and 11 append the hits, the warps from 12 on read the accumulators (warp w
+// may only read tensor-memory lanes 32 (w % 4) .. + 31; each four warps take a share of the queries).
+// They hand work over through mbarriers only.
+constexpr int kTcMmaWarp = 9;
+constexpr int kTcDrainWarp = 10;  // and the one after it: unit t's hits are appended by 10 + t % 2
+constexpr uint32_t kTcDrains = 2;
+constexpr int kTcEpiWarp = 12;
+// producers of a chunk buffer, with nb buffers
+__host__ __device__ constexpr uint32_t tc_group(uint32_t nb) { return nb == 3 ? 96u : 128u; }
 constexpr uint32_t kTcTmemCols = 512;  // all of tensor memory, in FP32 accumulators
 // Queries per launch and accumulators.  One CTA: 128 queries (N = 128, M = 128), four
 // accumulators of 128 columns.  A CTA pair (cta_group::2): 256 queries (N = 256, each CTA
@@ -56,6 +56,11 @@ template <bool PAIR>
 struct TcShape {
   static constexpr uint32_t Q = PAIR ? 2 * kTcQ : kTcQ;
   static constexpr uint32_t ACC = kTcTmemCols / Q;
+  // epilogue threads, 32 or 64 queries each: a warp's reads of an accumulator are a chain of
+  // latencies, and a pair's two accumulators leave little time for it (2M rows x 1024, 64M entries,
+  // 256 queries: 286 us with 8 warps, 278 with 16; 128 queries on one CTA: 203 and 215)
+  static constexpr uint32_t EPI = PAIR ? 512 : 256;
+  static constexpr uint32_t THREADS = kTcEpiWarp * 32 + EPI;
 };
 // mbarriers of a kernel with nb chunk buffers and acc accumulators: staged[nb] (producers ->
 // MMA), done[nb] (MMA -> producers), full[acc] (MMA -> epilogue), empty[acc] (epilogue -> MMA),
@@ -214,6 +219,12 @@ __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t da, uint64_t db, uin
         :: "r"(d), "l"(da), "l"(db), "r"(idesc), "r"(acc));
   }
 }
+// one thread of the warp, the same each time
+__device__ __forceinline__ bool tc_elect() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
+}
 // Arrives on `bar` once the MMAs issued so far complete.  PAIR: on the barrier at the same
 // offset in each CTA of ctamask (bit r: the pair's CTA of rank r).
 template <bool PAIR>
@@ -251,16 +262,14 @@ __device__ __forceinline__ void tc_dealloc(uint32_t tmem) {
 __device__ __forceinline__ void tc_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// 32 consecutive accumulator columns of this warp's 32 lanes (one row per thread)
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+// 16 consecutive accumulator columns of this warp's 32 lanes (one row per thread)
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
-      "%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
+      "%15}, [%16];"
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
         "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
-        "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
-        "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        "=r"(v[14]), "=r"(v[15])
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -303,6 +312,19 @@ struct TcQueue {
 __device__ __forceinline__ uint32_t tc_epi_row(uint32_t T) {
   return T * kTcRows + ((threadIdx.x >> 5) & 3u) * 32u + (threadIdx.x & 31u);
 }
+__device__ __forceinline__ float4 tc_lds4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+// The row's scale and sums on their way to L1 while its unit before is read, at no register: loaded
+// when they are needed, they held an epilogue warp for 1000 of a unit's 5500 cycles (4M rows x 1024 at
+// 8 bits, 512 queries, the whole call: 1726 -> 1674 us).
+__device__ __forceinline__ void tc_prefetch(const TcArgs& a, uint32_t row) {
+  if (row >= a.n_rows) return;
+  if (a.rowscale) asm volatile("prefetch.global.L1 [%0];" :: "l"(a.rowscale + row));
+  if (a.rowstat) asm volatile("prefetch.global.L1 [%0];" :: "l"(a.rowstat + row));
+}
 // two FP32 fused multiply-adds per instruction
 __device__ __forceinline__ void tc_fma2(float& x0, float& x1, float a0, float a1, float b, float c0,
                                         float c1) {
@@ -312,9 +334,8 @@ __device__ __forceinline__ void tc_fma2(float& x0, float& x1, float a0, float a1
 }
 // x[j] = score j times rs minus its bound (nthf: negated bounds, the same for every lane: 16-byte
 // broadcasts)
-__device__ __forceinline__ void tc_margin8(float (&x)[8], const uint32_t* v, float rs, const float* nthf) {
-  const float4 t0 = reinterpret_cast<const float4*>(nthf)[0];
-  const float4 t1 = reinterpret_cast<const float4*>(nthf)[1];
+__device__ __forceinline__ void tc_margin8(float (&x)[8], const uint32_t* v, float rs, float4 t0,
+                                           float4 t1) {
   tc_fma2(x[0], x[1], __uint_as_float(v[0]), __uint_as_float(v[1]), rs, t0.x, t0.y);
   tc_fma2(x[2], x[3], __uint_as_float(v[2]), __uint_as_float(v[3]), rs, t0.z, t0.w);
   tc_fma2(x[4], x[5], __uint_as_float(v[4]), __uint_as_float(v[5]), rs, t1.x, t1.y);
@@ -339,117 +360,133 @@ __device__ __forceinline__ float tc_limit(uint2 st, int centre, float E, float Q
 // queues every (row, query) score at or above the query's bound.  nthf holds the negated bounds on
 // rs * score (rs is the row's scale, or 1 without row scales, where the score is an exact integer),
 // so a score passes where fma(score, rs, -bound) >= lim (0, or what an approximate score of the row
-// may fall short by).  A block of 32 queries costs a fused
+// may fall short by).  A block of 16 queries costs a fused
 // multiply-add per two scores and the maximum of each group of eight (three-operand maxima); only
 // groups that reach 0 are looked at again, and take their queue slots with one atomic per block.  The accumulator goes back to the MMA role (an
 // arrive on `empty`) as soon as the thread's last load from it has completed.
 // The epilogue was the pass's longest stage: a block with a hit waited for the survivor counter's
 // atomic in device memory (over 1500 cycles; hits come in bursts, a long row passing for most of the
 // queries), and each score took three instructions.  With the queues and the fused compares
-// 2M rows x 1024, 64M entries, 256 queries: 748 -> 395 us (331 with tc_arrive_warp).
+// 2M rows x 1024, 64M entries, 256 queries: 748 -> 395 us (278 with the steps since).
 template <bool PAIR>
 __device__ __forceinline__ void tc_epilogue(const TcArgs& a, uint32_t T, uint32_t tmem,
                                             uint32_t dbuf, const float* nthf_all, uint32_t S,
                                             float rs, float lim, uint32_t empty,
                                             const TcQueue& hq) {
-  constexpr uint32_t Q = TcShape<PAIR>::Q, HALF = Q / 2;
+  constexpr uint32_t Q = TcShape<PAIR>::Q, PART = Q / (TcShape<PAIR>::EPI / 128);
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t g = warp & 3u, h = (warp - kTcEpiWarp) >> 2;
   const uint32_t row = tc_epi_row(T);
   const bool valid = row < a.n_rows;
   const uint32_t p = valid ? part_of(row, S, a.slice) : 0u;
-  const float* nthf = nthf_all + p * Q;
+  const uint32_t thaddr = tc_smem_u32(nthf_all + p * Q);
+  uint32_t mask = 0;  // a filter: hits of the block of 32 queries
 #pragma unroll 1
-  for (uint32_t col0 = h * HALF; col0 < h * HALF + HALF; col0 += 32u) {
-    uint32_t v[32];
+  for (uint32_t col0 = h * PART; col0 < h * PART + PART; col0 += 16u) {
+    uint32_t v[16];
+    float4 nt[4];  // read before the accumulator: both latencies pass together
+#pragma unroll
+    for (int j = 0; j < 4; j++) nt[j] = tc_lds4(thaddr + (col0 + 4u * j) * 4u);
     __syncwarp();  // tcgen05.ld needs the warp together again after a block with hits
-    tc_ld32(tmem + dbuf * Q + col0 + ((g * 32u) << 16), v);
-    if (col0 + 32u == h * HALF + HALF) {  // the last load of this unit has completed
+    tc_ld16(tmem + dbuf * Q + col0 + ((g * 32u) << 16), v);
+    if (col0 + 16u == h * PART + PART) {  // the last load of this unit has completed
       tc_fence_before();
       tc_arrive_warp<PAIR>(empty);
     }
-    if (col0 >= a.nq) continue;
-    float m[4];
+    float m[2];
 #pragma unroll
-    for (int j8 = 0; j8 < 4; j8++) {
+    for (int j8 = 0; j8 < 2; j8++) {
       float x[8];
-      tc_margin8(x, v + 8 * j8, rs, nthf + col0 + 8 * j8);
+      tc_margin8(x, v + 8 * j8, rs, nt[2 * j8], nt[2 * j8 + 1]);
       const float m0 = fmaxf(fmaxf(x[0], x[1]), x[2]), m1 = fmaxf(fmaxf(x[3], x[4]), x[5]);
       m[j8] = fmaxf(fmaxf(m0, m1), fmaxf(x[6], x[7]));
     }
-    if (fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])) >= lim && valid) {
+    if (fmaxf(m[0], m[1]) >= lim && valid && col0 < a.nq) {
       uint32_t hit = 0;
 #pragma unroll
-      for (int j8 = 0; j8 < 4; j8++) {
+      for (int j8 = 0; j8 < 2; j8++) {
         if (m[j8] >= lim) {
           float x[8];
-          tc_margin8(x, v + 8 * j8, rs, nthf + col0 + 8 * j8);
+          tc_margin8(x, v + 8 * j8, rs, nt[2 * j8], nt[2 * j8 + 1]);
 #pragma unroll
           for (int j = 0; j < 8; j++) hit |= (x[j] >= lim ? 1u : 0u) << (8 * j8 + j);
         }
       }
       if (a.rowstat) {
-        const uint32_t l = col0 / 32u, k = atomicAdd(hq.n + l, 1u);
-        if (k < hq.cap) hq.e[(size_t)l * hq.cap + k] = make_uint2(row, hit);
-        continue;
-      }
-      const uint32_t nh = __popc(hit);
-      uint32_t i = atomicAdd(hq.n, nh);
-      const uint32_t meta = col0 | (row % kTcRows) << 8;
-      if (i + nh <= hq.cap) {
-#pragma unroll
-        for (int j = 0; j < 32; j++)
-          if ((hit >> j) & 1u) hq.e[i++] = make_uint2(meta + j, v[j]);
+        mask |= hit << (col0 & 16u);
       } else {
-        for (; i < hq.cap; i++) hq.e[i] = make_uint2(kTcNoHit, 0u);
-        const size_t qp = (size_t)(a.q0 + col0) * S + p;
+        const uint32_t nh = __popc(hit);
+        uint32_t i = atomicAdd(hq.n, nh);
+        const uint32_t meta = col0 | (row % kTcRows) << 8;
+        if (i + nh <= hq.cap) {
 #pragma unroll
-        for (int j8 = 0; j8 < 4; j8++)
-          if ((hit >> (8 * j8)) & 255u)
-            tc_append<8>(a, S, qp + (size_t)(8 * j8) * S, row, v + 8 * j8, hit >> (8 * j8),
-                         a.rowscale ? rs : -1.0f);
+          for (int j = 0; j < 16; j++)
+            if ((hit >> j) & 1u) hq.e[i++] = make_uint2(meta + j, v[j]);
+        } else {
+          for (; i < hq.cap; i++) hq.e[i] = make_uint2(kTcNoHit, 0u);
+          const size_t qp = (size_t)(a.q0 + col0) * S + p;
+#pragma unroll
+          for (int j8 = 0; j8 < 2; j8++)
+            if ((hit >> (8 * j8)) & 255u)
+              tc_append<8>(a, S, qp + (size_t)(8 * j8) * S, row, v + 8 * j8, hit >> (8 * j8),
+                           a.rowscale ? rs : -1.0f);
+        }
       }
+    }
+    if (mask && (col0 & 16u)) {
+      const uint32_t l = col0 / 32u, k = atomicAdd(hq.n + l, 1u);
+      if (k < hq.cap) hq.e[(size_t)l * hq.cap + k] = make_uint2(row, mask);
+      mask = 0;
     }
   }
 }
 
-constexpr int kTcPer = 8;  // entries of a chunk a producer thread holds (2048 per chunk)
+constexpr int kTcPer = 12;  // entries of a chunk a producer thread holds (1536 per chunk or more)
 
-// A producer's share of one chunk's entries: v[u] = entry b + tid + 256 u for tid + 256 u < n
+// A producer's share of one chunk's entries, G threads to a chunk: v[u] = entry b + t + G u for
+// t + G u < n
+template <uint32_t G>
 struct TcEnt {
   uint32_t v[kTcPer];
   uint32_t b = 0, n = 0;
-  __device__ __forceinline__ void load(const uint32_t* ent, uint32_t b_, uint32_t n_, uint32_t tid) {
+  __device__ __forceinline__ void load(const uint32_t* ent, uint32_t b_, uint32_t n_, uint32_t t) {
     b = b_;
     n = n_;
 #pragma unroll
-    for (int u = 0; u < kTcPer; u++) {
-      const uint32_t i = tid + (uint32_t)u * kTcProducers;
-      v[u] = i < n ? __ldg(ent + b + i) : 0u;
+    for (int u0 = 0; u0 < kTcPer; u0 += 4) {
+      if (u0 * G >= n) break;  // the whole group's
+#pragma unroll
+      for (int u = u0; u < u0 + 4; u++) {
+        const uint32_t i = t + (uint32_t)u * G;
+        v[u] = i < n ? __ldg(ent + b + i) : 0u;
+      }
     }
   }
   // writes the entries' e4m3 bytes (or zeros) into a chunk buffer
-  __device__ __forceinline__ void stage(unsigned char* ab, const uint32_t* ent, uint32_t tid,
+  __device__ __forceinline__ void stage(unsigned char* ab, const uint32_t* ent, uint32_t t,
                                         bool clear) const {
 #pragma unroll
-    for (int u = 0; u < kTcPer; u++) {
-      const uint32_t i = tid + (uint32_t)u * kTcProducers;
-      if (i < n) ab[v[u] >> 16] = clear ? (uint8_t)0 : (uint8_t)v[u];
+    for (int u0 = 0; u0 < kTcPer; u0 += 4) {
+      if (u0 * G >= n) break;
+#pragma unroll
+      for (int u = u0; u < u0 + 4; u++)
+        if (t + (uint32_t)u * G < n) ab[v[u] >> 16] = clear ? (uint8_t)0 : (uint8_t)v[u];
     }
-    for (uint32_t i = tid + kTcPer * kTcProducers; i < n; i += kTcProducers) {
+    for (uint32_t i = t + kTcPer * G; i < n; i += G) {
       const uint32_t e = __ldg(ent + b + i);
       ab[e >> 16] = clear ? (uint8_t)0 : (uint8_t)e;
     }
   }
 };
 
-// OR of `fail` over the producer threads (named barrier 1)
-__device__ __forceinline__ bool tc_producers_any(bool fail) {
+// OR of `fail` over the G threads of a producer group (named barrier 1 + grp)
+template <uint32_t G>
+__device__ __forceinline__ bool tc_group_any(uint32_t grp, bool fail) {
   uint32_t r;
   asm volatile(
-      "{\n .reg .pred f, r;\n setp.ne.u32 f, %1, 0;\n bar.red.or.pred r, 1, %2, f;\n"
+      "{\n .reg .pred f, r;\n setp.ne.u32 f, %1, 0;\n bar.red.or.pred r, %3, %2, f;\n"
       " selp.u32 %0, 1, 0, r;\n}\n"
-      : "=r"(r) : "r"((uint32_t)fail), "n"(kTcProducers) : "memory");
+      : "=r"(r) : "r"((uint32_t)fail), "n"(G), "r"(1u + grp) : "memory");
   return r != 0;
 }
 
@@ -498,14 +535,14 @@ __device__ __forceinline__ void tc_drain_scores(const TcArgs& a, uint32_t S, con
 // accumulators back to the even CTA's barriers.  The two CTAs keep identical shared-memory
 // layouts, since an operand descriptor addresses the same offset in both.
 template <uint32_t NB, bool PAIR>
-__global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
+__global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a) {
   grid_wait();
   static_assert(NB == 2 || NB == 3, "two or three chunk buffers");
   constexpr uint32_t Q = TcShape<PAIR>::Q, ACC = TcShape<PAIR>::ACC;
   constexpr uint32_t kDone = NB, kFull = 2 * NB, kEmpty = 2 * NB + ACC;
   constexpr uint32_t kDrain = kEmpty + ACC, kQueued = kDrain + 1, kDrained = kQueued + kTcQueues;
   constexpr uint32_t kBars = tc_nbars(NB, ACC);
-  constexpr uint32_t R = NB + 2;  // producer ring: the chunks of every buffer and two ahead
+  constexpr uint32_t G = tc_group(NB);  // producers of a chunk buffer
   extern __shared__ __align__(16) unsigned char smem[];
   const uint32_t qbytes = (a.kpad / 16u) * 2048u;
   unsigned char* sq = smem;                     // query operand (PAIR: this CTA's 128 queries)
@@ -560,9 +597,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
       // one arrival per warp; PAIR: both CTAs' producers and epilogues arrive on the even CTA's
       // staged and empty barriers
       const uint32_t both = PAIR ? 2u : 1u;
-      const uint32_t cnt = (b < kDone) ? both * kTcProducers / 32
-                           : ((b >= kEmpty && b < kDrain) ? both * kTcEpilogue / 32
-                           : ((b >= kQueued && b < kDrained) ? (uint32_t)kTcEpilogue / 32 : 1u));
+      const uint32_t cnt = (b < kDone) ? both * G / 32
+                           : ((b >= kEmpty && b < kDrain) ? both * TcShape<PAIR>::EPI / 32
+                           : ((b >= kQueued && b < kDrained) ? TcShape<PAIR>::EPI / 32 : 1u));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(tc_smem_u32(bars + b)), "r"(cnt));
     }
     *gave_up = 0u;
@@ -582,75 +619,64 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
   const uint32_t total = ntl * a.nch;  // chunks of this CTA (PAIR: the same in both CTAs)
   bool ok = true;
 
-  if (warp < kTcProducers / 32) {
+  if (warp < NB * G / 32u) {
     // ---- producers ----------------------------------------------------------------------------
-    // Chunk i lives in ring set E[i % R], R = NB + 2 (indices fixed at compile time: the loop
-    // below is unrolled R ways).  Step i clears chunk i - NB, the last chunk of buffer i % NB,
-    // from E[(i + 2) % R], loads chunk i + 2 into that set and stages chunk i (loaded two steps
-    // earlier); a chunk's row offsets are read R steps before its entries.  So no register a
-    // store or a copy reads waits on a load in flight.
-    // chunk id of chunk i: tile tile_of(unit + (i / nch) units), chunk i % nch; kept
-    // incrementally for the look-ahead chunk (no division per step).  PAIR: the odd CTA's tile
-    // of the last unit may lie past the matrix; its chunks are empty.
-    uint32_t la_i = 0, la_t = tile_of(unit), la_c = 0;
-    auto ptr_next = [&](uint32_t& b, uint32_t& e) {  // offsets of chunk la_i, then advance it
+    // A group of G threads per chunk buffer: group g takes chunks g, g + NB, ...  Its step clears the
+    // buffer's last chunk once the MMAs have read it, stages the next one, whose entries were loaded a
+    // step earlier, and loads the one after.  A step is a chain of latencies (the wait, the
+    // clears, the group's barrier, the stores, the proxy fence: about 1300 cycles, more than a
+    // chunk's MMAs), so the groups' steps overlap; the loads come after the hand-over, since the
+    // stores would wait for them too.  One group of eight warps for all buffers: 318 us where this
+    // takes 290 (2M rows x 1024, 64M entries, 256 queries), 283 and 203 for 128.
+    const uint32_t grp = warp / (G / 32u), t = tid - grp * G;
+    unsigned char* const ab = sa + grp * kTcChunkBytes;
+    // PAIR: the odd CTA's tile of the last unit may lie past the matrix; its chunks are empty
+    uint32_t la_i = grp, la_t = tile_of(unit), la_c = grp;
+    auto ptr_next = [&](uint32_t& b, uint32_t& e) {  // offsets of chunk la_i, then on to la_i + NB
+      while (la_c >= a.nch) {
+        la_c -= a.nch;
+        la_t += PAIR ? 2u : 1u;
+      }
       const bool in = la_i < total && la_t < a.n_rtiles;
       const uint32_t j = la_t * a.nch + la_c;
       b = in ? __ldg(a.ptr + j) : 0u;
       e = in ? __ldg(a.ptr + j + 1) : 0u;
-      la_i++;
-      if (++la_c == a.nch) {
-        la_c = 0;
-        la_t += PAIR ? 2u : 1u;
-      }
+      la_i += NB;
+      la_c += NB;
     };
-    TcEnt E[R];
-    uint32_t Pb[R], Pe[R];  // P[j % R]: row offsets of chunk j, for j = i + 2 .. i + R + 1
-    {
-      uint32_t b, e;
-      ptr_next(b, e);
-      E[0].load(a.ent, b, e - b, tid);
-      ptr_next(b, e);
-      E[1].load(a.ent, b, e - b, tid);
-#pragma unroll
-      for (uint32_t j = 2; j < R + 2; j++) ptr_next(Pb[j % R], Pe[j % R]);
-    }
-    uint32_t buf = 0;  // i % NB
-    auto step = [&](uint32_t i, TcEnt& cur, TcEnt& old, uint32_t& pb, uint32_t& pe) -> bool {
-      unsigned char* ab = sa + buf * kTcChunkBytes;
-      if (i >= NB) {  // the MMAs of chunk i - NB have read this buffer: clear its entries
-        ok &= tc_wait(b_done + 8u * buf, ((i - NB) / NB) & 1u, gave_up);
-        if (ok) old.stage(ab, a.ent, tid, true);
+    TcEnt<G> E0, E1;
+    uint32_t pb, pe;
+    ptr_next(pb, pe);
+    E0.load(a.ent, pb, pe - pb, t);
+    ptr_next(pb, pe);
+    uint32_t j = 0;  // steps done: uses of the buffer
+    auto step = [&](TcEnt<G>& cur, TcEnt<G>& old) -> bool {
+      if (j > 0) {
+        ok &= tc_wait(b_done + 8u * grp, (j - 1u) & 1u, gave_up);
+        if (ok) old.stage(ab, a.ent, t, true);
       }
-      // every clear lands before any write of this chunk (they may share a byte); the
-      // producers leave together at the first failure
-      if (tc_producers_any(!ok)) return false;
-      old.load(a.ent, pb, pe - pb, tid);  // chunk i + 2
-      ptr_next(pb, pe);                   // chunk i + R + 2
-      cur.stage(ab, a.ent, tid, false);
+      // every clear lands before any write of this chunk (they may share a byte); the group's
+      // threads leave together at the first failure
+      if (tc_group_any<G>(grp, !ok)) return false;
+      cur.stage(ab, a.ent, t, false);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      tc_arrive_warp<PAIR>(b_staged + 8u * buf);
-      buf = buf + 1 == NB ? 0u : buf + 1;
+      tc_arrive_warp<PAIR>(b_staged + 8u * grp);
+      old.load(a.ent, pb, pe - pb, t);
+      ptr_next(pb, pe);
+      j++;
       return true;
     };
     bool go = true;
-    for (uint32_t i0 = 0; go && i0 < total; i0 += R) {
-#pragma unroll
-      for (uint32_t k = 0; k < R; k++) {
-        if (i0 + k >= total) break;
-        go = step(i0 + k, E[k], E[(k + 2) % R], Pb[(k + 2) % R], Pe[(k + 2) % R]);
-        if (!go) break;
-      }
+    for (uint32_t i = grp; go && i < total; i += 2u * NB) {
+      go = step(E0, E1);
+      if (go && i + NB < total) go = step(E1, E0);
     }
     // the odd CTA: before it leaves, the even CTA's commits for its last chunk buffers have landed
     // (those before them were waited for above, those of the accumulators by the epilogue)
-    if (PAIR && rank == 1 && tid == 0 && go) {
-      bool landed = true;
-      for (uint32_t j = min(NB, total); j >= 1 && landed && !*gave_up; j--)
-        landed = tc_wait_own(b_done + 8u * ((total - j) % NB), ((total - j) / NB) & 1u);
-      if (!landed) *gave_up = 1u;
+    if (PAIR && rank == 1 && t == 0 && go && j > 0) {
+      if (!tc_wait_own(b_done + 8u * grp, (j - 1u) & 1u)) *gave_up = 1u;
     }
-  } else if (warp < kTcEpiWarp + kTcEpilogue / 32) {
+  } else if (warp >= kTcEpiWarp) {
     // ---- epilogue -----------------------------------------------------------------------------
     const int centre = a.rowstat ? tc_centre(a.qstat) : 0;
     const float qE = a.rowstat ? (float)a.qstat[2] : 0.0f, qQ = a.rowstat ? (float)a.qstat[3] : 0.0f;
@@ -663,6 +689,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
       // without row scales rs = 1: f * 1 is f exactly, so every score takes one path
       const float rs = a.rowscale ? (row < a.n_rows ? __ldg(a.rowscale + row) : 0.0f) : 1.0f;
       const uint2 st = a.rowstat && row < a.n_rows ? __ldg(a.rowstat + row) : make_uint2(0u, 0u);
+      tc_prefetch(a, tc_epi_row(tile_of(unit + tl + 1u)));
       const float lim = a.rowstat ? tc_limit(st, centre, qE, qQ, rs) : 0.0f;
       if (ok) ok &= tc_wait(b_full + 8u * d, (tl / ACC) & 1u, gave_up);
       ok = __all_sync(0xFFFFFFFFu, ok);  // tcgen05.ld needs the whole warp
@@ -673,7 +700,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
                                   : TcQueue{hq_e + (size_t)hb * a.queue_cap, hq_n + hb, a.queue_cap});
       if (!a.rowstat) tc_arrive_warp<false>(b_queued + 8u * hb);
     }
-  } else if (warp >= kTcDrainWarp) {
+  } else if (warp >= kTcDrainWarp && warp < kTcDrainWarp + kTcDrains) {
     // ---- drain: appends the queued hits of every third unit, four per lane at a time -----------
     const uint32_t lane = tid & 31u;
     for (uint32_t tl = warp - kTcDrainWarp; tl < ntl && !a.rowstat; tl += kTcDrains) {
@@ -689,26 +716,35 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
         tc_arrive(b_drained + 8u * b);
       }
     }
-  } else if ((tid & 31u) == 0 && rank == 0) {
-    // ---- MMA issue (one thread; PAIR: of the even CTA) ----------------------------------------
+  } else if (warp == kTcMmaWarp && rank == 0) {
+    // ---- MMA issue (one thread of the warp; PAIR: of the even CTA) -----------------------------
+    // The warp keeps together but for the issue itself, so that descriptors and addresses are uniform
+    // values; a chunk's eight MMAs differ by constants.  Issued from a thread on its own, with the
+    // descriptors built for each, an MMA took 122 cycles to issue (now 53), twice what one of 128
+    // queries takes to run.
     // instruction descriptor: FP32 accumulator, e4m3 x e4m3, both K-major, N = Q (one CTA: no more
     // than the queries need), M = 128 (256 over a pair)
     const uint32_t n = PAIR ? Q : (min(a.nq, Q) + 15u) & ~15u;
     const uint32_t idesc = (1u << 4) | ((n >> 3) << 17) | (((PAIR ? 2u : 1u) * kTcRows >> 4) << 24);
-    const uint32_t sq_addr = tc_smem_u32(sq), sa_addr = tc_smem_u32(sa);
+    const uint64_t da0 = tc_desc(tc_smem_u32(sa)), db0 = tc_desc(tc_smem_u32(sq));
+    const bool lead = tc_elect();
     uint32_t tl = 0, c = 0, issued = 0;
     for (uint32_t i = 0; i < total && !a.mma_idle; i++) {
       const uint32_t buf = i % NB, d = tl % ACC;
       if (c == 0 && tl >= ACC) ok &= tc_wait(b_empty + 8u * d, ((tl - ACC) / ACC) & 1u, gave_up);
       if (ok) ok &= tc_wait(b_staged + 8u * buf, (i / NB) & 1u, gave_up);
-      if (!ok) break;
+      if (!__all_sync(0xFFFFFFFFu, ok)) break;
       tc_fence_after();
       const uint32_t nk = min(kTcChunkK, a.kpad - c * kTcChunkK) / 32u;
-      for (uint32_t kk = 0; kk < nk; kk++)
-        tc_mma<PAIR>(tmem + d * Q, tc_desc(sa_addr + buf * kTcChunkBytes + kk * 4096u),
-                     tc_desc(sq_addr + (c * 16u + 2u * kk) * 2048u), idesc, (c | kk) != 0);
-      tc_commit<PAIR>(b_done + 8u * buf);
-      if (c == a.nch - 1) tc_commit<PAIR>(b_full + 8u * d);
+      const uint64_t da = da0 + buf * (kTcChunkBytes >> 4), db = db0 + c * (kTcChunkBytes >> 4);
+      if (lead) {
+#pragma unroll
+        for (uint32_t kk = 0; kk < kTcChunkK / 32u; kk++)
+          if (kk < nk) tc_mma<PAIR>(tmem + d * Q, da + kk * 256u, db + kk * 256u, idesc, (c | kk) != 0);
+        tc_commit<PAIR>(b_done + 8u * buf);
+        if (c == a.nch - 1) tc_commit<PAIR>(b_full + 8u * d);
+      }
+      __syncwarp();
       issued = i + 1;
       if (++c == a.nch) {
         c = 0;
@@ -726,7 +762,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cand_tc(TcArgs a) {
       const uint32_t tiles_full = issued / a.nch;  // units whose accumulator commit was issued
       for (uint32_t j = 1; j <= ACC && j <= tiles_full; j++)  // the last use of each accumulator
         drained &= tc_wait_own(b_full + 8u * ((tiles_full - j) % ACC), ((tiles_full - j) / ACC) & 1u);
-      tc_commit<PAIR>(tc_smem_u32(bars + kDrain), 1);
+      if (lead) tc_commit<PAIR>(tc_smem_u32(bars + kDrain), 1);
       drained &= tc_wait_own(tc_smem_u32(bars + kDrain), 0u);
       if (!drained) *gave_up = 1u;
     }
