@@ -722,10 +722,11 @@ int Engine::apply_config(const Config& c) {
   // Auto batches: up to this many queries the four-query pass, above it blocks of 128.  Whole calls,
   // four-query pass against 128-query block: 8-bit, 40 queries 290 / 298 us (1M rows x 20 entries),
   // 48 queries 730 / 829 us (4M); 6-bit, 64 queries 395 / 449 us (1M); 4-bit 428 / 459 us.  The
-  // tensor-core pass costs less per entry the larger the matrix: 24 queries 201 / 286 us (1M x 32).
-  // The filter form: 48 queries 301 / 303 us (6-bit, 1M), 709 / 708 us (8-bit, 4M), 164 / 142 us
-  // (400k x 500); 4-bit 32 queries 241 / 245 us.
-  multi_max = use_tc ? 24 : (use_tf ? (bits == 4 ? 32 : 44) : (bits == 8 ? 48 : 64));
+  // tensor-core passes, four-query pass first, 4-bit 1M x 32: 12 queries 118 / 134 us, 16 139 / 134 us
+  // (300k x 20: 83 / 72 us and 96 / 72 us).  The filter form, 8-bit: 32 queries 170 / 186 us (1M),
+  // 277 / 281 us (2M), 482 / 459 us (4M), 40 queries 208 / 203, 336 / 302 and 597 / 488 us; 6-bit
+  // 400k x 500 117 / 112 us and 137 / 128 us; 4-bit 1M x 32: 20 queries 162 / 172 us, 24 183 / 171 us.
+  multi_max = use_tc ? 12 : (use_tf ? (bits == 4 ? 20 : 32) : (bits == 8 ? 48 : 64));
   if (batch_mode != 1) {
     batch_smem = batch_smem_bytes((int)bits, cols, split, batch_warps_n);
     int occb = 0;
@@ -910,7 +911,7 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
 
 // The tensor-core layout and exact values behind the filter form of the batched pass (8 bytes per
 // entry and 24 per row), made on the device from the FP32 CSR: for handles whose batches can reach
-// it (above 64 queries), without a memory limit, and only where a quarter of the memory left over
+// it (above 64 queries; smaller handles keep their memory), without a memory limit, and only where a quarter of the memory left over
 // holds it.  Not for pre-quantised matrices, nor where a row repeats a column (the dense tile
 // would keep one of the values).
 int Engine::build_tf(const HostCSR& m, const aes_params& p, float gmax, size_t planned, size_t config) {

@@ -155,6 +155,7 @@ def test_fp32_only_batches(rows, cols, kind, p0, p1, nq, k, ck, stride):
     (4000, 1024, 0, 1, 200, 4000, 0),   # every score passes: the hit queues overflow
     (90000, 256, 0, 1, 130, 64, 300),   # rows that pass for every query, in one tile
     (90000, 256, 1, 4, 256, 64, 300),   # with row scales and partitions
+    (5000, 100, 0, 1, 17, 64, 50),      # a launch of a column more than a warp's block
     (3000, 96, 1, 1, 25, 100, 40),      # one block of few queries
 ])
 def test_tensor_hit_queues(rows, cols, quant, split, nq, ck, hot):
@@ -213,9 +214,10 @@ def _filter_case(rows, cols, lo, hi, bits, quant, seed, signed):
     (40001, 500, 5, 25, 32, 150, "dense"),    # a CTA pair; partitions
     (9000, 333, 100, 300, 3, 300, "mixed"),   # a pair and a single launch; rows of many pieces
     (130, 40, 2, 8, 1, 129, "mixed"),         # two row tiles
+    (20000, 128, 5, 25, 2, 40, "dense"),      # part of a launch's columns
 ])
 def test_filter_pass(bits, quant, rows, cols, lo, hi, split, nq, kind):
-    """Batches above 64 queries of a handle without a memory limit: approximate FP8 scores filter
+    """Batches of a handle for more than 64 queries without a memory limit: approximate FP8 scores filter
     the rows and an exact integer check follows; with a memory limit the dp4a pass runs.  Both give
     the oracle's candidates and Top-K."""
     ck, k = max(96, 3 * split), 25
@@ -230,7 +232,7 @@ def test_filter_pass(bits, quant, rows, cols, lo, hi, split, nq, kind):
         Q[3::5] *= rng.random((len(Q[3::5]), cols)) < 0.1
     m = orc.Matrix(rows, cols, ptr, col, val, bits, quant)
     kw = dict(ptr=ptr, col=col, val=val, bits=bits, quant=quant, split=split, ck=ck, k_max=k,
-              max_batch=nq, batch_tile=128)
+              max_batch=max(nq, 65), batch_tile=128)
     eng = E.SpMV(rows, cols, **kw)
     lim = E.SpMV(rows, cols, mem_limit=1 << 40, **kw)
     assert eng.info()["device_bytes"] > lim.info()["device_bytes"]
