@@ -890,7 +890,10 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
   for (int sample = 0; sample < 2; sample++)
     AES_CK(raise_smem((const void*)pick_multi((int)bits, sgn, d_rowscale != nullptr, sample)));
   AES_CK(raise_smem((const void*)k_final));
-  AES_CK(raise_smem((const void*)k_exact_multi<8>));
+  for (const void* f : {(const void*)k_exact_multi<4, false>, (const void*)k_exact_multi<4, true>,
+                        (const void*)k_exact_multi<8, false>, (const void*)k_exact_multi<8, true>,
+                        (const void*)k_exact_multi<16, false>, (const void*)k_exact_multi<16, true>})
+    AES_CK(raise_smem(f));
   if (tc_ready || tf_ready) {
     AES_CK(raise_smem((const void*)k_cand_tc<2, false>));
     AES_CK(raise_smem((const void*)k_cand_tc<3, false>));
@@ -1960,7 +1963,7 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     AES_CK(cudaGetLastError());
     AES_CK(e.chain(k_threshold, dim3(1, n), kThreadsThr, 0, s, e.d_allkeys, ns, 0, e.d_exact_aux, 1,
                       e.d_exact_aux + 2, e.d_thr, e.d_cnt));
-    for (uint32_t i = 0; i < n;) {  // groups of eight queries, then four, a last one alone
+    for (uint32_t i = 0; i < n;) {  // groups of 16 queries, then the rest, one alone
       ExactArgs x{};
       x.ptr = e.d_csr_ptr;
       x.col = e.d_csr_col;
@@ -1974,14 +1977,16 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
       x.surv = e.d_surv + (size_t)i * e.cap;
       x.cap = e.cap;
       const uint32_t left = n - i;
-      if (left > 4) {
-        const uint32_t g = left >= 8 ? left / 8 : 1;
-        x.nq = std::min(left, 8 * g);
-        k_exact_multi<8><<<dim3((4 * e.sm_count + g - 1) / g, g), kExactWarps * 32,
-                           exact_multi_smem_bytes<8>(e.cols), s>>>(x);
+      if (left > 8) {
+        const uint32_t g = std::max<uint32_t>(1, left / 16 + (left % 16 > 8 ? 1 : 0));
+        x.nq = std::min(left, 16 * g);
+        launch_exact_multi<16>(x, g, e.nnz, e.sm_count, s);
+      } else if (left > 4) {
+        x.nq = left;
+        launch_exact_multi<8>(x, 1, e.nnz, e.sm_count, s);
       } else if (left > 1) {
         x.nq = left;
-        k_exact_multi<4><<<4 * e.sm_count, kExactWarps * 32, exact_multi_smem_bytes<4>(e.cols), s>>>(x);
+        launch_exact_multi<4>(x, 1, e.nnz, e.sm_count, s);
       } else {
         x.nq = 1;
         k_exact_all<true><<<e.sm_count * 8, kExactWarps * 32, exact_all_smem_bytes(e.cols), s>>>(

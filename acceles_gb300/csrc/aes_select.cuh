@@ -10,6 +10,8 @@
 //   k_exact_sample, k_exact_all, k_exact_multi   the FP32-only Top-K of every row
 #pragma once
 
+#include <algorithm>
+
 #include "aes_kernels.cuh"
 
 namespace aes {
@@ -1113,90 +1115,158 @@ struct ExactArgs {
   uint32_t cap;
 };
 
-__device__ __forceinline__ void exact_emit(const ExactArgs& a, uint32_t q, uint32_t row, float score,
-                                           uint32_t th) {
-  const uint32_t key = key_f32(score);
-  if (key >= th) {
-    const uint32_t i = atomicAdd(a.cnt + q, 1u);
-    if (i < a.cap) a.surv[(size_t)q * a.cap + i] = make_uint2(key, row);
+// Bound by shared memory: an entry gathers T queries' values of its column.  T / 4 lanes walk a row
+// in column order, four queries each, so the 16-byte loads of eight lanes cover 32 / T rows' columns;
+// the table keeps a column's T values 32 / T times side by side, 128 bytes in all, and each of the
+// rows reads its own copy: no two lanes meet in a bank whatever the columns (one copy with a lane
+// per row, two loads for eight queries: 2.7 wavefronts instead of one per eight lanes).  A warp
+// stages its 128 / T rows' entries (contiguous in the CSR) in chunks, the next chunk's loads under
+// way while it walks.  1M rows x 20 entries, 16 queries: 205 -> 106 us.  blockIdx.y: the group of T
+// queries.
+// Two forms: 32 warps with 256 staged entries each, or 16 with 512 (LONG) where a warp's rows have more
+// than 256 on average (exact_multi_long): eight queries, 16 rows to a warp, 1M x 20 127 / 112 us,
+// 3M x 8.5 130 / 163 us; 16 queries, 8 rows to a warp, 1M x 20 151 / 162 us, 1M x 40 289 / 222 us.
+template <int T, bool LONG>
+struct ExMulti {
+  static constexpr uint32_t WARPS = LONG ? 16 : 32;
+  static constexpr uint32_t CHUNK = LONG ? 512 : 256;  // entries per warp and chunk
+  static constexpr uint32_t HITS = 64;  // hits a warp collects before it appends them, 32 at a time or more
+  __host__ static size_t smem(uint32_t cols) {
+    return (size_t)cols * 128 + (size_t)WARPS * (CHUNK * 8 + HITS * 12);
   }
+};
+template <int T>
+__host__ inline bool exact_multi_long(uint64_t nnz, uint32_t rows) {
+  return nnz * (128 / T) > 256ull * rows;
+}
+template <int T, bool LONG>
+__global__ void __launch_bounds__(ExMulti<T, LONG>::WARPS * 32, 1) k_exact_multi(ExactArgs a) {
+  static_assert(T == 4 || T == 8 || T == 16, "queries per walk");
+  constexpr uint32_t kWarps = ExMulti<T, LONG>::WARPS, kChunk = ExMulti<T, LONG>::CHUNK;
+  constexpr uint32_t kHits = ExMulti<T, LONG>::HITS;
+  constexpr uint32_t L = T / 4, R = 32 / L, COPIES = 32 / T, U = kChunk / 32;
+  extern __shared__ __align__(128) unsigned char xsm[];
+  float* qs = reinterpret_cast<float*>(xsm);  // [cols][COPIES][T]
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  uint2* st = reinterpret_cast<uint2*>(xsm + (size_t)a.cols * 128) + warp * kChunk;
+  // hits {query, key, row}: one atomic round trip for 32 of them, not one for each block of rows with a
+  // hit (100k rows, 64 queries, the whole call: 352 -> 192 us)
+  uint32_t* hits = reinterpret_cast<uint32_t*>(xsm + (size_t)a.cols * 128 + (size_t)kWarps * kChunk * 8) +
+                   warp * kHits * 3;
+  uint32_t nh = 0;
+  auto flush = [&]() {
+    __syncwarp();
+    for (uint32_t i = lane; i < nh; i += 32) {
+      const uint32_t q = hits[i], at = atomicAdd(a.cnt + q, 1u);
+      if (at < a.cap)
+        a.surv[(size_t)q * a.cap + at] = make_uint2(hits[kHits + i], hits[2 * kHits + i]);
+    }
+    __syncwarp();
+    nh = 0;
+  };
+  const uint32_t q0 = blockIdx.y * T, nq = min((uint32_t)T, a.nq - q0);
+  {  // a thread takes one query's value of every COPIES-th group of columns; writes without conflicts
+    const uint32_t t = lane % T, sub = lane / T;
+    const float* x = a.q + (size_t)(q0 + min(t, nq - 1u)) * a.ld;
+#pragma unroll 8
+    for (uint32_t j = warp * COPIES + sub; j < a.cols; j += kWarps * COPIES) {
+      const float v = x[j];
+#pragma unroll
+      for (uint32_t k = 0; k < COPIES; k++) qs[j * 32u + (sub + k) % COPIES * T + t] = v;
+    }
+  }
+  const uint32_t g = lane / L, l = lane % L;
+  uint32_t th[4];
+#pragma unroll
+  for (uint32_t t = 0; t < 4; t++) th[t] = 4 * l + t < nq ? a.thr[q0 + 4 * l + t] : 0xFFFFFFFFu;
+  const unsigned char* mine = xsm + lane % 8u * 16u;  // the row's copy, this lane's queries
+  __syncthreads();
+  const uint32_t nblk = (a.rows + R - 1) / R, stride = gridDim.x * kWarps;
+  // this lane's row of block blk (past the matrix: empty)
+  auto bounds = [&](uint64_t blk, uint32_t& s, uint32_t& e) {
+    const uint64_t r = blk * R + g;
+    s = a.ptr[min(r, (uint64_t)a.rows)];
+    e = a.ptr[min(r + 1, (uint64_t)a.rows)];
+  };
+  float lv[U];
+  uint32_t lc[U];
+  auto load = [&](uint32_t c, uint32_t E1) {
+    const uint32_t n = min(kChunk, E1 - c);
+#pragma unroll
+    for (uint32_t u = 0; u < U; u++) {
+      const uint32_t i = u * 32 + lane;
+      lv[u] = i < n ? __ldg(a.val + c + i) : 0.0f;
+      lc[u] = i < n ? (uint32_t)__ldg(a.col + c + i) : 0u;
+    }
+  };
+  uint32_t blk = warp * gridDim.x + blockIdx.x;  // (a small matrix spreads over the CTAs)
+  uint32_t s, e, sn, en;
+  bounds(blk, s, e);
+  bounds((uint64_t)blk + stride, sn, en);
+  uint32_t c = __shfl_sync(0xFFFFFFFFu, s, 0), E1 = __shfl_sync(0xFFFFFFFFu, e, 31);
+  load(c, E1);
+  while (blk < nblk) {
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (bool more = true; more;) {
+      const uint32_t n = min(kChunk, E1 - c), c0 = c, e0 = c + n;
+      __syncwarp();
+#pragma unroll
+      for (uint32_t u = 0; u < U; u++)
+        if (u * 32 < n) st[u * 32 + lane] = make_uint2(__float_as_uint(lv[u]), lc[u] * 128u);
+      __syncwarp();
+      more = E1 - c > kChunk;
+      if (more) {
+        c += kChunk;
+      } else {
+        c = __shfl_sync(0xFFFFFFFFu, sn, 0);
+        E1 = __shfl_sync(0xFFFFFFFFu, en, 31);
+      }
+      load(c, E1);
+      const uint32_t d = min(e, e0);
+#pragma unroll 4
+      for (uint32_t i = max(s, c0); i < d; i++) {
+        const uint2 w = st[i - c0];
+        const float v = __uint_as_float(w.x);
+        const float4 x = *reinterpret_cast<const float4*>(mine + w.y);
+        acc[0] = __fadd_rn(acc[0], __fmul_rn(v, x.x));
+        acc[1] = __fadd_rn(acc[1], __fmul_rn(v, x.y));
+        acc[2] = __fadd_rn(acc[2], __fmul_rn(v, x.z));
+        acc[3] = __fadd_rn(acc[3], __fmul_rn(v, x.w));
+      }
+    }
+    const uint32_t r = blk * R + g;
+#pragma unroll
+    for (uint32_t t = 0; t < 4; t++) {
+      const uint32_t key = key_f32(acc[t]);
+      const bool hit = key >= th[t] && r < a.rows && 4 * l + t < nq;
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit);
+      if (!m) continue;
+      if (nh + __popc(m) > kHits) flush();
+      if (hit) {
+        const uint32_t at = nh + __popc(m & ((1u << lane) - 1u));
+        hits[at] = q0 + 4 * l + t;
+        hits[kHits + at] = key;
+        hits[2 * kHits + at] = r;
+      }
+      nh += __popc(m);
+    }
+    s = sn;
+    e = en;
+    if (nblk - blk <= stride) break;
+    blk += stride;
+    bounds((uint64_t)blk + stride, sn, en);
+  }
+  flush();
 }
 
-// Bound by shared memory: a lane walks its row's entries in column order (values and columns
-// staged from the CSR, 32 rows' entries being contiguous) and gathers the T queries' values of a
-// column with 16-byte loads, about 11 wavefronts each over random columns against 6.5 for the
-// entry itself; so eight queries per walk, or four for a last few.  1M rows x 20 entries: 43 us
-// for a query alone (and a key array to filter), 102 us for eight.  blockIdx.y: the group of T queries.
+// One CTA per SM, shared out over g groups of T queries
 template <int T>
-__host__ inline size_t exact_multi_smem_bytes(uint32_t cols) {
-  return (size_t)cols * T * 4 + (size_t)kExactWarps * kExactChunk * 6;
-}
-template <int T>
-__global__ void __launch_bounds__(kExactWarps * 32) k_exact_multi(ExactArgs a) {
-  grid_wait();
-  static_assert(T == 4 || T == 8, "queries per walk");
-  extern __shared__ __align__(16) unsigned char xsm[];
-  float4* qs = reinterpret_cast<float4*>(xsm);  // [T / 4][cols]
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  float* sv = reinterpret_cast<float*>(xsm + (size_t)a.cols * T * 4) + warp * kExactChunk;
-  uint16_t* sc = reinterpret_cast<uint16_t*>(xsm + (size_t)a.cols * T * 4 +
-                                             (size_t)kExactWarps * kExactChunk * 4) + warp * kExactChunk;
-  const uint32_t q0 = blockIdx.y * T, nq = min((uint32_t)T, a.nq - q0);
-  uint32_t th[T];
-#pragma unroll
-  for (int t = 0; t < T; t++) {
-    th[t] = (uint32_t)t < nq ? a.thr[q0 + t] : 0xFFFFFFFFu;
-    const float* x = a.q + (size_t)(q0 + ((uint32_t)t < nq ? t : 0u)) * a.ld;
-    for (uint32_t j = threadIdx.x; j < a.cols; j += blockDim.x)
-      reinterpret_cast<float*>(qs)[((size_t)(t / 4) * a.cols + j) * 4 + t % 4] = x[j];
-  }
-  __syncthreads();
-  const uint32_t nblk = (a.rows + 31) / 32;
-  for (uint32_t blk = blockIdx.x * kExactWarps + warp; blk < nblk; blk += gridDim.x * kExactWarps) {
-    const uint32_t r0 = blk * 32, r = r0 + lane;
-    const uint32_t rend = min(r0 + 32u, a.rows);
-    const uint32_t E0 = a.ptr[r0], E1 = a.ptr[rend];
-    const uint32_t s = r < a.rows ? a.ptr[r] : E1, e = r < a.rows ? a.ptr[r + 1] : E1;
-    float acc[T];
-#pragma unroll
-    for (int t = 0; t < T; t++) acc[t] = 0.0f;
-    for (uint32_t c = E0; c < E1; c += kExactChunk) {
-      const uint32_t n = min(kExactChunk, E1 - c);
-      float lv[kExactChunk / 32];
-      uint16_t lc[kExactChunk / 32];
-#pragma unroll
-      for (uint32_t u = 0; u < kExactChunk / 32; u++) {
-        const uint32_t i = u * 32 + lane;
-        lv[u] = i < n ? __ldg(a.val + c + i) : 0.0f;
-        lc[u] = i < n ? __ldg(a.col + c + i) : (uint16_t)0;
-      }
-#pragma unroll
-      for (uint32_t u = 0; u < kExactChunk / 32; u++) {
-        sv[u * 32 + lane] = lv[u];
-        sc[u * 32 + lane] = lc[u];
-      }
-      __syncwarp();
-      const uint32_t b = max(s, c), d = min(e, c + n);
-      for (uint32_t i = b; i < d; i++) {
-        const float v = sv[i - c];
-        const uint32_t j = sc[i - c];
-#pragma unroll
-        for (int g = 0; g < T / 4; g++) {
-          const float4 x = qs[(size_t)g * a.cols + j];
-          acc[4 * g + 0] = __fadd_rn(acc[4 * g + 0], __fmul_rn(v, x.x));
-          acc[4 * g + 1] = __fadd_rn(acc[4 * g + 1], __fmul_rn(v, x.y));
-          acc[4 * g + 2] = __fadd_rn(acc[4 * g + 2], __fmul_rn(v, x.z));
-          acc[4 * g + 3] = __fadd_rn(acc[4 * g + 3], __fmul_rn(v, x.w));
-        }
-      }
-      __syncwarp();
-    }
-    if (r < a.rows) {
-#pragma unroll
-      for (int t = 0; t < T; t++)
-        if ((uint32_t)t < nq) exact_emit(a, q0 + t, r, acc[t], th[t]);
-    }
-  }
+__host__ inline void launch_exact_multi(const ExactArgs& x, uint32_t g, uint64_t nnz, int sm_count, cudaStream_t s) {
+  const dim3 grid(std::max<uint32_t>(1, (uint32_t)sm_count / g), g);
+  if (exact_multi_long<T>(nnz, x.rows))
+    k_exact_multi<T, true><<<grid, ExMulti<T, true>::WARPS * 32, ExMulti<T, true>::smem(x.cols), s>>>(x);
+  else
+    k_exact_multi<T, false><<<grid, ExMulti<T, false>::WARPS * 32, ExMulti<T, false>::smem(x.cols), s>>>(x);
 }
 
 // FP32 keys of rows 0, S, 2 S, ... (ns of them) per query (blockIdx.y): keys[nq][ns].  A warp takes

@@ -125,12 +125,15 @@ def test_four_query_pass(bits, quant, rows, cols, lo, hi, split, nq):
 
 @pytest.mark.parametrize("rows,cols,kind,p0,p1,nq,k,ck,stride", [
     (30000, 1024, E.GEN_UNIFORM_DEG, 10, 30, 1, 100, 512, 0),   # one query: rows filtered as scored
-    (30001, 1024, E.GEN_UNIFORM_DEG, 0, 30, 17, 100, 512, 0),   # two groups of eight and one; empty rows
-    (30000, 333, E.GEN_UNIFORM_DEG, 10, 30, 12, 7, 512, 0),     # eight and four
+    (30001, 1024, E.GEN_UNIFORM_DEG, 0, 30, 17, 100, 512, 0),   # a group of 16 and one; empty rows
+    (30000, 333, E.GEN_UNIFORM_DEG, 10, 30, 12, 7, 512, 0),     # twelve in a group of 16
     (29999, 777, E.GEN_UNIFORM_DEG, 1, 3, 6, 33, 512, 0),       # six in a group of eight
     (6000, 1024, E.GEN_GAMMA_DEG, 200, 1024, 11, 20, 512, 0),   # rows longer than a staged chunk's share
+    (9001, 100, E.GEN_UNIFORM_DEG, 0, 12, 4, 50, 128, 0),        # a lane per row; short and empty rows
+    (9000, 200, E.GEN_UNIFORM_DEG, 20, 60, 3, 50, 128, 0),       # long chunks, by four and by eight
+    (9000, 200, E.GEN_UNIFORM_DEG, 20, 60, 8, 50, 128, 0),
     (31, 64, E.GEN_UNIFORM_DEG, 1, 9, 3, 40, 64, 0),            # fewer rows than results: no sample
-    (30000, 256, E.GEN_UNIFORM_DEG, 4, 9, 70, 100, 128, 256),   # more queries than one chunk takes
+    (30000, 256, E.GEN_UNIFORM_DEG, 4, 9, 70, 100, 128, 256),   # four groups of 16 and six
 ])
 def test_fp32_only_batches(rows, cols, kind, p0, p1, nq, k, ck, stride):
     ptr, col, val = E.gen_matrix(kind, rows, cols, p0, p1, seed=rows + nq)
