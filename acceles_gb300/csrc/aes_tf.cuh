@@ -253,6 +253,9 @@ struct TfCheck {
 };
 
 constexpr int kThreadsCheck = 256;
+// groups of eight rows whose first loads are in flight together (1: 40 registers and not 80, twice the
+// warps; 512 queries on 4M x 1024 1558 us for 1541, 100 on 400k x 500 200 for 196)
+constexpr int kCheckRows = 4;
 // bytes per query in shared memory: a word more than the row, so that the bytes of several queries at
 // one column (hits of one row) lie in different banks
 __host__ __device__ inline uint32_t check_ld(uint32_t ld8) { return ld8 + 4u; }
@@ -332,28 +335,44 @@ __global__ void __launch_bounds__(kThreadsCheck) k_recheck(TfCheck a) {
         score = a.sgn ? (int)qs[q * ld + c] : (int)csm[q * ld + c];
       }
 #pragma unroll
-      for (int j0 = 0; j0 < 32; j0 += 8) {
-        const int j = j0 + (int)(lane >> 2);
-        const uint32_t n4j = __shfl_sync(0xFFFFFFFFu, n4, j), nj = h0 + j < total ? n4j : 0u;
-        const uint4* src = a.q + __shfl_sync(0xFFFFFFFFu, src_h, j) + (lane & 3u);
-        const int8_t* qj = qs + __shfl_sync(0xFFFFFFFFu, q, j) * ld;
-        auto val = [&](uint32_t x) {
-          const uint32_t o = x & 0xFFFFu;
-          return ((int)x >> 16) * (a.sgn ? (int)qj[o] : (int)(uint8_t)qj[o]);
-        };
-        auto dot = [&](uint4 x) { return val(x.x) + val(x.y) + val(x.z) + val(x.w); };
-        int x = 0;
-        for (uint32_t k4 = lane & 3u; k4 < nj; k4 += 8, src += 8) {
-          const uint4 x0 = __ldg(src);
-          const uint4 x1 = k4 + 4 < nj ? __ldg(src + 4) : make_uint4(0u, 0u, 0u, 0u);
-          x += dot(x0) + dot(x1);
+      for (int j0 = 0; j0 < 32; j0 += 8 * kCheckRows) {
+        if (h0 + j0 >= total) break;
+        // the first 32 entries of each row in flight together
+        uint32_t nj[kCheckRows];
+        const uint4* src[kCheckRows];
+        uint4 x0[kCheckRows], x1[kCheckRows];
+#pragma unroll
+        for (int w = 0; w < kCheckRows; w++) {
+          const int j = j0 + 8 * w + (int)(lane >> 2);
+          const uint32_t n4j = __shfl_sync(0xFFFFFFFFu, n4, j);
+          nj[w] = h0 + j < total ? n4j : 0u;
+          src[w] = a.q + __shfl_sync(0xFFFFFFFFu, src_h, j);
+          const uint32_t k4 = lane & 3u;
+          x0[w] = k4 < nj[w] ? __ldg(src[w] + k4) : make_uint4(0u, 0u, 0u, 0u);
+          x1[w] = k4 + 4 < nj[w] ? __ldg(src[w] + k4 + 4) : make_uint4(0u, 0u, 0u, 0u);
         }
-        __syncwarp();
-        x += __shfl_xor_sync(0xFFFFFFFFu, x, 1);
-        x += __shfl_xor_sync(0xFFFFFFFFu, x, 2);
-        // lane j0 + g takes the sum of the four lanes 4 g .. 4 g + 3
-        const int y = __shfl_sync(0xFFFFFFFFu, x, (int)(lane & 7u) * 4);
-        if ((int)(lane >> 3) == j0 / 8) score += y;
+#pragma unroll
+        for (int w = 0; w < kCheckRows; w++) {
+          const int j = j0 + 8 * w + (int)(lane >> 2);
+          const int8_t* qj = qs + __shfl_sync(0xFFFFFFFFu, q, j) * ld;
+          auto val = [&](uint32_t x) {
+            const uint32_t o = x & 0xFFFFu;
+            return ((int)x >> 16) * (a.sgn ? (int)qj[o] : (int)(uint8_t)qj[o]);
+          };
+          auto dot = [&](uint4 x) { return val(x.x) + val(x.y) + val(x.z) + val(x.w); };
+          int x = dot(x0[w]) + dot(x1[w]);
+          for (uint32_t k4 = (lane & 3u) + 8; k4 < nj[w]; k4 += 8) {
+            const uint4 y0 = __ldg(src[w] + k4);
+            const uint4 y1 = k4 + 4 < nj[w] ? __ldg(src[w] + k4 + 4) : make_uint4(0u, 0u, 0u, 0u);
+            x += dot(y0) + dot(y1);
+          }
+          __syncwarp();
+          x += __shfl_xor_sync(0xFFFFFFFFu, x, 1);
+          x += __shfl_xor_sync(0xFFFFFFFFu, x, 2);
+          // lane j0 + 8 w + g takes the sum of the four lanes 4 g .. 4 g + 3
+          const int y = __shfl_sync(0xFFFFFFFFu, x, (int)(lane & 7u) * 4);
+          if ((int)(lane >> 3) == j0 / 8 + w) score += y;
+        }
       }
       const uint32_t key = a.rowscale && h < total
           ? key_f32(__fmul_rn(__int2float_rn(score), __ldg(a.rowscale + row))) : key_i32(score);
