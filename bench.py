@@ -623,6 +623,9 @@ def main():
     batch_launch_ms, cand_per_step = cand_launch_ms(eng, Bb)
     blocks = (Bb + 127) // 128
 
+    # with room for its layout the batched pass is the tensor-core filter (a launch per two blocks of
+    # 128 queries, then an exact check), else the dp4a pass (one launch for all blocks)
+    filtered = cand_per_step > 1
     # dominant kernel of the batched path: the batched candidate pass; algorithmic bytes of one
     # 128-query block = Ultra-CSR packets + tile row bases + the block's query table
     alg_bytes = info["packets"] * 64 + (info["tiles"] + 1) * 4 + COLS * 128
@@ -634,13 +637,13 @@ def main():
     # the committed ncu summaries are of the 8-bit, one-partition workload at 10M rows
     profiled = BITS == 8 and args.split == 1 and rows == ROWS
     traffic = (profile_traffic("cand_batch_10Mx1024_b8.md", "traffic_bytes_per_block")
-               if profiled else None)
-    # the batched pass is bound by instruction issue, not HBM: warp instructions per group of
+               if profiled and not filtered else None)
+    # the dp4a pass is bound by instruction issue, not HBM: warp instructions per group of
     # four entries (ncu instruction count of the capture) x the groups of one block, over the
     # live time per block at the sampled SM clock; an SM issues at most 4 warp instructions a cycle
     issue = None
     ipg = (profile_number("cand_batch_10Mx1024_b8.md", "warp_instructions_per_group")
-           if profiled and profile_current("cand_batch_10Mx1024_b8.md") else None)
+           if profiled and not filtered and profile_current("cand_batch_10Mx1024_b8.md") else None)
     if ipg:
         groups = info["tiles"] * 32 * (511 // (BITS + 11)) // 4
         sms = torch.cuda.get_device_properties(local).multi_processor_count
@@ -738,16 +741,19 @@ def main():
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "int32",
             "data": "synthetic (seeded; reference matrices not shipped)",
             "config": headline_config(rows, info["nnz"], args.split, Bb),
-            "path": "batched (one candidate pass per 128 queries)",
+            "path": "batched (candidate passes over blocks of 128 queries)",
             "plain_leg": {"batch": Bp, "steps": args.steps, "ms_per_step": ms_p / args.steps},
             "parallelism": f"replicas x{world}",
             "batched_qps": qps, "plain_qps": plain_qps, "batched_over_plain": qps / plain_qps,
             "hbm_gbs_batched_pass": achieved, "hbm_gbs_plain_pass": plain_achieved,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": f"k_cand_batch<{BITS},signed,FILTER> (128 queries per matrix read)",
-                         "limiter": "CUDA-core integer issue (gathers, byte transposes, dp4a); "
-                                    "one matrix read serves 128 queries",
+                         "kernel": ("k_cand_tc (approximate FP8 scores with a bound; CTA pairs, 256 queries "
+                                    "per matrix read), then k_recheck" if filtered else
+                                    f"k_cand_batch<{BITS},signed,FILTER> (128 queries per matrix read)"),
+                         "limiter": ("FP8 products of the densified rows and their epilogue" if filtered else
+                                     "CUDA-core integer issue (gathers, byte transposes, dp4a); "
+                                     "one matrix read serves 128 queries"),
                          "alg_bytes_per_block": alg_bytes, "ms_per_block": cand_ms,
                          "launches_per_step": cand_per_step, "blocks_per_step": blocks,
                          "issue": issue},

@@ -56,7 +56,9 @@ typedef struct aes_params {
                              Top-CK (SPLIT, quantify_util.py:173-196 / SPMV_PARTITIONS) */
   uint32_t ck;            /* candidates kept (APPROXIMATE_K, types.hpp:149) */
   uint32_t k_max;         /* largest K a run may request (<= 1024) */
-  uint32_t max_batch;     /* most queries per aes_set_query / aes_run_device call */
+  uint32_t max_batch;     /* most queries per aes_set_query / aes_run_device call; above 64 and
+                             without mem_limit the handle also holds the tensor-core filter's
+                             layout (8 B per entry, 24 per row) where memory is ample */
   uint32_t pack_parts;    /* Ultra-CSR packing partitions (SPMV_PARTITIONS = 32) */
   uint32_t sample_stride; /* threshold sample: one 32-packet tile in this many (0 = auto) */
   uint32_t batch_tile;    /* queries per matrix pass: 1 = one; 0 = auto: four for a few queries,
@@ -82,7 +84,8 @@ typedef struct aes_params {
                                cores at creation (4 B per entry) and run the batched candidate
                                pass as FP8 tcgen05 products of 128-row tiles; the integers are
                                exact in FP8 and the scores exact in FP32, so results equal the
-                               dp4a pass.  Ignored for 6- and 8-bit matrices, for matrices with
+                               dp4a pass.  Ignored for 6- and 8-bit matrices (whose larger
+                               batches use such products as a filter without the flag), for matrices with
                                duplicate (row, col) entries and for split > 32 */
 
 #define AES_FLAG_TEST_IDLE_MMA 16u /* failure-path tests only: the tensor-core pass's MMA role
