@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(256) k_tf_rows(TfMatrix a) {
       }
     }
     if (!__any_sync(0xFFFFFFFFu, any)) {  // a row left empty gets one entry
+      __syncwarp();  // (after the zero that another lane stored in its place: a vote orders no memory)
       if (s == e) {
         r2 = lane == 0;
         rs = lane == 0;
