@@ -143,7 +143,7 @@ struct BatchRows {
 #pragma unroll
         for (int t = 0; t < 4; t++) {
           const uint32_t q = 4 * lane + t;
-          th[t] = q < nq ? __ldg(a.thr + (size_t)(q0 + q) * a.split + p) : 0xFFFFFFFFu;
+          th[t] = q < nq ? a.thr[(size_t)(q0 + q) * a.split + p] : 0xFFFFFFFFu;
         }
       }
       const bool hit = (key[0] >= th[0]) | (key[1] >= th[1]) | (key[2] >= th[2]) | (key[3] >= th[3]);
@@ -161,7 +161,7 @@ struct BatchRows {
     if (a.split <= 1) return thr4[t];
     if (thr_s) return thr_s[p * kBatchQ + 4 * lane + t];
     const uint32_t q = 4 * lane + t;
-    return q < nq ? __ldg(a.thr + (size_t)(q0 + q) * a.split + p) : 0xFFFFFFFFu;
+    return q < nq ? a.thr[(size_t)(q0 + q) * a.split + p] : 0xFFFFFFFFu;
   }
   // integer keys: per query, the lowest score bound over the partitions of rows r0 .. r1 (one
   // partition for almost every tile: the partitions are contiguous row ranges)
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kWarpsBatchMax * 32, 1) k_cand_batch(BatchArgs
 #pragma unroll
       for (int u = 0; u < 8; u++) {
         const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
-        if (i < n) v[u] = __ldg(src + i);
+        if (i < n) v[u] = src[i];
       }
 #pragma unroll
       for (int u = 0; u < 8; u++) {
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(kWarpsBatchMax * 32, 1) k_cand_batch(BatchArgs
 // contiguously instead of one 32-byte sector per key.  A CTA moves 32 rows x 128 queries of one
 // block (blockIdx.y) through shared memory; both the reads and the writes are coalesced.
 constexpr uint32_t kTransposeRows = 32;
-__global__ void __launch_bounds__(256) k_keys_transpose(const uint32_t* __restrict__ in,
+__global__ void __launch_bounds__(256) k_keys_transpose(const uint32_t* in,
                                                         uint32_t n_rows, uint32_t nq,
                                                         uint32_t* __restrict__ out) {
   grid_wait();
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(256) k_keys_transpose(const uint32_t* __restri
 // qtab[blk][col][33] words: byte t of word (blk, col, l) = quantised query 128 blk + 4l + t at
 // col (0 past nq); word 32 of each column and the padding to a 16-byte slot are zero.  Every
 // block of the batch in one launch.
-__global__ void k_qtable(const int8_t* __restrict__ q8, uint32_t ld8, uint32_t cols, uint32_t nq,
+__global__ void k_qtable(const int8_t* q8, uint32_t ld8, uint32_t cols, uint32_t nq,
                          uint32_t* __restrict__ qtab) {
   grid_wait();
   grid_next();

@@ -27,7 +27,9 @@ __host__ __device__ constexpr int plain_threads(int B) { return plain_warps(B) *
 // predecessor drains; it touches nothing that other kernels write before grid_wait(), which returns
 // once the predecessor is complete and its writes are visible.  grid_next() lets the next kernel start
 // in turn.  Kernels call it at their top after the wait, so what lies two kernels back is complete when
-// a kernel starts at all.  It hides the launch and drain between the short kernels around the
+// a kernel starts at all.  What the predecessor writes is read with plain loads, never
+// through the read-only path (__ldg, const __restrict__ parameters): that path is for memory that does
+// not change while the kernel runs, and its loads may be moved across the wait.  It hides the launch and drain between the short kernels around the
 // candidate pass, some 2 us each (one query of a small matrix 87 -> 75 us per call).  The long passes
 // over a whole batch leave it out: the next kernel then starts at their end.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -124,7 +126,7 @@ struct Emitter {
   // filter with integer keys (no row scales), any number of partitions
   __device__ __forceinline__ bool int_keys() const { return MODE == MODE_FILTER && !a.rowscale; }
   __device__ __forceinline__ uint32_t thr_of(uint32_t p) const {
-    return a.split <= 1 ? thr0 : (a.split <= kThrSmemMax ? thr_s[p] : __ldg(a.thr + p));
+    return a.split <= 1 ? thr0 : (a.split <= kThrSmemMax ? thr_s[p] : a.thr[p]);
   }
   // the lowest score bound over the partitions of rows r0 .. r1 (one partition for almost every
   // tile: the partitions are contiguous row ranges)
@@ -152,7 +154,7 @@ struct Emitter {
       uint32_t p = 0, th = thr0;
       if (a.split > 1) {
         p = part_of(row, a.split, a.slice);
-        th = (a.split <= kThrSmemMax) ? thr_s[p] : __ldg(a.thr + p);
+        th = (a.split <= kThrSmemMax) ? thr_s[p] : a.thr[p];
       }
       if (key >= th) {
         uint32_t i = atomicAdd(a.cnt + p, 1u);

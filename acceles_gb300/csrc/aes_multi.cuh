@@ -53,7 +53,7 @@ struct MultiEmit {
   uint32_t q0, nq;        // first query, queries (1 .. 4)
   __device__ __forceinline__ uint32_t thr_key(uint32_t p, int t) const {
     if (thr_s) return thr_s[p * kMultiQ + t];
-    return (uint32_t)t < nq ? __ldg(a.thr + (size_t)(q0 + t) * a.split + p) : 0xFFFFFFFFu;
+    return (uint32_t)t < nq ? a.thr[(size_t)(q0 + t) * a.split + p] : 0xFFFFFFFFu;
   }
   // the bound of a key threshold: x >= bound (signed, or FP32 bits) <=> key(x) >= th
   __device__ __forceinline__ static int32_t bound(uint32_t th) {
@@ -89,10 +89,13 @@ struct MultiEmit {
     const bool hit = (x[0] >= b[0]) | (x[1] >= b[1]) | (x[2] >= b[2]) | (x[3] >= b[3]);
     if (valid && hit) {
       const uint32_t p = part_of(row, a.split, a.slice);
+      uint32_t th[kMultiQ];  // all four in flight, before the atomics
+#pragma unroll
+      for (int t = 0; t < kMultiQ; t++) th[t] = thr_key(p, t);
 #pragma unroll
       for (int t = 0; t < kMultiQ; t++) {
         const uint32_t key = SCALED ? key_f32(__uint_as_float((uint32_t)x[t])) : key_i32(x[t] >> SHIFT);
-        if (key >= thr_key(p, t) && (uint32_t)t < nq) {
+        if (key >= th[t] && (uint32_t)t < nq) {
           const size_t qp = (size_t)(q0 + t) * a.split + p;
           const uint32_t i = atomicAdd(a.cnt + qp, 1u);
           if (i < a.cap) a.surv[qp * a.cap + i] = make_uint2(key, row);

@@ -184,7 +184,7 @@ constexpr uint32_t kThrListMax = 1024;
 
 template <int N>
 __global__ void __launch_bounds__(kThrWarps * 32) k_threshold_warp(
-    const uint32_t* __restrict__ keys_all, uint32_t ld_keys, const uint32_t* __restrict__ part_begin,
+    const uint32_t* keys_all, uint32_t ld_keys, const uint32_t* __restrict__ part_begin,
     uint32_t split, uint32_t pairs, const uint32_t* __restrict__ r_part, uint32_t* __restrict__ thr,
     uint32_t* __restrict__ cnt) {
   grid_wait();
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kThrWarps * 32) k_threshold_warp(
 // few others do, so the few threads at or above it gather their keys of at least that bound, and
 // the r-th largest of the gathered keys is the answer.  One read of the keys, where two
 // histograms took three: 27 -> 12.8 us for 39k keys, r = 24.  Larger ranks: two histograms.
-__global__ void __launch_bounds__(kThreadsThr, 2) k_threshold(const uint32_t* __restrict__ keys_all, uint32_t ld_keys, uint32_t qblk,
+__global__ void __launch_bounds__(kThreadsThr, 2) k_threshold(const uint32_t* keys_all, uint32_t ld_keys, uint32_t qblk,
                             const uint32_t* __restrict__ part_begin, uint32_t split,
                             const uint32_t* __restrict__ r_part, uint32_t* __restrict__ thr,
                             uint32_t* __restrict__ cnt) {
@@ -1053,7 +1053,7 @@ template <bool FILTER>
 __global__ void __launch_bounds__(kExactWarps * 32) k_exact_all(
     const uint32_t* __restrict__ ptr, const uint16_t* __restrict__ col,
     const float* __restrict__ val, const float* __restrict__ q, uint32_t cols, uint32_t rows,
-    uint32_t* __restrict__ keys, const uint32_t* __restrict__ thr, uint32_t* __restrict__ cnt,
+    uint32_t* __restrict__ keys, const uint32_t* thr, uint32_t* __restrict__ cnt,
     uint2* __restrict__ surv, uint32_t cap) {
   grid_wait();
   extern __shared__ __align__(16) unsigned char xsm[];

@@ -89,7 +89,7 @@ __host__ inline uint32_t tc_bufs(uint32_t cols, uint32_t split, size_t smem_limi
 }
 
 // e4m3 query operand of queries q0 .. q0 + nq - 1 (zero past nq and past cols)
-__global__ void k_qtable_tc(const int8_t* __restrict__ q8, uint32_t ld8, uint32_t cols, uint32_t q0,
+__global__ void k_qtable_tc(const int8_t* q8, uint32_t ld8, uint32_t cols, uint32_t q0,
                             uint32_t nq, uint8_t* __restrict__ qt) {
   grid_wait();
   grid_next();
@@ -283,7 +283,7 @@ __device__ __forceinline__ void tc_append(const TcArgs& a, uint32_t S, size_t qp
                                           const uint32_t* score, uint32_t hit, float rs) {
   uint32_t key[N], th[N], ix[N];
 #pragma unroll
-  for (int j = 0; j < N; j++) th[j] = (hit >> j) & 1u ? __ldg(a.thr + qp + (size_t)j * S) : 0xFFFFFFFFu;
+  for (int j = 0; j < N; j++) th[j] = (hit >> j) & 1u ? a.thr[qp + (size_t)j * S] : 0xFFFFFFFFu;
 #pragma unroll
   for (int j = 0; j < N; j++) {
     const float f = __uint_as_float(score[j]);
@@ -515,7 +515,7 @@ __device__ __forceinline__ void tc_drain_scores(const TcArgs& a, uint32_t S, con
       if (meta[u] != kTcNoHit) {
         const uint32_t row = T * kTcRows + (meta[u] >> 8);
         qp[u] = (size_t)(a.q0 + (meta[u] & 255u)) * S + part_of(row, S, a.slice);
-        th[u] = __ldg(a.thr + qp[u]);
+        th[u] = a.thr[qp[u]];
         const float f = __uint_as_float(score[u]);
         key[u] = a.rowscale ? key_f32(__fmul_rn(f, __ldg(a.rowscale + row))) : key_i32(__float2int_rn(f));
       }

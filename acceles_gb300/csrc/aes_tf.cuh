@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256) k_tf_tiles(TfMatrix a) {
 // every query value, then E and Q.
 constexpr uint32_t kTfStats = 4;
 
-__global__ void __launch_bounds__(256) k_tf_qstats(const int8_t* __restrict__ q8, uint32_t ld8,
+__global__ void __launch_bounds__(256) k_tf_qstats(const int8_t* q8, uint32_t ld8,
                                                    uint32_t cols, uint32_t sgn, uint32_t* st) {
   grid_wait();
   grid_next();
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(256) k_tf_qstats(const int8_t* __restrict__ q8
 // e4m3 operands of every 128-query block, and E and Q.  A thread takes 16 columns of a query, 16
 // bytes of both layouts (rows of q8 are padded to 16, and the operand's k 16 j .. 16 j + 15 of one
 // query are contiguous).
-__global__ void __launch_bounds__(256) k_tf_qtable(const int8_t* __restrict__ q8, uint32_t ld8,
+__global__ void __launch_bounds__(256) k_tf_qtable(const int8_t* q8, uint32_t ld8,
                                                    uint32_t cols, uint32_t nq, uint32_t nblk, uint32_t sgn,
                                                    uint32_t* st, uint8_t* __restrict__ qt) {
   grid_wait();
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kThreadsCheck) k_recheck(TfCheck a) {
       const uint32_t n4 = (__shfl_sync(0xFFFFFFFFu, m, e) + 3u) >> 2;
       const uint64_t src_h = __shfl_sync(0xFFFFFFFFu, at, e);
       const size_t qp = (size_t)(qb + q) * a.split + part_of(row, a.split, a.slice);
-      const uint32_t th = h < total ? __ldg(a.thr + qp) : 0xFFFFFFFFu;
+      const uint32_t th = h < total ? __ldg(a.thr + qp) : 0xFFFFFFFFu;  // (not a dependent launch)
       int32_t score = 0;
       if (h < total && n4 == 0) {
         const uint32_t c = (uint32_t)(tf_mix(a.seed ^ (uint64_t)row) % (uint64_t)a.cols);
