@@ -141,19 +141,35 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {
 // Waits for the phase of the given parity to complete, for about a second at most, whether or
 // not another role has given up: the MMA thread's wait for its own MMAs in flight before the CTA
 // frees its tensor memory and leaves.
+// Scope: what crosses the CTAs of a pair is waited for at cluster scope, with an acquire for shared
+// memory and relaxed where a tcgen05 fence follows.
+enum TcScope { TC_CTA, TC_CLUSTER, TC_CLUSTER_RELAXED };
+template <TcScope SCOPE = TC_CTA>
 __device__ __forceinline__ uint32_t tc_try(uint32_t bar, uint32_t parity) {
   uint32_t done;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  if constexpr (SCOPE == TC_CTA)
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  else if constexpr (SCOPE == TC_CLUSTER)
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  else
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done;
 }
+template <TcScope SCOPE = TC_CTA>
 __device__ __forceinline__ bool tc_wait_own(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();
   uint32_t done = 0;
   while (!done) {
-    done = tc_try(bar, parity);
+    done = tc_try<SCOPE>(bar, parity);
     if (!done && clock64() - t0 > (1ll << 31)) return false;
   }
   return true;
@@ -161,11 +177,12 @@ __device__ __forceinline__ bool tc_wait_own(uint32_t bar, uint32_t parity) {
 // Waits for the phase of the given parity to complete.  Gives up after about a second, or as
 // soon as another thread of the CTA has given up (*gave_up set), so that every role leaves its
 // loop instead of waiting on a partner that has left.
+template <TcScope SCOPE = TC_CTA>
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up) {
   const long long t0 = clock64();
   uint32_t done = 0;
   while (!done) {
-    done = tc_try(bar, parity);
+    done = tc_try<SCOPE>(bar, parity);
     if (done) break;
     if (*gave_up) return false;
     if (clock64() - t0 > (1ll << 31)) {
@@ -184,21 +201,25 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// A warp's arrival, once for its 32 threads, on a barrier of the pair's even CTA (the one whose
-// thread issues the MMAs), through its shared::cluster address; one CTA: a local arrive.  The
-// default scope: what the arrival orders is shared memory that each CTA wrote itself and handed to
-// the async proxy (fence.proxy.async) or tensor memory that it has read (tcgen05 fence).  A release
-// at cluster scope waits for the thread's global accesses in flight, about 900 cycles, and had to be
-// kept off these paths by threads that forwarded each phase: 2M rows x 1024, 64M entries, 256
-// queries: 395 us so, 331 now.
-template <bool PAIR>
+// A warp's arrival, once for its 32 threads.  PAIR: on the barrier at the same offset in the pair's even
+// CTA (the one whose thread issues the MMAs), through its shared::cluster address and at cluster scope.
+// RELAXED where only tensor-memory reads are handed over: tcgen05.fence orders those, the arrival gives
+// the execution order.  Operand bytes in shared memory want a release, and a release at cluster
+// scope holds the arriving warp up: from the producers it cost 256 queries of 2M rows x 1024, 64M
+// entries 14 us (435 us the whole call for 421 with arrivals at CTA scope, which order nothing
+// between CTAs).  So the odd CTA's producers arrive on their own CTA's barrier, and its MMA warp,
+// which has no MMAs to issue, passes each phase on: 428 us.
+template <bool PAIR, bool RELAXED>
 __device__ __forceinline__ void tc_arrive_warp(uint32_t bar) {
   __syncwarp();
   if ((threadIdx.x & 31u) == 0) {
     if constexpr (PAIR) {
       uint32_t ra;
       asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(ra) : "r"(bar));
-      asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(ra) : "memory");
+      if constexpr (RELAXED)
+        asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(ra) : "memory");
+      else
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(ra) : "memory");
     } else {
       tc_arrive(bar);
     }
@@ -395,7 +416,7 @@ __device__ __forceinline__ void tc_epilogue(const TcArgs& a, uint32_t T, uint32_
     tc_ld16(tmem + dbuf * Q + col0 + ((g * 32u) << 16), v);
     if (col0 + 16u == end) {  // the last load of this unit has completed
       tc_fence_before();
-      tc_arrive_warp<PAIR>(empty);
+      tc_arrive_warp<PAIR, true>(empty);
     }
     float m[2];
 #pragma unroll
@@ -535,8 +556,8 @@ __device__ __forceinline__ void tc_drain_scores(const TcArgs& a, uint32_t S, con
 // unit i / nch; chunk buffer i % NB; accumulator (unit t) t % ACC.
 // PAIR: the even CTA's MMA thread issues cta_group::2 MMAs with M = 256 (the two CTAs' row tiles
 // from their own chunk buffers) and N = 256 (the two CTAs' 128-query operands), and commits them
-// to the barriers of both CTAs; both CTAs' producers and epilogues hand their buffers and
-// accumulators back to the even CTA's barriers.  The two CTAs keep identical shared-memory
+// to the barriers of both CTAs; both CTAs' epilogues hand their accumulators back to the even CTA's
+// barriers, and the odd CTA's staged chunks are passed on to them.  The two CTAs keep identical shared-memory
 // layouts, since an operand descriptor addresses the same offset in both.
 template <uint32_t NB, bool PAIR>
 __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a) {
@@ -547,6 +568,8 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
   constexpr uint32_t kDrain = kEmpty + ACC, kQueued = kDrain + 1, kDrained = kQueued + kTcQueues;
   constexpr uint32_t kBars = tc_nbars(NB, ACC);
   constexpr uint32_t G = tc_group(NB);  // producers of a chunk buffer
+  // what crosses the pair is waited for at cluster scope (tc_arrive_warp)
+  constexpr TcScope kAcq = PAIR ? TC_CLUSTER : TC_CTA, kRlx = PAIR ? TC_CLUSTER_RELAXED : TC_CTA;
   extern __shared__ __align__(16) unsigned char smem[];
   const uint32_t qbytes = (a.kpad / 16u) * 2048u;
   unsigned char* sq = smem;                     // query operand (PAIR: this CTA's 128 queries)
@@ -598,10 +621,10 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
   }
   if (tid == 0) {
     for (uint32_t b = 0; b < kBars; b++) {
-      // one arrival per warp; PAIR: both CTAs' producers and epilogues arrive on the even CTA's
-      // staged and empty barriers
+      // one arrival per warp; PAIR: both CTAs' epilogues arrive on the even CTA's empty barriers, and
+      // the odd CTA's MMA warp once on its staged barriers
       const uint32_t both = PAIR ? 2u : 1u;
-      const uint32_t cnt = (b < kDone) ? both * G / 32
+      const uint32_t cnt = (b < kDone) ? G / 32 + (PAIR && rank == 0 ? 1u : 0u)
                            : ((b >= kEmpty && b < kDrain) ? both * TcShape<PAIR>::EPI / 32
                            : ((b >= kQueued && b < kDrained) ? TcShape<PAIR>::EPI / 32 : 1u));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(tc_smem_u32(bars + b)), "r"(cnt));
@@ -656,7 +679,7 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
     uint32_t j = 0;  // steps done: uses of the buffer
     auto step = [&](TcEnt<G>& cur, TcEnt<G>& old) -> bool {
       if (j > 0) {
-        ok &= tc_wait(b_done + 8u * grp, (j - 1u) & 1u, gave_up);
+        ok &= tc_wait<kAcq>(b_done + 8u * grp, (j - 1u) & 1u, gave_up);
         if (ok) old.stage(ab, a.ent, t, true);
       }
       // every clear lands before any write of this chunk (they may share a byte); the group's
@@ -664,7 +687,7 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
       if (tc_group_any<G>(grp, !ok)) return false;
       cur.stage(ab, a.ent, t, false);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      tc_arrive_warp<PAIR>(b_staged + 8u * grp);
+      tc_arrive_warp<false, false>(b_staged + 8u * grp);
       old.load(a.ent, pb, pe - pb, t);
       ptr_next(pb, pe);
       j++;
@@ -678,7 +701,7 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
     // the odd CTA: before it leaves, the even CTA's commits for its last chunk buffers have landed
     // (those before them were waited for above, those of the accumulators by the epilogue)
     if (PAIR && rank == 1 && t == 0 && go && j > 0) {
-      if (!tc_wait_own(b_done + 8u * grp, (j - 1u) & 1u)) *gave_up = 1u;
+      if (!tc_wait_own<kAcq>(b_done + 8u * grp, (j - 1u) & 1u)) *gave_up = 1u;
     }
   } else if (warp >= kTcEpiWarp) {
     // ---- epilogue -----------------------------------------------------------------------------
@@ -695,14 +718,14 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
       const uint2 st = a.rowstat && row < a.n_rows ? __ldg(a.rowstat + row) : make_uint2(0u, 0u);
       tc_prefetch(a, tc_epi_row(tile_of(unit + tl + 1u)));
       const float lim = a.rowstat ? tc_limit(st, centre, qE, qQ, rs) : 0.0f;
-      if (ok) ok &= tc_wait(b_full + 8u * d, (tl / ACC) & 1u, gave_up);
+      if (ok) ok &= tc_wait<kRlx>(b_full + 8u * d, (tl / ACC) & 1u, gave_up);
       ok = __all_sync(0xFFFFFFFFu, ok);  // tcgen05.ld needs the whole warp
       if (!ok) break;
       tc_fence_after();
       tc_epilogue<PAIR>(a, T, tmem, d, thf, S, rs, lim, b_empty + 8u * d,
                         a.rowstat ? TcQueue{hq_e, hq_n, a.queue_cap}
                                   : TcQueue{hq_e + (size_t)hb * a.queue_cap, hq_n + hb, a.queue_cap});
-      if (!a.rowstat) tc_arrive_warp<false>(b_queued + 8u * hb);
+      if (!a.rowstat) tc_arrive_warp<false, false>(b_queued + 8u * hb);
     }
   } else if (warp >= kTcDrainWarp && warp < kTcDrainWarp + kTcDrains) {
     // ---- drain: appends the queued hits of every third unit, four per lane at a time -----------
@@ -720,6 +743,14 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
         tc_arrive(b_drained + 8u * b);
       }
     }
+  } else if (PAIR && warp == kTcMmaWarp && rank == 1) {
+    // ---- the odd CTA's staged chunks, passed on to the even CTA (tc_arrive_warp) ----------------
+    for (uint32_t i = 0; i < total; i++) {
+      const uint32_t buf = i % NB;
+      ok = tc_wait(b_staged + 8u * buf, (i / NB) & 1u, gave_up);
+      if (!__all_sync(0xFFFFFFFFu, ok)) break;
+      tc_arrive_warp<true, false>(b_staged + 8u * buf);
+    }
   } else if (warp == kTcMmaWarp && rank == 0) {
     // ---- MMA issue (one thread of the warp; PAIR: of the even CTA) -----------------------------
     // The warp keeps together but for the issue itself, so that descriptors and addresses are uniform
@@ -735,8 +766,8 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
     uint32_t tl = 0, c = 0, issued = 0;
     for (uint32_t i = 0; i < total && !a.mma_idle; i++) {
       const uint32_t buf = i % NB, d = tl % ACC;
-      if (c == 0 && tl >= ACC) ok &= tc_wait(b_empty + 8u * d, ((tl - ACC) / ACC) & 1u, gave_up);
-      if (ok) ok &= tc_wait(b_staged + 8u * buf, (i / NB) & 1u, gave_up);
+      if (c == 0 && tl >= ACC) ok &= tc_wait<kRlx>(b_empty + 8u * d, ((tl - ACC) / ACC) & 1u, gave_up);
+      if (ok) ok &= tc_wait<kAcq>(b_staged + 8u * buf, (i / NB) & 1u, gave_up);
       if (!__all_sync(0xFFFFFFFFu, ok)) break;
       tc_fence_after();
       const uint32_t nk = min(kTcChunkK, a.kpad - c * kTcChunkK) / 32u;
@@ -762,12 +793,12 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
     if (issued >= 1) {
       bool drained = true;
       for (uint32_t j = 1; j <= NB && j <= issued; j++)  // the last use of each chunk buffer
-        drained &= tc_wait_own(b_done + 8u * ((issued - j) % NB), ((issued - j) / NB) & 1u);
+        drained &= tc_wait_own<kRlx>(b_done + 8u * ((issued - j) % NB), ((issued - j) / NB) & 1u);
       const uint32_t tiles_full = issued / a.nch;  // units whose accumulator commit was issued
       for (uint32_t j = 1; j <= ACC && j <= tiles_full; j++)  // the last use of each accumulator
-        drained &= tc_wait_own(b_full + 8u * ((tiles_full - j) % ACC), ((tiles_full - j) / ACC) & 1u);
+        drained &= tc_wait_own<kRlx>(b_full + 8u * ((tiles_full - j) % ACC), ((tiles_full - j) / ACC) & 1u);
       if (lead) tc_commit<PAIR>(tc_smem_u32(bars + kDrain), 1);
-      drained &= tc_wait_own(tc_smem_u32(bars + kDrain), 0u);
+      drained &= tc_wait_own<kRlx>(tc_smem_u32(bars + kDrain), 0u);
       if (!drained) *gave_up = 1u;
     }
   }

@@ -58,3 +58,21 @@ def test_dependent_kernels_take_no_read_only_parameters():
         for p in re.findall(r"const\s+\w+\*\s+__restrict__\s+(\w+)", kernels[k][0]):
             assert p in RESIDENT, (k, p)
         assert "grid_wait();" in kernels[k][1], k
+
+
+def test_pair_barriers_are_used_at_cluster_scope():
+    """What crosses the CTAs of a pair is handed over at cluster scope; a barrier operation without a
+    scope orders the threads of one CTA only."""
+    text = _src("aes_tc.cuh")
+    arrives = re.findall(r"mbarrier\.arrive([.\w:]*)\.b64", text)
+    assert any("shared::cluster" in a for a in arrives)
+    for a in arrives:
+        if "shared::cluster" in a:
+            assert re.match(r"\.(release|relaxed)\.cluster\.", a), a
+    body = text[text.index("k_cand_tc(TcArgs a)"):]
+    waits = re.findall(r"tc_wait(?:_own)?(<\w+>)?\((b_\w+)", body)
+    for scope, bar in waits:
+        if bar in ("b_done", "b_full", "b_empty"):
+            assert scope in ("<kAcq>", "<kRlx>"), (bar, scope)
+    staged = [scope for scope, bar in waits if bar == "b_staged"]
+    assert sorted(staged) == ["", "<kAcq>"], staged  # the odd CTA's own phases; the MMA role's
