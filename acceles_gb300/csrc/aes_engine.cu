@@ -218,16 +218,16 @@ struct Engine {
     uint32_t* idx;
     float* score;
     cudaStream_t s;
-    bool pre, host_q;
+    bool pre, host_q, filter;
     bool operator<(const GraphKey& o) const {
-      return std::tie(q, nq, k, idx, score, s, pre, host_q) <
-             std::tie(o.q, o.nq, o.k, o.idx, o.score, o.s, o.pre, o.host_q);
+      return std::tie(q, nq, k, idx, score, s, pre, host_q, filter) <
+             std::tie(o.q, o.nq, o.k, o.idx, o.score, o.s, o.pre, o.host_q, o.filter);
     }
   };
   struct Graph {
     cudaGraphExec_t ex;
     uint64_t launches, cands;  // kernels inside
-    bool batched, tf;          // the forms it runs
+    bool batched;              // the form it runs
   };
   std::map<GraphKey, Graph> graphs;
   uint64_t n_graph_launch = 0;
@@ -247,9 +247,12 @@ struct Engine {
   int batch_warps_n = 0, batch_grid = 0;
   size_t batch_smem = 0;
   uint32_t batch_mode = 0;        // 0 auto, 1 never, else always
-  uint32_t multi_max = 0;         // auto: the most queries that take the four-query pass
+  // auto: the most queries that take the four-query pass, without and with the filter
+  uint32_t multi_max = 0, multi_max_tf = 0;
   bool use_tc = false;            // batched candidate pass on the tensor cores
   bool use_tf = false;            // ... as a filter with an exact check
+  // batches in a row whose rows overflowed the filter's lists, and batches that still go without it
+  uint32_t tf_over = 0, tf_rest = 0;
   bool last_tf = false, last_pre = false;  // of the last run
   uint8_t* d_qtab_tc = nullptr;   // [blocks][tc_qtab_bytes(cols)] e4m3 query operands
   size_t tc_smem = 0;
@@ -363,10 +366,22 @@ struct Engine {
   // d_q: the FP32 queries, or null when there are none (pre-quantised queries alone); pre: the
   // quantised queries are already in d_q8
   // host_q: the queries are still in h_q32 only (d_q == d_q32 is filled on the way)
+  // filter: blocks of 128 take the filter (filter_turn)
   int enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score,
-              cudaStream_t s, bool pre = false, bool host_q = false);
+              cudaStream_t s, bool pre, bool host_q, bool filter);
   int enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score,
-                    cudaStream_t s, bool pre = false, bool host_q = false);
+                    cudaStream_t s, bool pre, bool host_q, bool filter);
+  // blocks of 128 queries, and not the passes of fewer
+  bool takes_blocks(uint32_t nq, bool filter) const {
+    return batch_mode != 1 && (batch_mode != 0 || nq > (filter ? multi_max_tf : multi_max));
+  }
+  // This batch takes the filter: there is one, the batch is large enough, and it is not resting
+  bool filter_turn(uint32_t nq) {
+    if (!use_tf || !takes_blocks(nq, true)) return false;
+    if (!tf_rest) return true;
+    tf_rest--;
+    return false;
+  }
   // CTAs per query of k_final (FinalArgs::comp and done set in `scratch`, nq queries, where more
   // than one)
   uint32_t final_grid(uint32_t nq, void* scratch, size_t scratch_bytes, FinalArgs* fa) const;
@@ -691,6 +706,7 @@ int Engine::apply_config(const Config& c) {
   AES_AL(d_qtab, (size_t)((maxB + kBatchQ - 1) / kBatchQ) * batch_qtab_words(cols));
   use_tc = tc_usable(p, split);
   use_tf = !use_tc && tf_usable(p, split);
+  tf_over = tf_rest = 0;
   if (use_tf) {
     tf_list_cap = tf_list_entries(cap, split);
     AES_AL(d_tf_list, (size_t)sm_count * kTcLists * tf_list_cap);
@@ -729,7 +745,8 @@ int Engine::apply_config(const Config& c) {
   // (300k x 20: 83 / 72 us and 96 / 72 us).  The filter form, 8-bit: 32 queries 170 / 186 us (1M),
   // 277 / 281 us (2M), 482 / 459 us (4M), 40 queries 208 / 203, 336 / 302 and 597 / 488 us; 6-bit
   // 400k x 500 117 / 112 us and 137 / 128 us; 4-bit 1M x 32: 20 queries 162 / 172 us, 24 183 / 171 us.
-  multi_max = use_tc ? 12 : (use_tf ? (bits == 4 ? 20 : 32) : (bits == 8 ? 48 : 64));
+  multi_max = use_tc ? 12 : (bits == 8 ? 48 : 64);
+  multi_max_tf = bits == 4 ? 20 : 32;
   if (batch_mode != 1) {
     batch_smem = batch_smem_bytes((int)bits, cols, split, batch_warps_n);
     int occb = 0;
@@ -1225,10 +1242,10 @@ int Engine::run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s) {
 }
 
 int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score,
-                    cudaStream_t s, bool pre, bool host_q) {
-  const bool batched = batch_mode != 1 && (batch_mode != 0 || nq > multi_max);
+                    cudaStream_t s, bool pre, bool host_q, bool filter) {
+  const bool batched = takes_blocks(nq, filter);
   last_batched = batched;
-  const bool tc = batched && (use_tc || use_tf), tf = batched && use_tf;
+  const bool tf = batched && filter, tc = tf || (batched && use_tc);
   last_tf = tf;
   last_pre = pre;
   // memsets first: the kernels that follow start one out of the other (chain)
@@ -1382,8 +1399,8 @@ uint32_t Engine::final_grid(uint32_t nq, void* scratch, size_t scratch_bytes, Fi
 // Replays the launch sequence of enqueue() as one CUDA graph (captured on first use for these
 // arguments).  Profiling events are not recorded inside graphs.
 int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx,
-                          float* d_score, cudaStream_t s, bool pre, bool host_q) {
-  GraphKey key{d_q, nq, k, d_idx, d_score, s, pre, host_q};
+                          float* d_score, cudaStream_t s, bool pre, bool host_q, bool filter) {
+  GraphKey key{d_q, nq, k, d_idx, d_score, s, pre, host_q, filter};
   auto it = graphs.find(key);
   if (it == graphs.end()) {
     if (graphs.size() >= 64) drop_graphs();
@@ -1392,7 +1409,7 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
     const uint64_t saved_launch = n_launch, saved_cand = n_cand;
     AES_CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     capturing = true;
-    int rc = enqueue(d_q, nq, k, d_idx, d_score, s, pre, host_q);
+    int rc = enqueue(d_q, nq, k, d_idx, d_score, s, pre, host_q, filter);
     capturing = false;
     cudaGraph_t graph = nullptr;
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
@@ -1406,8 +1423,7 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
     ce = cudaGraphInstantiate(&ex, graph, 0);
     cudaGraphDestroy(graph);
     if (ce != cudaSuccess) return ::aes::fail(AES_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ce));
-    it = graphs.emplace(key, Graph{ex, n_launch - saved_launch, n_cand - saved_cand, last_batched,
-                                   last_tf}).first;
+    it = graphs.emplace(key, Graph{ex, n_launch - saved_launch, n_cand - saved_cand, last_batched}).first;
     n_launch = saved_launch;
     n_cand = saved_cand;
   }
@@ -1415,7 +1431,7 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
   n_launch += it->second.launches;
   n_cand += it->second.cands;
   last_batched = it->second.batched;
-  last_tf = it->second.tf;
+  last_tf = filter;
   last_pre = pre;
   n_graph_launch++;
   return AES_OK;
@@ -1433,18 +1449,24 @@ int Engine::repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cud
     if (h_status[q] & ST_DEVICE)
       return fail(AES_ERR_CUDA, "tensor-core candidate pass: a bounded wait gave up");
   }
-  // The filter lets through more rows than reach the thresholds; where that overflows the survivor
-  // buffers of more than a few queries, its bounds are too wide for this data: the batch is run
-  // again, and later ones are run, with the dp4a pass.
+  // The filter lets through more rows than reach the thresholds.  Where that overflows its lists,
+  // its bounds are too wide for these queries, or rows tie at a threshold (every row of a query of
+  // zeros does): the block of 32 queries has no result, and the batch is run again without the filter
+  // (256 queries of 4M x 1024, 8 bits: 1.7 ms; the slow path takes 8.5 ms for one query there).
+  // After one such batch the next tries it again; after the n-th in a row it rests for 2^(n-1)
+  // batches, 128 at most, so that queries that never suit it hardly pay for it.
   if (last_tf) {
-    uint32_t over = 0;
-    for (uint32_t q = 0; q < nq; q++) over += (h_status[q] & ST_OVERFLOW) ? 1u : 0u;
-    if (over * 16 > nq) {
-      use_tf = false;
-      drop_graphs();
-      int rc = enqueue(last_q32, nq, k, d_idx, d_score, s, last_pre);
+    bool over = false;
+    for (uint32_t q = 0; q < nq; q++) over |= (h_status[q] & ST_LIST) != 0;
+    if (over) {
+      tf_over = std::min(tf_over + 1, 8u);
+      tf_rest = tf_over > 1 ? 1u << (tf_over - 1) : 0u;
+      int rc = enqueue(last_q32, nq, k, d_idx, d_score, s, last_pre, false, false);
       if (rc) return rc;
+      AES_CK(cudaEventRecord(ev1, s));  // (aes_run: its time counts)
       AES_CK(cudaStreamSynchronize(s));
+    } else {
+      tf_over = 0;
     }
   }
   for (uint32_t q = 0; q < nq; q++) {
@@ -1784,9 +1806,10 @@ int aes_run(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score, uint
   e.last_q32 = dq;
   e.last_int_final = e.int_final(dq);
   AES_CK(cudaEventRecord(e.ev0, e.stream));
+  const bool filter = e.filter_turn(nq);
   int rc = (e.prm.flags & AES_FLAG_GRAPHS)
-               ? e.enqueue_graph(dq, nq, k, e.h_out_idx, e.h_out_score, e.stream, e.q_pre, host_q)
-               : e.enqueue(dq, nq, k, e.h_out_idx, e.h_out_score, e.stream, e.q_pre, host_q);
+               ? e.enqueue_graph(dq, nq, k, e.h_out_idx, e.h_out_score, e.stream, e.q_pre, host_q, filter)
+               : e.enqueue(dq, nq, k, e.h_out_idx, e.h_out_score, e.stream, e.q_pre, host_q, filter);
   if (rc) return rc;
   AES_CK(cudaEventRecord(e.ev1, e.stream));
   uint32_t rep = 0;
@@ -1824,8 +1847,10 @@ int aes_run_device(aes_handle* h, const float* d_queries, uint32_t nq, uint32_t 
   }
   e.last_q32 = d_queries;
   e.last_int_final = e.int_final(d_queries);
-  int rc = (e.prm.flags & AES_FLAG_GRAPHS) ? e.enqueue_graph(d_queries, nq, k, d_idx, d_score, s)
-                                           : e.enqueue(d_queries, nq, k, d_idx, d_score, s);
+  const bool filter = e.filter_turn(nq);
+  int rc = (e.prm.flags & AES_FLAG_GRAPHS)
+               ? e.enqueue_graph(d_queries, nq, k, d_idx, d_score, s, false, false, filter)
+               : e.enqueue(d_queries, nq, k, d_idx, d_score, s, false, false, filter);
   if (rc) return rc;
   e.last_nq = nq;
   e.last_k = k;

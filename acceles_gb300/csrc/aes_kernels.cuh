@@ -44,6 +44,7 @@ constexpr uint32_t ST_OVERFLOW = 1u;  // survivors exceeded the buffer
 constexpr uint32_t ST_MISS = 2u;      // fewer survivors than candidates needed
 constexpr uint32_t ST_QUERY = 4u;     // query rejected by the quantiser
 constexpr uint32_t ST_DEVICE = 8u;    // a bounded wait on the tensor pipe gave up
+constexpr uint32_t ST_LIST = 16u;     // rows that the filter let through exceeded its lists
 
 __host__ __device__ constexpr int packet_elems(int B) { return 511 / (B + 11); }
 

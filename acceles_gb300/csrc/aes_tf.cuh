@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kThreadsCheck) k_recheck(TfCheck a) {
   for (uint32_t l = threadIdx.x; l < a.ctas; l += kThreadsCheck) atomicMax(&s_most, a.list_n[l * kTcLists + blk]);
   __syncthreads();
   if (s_most > a.list_cap) {
-    if (threadIdx.x < nb && blockIdx.y == 0) atomicOr(a.status + qb + threadIdx.x, ST_OVERFLOW);
+    if (threadIdx.x < nb && blockIdx.y == 0) atomicOr(a.status + qb + threadIdx.x, ST_LIST);
     return;
   }
   // pieces of 32 entries, the j-th of every list before the next, over all warps of the block's CTAs

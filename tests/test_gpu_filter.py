@@ -41,3 +41,63 @@ def test_rows_left_empty(bits, quant):
     eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=bits, quant=quant, split=1, ck=ck, k_max=k,
                  max_batch=nq, batch_tile=128)
     _check(m, eng, Q, 1, ck, k, every=9)
+
+
+def _wide(rows=150_000, nq=70):
+    """Rows and queries whose scores lie closer together than the filter's bounds."""
+    cols, deg = 512, 120
+    rng = np.random.default_rng(5)
+    ptr = (np.arange(rows + 1) * deg).astype(np.uint64)
+    start = rng.integers(0, cols - deg, rows)
+    col = (start[:, None] + np.arange(deg)[None, :]).astype(np.uint32).reshape(-1)
+    val = (115 + rng.integers(-1, 2, rows * deg)).astype(np.float32)
+    val[0] = 127
+    Q = (115 + rng.integers(-1, 2, (nq, cols))).astype(np.float32)
+    Q[:, 0] = 127
+    kw = dict(ptr=ptr, col=col, val=val, bits=8, split=1, ck=8, k_max=8, max_batch=nq, sample_stride=4)
+    return rows, cols, Q, kw
+
+
+def _launches(eng, Q, k):
+    eng.Q_reset(Q)
+    eng.stats(reset=True)
+    ns = eng(k=k)
+    return eng.stats(reset=True)["launches"], ns
+
+
+@pytest.mark.parametrize("rows", [150_000, 600_000])
+def test_ties_leave_the_filter_on(rows):
+    """Queries of zeros tie every row: their survivors (and the filter's lists) overflow whatever the pass.
+    The batch after such a one takes the filter again."""
+    cols, nq, ck, k = 256, 80, 64, 20
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 4, 10, seed=rows)
+    Q = np.random.default_rng(1).random((nq, cols)).astype(np.float32)
+    Z = Q.copy()
+    Z[::10] = 0
+    m = orc.Matrix(rows, cols, ptr, col, val, 8, 0)
+    eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=8, split=1, ck=ck, k_max=k, max_batch=nq)
+    base, _ = _launches(eng, Q, k)
+    _check(m, eng, Z, 1, ck, k, every=5)
+    assert _launches(eng, Q, k)[0] == base
+    _check(m, eng, Q, 1, ck, k, every=16)
+
+
+def test_lists_that_overflow():
+    """The batch is run again without the filter, the second run counts in its time, and a batch that
+    is small enough for it takes the four-query pass while the filter rests."""
+    rows, cols, Q, kw = _wide()
+    eng, dp4a = E.SpMV(rows, cols, **kw), E.SpMV(rows, cols, mem_limit=1 << 40, **kw)
+    assert eng.info()["device_bytes"] > dp4a.info()["device_bytes"] + 8 * 120 * rows  # it has the layout
+    one, _ = _launches(dp4a, Q, 8)
+    ns1 = min(_launches(dp4a, Q, 8)[1] for _ in range(3))
+    two, ns2 = _launches(eng, Q, 8)
+    assert two > one and eng.stats()["repaired"] == 0
+    assert ns2 > ns1
+    assert _launches(eng, Q, 8)[0] == two  # the second in a row; the filter rests for two batches
+    four, _ = _launches(dp4a, Q[:40], 8)
+    assert _launches(eng, Q[:40], 8)[0] == four
+    assert _launches(eng, Q, 8)[0] == one
+    assert _launches(eng, Q, 8)[0] == two
+    m = orc.Matrix(rows, cols, kw["ptr"], kw["col"], kw["val"], 8, 0)
+    for _ in range(2):
+        _check(m, eng, Q, 1, 8, 8, every=30)
