@@ -412,10 +412,11 @@ struct Engine {
     return tf_ready && p.max_batch > 64 && !p.mem_limit && tc_fits(p, S);
   }
   // entries of a filter CTA's list per block of 32 queries: twice its share of what the survivor
-  // buffers of 32 queries hold, or every row it can meet
+  // buffers of 32 queries hold, or every row it can meet, twice: where the epilogue's shares are odd
+  // multiples of 16 queries (65 to 96 on one CTA), two warps append rows to one list
   uint32_t tf_list_entries(uint32_t c, uint32_t S) const {
     const uint64_t share = 2ull * 32 * S * c / (uint32_t)sm_count + 512;
-    const uint64_t all = ((uint64_t)tc_rtiles / std::max(1, sm_count - 1) + 2) * kTcRows;
+    const uint64_t all = 2 * ((uint64_t)tc_rtiles / std::max(1, sm_count - 1) + 2) * kTcRows;
     return (uint32_t)std::min(share, all);
   }
   int build_tf(const HostCSR& m, const aes_params& p, float gmax, size_t planned, size_t config);

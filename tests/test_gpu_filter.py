@@ -101,3 +101,16 @@ def test_lists_that_overflow():
     m = orc.Matrix(rows, cols, kw["ptr"], kw["col"], kw["val"], 8, 0)
     for _ in range(2):
         _check(m, eng, Q, 1, 8, 8, every=30)
+
+
+def test_lists_hold_every_row_twice():
+    """80 queries: the second 32 are shared by two epilogue warps, which append the same rows to one list;
+    where every row passes, the lists still hold them and the batch is not run again."""
+    rows, cols, ck, k = 20000, 128, 4096, 20
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 4, 10, seed=3)
+    Q = np.random.default_rng(1).random((100, cols)).astype(np.float32)
+    m = orc.Matrix(rows, cols, ptr, col, val, 8, 0)
+    eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=8, split=1, ck=ck, k_max=k, max_batch=100)
+    base, _ = _launches(eng, Q, k)
+    assert _launches(eng, Q[:80], k)[0] == base
+    _check(m, eng, Q[:80], 1, ck, k, every=13)
