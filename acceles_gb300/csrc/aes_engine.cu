@@ -419,7 +419,7 @@ struct Engine {
     const uint64_t all = 2 * ((uint64_t)tc_rtiles / std::max(1, sm_count - 1) + 2) * kTcRows;
     return (uint32_t)std::min(share, all);
   }
-  int build_tf(const HostCSR& m, const aes_params& p, float gmax, size_t planned, size_t config);
+  int build_tf(const HostCSR& m, const PackedMatrix& pm, const aes_params& p, size_t planned, size_t config);
 };
 
 // CUDA events around one full candidate-pass launch (AES_FLAG_PROFILE)
@@ -892,7 +892,7 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
       AES_CK(cudaMemcpy(d_tc_ent, pm.tc_ent.data(), pm.tc_ent.size() * 4, cudaMemcpyHostToDevice));
   }
 
-  if ((rc = build_tf(m, p, pm.gmax, plan, c.plan))) return rc;
+  if ((rc = build_tf(m, pm, p, plan, c.plan))) return rc;
   if (tf_ready && (rc = plan_config(p, &c))) return rc;  // (with the filter's lists)
 
   // the shared-memory limit is an attribute of the kernel, shared by every handle: raise it to
@@ -937,9 +937,10 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
 // entry and 24 per row), made on the device from the FP32 CSR: for handles whose batches can reach
 // it (above 64 queries; smaller handles keep their memory), without a memory limit, and only where a quarter of the memory left over
 // holds it.  Not for pre-quantised matrices, nor where a row repeats a column (the dense tile
-// would keep one of the values).
-int Engine::build_tf(const HostCSR& m, const aes_params& p, float gmax, size_t planned, size_t config) {
-  if (p.max_batch <= 64 || p.mem_limit || !has_f32 || m.prequantized || tc_ready || nnz == 0 ||
+// would keep one of the values), nor with infinite or NaN values, whose integers are those of the
+// packer's floating-point arithmetic and not of k_tf_rows' integer arithmetic.
+int Engine::build_tf(const HostCSR& m, const PackedMatrix& pm, const aes_params& p, size_t planned, size_t config) {
+  if (p.max_batch <= 64 || p.mem_limit || !has_f32 || m.prequantized || !pm.finite || tc_ready || nnz == 0 ||
       p.batch_tile == 1)
     return AES_OK;
   const size_t need = nnz * 4 + tf_row_words(nnz, rows) * 4 + rows * 8ull + ((size_t)tc_rtiles * tc_nch + 1) * 4 + config;
@@ -968,7 +969,7 @@ int Engine::build_tf(const HostCSR& m, const aes_params& p, float gmax, size_t p
   a.nch = tc_nch;
   a.bits = (int)bits;
   a.quant = (int)quant;
-  a.gmax = gmax;
+  a.gmax = pm.gmax;
   a.q = d_tf_q;
   a.rowstat = d_tf_rowstat;
   a.ent = d_tf_ent;

@@ -255,27 +255,30 @@ int quantize_and_pack(const HostCSR& m, const aes_params& p, PackedMatrix* out) 
   if (!preq) {
     unsigned nt = std::max(1u, std::thread::hardware_concurrency());
     std::vector<double> part(nt, 0.0);
-    std::vector<char> neg(nt, 0);
+    std::vector<char> neg(nt, 0), inf(nt, 0);
     std::vector<std::thread> th;
     uint64_t chunk = (nnz + nt - 1) / nt;
     for (unsigned t = 0; t < nt; t++) {
       th.emplace_back([&, t] {
         uint64_t b = (uint64_t)t * chunk, e = std::min(nnz, b + chunk);
         double mx = 0.0;
-        char ng = 0;
+        char ng = 0, nf = 0;
         for (uint64_t i = b; i < e; i++) {
           double a = std::fabs((double)m.val[i]);
           if (a > mx) mx = a;
           if (m.val[i] < 0.0f) ng = 1;
+          if (!std::isfinite(m.val[i])) nf = 1;
         }
         part[t] = mx;
         neg[t] = ng;
+        inf[t] = nf;
       });
     }
     for (auto& x : th) x.join();
     for (unsigned t = 0; t < nt; t++) {
       gmax = std::max(gmax, part[t]);
       negative |= (neg[t] != 0);
+      if (inf[t]) out->finite = false;
     }
   }
   out->gmax = (float)gmax;  // (an FP32 value)

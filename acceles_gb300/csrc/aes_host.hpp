@@ -56,7 +56,8 @@ struct PackedMatrix {
   // e4m3 value.  tc_ptr[t * tc_nch + c] is the first entry of (tile t, chunk c).
   std::vector<uint32_t> tc_ptr, tc_ent;
   uint32_t tc_nch = 0;
-  float gmax = 0.0f;  // max |v| of the FP32 values
+  float gmax = 0.0f;   // max |v| of the FP32 values
+  bool finite = true;  // none of them is infinite or NaN
 };
 
 // Quantise (quantify_util.py:8-28 or the per-row variant), drop zero results

@@ -114,3 +114,24 @@ def test_lists_hold_every_row_twice():
     base, _ = _launches(eng, Q, k)
     assert _launches(eng, Q[:80], k)[0] == base
     _check(m, eng, Q[:80], 1, ck, k, every=13)
+
+
+@pytest.mark.parametrize("bits,quant,bad", [(8, 1, np.nan), (6, 0, np.nan), (8, 0, np.inf), (8, 1, np.inf)])
+def test_not_for_values_that_are_not_finite(bits, quant, bad):
+    """An infinite or NaN value leaves its row's (or the matrix's) integers to the packer alone: the
+    candidates are those of the dp4a pass."""
+    rows, cols, nq, ck, k = 4000, 300, 70, 64, 20
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 5, 15, seed=4)
+    for r in range(0, rows, 5):
+        val[int(ptr[r])] = bad
+    kw = dict(ptr=ptr, col=col, val=val, bits=bits, quant=quant, split=1, ck=ck, k_max=k, max_batch=nq,
+              batch_tile=128)
+    Q = np.random.default_rng(2).random((nq, cols)).astype(np.float32)
+    got = []
+    for e in (E.SpMV(rows, cols, **kw), E.SpMV(rows, cols, mem_limit=1 << 40, **kw)):
+        e.Q_reset(Q)
+        e(k=k)
+        got.append([e.read_topk()[0]] + [e.read_candidates(i)[:2] for i in range(0, nq, 9)])
+    assert np.array_equal(got[0][0], got[1][0])
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
