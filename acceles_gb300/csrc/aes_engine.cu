@@ -77,6 +77,9 @@ static PlainKernel pick_plain(int bits, bool sgn, int mode) {
 
 constexpr uint64_t kMultiSampleMax = 16 * 1024;  // sample tiles x groups of four queries
 
+// more device memory that the denser sampling rules may cost a handle
+constexpr size_t kDenseBytes = (size_t)256 << 20;
+
 typedef void (*MultiKernel)(MultiArgs);
 template <int B, bool SAMPLE>
 static MultiKernel multi_kernel(bool sgn, bool scaled) {
@@ -124,6 +127,103 @@ struct SharedAllocs {
   }
 };
 
+// The filter's layout of one matrix (aes_tf.cuh), shared by the handle that built it and its views.
+// Optional memory: where a create, a view or a retune would not fit, the layouts of its device that no
+// batch is on are given back (give_back_layout), and their handles go on with the dp4a pass.
+struct TfLayout {
+  int device = -1;
+  uint32_t *q = nullptr, *ptr = nullptr, *ent = nullptr;  // quantised rows; tile offsets, entries
+  uint2* rowstat = nullptr;
+  size_t bytes = 0;
+
+  ~TfLayout() { free_arrays(); }
+  bool enter() {  // a handle puts a batch on it; false: given back
+    std::lock_guard<std::mutex> lk(mu);
+    if (gone) return false;
+    users++;
+    return true;
+  }
+  void leave() {
+    std::lock_guard<std::mutex> lk(mu);
+    users--;
+  }
+  void keep() {  // a caller's graph holds its addresses
+    std::lock_guard<std::mutex> lk(mu);
+    kept = true;
+  }
+  size_t held() {
+    std::lock_guard<std::mutex> lk(mu);
+    return gone ? 0 : bytes;
+  }
+  bool give_back() {
+    std::lock_guard<std::mutex> lk(mu);
+    if (gone || kept || users) return false;
+    // (a batch of aes_run_device whose handle has run another since may still be on the device)
+    if (cudaSetDevice(device) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    free_arrays();
+    gone = true;
+    return true;
+  }
+
+ private:
+  void free_arrays() {
+    if (device >= 0) cudaSetDevice(device);
+    for (void* p : {(void*)q, (void*)ptr, (void*)ent, (void*)rowstat}) cudaFree(p);
+    q = ptr = ent = nullptr;
+    rowstat = nullptr;
+  }
+  std::mutex mu;
+  uint32_t users = 0;  // handles with a batch on it
+  bool kept = false, gone = false;
+};
+
+static std::mutex g_layouts_mu;
+static std::vector<std::weak_ptr<TfLayout>> g_layouts;  // of every handle of the process
+
+// Frees one idle layout of the device; false: there is none.
+static bool give_back_layout(int device) {
+  std::vector<std::shared_ptr<TfLayout>> all;
+  {
+    std::lock_guard<std::mutex> lk(g_layouts_mu);
+    for (size_t i = 0; i < g_layouts.size();) {
+      if (auto t = g_layouts[i].lock()) {
+        all.push_back(t);
+        i++;
+      } else {
+        g_layouts.erase(g_layouts.begin() + i);
+      }
+    }
+  }
+  for (auto& t : all)
+    if (t->device == device && t->give_back()) return true;
+  return false;
+}
+
+// per-query scratch of aes_run_noalloc
+static constexpr size_t kNoAllocScratchBytes = (size_t)16 << 20;  // 16 MiB
+struct NoAllocLayout {
+  size_t q8, skeys, thr, cnt, surv, cand, cand_key, status, total;
+};
+static NoAllocLayout noalloc_layout(uint32_t ld8, uint32_t n_sample_rows, uint32_t split, uint32_t cap,
+                                    uint32_t nslots) {
+  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  NoAllocLayout L{};
+  size_t o = 0;
+  L.q8 = o;       o += up(ld8);
+  L.skeys = o;    o += up((size_t)std::max<uint32_t>(n_sample_rows, 1) * 4);
+  L.thr = o;      o += up((size_t)split * 4);
+  L.cnt = o;      o += up((size_t)split * 4);
+  L.surv = o;     o += up((size_t)split * cap * 8);
+  L.cand = o;     o += up((size_t)std::max<uint32_t>(nslots, 1) * 4);
+  L.cand_key = o; o += up((size_t)std::max<uint32_t>(nslots, 1) * 4);
+  L.status = o;   o += 256;
+  L.total = o;
+  return L;
+}
+
 struct Engine {
   aes_params prm{};
   int device = 0;
@@ -143,11 +243,10 @@ struct Engine {
   uint32_t* d_tc_ent = nullptr;
   uint32_t tc_nch = 0, tc_rtiles = 0;
   bool tc_ready = false;
-  // the tensor-core pass as a filter (aes_tf.cuh): quantised rows, row sums, layout
-  uint32_t* d_tf_q = nullptr;
-  uint2* d_tf_rowstat = nullptr;
-  uint32_t *d_tf_ptr = nullptr, *d_tf_ent = nullptr;
-  bool tf_ready = false;
+  // the tensor-core pass as a filter (aes_tf.cuh), or null
+  std::shared_ptr<TfLayout> tf;
+  bool tf_mine = false;  // built by this handle: counted in its device bytes
+  bool tf_in = false;    // this handle has a batch on it
   uint2* d_tf_list = nullptr;  // of the configuration: the filter's lists
   uint32_t* d_tf_list_n = nullptr;
   uint32_t tf_list_cap = 0;
@@ -162,6 +261,7 @@ struct Engine {
     uint32_t split = 1, slice = 0, ntop = 0, nslots = 0, ck_eff = 0, cap = 0;
     uint32_t ss = 1, n_sample_tiles = 0, n_sample_rows = 0, maxB = 1;
     std::vector<uint32_t> sample_first, part_begin, part_r;
+    bool tf = false;  // with the filter's lists
     size_t plan = 0;  // device bytes of the configuration's buffers
   };
   Config cur;
@@ -313,6 +413,8 @@ struct Engine {
     free_config();
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
+    tf_leave();
+    tf.reset();
     mat_store.reset();
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -326,6 +428,10 @@ struct Engine {
     size_t b = std::max<size_t>(n * sizeof(T), 16);
     void* q = nullptr;
     cudaError_t e = cudaMalloc(&q, b);
+    while (e == cudaErrorMemoryAllocation && give_back_layout(device)) {
+      cudaGetLastError();
+      e = cudaMalloc(&q, b);
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(AES_ERR_NOMEM, std::string("cudaMalloc refused: ") + cudaGetErrorString(e));
@@ -360,7 +466,11 @@ struct Engine {
   bool capturing = false;
   int build(const HostCSR& m, const aes_params& p);
   int build_view(const Engine& base, const aes_params& p);
-  int plan_config(const aes_params& p, Config* c) const;
+  // lean: the smallest buffers, those of a handle with a memory limit
+  int plan_config(const aes_params& p, bool lean, Config* c) const;
+  int plan_stride(const aes_params& p, uint32_t stride, bool lean, Config* c) const;
+  int admit(const aes_params& p, size_t more, size_t freed, const char* what, Config* c);
+  int apply_or_lean(Config* c);
   int apply_config(const Config& c);
   int retune(const aes_params& p);
   // d_q: the FP32 queries, or null when there are none (pre-quantised queries alone); pre: the
@@ -378,9 +488,16 @@ struct Engine {
   // This batch takes the filter: there is one, the batch is large enough, and it is not resting
   bool filter_turn(uint32_t nq) {
     if (!use_tf || !takes_blocks(nq, true)) return false;
-    if (!tf_rest) return true;
-    tf_rest--;
-    return false;
+    if (tf_rest) {
+      tf_rest--;
+      return false;
+    }
+    if (!tf_in && !tf->enter()) return use_tf = false;
+    return tf_in = true;
+  }
+  void tf_leave() {
+    if (tf_in) tf->leave();
+    tf_in = false;
   }
   // CTAs per query of k_final (FinalArgs::comp and done set in `scratch`, nq queries, where more
   // than one)
@@ -409,7 +526,7 @@ struct Engine {
   }
   // ... as a filter (build_tf has the reasons)
   bool tf_usable(const aes_params& p, uint32_t S) const {
-    return tf_ready && p.max_batch > 64 && !p.mem_limit && tc_fits(p, S);
+    return tf && p.max_batch > 64 && !p.mem_limit && tc_fits(p, S) && tf->held() != 0;
   }
   // entries of a filter CTA's list per block of 32 queries: twice its share of what the survivor
   // buffers of 32 queries hold, or every row it can meet, twice: where the epilogue's shares are odd
@@ -451,9 +568,9 @@ int Engine::prof_close(cudaStream_t s) {
 static_assert(kTcQ == kBatchQ, "tensor-core and dp4a passes use the same query blocks");
 int Engine::run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair) {
   TcArgs a{};
-  a.ent = use_tf ? d_tf_ent : d_tc_ent;
-  a.ptr = use_tf ? d_tf_ptr : d_tc_ptr;
-  a.rowstat = use_tf ? d_tf_rowstat : nullptr;
+  a.ent = use_tf ? tf->ent : d_tc_ent;
+  a.ptr = use_tf ? tf->ptr : d_tc_ptr;
+  a.rowstat = use_tf ? tf->rowstat : nullptr;
   a.qstat = d_exact_aux + 4;
   a.n_rtiles = tc_rtiles;
   a.nch = tc_nch;
@@ -514,7 +631,7 @@ int Engine::run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair) {
 int Engine::run_check(uint32_t q0, uint32_t n, cudaStream_t s, uint32_t ctas) {
   TfCheck c{};
   c.ptr = d_csr_ptr;
-  c.q = reinterpret_cast<const uint4*>(d_tf_q);
+  c.q = reinterpret_cast<const uint4*>(tf->q);
   c.cols = cols;
   c.seed = prm.seed;
   c.q8 = d_q8;
@@ -567,7 +684,41 @@ static size_t matrix_plan(uint64_t tiles, uint32_t rows, uint64_t nnz, uint32_t 
 
 // Host-only: selection geometry, sample tiles, per-partition sample ranks and the device bytes
 // of the configuration's buffers.  Needs rows, cols, tiles and h_tile_rowbase.
-int Engine::plan_config(const aes_params& p, Config* c) const {
+int Engine::plan_config(const aes_params& p, bool lean, Config* c) const {
+  // auto: every tile of a tiny matrix, else one tile in 64, or in 256 of a large matrix with one
+  // partition (a 512-query batch of 95k tiles: 1.92 ms at 256, 2.02 at 128).  Several partitions keep Top-(CK/split) each: the bound of so few candidates from a
+  // sparse sample sits far below the boundary and lets many rows through to the survivor buffers
+  // (10M x 1024, 8-bit, 32 partitions: 99 us per pass at one tile in 256, 85 us at 64), so partitions
+  // of fewer rows are sampled up to one tile in 16, for some 780 rows each (100 queries of
+  // 400k x 500, 6-bit, 32 partitions: 278 us per call at 64, 223 us at 16).
+  // Under a memory limit, or where memory is short (admit), the sparser rule, whose buffers are smaller:
+  // one in 64 and, above 16384 tiles with one partition, 256.  That rule also where the denser one takes
+  // the handle past aes_run_noalloc's scratch or costs it more than kDenseBytes.
+  if (p.sample_stride) return plan_stride(p, p.sample_stride, lean, c);
+  const uint32_t S = p.split <= 1 ? 1 : p.split, rows_part = rows / S;
+  const uint32_t sparse = tiles <= 64 ? 1 : ((tiles <= 16384 || S > 1) ? 64 : 256);
+  uint32_t dense = sparse;
+  if (!lean && !p.mem_limit && tiles > 64) {
+    if (S > 1)
+      while (dense > 16 && rows_part / dense < 780) dense /= 2;
+    else if (tiles <= 65536)
+      dense = 64;
+  }
+  int rc = plan_stride(p, sparse, lean, c);
+  if (rc || dense == sparse) return rc;
+  Config d;
+  if ((rc = plan_stride(p, dense, lean, &d))) return rc;
+  auto scratch = [&](const Config& x) {
+    return noalloc_layout(ld8, x.n_sample_rows, x.split, x.cap, x.nslots).total;
+  };
+  if (d.plan <= c->plan + kDenseBytes &&
+      (scratch(d) <= kNoAllocScratchBytes || scratch(*c) > kNoAllocScratchBytes))
+    *c = std::move(d);
+  return AES_OK;
+}
+
+// ... with every stride-th tile sampled
+int Engine::plan_stride(const aes_params& p, uint32_t stride, bool lean, Config* c) const {
   c->p = p;
   const uint32_t S = p.split <= 1 ? 1 : p.split;
   c->split = S;
@@ -583,23 +734,7 @@ int Engine::plan_config(const aes_params& p, Config* c) const {
   }
 
   // sample tiles: every ss-th tile, with the rows each one owns
-  // auto: every tile of a tiny matrix, else one tile in 64, or in 256 of a large matrix with one
-  // partition (a 512-query batch of 95k tiles: 1.92 ms at 256, 2.02 at 128).  Several partitions keep Top-(CK/split) each: the bound of so few candidates from a
-  // sparse sample sits far below the boundary and lets many rows through to the survivor buffers
-  // (10M x 1024, 8-bit, 32 partitions: 99 us per pass at one tile in 256, 85 us at 64), so partitions
-  // of fewer rows are sampled up to one tile in 16, for some 780 rows each (100 queries of
-  // 400k x 500, 6-bit, 32 partitions: 278 us per call at 64, 223 us at 16).
-  // Under a memory limit the sparser rule, whose buffers are smaller: one in 64 and, above 16384
-  // tiles with one partition, 256.
-  if (p.sample_stride) c->ss = p.sample_stride;
-  else if (tiles <= 64) c->ss = 1;
-  else if (p.mem_limit) c->ss = (tiles <= 16384 || S > 1) ? 64 : 256;
-  else if (S > 1) {
-    c->ss = 64;
-    while (c->ss > 16 && c->slice / c->ss < 780) c->ss /= 2;
-  } else {
-    c->ss = tiles <= 65536 ? 64 : 256;
-  }
+  c->ss = stride;
   const uint32_t ss_ = c->ss;
   c->n_sample_tiles = (uint32_t)((tiles + ss_ - 1) / ss_);
   auto owned_begin = [&](uint64_t t) -> uint64_t {
@@ -659,8 +794,9 @@ int Engine::plan_config(const aes_params& p, Config* c) const {
   plan += maxB * (size_t)c->n_sample_rows * 4;  // the same keys, query-major
   plan += maxB * (ld32 * 4ull + ld8 + S * 8ull + (size_t)S * c->cap * 8 + c->nslots * 8ull + 4);
   plan += nblk * batch_qtab_words(cols) * 4;
-  if (tc_usable(p, S) || tf_usable(p, S)) plan += nblk * tc_qtab_bytes(cols);
-  if (!tc_usable(p, S) && tf_usable(p, S)) plan += (size_t)sm_count * kTcLists * (tf_list_entries(c->cap, S) * 8ull + 4);
+  c->tf = !lean && !tc_usable(p, S) && tf_usable(p, S);
+  if (tc_usable(p, S) || c->tf) plan += nblk * tc_qtab_bytes(cols);
+  if (c->tf) plan += (size_t)sm_count * kTcLists * (tf_list_entries(c->cap, S) * 8ull + 4);
   plan += p.k_max * 8ull;
   c->plan = plan;
 
@@ -668,6 +804,40 @@ int Engine::plan_config(const aes_params& p, Config* c) const {
   if (psmem > (size_t)smem_optin)
     return fail(AES_ERR_UNSUPPORTED, "shared memory of the candidate pass exceeds the device limit");
   return AES_OK;
+}
+
+// Plans a configuration that fits the free memory beside `more` bytes, with `freed` bytes that it will
+// free first: the full one, else the lean one, else the lean one with layouts given back.
+int Engine::admit(const aes_params& p, size_t more, size_t freed, const char* what, Config* c) {
+  size_t freeb = 0;
+  for (const bool lean : {false, true}) {
+    int rc = plan_config(p, lean, c);
+    if (rc) return rc;
+    if (p.mem_limit && more + c->plan > p.mem_limit)
+      return fail(AES_ERR_NOMEM, std::string(what) + " needs " + std::to_string(more + c->plan) +
+                                     " device bytes, over the handle limit " +
+                                     std::to_string(p.mem_limit));
+    do {
+      size_t totalb = 0;
+      AES_CK(cudaMemGetInfo(&freeb, &totalb));
+      if (more + c->plan + (64ull << 20) <= freeb + freed) return AES_OK;
+    } while (lean && give_back_layout(device));
+  }
+  return fail(AES_ERR_NOMEM, std::string(what) + " needs " + std::to_string(more + c->plan) +
+                                 " device bytes, " + std::to_string(freeb + freed) + " free");
+}
+
+// apply_config; where an allocation is refused all the same, the lean form of the same configuration
+int Engine::apply_or_lean(Config* c) {
+  int rc = apply_config(*c);
+  if (rc != AES_ERR_NOMEM) return rc;
+  const std::string why = last_error_cstr();
+  free_config();
+  Config lean;
+  const aes_params p = c->p;
+  if (plan_config(p, true, &lean) != AES_OK || lean.plan >= c->plan) return fail(rc, why);
+  *c = lean;
+  return apply_config(*c);
 }
 
 // Allocates the configuration's buffers, uploads its sample metadata and sets launch geometry.
@@ -706,7 +876,7 @@ int Engine::apply_config(const Config& c) {
   AES_AL(d_status, maxB);
   AES_AL(d_qtab, (size_t)((maxB + kBatchQ - 1) / kBatchQ) * batch_qtab_words(cols));
   use_tc = tc_usable(p, split);
-  use_tf = !use_tc && tf_usable(p, split);
+  use_tf = c.tf;
   tf_over = tf_rest = 0;
   if (use_tf) {
     tf_list_cap = tf_list_entries(cap, split);
@@ -836,21 +1006,12 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
   tc_rtiles = (uint32_t)((rows + kTcRows - 1) / kTcRows);
   const size_t tc_bytes = tc_ready ? (pm.tc_ptr.size() + pm.tc_ent.size()) * 4 : 0;
 
-  Config c;
-  rc = plan_config(p, &c);
-  if (rc) return rc;
-
   // ---- memory plan and admission: nothing is allocated unless all of it fits ---------------
-  const size_t plan = matrix_plan(tiles, rows, nnz, quant, has_f32) + tc_bytes + c.plan;
-  if (p.mem_limit && plan > p.mem_limit)
-    return fail(AES_ERR_NOMEM, "matrix needs " + std::to_string(plan) +
-                                   " device bytes, over the handle limit " +
-                                   std::to_string(p.mem_limit));
-  size_t freeb = 0, totalb = 0;
-  AES_CK(cudaMemGetInfo(&freeb, &totalb));
-  if (plan + (64ull << 20) > freeb)
-    return fail(AES_ERR_NOMEM, "matrix needs " + std::to_string(plan) + " device bytes, " +
-                                   std::to_string(freeb) + " free");
+  Config c;
+  const size_t mat_plan = matrix_plan(tiles, rows, nnz, quant, has_f32) + tc_bytes;
+  rc = admit(p, mat_plan, 0, "matrix", &c);
+  if (rc) return rc;
+  const size_t plan = mat_plan + c.plan;
 
   int rc2 = 0;
 #define AES_AL(ptr, n) if ((rc2 = dalloc(&(ptr), (n))) != AES_OK) return rc2
@@ -893,7 +1054,7 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
   }
 
   if ((rc = build_tf(m, pm, p, plan, c.plan))) return rc;
-  if (tf_ready && (rc = plan_config(p, &c))) return rc;  // (with the filter's lists)
+  if (tf && (rc = plan_config(p, false, &c))) return rc;  // (with the filter's lists)
 
   // the shared-memory limit is an attribute of the kernel, shared by every handle: raise it to
   // the device maximum (less the kernel's static shared memory) once, not to this handle's size
@@ -915,7 +1076,7 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
                         (const void*)k_exact_multi<8, false>, (const void*)k_exact_multi<8, true>,
                         (const void*)k_exact_multi<16, false>, (const void*)k_exact_multi<16, true>})
     AES_CK(raise_smem(f));
-  if (tc_ready || tf_ready) {
+  if (tc_ready || tf) {
     AES_CK(raise_smem((const void*)k_cand_tc<2, false>));
     AES_CK(raise_smem((const void*)k_cand_tc<3, false>));
     AES_CK(raise_smem((const void*)k_cand_tc<2, true>));
@@ -927,16 +1088,17 @@ int Engine::build(const HostCSR& m, const aes_params& p) {
   std::vector<void*> own;
   for (void* q : allocs) (q == (void*)d_allkeys ? own : mat_store->ptrs).push_back(q);
   allocs.swap(own);
-  rc = apply_config(c);
+  rc = apply_or_lean(&c);
   if (rc) return rc;
   AES_CK(cudaDeviceSynchronize());
   return AES_OK;
 }
 
 // The tensor-core layout and exact values behind the filter form of the batched pass (8 bytes per
-// entry and 24 per row), made on the device from the FP32 CSR: for handles whose batches can reach
-// it (above 64 queries; smaller handles keep their memory), without a memory limit, and only where a quarter of the memory left over
-// holds it.  Not for pre-quantised matrices, nor where a row repeats a column (the dense tile
+// entry and 24 per row), made on the device from the FP32 CSR: for handles of more than 64 queries,
+// without a memory limit, and only where a quarter of the memory left over holds it.  64 is no
+// line of speed (that lies at 20 to 32 queries, multi_max_tf): below it a handle takes no more memory
+// than with a limit, so that a budget may be measured on a handle without one.  Not for pre-quantised matrices, nor where a row repeats a column (the dense tile
 // would keep one of the values), nor with infinite or NaN values, whose integers are those of the
 // packer's floating-point arithmetic and not of k_tf_rows' integer arithmetic.
 int Engine::build_tf(const HostCSR& m, const PackedMatrix& pm, const aes_params& p, size_t planned, size_t config) {
@@ -956,10 +1118,17 @@ int Engine::build_tf(const HostCSR& m, const PackedMatrix& pm, const aes_params&
     if (d) dup = true;
   });
   if (dup) return AES_OK;
-  int rc = AES_OK;
-  if ((rc = dalloc(&d_tf_q, tf_row_words(nnz, rows))) || (rc = dalloc(&d_tf_rowstat, rows)) ||
-      (rc = dalloc(&d_tf_ent, nnz)) || (rc = dalloc(&d_tf_ptr, (size_t)tc_rtiles * tc_nch + 1)))
-    return rc;
+  auto t = std::make_shared<TfLayout>();
+  t->device = device;
+  auto get = [&](auto** ptr, size_t n) {
+    t->bytes += n * sizeof(**ptr);
+    return cudaMalloc((void**)ptr, n * sizeof(**ptr));
+  };
+  if (get(&t->q, tf_row_words(nnz, rows)) != cudaSuccess || get(&t->rowstat, rows) != cudaSuccess ||
+      get(&t->ent, nnz) != cudaSuccess || get(&t->ptr, (size_t)tc_rtiles * tc_nch + 1) != cudaSuccess) {
+    cudaGetLastError();  // no filter then
+    return AES_OK;
+  }
   TfMatrix a{};
   a.ptr = d_csr_ptr;
   a.col = d_csr_col;
@@ -970,17 +1139,21 @@ int Engine::build_tf(const HostCSR& m, const PackedMatrix& pm, const aes_params&
   a.bits = (int)bits;
   a.quant = (int)quant;
   a.gmax = pm.gmax;
-  a.q = d_tf_q;
-  a.rowstat = d_tf_rowstat;
-  a.ent = d_tf_ent;
-  a.tptr = d_tf_ptr;
+  a.q = t->q;
+  a.rowstat = t->rowstat;
+  a.ent = t->ent;
+  a.tptr = t->ptr;
   // (the default stream: after the uploads)
-  AES_CK(cudaMemsetAsync(d_tf_q, 0, tf_row_words(nnz, rows) * 4, 0));
+  AES_CK(cudaMemsetAsync(t->q, 0, tf_row_words(nnz, rows) * 4, 0));
   k_tf_rows<<<std::min<uint32_t>((rows + 7) / 8, 16u * (uint32_t)sm_count), 256>>>(a);
   AES_CK(cudaGetLastError());
   k_tf_tiles<<<std::min<uint32_t>(tc_rtiles, 8u * (uint32_t)sm_count), 256>>>(a);
   AES_CK(cudaGetLastError());
-  tf_ready = true;
+  AES_CK(cudaStreamSynchronize(0));
+  tf = t;
+  tf_mine = true;
+  std::lock_guard<std::mutex> lk(g_layouts_mu);
+  g_layouts.push_back(tf);
   return AES_OK;
 }
 
@@ -1004,28 +1177,17 @@ int Engine::build_view(const Engine& b, const aes_params& p) {
   d_tiles = b.d_tiles; d_tile_rowbase = b.d_tile_rowbase; d_rowscale = b.d_rowscale;
   d_tc_ptr = b.d_tc_ptr; d_tc_ent = b.d_tc_ent; tc_nch = b.tc_nch; tc_rtiles = b.tc_rtiles;
   tc_ready = b.tc_ready;
-  d_tf_q = b.d_tf_q; d_tf_rowstat = b.d_tf_rowstat; d_tf_ptr = b.d_tf_ptr; d_tf_ent = b.d_tf_ent;
-  tf_ready = b.tf_ready;
+  tf = b.tf;
   d_csr_ptr = b.d_csr_ptr; d_csr_col = b.d_csr_col; d_csr_val = b.d_csr_val;
   has_f32 = b.has_f32;
   ld32 = b.ld32; ld8 = b.ld8;
   h_tile_rowbase = b.h_tile_rowbase;
   mat_store = b.mat_store;
   Config c;
-  int rc = plan_config(p, &c);
+  int rc = admit(p, rows * 4ull, 0, "view", &c);
   if (rc) return rc;
-  const size_t plan = rows * 4ull + c.plan;
-  if (p.mem_limit && plan > p.mem_limit)
-    return fail(AES_ERR_NOMEM, "view needs " + std::to_string(plan) +
-                                   " device bytes, over the handle limit " +
-                                   std::to_string(p.mem_limit));
-  size_t freeb = 0, totalb = 0;
-  AES_CK(cudaMemGetInfo(&freeb, &totalb));
-  if (plan + (64ull << 20) > freeb)
-    return fail(AES_ERR_NOMEM, "view needs " + std::to_string(plan) + " device bytes, " +
-                                   std::to_string(freeb) + " free");
   if ((rc = dalloc(&d_allkeys, rows)) != AES_OK) return rc;
-  rc = apply_config(c);
+  rc = apply_or_lean(&c);
   if (rc) return rc;
   AES_CK(cudaDeviceSynchronize());
   return AES_OK;
@@ -1040,28 +1202,24 @@ int Engine::retune(const aes_params& p) {
     return fail(AES_ERR_INVALID,
                 "bits, quant, pack_parts, seed and device are fixed by the packed matrix");
   AES_CK(cudaSetDevice(device));
-  Config c;
-  int rc = plan_config(p, &c);
-  if (rc) return rc;
-  if (p.mem_limit && mat_bytes + c.plan > p.mem_limit)
-    return fail(AES_ERR_NOMEM, "configuration needs " + std::to_string(mat_bytes + c.plan) +
-                                   " device bytes, over the handle limit " +
-                                   std::to_string(p.mem_limit));
   AES_CK(cudaDeviceSynchronize());  // runs on caller streams may still read the old buffers
-  size_t freeb = 0, totalb = 0;
-  AES_CK(cudaMemGetInfo(&freeb, &totalb));
-  if (c.plan + (64ull << 20) > freeb + cfg_bytes)
-    return fail(AES_ERR_NOMEM, "configuration needs " + std::to_string(c.plan) +
-                                   " device bytes, " + std::to_string(freeb + cfg_bytes) +
-                                   " available");
+  tf_leave();
+  Config c;
+  // (the matrix arrays count against the limit and are there already)
+  int rc = admit(p, mat_bytes, mat_bytes + cfg_bytes, "configuration", &c);
+  if (rc) return rc;
   Config old = cur;
   free_config();
-  rc = apply_config(c);
+  rc = apply_or_lean(&c);
   if (rc) {
     std::string why = last_error_cstr();
     free_config();
     if (apply_config(old) != AES_OK) free_config();
     return fail(rc, why);
+  }
+  if (p.mem_limit) {  // the limit leaves no room for the layout (views may go on with it)
+    tf.reset();
+    tf_mine = false;
   }
   AES_CK(cudaDeviceSynchronize());
   return AES_OK;
@@ -1444,6 +1602,7 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
 int Engine::repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cudaStream_t s,
                    uint32_t* repaired) {
   AES_CK(cudaStreamSynchronize(s));  // (k_final has written the status words to h_status)
+  tf_leave();
   uint32_t nrep = 0;
   for (uint32_t q = 0; q < nq; q++) {
     if (h_status[q] & ST_QUERY) return fail(AES_ERR_QUERY, "query " + std::to_string(q) +
@@ -1735,7 +1894,7 @@ int aes_get_info(const aes_handle* h, aes_info* info) {
   info->packets = e.packets;
   info->tiles = e.tiles;
   info->packet_bytes = e.packets * 64ull;
-  info->device_bytes = e.bytes;
+  info->device_bytes = e.bytes + (e.tf_mine ? e.tf->held() : 0);
   info->split = e.split;
   info->ck = e.nslots;
   info->ck_effective = e.ck_eff;
@@ -1850,6 +2009,11 @@ int aes_run_device(aes_handle* h, const float* d_queries, uint32_t nq, uint32_t 
   e.last_q32 = d_queries;
   e.last_int_final = e.int_final(d_queries);
   const bool filter = e.filter_turn(nq);
+  if (filter) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    AES_CK(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) e.tf->keep();
+  }
   int rc = (e.prm.flags & AES_FLAG_GRAPHS)
                ? e.enqueue_graph(d_queries, nq, k, d_idx, d_score, s, false, false, filter)
                : e.enqueue(d_queries, nq, k, d_idx, d_score, s, false, false, filter);
@@ -2132,7 +2296,7 @@ int aes_read_candidates(aes_handle* h, uint32_t query, uint32_t* idx, int32_t* s
 // Per-query scratch of aes_run_noalloc lives in this fixed device array instead of memory the
 // call allocates.  The array is part of the library's device image: every GPU that loads the
 // library holds these bytes until the process exits.
-static constexpr size_t kNoAllocScratchBytes = (size_t)16 << 20;  // 16 MiB
+using aes::kNoAllocScratchBytes;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
 namespace {
@@ -2156,26 +2320,6 @@ int noalloc_scratch(int dev, unsigned char** out) {
   return AES_OK;
 }
 
-struct NoAllocLayout {
-  size_t q8, skeys, thr, cnt, surv, cand, cand_key, status, total;
-};
-
-NoAllocLayout noalloc_layout(const aes::Engine& e) {
-  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  NoAllocLayout L{};
-  size_t o = 0;
-  L.q8 = o;       o += up(e.ld8);
-  L.skeys = o;    o += up((size_t)std::max<uint32_t>(e.n_sample_rows, 1) * 4);
-  L.thr = o;      o += up((size_t)e.split * 4);
-  L.cnt = o;      o += up((size_t)e.split * 4);
-  L.surv = o;     o += up((size_t)e.split * e.cap * 8);
-  L.cand = o;     o += up((size_t)std::max<uint32_t>(e.nslots, 1) * 4);
-  L.cand_key = o; o += up((size_t)std::max<uint32_t>(e.nslots, 1) * 4);
-  L.status = o;   o += 256;
-  L.total = o;
-  return L;
-}
-
 }  // namespace
 
 extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, uint32_t* d_idx,
@@ -2186,7 +2330,7 @@ extern "C" int aes_run_noalloc(aes_handle* h, const float* d_query, uint32_t k, 
   if (!e.configured) return aes::fail(AES_ERR_STATE, kUnconfigured);
   if (k == 0 || k > e.prm.k_max) return aes::fail(AES_ERR_INVALID, "k must be in [1, k_max]");
   AES_CK(cudaSetDevice(e.device));
-  const NoAllocLayout L = noalloc_layout(e);
+  const aes::NoAllocLayout L = aes::noalloc_layout(e.ld8, e.n_sample_rows, e.split, e.cap, e.nslots);
   if (L.total > kNoAllocScratchBytes)
     return aes::fail(AES_ERR_UNSUPPORTED,
                      "aes_run_noalloc: this matrix needs " + std::to_string(L.total) +

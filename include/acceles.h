@@ -57,8 +57,11 @@ typedef struct aes_params {
   uint32_t ck;            /* candidates kept (APPROXIMATE_K, types.hpp:149) */
   uint32_t k_max;         /* largest K a run may request (<= 1024) */
   uint32_t max_batch;     /* most queries per aes_set_query / aes_run_device call; above 64 and
-                             without mem_limit the handle also holds the tensor-core filter's
-                             layout (8 B per entry, 24 per row) where memory is ample */
+                             without mem_limit (any value refuses it) the handle also holds the
+                             tensor-core filter's layout (8 B per entry, 24 per row) where memory is
+                             ample.  It is given back, and the handle goes on with the dp4a pass,
+                             where a later create, view or retune needs the memory, or at a retune
+                             with a mem_limit */
   uint32_t pack_parts;    /* Ultra-CSR packing partitions (SPMV_PARTITIONS = 32) */
   uint32_t sample_stride; /* threshold sample: one 32-packet tile in this many (0 = auto) */
   uint32_t batch_tile;    /* queries per matrix pass: 1 = one; 0 = auto: four for a few queries,

@@ -1,5 +1,7 @@
 """GPU tests of the tensor-core filter (6- and 8-bit batches) beside its forms: rows and values at
 its edges, its memory, and how it gives way to the dp4a pass.  Results must equal the oracle's."""
+import contextlib
+
 import numpy as np
 import pytest
 
@@ -135,3 +137,98 @@ def test_not_for_values_that_are_not_finite(bits, quant, bad):
     assert np.array_equal(got[0][0], got[1][0])
     for a, b in zip(got[0][1:], got[1][1:]):
         assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@contextlib.contextmanager
+def _memory_short(left):
+    """Holds device memory so that about `left` bytes stay free."""
+    import torch
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    hold = torch.empty(max(0, (free - left) >> 21) << 21, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        hold.untyped_storage().resize_(0)
+        torch.cuda.empty_cache()
+
+
+def test_layout_is_given_back_where_memory_is_short():
+    """A matrix that fits beside the others' own memory is accepted: the layouts that nobody is using make
+    room, and their handles go on with the dp4a pass."""
+    rows, cols, nq, ck, k = 3_000_000, 256, 80, 64, 20
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 15, 25, seed=8)
+    Q = np.random.default_rng(1).random((nq, cols)).astype(np.float32)
+    kw = dict(ptr=ptr, col=col, val=val, bits=8, split=1, ck=ck, k_max=k, max_batch=nq)
+    m = orc.Matrix(rows, cols, ptr, col, val, 8, 0)
+    probe = E.SpMV(rows, cols, mem_limit=1 << 40, **kw)
+    alone = probe.info()["device_bytes"]
+    dp4a, _ = _launches(probe, Q, k)
+    probe.close()
+    first = E.SpMV(rows, cols, flags=E.FLAG_GRAPHS, **kw)
+    layout = first.info()["device_bytes"] - alone
+    assert layout > 8 * int(ptr[-1])
+    other = first.view()
+    for e in (first, other):
+        _check(m, e, Q, 1, ck, k, every=40)
+    with _memory_short(alone + (64 << 20) - layout // 2):
+        second = E.SpMV(rows, cols, **kw)
+        assert first.info()["device_bytes"] <= alone + layout - 8 * int(ptr[-1])
+        for e in (first, other, second):
+            _check(m, e, Q, 1, ck, k, every=40)
+            assert _launches(e, Q, k)[0] == dp4a
+
+
+def test_lean_buffers_where_memory_is_short():
+    """A view (and a retune) whose full buffers do not fit is made with the buffers of a limited handle."""
+    rows, cols, nq, ck, k = 400_000, 256, 80, 1024, 20
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 15, 25, seed=9)
+    Q = np.random.default_rng(1).random((nq, cols)).astype(np.float32)
+    m = orc.Matrix(rows, cols, ptr, col, val, 8, 0)
+    base = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=8, split=1, ck=ck, k_max=k, max_batch=nq)
+    v = base.view()
+    full = v.info()["device_bytes"]
+    v.close()
+    v = base.view(mem_limit=1 << 40)
+    lean = v.info()["device_bytes"]
+    v.close()
+    assert full > lean + (20 << 20)
+    small = base.view(max_batch=1)
+    _check(m, base, Q, 1, ck, k, every=40)
+    with _memory_short((64 << 20) + (full + lean) // 2):
+        small.retune(max_batch=nq)
+        assert small.info()["device_bytes"] == lean
+        _check(m, small, Q, 1, ck, k, every=40)
+        small.close()
+        v = base.view()
+        assert v.info()["device_bytes"] == lean
+        _check(m, v, Q, 1, ck, k, every=40)
+
+
+def test_memory_limit_at_a_retune_leaves_no_layout():
+    rows, cols, nq = 100_000, 256, 80
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 15, 25, seed=10)
+    kw = dict(ptr=ptr, col=col, val=val, bits=8, split=1, ck=64, k_max=10, max_batch=nq)
+    eng, lim = E.SpMV(rows, cols, **kw), E.SpMV(rows, cols, mem_limit=1 << 40, **kw)
+    need = lim.info()["device_bytes"]
+    eng.retune(mem_limit=need + (1 << 20))
+    assert eng.info()["device_bytes"] <= need + (1 << 20)
+
+
+def test_denser_sampling_keeps_the_fixed_scratch():
+    """Many partitions: a denser sample would take this handle past the scratch of aes_run_noalloc."""
+    import torch
+    rows, cols, split, k = 1_500_000, 64, 2000, 10
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 5, 10, seed=3)
+    eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=8, split=split, ck=split, k_max=k)
+    q = np.random.default_rng(1).random(cols).astype(np.float32)
+    dq = torch.from_numpy(q).cuda()
+    oi = torch.empty(k, dtype=torch.int32, device="cuda")
+    os_ = torch.empty(k, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    eng.run_noalloc(dq.data_ptr(), k, oi.data_ptr(), os_.data_ptr())
+    eng.Q_reset(q)
+    eng(k=k)
+    idx, sc = eng.read_topk()
+    assert np.array_equal(oi.cpu().numpy().view(np.uint32), idx[0])
+    assert np.array_equal(os_.cpu().numpy(), sc[0])
