@@ -36,7 +36,6 @@ struct BatchArgs {
   const uint32_t* qtab;         // [blocks][cols][33] words: bytes of queries 128 b + 4l .. 4l+3 at
                                 // (col, lane l)
   uint32_t nq;                  // queries of the batch (blocks = ceil(nq / 128))
-  uint32_t blk0;                // blocks blk0 .. blk0 + gridDim.y - 1 in this launch
   const float* rowscale;
   uint32_t split, slice;
   const uint32_t* thr;          // [nq][split] (MODE_FILTER)
@@ -384,7 +383,7 @@ __global__ void __launch_bounds__(kWarpsBatchMax * 32, 1) k_cand_batch(BatchArgs
   const uint32_t nwp = gridDim.x * wpc;
   // blockIdx.y selects the block of 128 queries: the blocks of a batch run as successive waves
   // of one launch, each CTA loading its block's query table once
-  const uint32_t blk = a.blk0 + blockIdx.y;
+  const uint32_t blk = blockIdx.y;
   const uint32_t q0 = blk * kBatchQ;
   const uint32_t nq = min((uint32_t)kBatchQ, a.nq - q0);
   {

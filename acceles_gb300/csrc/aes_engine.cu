@@ -507,7 +507,7 @@ struct Engine {
   int repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cudaStream_t s,
              uint32_t* repaired);
   int run_plain(int mode, uint32_t q, cudaStream_t s, uint32_t nq_y = 1, bool first = false);
-  int run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0 = 0, uint32_t nblk = 0);
+  int run_batch(int mode, uint32_t nq, cudaStream_t s);
   int run_multi(uint32_t nq, cudaStream_t s, bool sample = false, bool first = false);
   int run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint32_t* cnt, cudaStream_t s);
   int run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s);
@@ -1275,7 +1275,7 @@ int Engine::run_plain(int mode, uint32_t q, cudaStream_t s, uint32_t nq_y, bool 
 
 // The batched pass of mode over every 128-query block of an nq-query batch in one persistent
 // launch (blocks walked one after another; each CTA loads a block's query table once)
-int Engine::run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0, uint32_t nblk) {
+int Engine::run_batch(int mode, uint32_t nq, cudaStream_t s) {
   BatchArgs a{};
   a.tiles = d_tiles;
   a.tile_rowbase = d_tile_rowbase;
@@ -1284,8 +1284,7 @@ int Engine::run_batch(int mode, uint32_t nq, cudaStream_t s, uint32_t blk0, uint
   a.cols = cols;
   a.qtab = d_qtab;
   a.nq = nq;
-  a.blk0 = blk0;
-  if (!nblk) nblk = (nq + kBatchQ - 1) / kBatchQ - blk0;
+  const uint32_t nblk = (nq + kBatchQ - 1) / kBatchQ;
   a.rowscale = d_rowscale;
   a.split = split;
   a.slice = slice;
@@ -1380,7 +1379,7 @@ int Engine::run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint
     AES_CK(chain(k, g, kThrWarps * 32, 0, s, keys, n_sample_rows, d_part_sample_begin, split,
                  (uint32_t)pairs, d_part_r, thr, cnt));
   } else {
-    AES_CK(chain(k_threshold, dim3(split, nq), kThreadsThr, 0, s, keys, n_sample_rows, 0,
+    AES_CK(chain(k_threshold, dim3(split, nq), kThreadsThr, 0, s, keys, n_sample_rows,
                  d_part_sample_begin, split, d_part_r, thr, cnt));
   }
   return AES_OK;
@@ -2155,7 +2154,7 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     k_exact_sample<<<dim3(groups, n), kThreadsExSample, exact_sample_smem_bytes(e.cols), s>>>(
         fa, S, ns, e.d_allkeys);
     AES_CK(cudaGetLastError());
-    AES_CK(e.chain(k_threshold, dim3(1, n), kThreadsThr, 0, s, e.d_allkeys, ns, 0, e.d_exact_aux, 1,
+    AES_CK(e.chain(k_threshold, dim3(1, n), kThreadsThr, 0, s, e.d_allkeys, ns, e.d_exact_aux, 1,
                       e.d_exact_aux + 2, e.d_thr, e.d_cnt));
     for (uint32_t i = 0; i < n;) {  // groups of 16 queries, then the rest, one alone
       ExactArgs x{};

@@ -214,16 +214,14 @@ __global__ void __launch_bounds__(kThrWarps * 32) k_threshold_warp(
   }
 }
 
-// Sample keys of query q: keys[base(q) + i * stride] with base(q) = q * ld_keys and stride 1
-// (one query per pass), or, when qblk > 0 (batched passes of qblk queries),
-// base(q) = (q / qblk) * qblk * ld_keys + q % qblk and stride qblk.
+// Sample keys of query q: keys_all[q * ld_keys + i].
 //
 // Ranks up to kThrRankMax: every thread's largest key is found in one pass; the r-th largest of
 // those maxima (of groups of two or four threads where r is small) is a bound that r keys reach and
 // few others do, so the few threads at or above it gather their keys of at least that bound, and
 // the r-th largest of the gathered keys is the answer.  One read of the keys, where two
 // histograms took three: 27 -> 12.8 us for 39k keys, r = 24.  Larger ranks: two histograms.
-__global__ void __launch_bounds__(kThreadsThr, 2) k_threshold(const uint32_t* keys_all, uint32_t ld_keys, uint32_t qblk,
+__global__ void __launch_bounds__(kThreadsThr, 2) k_threshold(const uint32_t* keys_all, uint32_t ld_keys,
                             const uint32_t* __restrict__ part_begin, uint32_t split,
                             const uint32_t* __restrict__ r_part, uint32_t* __restrict__ thr,
                             uint32_t* __restrict__ cnt) {
@@ -233,14 +231,7 @@ __global__ void __launch_bounds__(kThreadsThr, 2) k_threshold(const uint32_t* ke
   __shared__ uint32_t smin[kThreadsThr / 32], smax[kThreadsThr / 32], sh[kThreadsThr / 32 + 3];
   __shared__ uint32_t s_bound, s_n;
   const uint32_t p = blockIdx.x, q = blockIdx.y;
-  const uint32_t stride = qblk ? qblk : 1u;
-  const uint32_t* kb = keys_all + (qblk ? (size_t)(q / qblk) * qblk * ld_keys + q % qblk
-                                        : (size_t)q * ld_keys);
-  struct Strided {
-    const uint32_t* b;
-    uint32_t s;
-    __device__ __forceinline__ uint32_t operator[](uint32_t i) const { return b[(size_t)i * s]; }
-  } kk{kb, stride};
+  const uint32_t* kk = keys_all + (size_t)q * ld_keys;
   const uint32_t a = part_begin[p], b = part_begin[p + 1];
   const uint32_t n = b - a;
   const uint32_t r = r_part[p];
