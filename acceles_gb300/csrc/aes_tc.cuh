@@ -1,4 +1,5 @@
-// aes_tc.cuh -- candidate pass of 4-bit matrices on the tensor cores (tcgen05).
+// aes_tc.cuh -- candidate pass on the tensor cores (tcgen05): exact for 4-bit matrices, and the kernel of
+// the filter for the other widths (aes_tf.cuh).
 //
 // The batched candidate pass of aes_batch.cuh scores 128 queries per matrix read with dp4a and is
 // bound by instruction issue.  For B = 4 every matrix value (signed [-8, 7], unsigned [0, 15]) and
@@ -13,12 +14,12 @@
 //     holding the entry's byte offset inside the chunk's operand layout and its e4m3 byte;
 //   - producer warps write a chunk's entries into one of two or three zeroed 32 KB chunk buffers
 //     (and write them back to zero once the MMAs of that chunk have read the buffer);
-//   - one thread issues the chunk's tcgen05.mma (kind::f8f6f4, M = 128, N = 128, K = 32 each)
-//     into one of four 128-column FP32 accumulators in tensor memory; tcgen05.commit signals
-//     mbarriers when a chunk buffer is read and when a tile's accumulator is complete;
+//   - the MMA warp's elected thread issues the chunk's tcgen05.mma (kind::f8f6f4, M = 128, N = 128,
+//     K = 32 each) into one of four 128-column FP32 accumulators in tensor memory; tcgen05.commit
+//     signals mbarriers when a chunk buffer is read and when a tile's accumulator is complete;
 //   - epilogue warps read a complete accumulator with tcgen05.ld while the next tiles' MMAs run and
 //     compare every (row, query) score with the query's threshold; a hit goes into the CTA's queue
-//     (device memory, in practice L2);
+//     (device memory, in practice L2), a filter's into its lists for k_recheck;
 //   - two warps drain the queues, appending the hits to the queries' survivors as the same
 //     candidate keys as in the other passes, so that no epilogue warp waits on an atomic's round trip.
 // Two blocks of 128 queries run together on CTA pairs (cta_group::2, M = 256 over the pair's two
@@ -106,7 +107,7 @@ struct TcArgs {
   const uint32_t* ptr;   // [n_rtiles * nch + 1] first entry of (row tile, chunk)
   uint32_t n_rtiles, nch, kpad, n_rows;
   const uint8_t* qt;     // e4m3 query operand of this launch, tc_qtab_bytes(cols)
-  uint32_t q0, nq;       // this launch scores queries q0 .. q0 + nq - 1 (nq <= 128)
+  uint32_t q0, nq;       // this launch scores queries q0 .. q0 + nq - 1 (nq <= 128, on pairs 256)
   const float* rowscale;
   // filter of approximate scores (aes_tf.cuh), or null: per row {sum |v'| << 13 | ceil(sum |d| / 2),
   // sum v}, and the launch's query statistics
@@ -369,7 +370,14 @@ __device__ __forceinline__ int tc_centre(const uint32_t* st) {
 }
 // Filter of approximate scores: minus what rs times the score may exceed rs times the approximate
 // one by, rounded away from zero: c sum v + E sum |v'| + Q sum |d|, and for the FP32 arithmetic
-// (the accumulator's, this one's and the compare's) 2^-12 of what the products can add up to.
+// (the accumulator's, this one's and the compare's) 2^-12 of Q sum |v'| + |c sum v|.
+// The accumulator takes a K = 32 step at a time, at most 32 of them (1024 columns), and each may
+// lose 2^-23 of it, which stays below P = sum |v' q'| <= (Q + E) sum |v'| <= 1.1 Q sum |v'|: 2^-18 P in
+// all.  That counts on sums that keep 24 bits within a step too, which PTX leaves open; measured, all
+// of 1.4M accumulators equalled the exact sum (1024 columns; operands of 256 x 128, random, of
+// alternating sign, ones after products of 27000, up to 2^25; every sum below 2^24 is then exact).
+// The multiply-add and the compare round the score's distance from the bound by 2^-24 of it.  So 2^-12
+// leaves a factor above 50.
 __device__ __forceinline__ float tc_limit(uint2 st, int centre, float E, float Q, float rs) {
   const float r1 = (float)(st.x >> 13), r2 = 2.0f * (float)(st.x & 0x1FFFu);
   const float c = __fmul_ru((float)centre, __int2float_ru((int)st.y));
@@ -466,7 +474,7 @@ __device__ __forceinline__ void tc_epilogue(const TcArgs& a, uint32_t T, uint32_
   }
 }
 
-constexpr int kTcPer = 12;  // entries of a chunk a producer thread holds (1536 per chunk or more)
+constexpr int kTcPer = 12;  // entries of a chunk a producer thread holds (1536 per chunk with two buffers, 1152 with three)
 
 // A producer's share of one chunk's entries, G threads to a chunk: v[u] = entry b + t + G u for
 // t + G u < n
@@ -728,7 +736,7 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
       if (!a.rowstat) tc_arrive_warp<false, false>(b_queued + 8u * hb);
     }
   } else if (warp >= kTcDrainWarp && warp < kTcDrainWarp + kTcDrains) {
-    // ---- drain: appends the queued hits of every third unit, four per lane at a time -----------
+    // ---- drain: the two warps append the queued hits of every other unit, four per lane at a time
     const uint32_t lane = tid & 31u;
     for (uint32_t tl = warp - kTcDrainWarp; tl < ntl && !a.rowstat; tl += kTcDrains) {
       const uint32_t b = tl % kTcQueues, T = tile_of(unit + tl);

@@ -232,3 +232,30 @@ def test_denser_sampling_keeps_the_fixed_scratch():
     idx, sc = eng.read_topk()
     assert np.array_equal(oi.cpu().numpy().view(np.uint32), idx[0])
     assert np.array_equal(os_.cpu().numpy(), sc[0])
+
+
+@pytest.mark.parametrize("quant,split", [(2, 1), (1, 3), (0, 1)])
+def test_full_rows_of_large_values(quant, split):
+    """Rows with an entry in every column, values and queries near the largest of 8 bits: scores near 2^26
+    a few parts in a thousand apart, where the FP32 accumulation of the filter rounds most."""
+    rows, cols, nq, ck, k = 3000, 1024, 70, 96, 30
+    rng = np.random.default_rng(quant)
+    ptr = np.arange(rows + 1, dtype=np.uint64) * cols
+    col = np.tile(np.arange(cols, dtype=np.uint32), rows)
+    val = (0.9 + 0.1 * rng.random(rows * cols)).astype(np.float32)
+    Q = (0.9 + 0.1 * rng.random((nq, cols))).astype(np.float32)
+    Q[1::2] = rng.random((len(Q[1::2]), cols))
+    if quant == 0:
+        val *= np.where(rng.random(len(val)) < 0.2, -1, 1).astype(np.float32)
+    m = orc.Matrix(rows, cols, ptr, col, val, 8, quant)
+    kw = dict(ptr=ptr, col=col, val=val, bits=8, quant=quant, split=split, ck=ck, k_max=k, max_batch=nq)
+    eng, lim = E.SpMV(rows, cols, **kw), E.SpMV(rows, cols, mem_limit=1 << 40, **kw)
+    assert eng.info()["device_bytes"] > lim.info()["device_bytes"] + 8 * int(ptr[-1])
+    _check(m, eng, Q, split, ck, k, every=7)
+    lim.Q_reset(Q)
+    lim(k=k)
+    for a, b in zip(eng.read_topk(), lim.read_topk()):
+        assert np.array_equal(a, b)
+    for i in range(nq):
+        for a, b in zip(eng.read_candidates(i), lim.read_candidates(i)):
+            assert np.array_equal(a, b)
