@@ -309,6 +309,7 @@ struct Engine {
   uint32_t* last_idx = nullptr;      // device outputs of the last run
   float* last_score = nullptr;
   cudaStream_t last_stream = nullptr;
+  uint32_t settled = 0;              // queries repaired for an aes_run_device before its aes_finish
   bool ran = false;
 
   // CUDA graphs of the per-batch launch sequence, keyed by its arguments
@@ -404,6 +405,7 @@ struct Engine {
     nq_loaded = 0;
     ran = false;
     last_from_device = false;
+    settled = 0;
   }
 
   void release() {
@@ -890,7 +892,7 @@ int Engine::apply_config(const Config& c) {
 #undef AES_AL
   AES_CK(cudaMallocHost(&h_q32, (size_t)maxB * ld32 * sizeof(float)));
   AES_CK(cudaMallocHost(&h_q8, (size_t)maxB * ld8));
-  AES_CK(cudaMallocHost(&h_status, (size_t)maxB * sizeof(uint32_t)));
+  AES_CK(cudaMallocHost(&h_status, 2 * (size_t)maxB * sizeof(uint32_t)));  // (the second half: aes_run_exact's)
   AES_CK(cudaMallocHost(&h_out_idx, (size_t)maxB * std::max<uint32_t>(p.k_max, 1) * sizeof(uint32_t)));
   AES_CK(cudaMallocHost(&h_out_score, (size_t)maxB * std::max<uint32_t>(p.k_max, 1) * sizeof(float)));
   if (n_sample_tiles)
@@ -2023,6 +2025,7 @@ int aes_run_device(aes_handle* h, const float* d_queries, uint32_t nq, uint32_t 
   e.last_score = d_score;
   e.last_stream = s;
   e.last_from_device = true;
+  e.settled = 0;
   e.ran = true;
   return AES_OK;
 }
@@ -2030,7 +2033,8 @@ int aes_run_device(aes_handle* h, const float* d_queries, uint32_t nq, uint32_t 
 int aes_finish(aes_handle* h, uint32_t* repaired) {
   if (!h) return aes::fail(AES_ERR_INVALID, "NULL handle");
   Engine& e = h->e;
-  if (repaired) *repaired = 0;
+  if (repaired) *repaired = e.settled;
+  e.settled = 0;
   if (!e.last_from_device) return AES_OK;
   cudaSetDevice(e.device);
   int rc = e.repair(e.last_nq, e.last_k, e.last_idx, e.last_score, e.last_stream, repaired);
@@ -2068,7 +2072,14 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
   AES_CK(cudaSetDevice(e.device));
   const uint32_t nq = e.nq_loaded;
   cudaStream_t s = e.stream;
+  // its own status words: an aes_run_device may still want its ones at aes_finish
+  uint32_t* const h_status = e.h_status + e.maxB;
   if (!e.q32_on_device) {
+    if (e.last_from_device && e.last_q32 == e.d_q32) {  // its queries are staged there: settle it first
+      int rc = e.repair(e.last_nq, e.last_k, e.last_idx, e.last_score, e.last_stream, &e.settled);
+      if (rc) return rc;
+      e.last_from_device = false;
+    }
     AES_CK(cudaMemcpyAsync(e.d_q32, e.h_q32, (size_t)nq * e.ld32 * 4, cudaMemcpyHostToDevice, s));
     e.q32_on_device = true;
   }
@@ -2112,7 +2123,7 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
   sa.slice = e.rows;
   sa.n_rows = e.rows;
   sa.ntop = k;
-  sa.status = e.d_status;
+  sa.status = e.d_exact_aux + 3;
   // every row of query q: keys, the select over all of them
   auto all_rows = [&](uint32_t q) -> int {
     k_exact_all<false><<<e.sm_count * 8, kExactWarps * 32, exact_all_smem_bytes(e.cols), s>>>(
@@ -2135,11 +2146,11 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     return AES_OK;
   };
   // the sampled rows' keys live in the key array (S queries' samples fit in it), the selected
-  // candidates in the sample keys' memory of the low-bit pass, else one query at a time
+  // candidates and the status words in the sample keys' memory of the low-bit pass, else one query
+  // at a time
   const uint32_t ns = S ? (e.rows + S - 1) / S : 0;
-  uint32_t chunk = S ? (uint32_t)std::min<uint64_t>({e.rows / ns, e.tail_bytes / (k * 8ull), nq}) : 0;
+  uint32_t chunk = S ? (uint32_t)std::min<uint64_t>({e.rows / ns, e.tail_bytes / (k * 8ull + 4), nq}) : 0;
   chunk = std::max<uint32_t>(chunk, 1);
-  AES_CK(cudaMemsetAsync(e.d_status, 0, nq * 4ull, s));
   AES_CK(cudaEventRecord(e.ev0, s));
   for (uint32_t q0 = 0; q0 < nq; q0 += chunk) {
     if (!S) {
@@ -2148,6 +2159,8 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
       continue;
     }
     const uint32_t n = std::min(chunk, nq - q0);
+    uint32_t* const d_status = n > 1 ? e.d_sample_keys + 2 * (size_t)n * k : e.d_exact_aux + 3;
+    AES_CK(cudaMemsetAsync(d_status, 0, n * 4ull, s));
     const float* q32 = e.d_q32 + (size_t)q0 * e.ld32;
     fa.q32 = q32;
     const uint32_t groups = (ns + kExSampleRows - 1) / kExSampleRows;
@@ -2192,7 +2205,7 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     sa.surv = e.d_surv;
     sa.cnt = e.d_cnt;
     sa.cap = e.cap;
-    sa.status = e.d_status + q0;
+    sa.status = d_status;
     sa.cand = n > 1 ? e.d_sample_keys : e.d_exact_cand;
     sa.cand_key = n > 1 ? e.d_sample_keys + (size_t)n * k : e.d_exact_key;
     AES_CK(e.chain(k_select<false>, dim3(1, n), kThreadsSel, 0, s, sa));
@@ -2200,17 +2213,16 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     fa.cand_key = sa.cand_key;
     fa.out_idx = e.h_out_idx + (size_t)q0 * k;
     fa.out_score = e.h_out_score + (size_t)q0 * k;
-    fa.status = e.d_status + q0;
-    fa.status_out = e.h_status + q0;
+    fa.status = d_status;
+    fa.status_out = h_status + q0;
     AES_CK(e.chain(k_final, dim3(1, n), kThreadsFinal, e.final_smem, s, fa));
   }
   AES_CK(cudaEventRecord(e.ev1, s));
   AES_CK(cudaStreamSynchronize(s));
   float total_ms = 0.0f;
   AES_CK(cudaEventElapsedTime(&total_ms, e.ev0, e.ev1));
-  sa.status = e.d_status;
   for (uint32_t q = 0; S && q < nq; q++) {  // the sample bound missed or the buffer overflowed
-    if (!e.h_status[q]) continue;
+    if (!h_status[q]) continue;
     AES_CK(cudaEventRecord(e.ev0, s));
     int rc = all_rows(q);
     if (rc) return rc;
