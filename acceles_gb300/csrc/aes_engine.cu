@@ -328,7 +328,7 @@ struct Engine {
   struct Graph {
     cudaGraphExec_t ex;
     uint64_t launches, cands;  // kernels inside
-    bool batched;              // the form it runs
+    uint32_t pass;             // the form it runs
   };
   std::map<GraphKey, Graph> graphs;
   uint64_t n_graph_launch = 0;
@@ -365,7 +365,7 @@ struct Engine {
   size_t tc_smem2 = 0;
   int tc_grid2 = 0;
   uint32_t tc_nb2 = 2;
-  bool last_batched = false;
+  uint32_t last_pass = AES_PASS_NONE;
   std::vector<uint32_t> h_tile_rowbase;  // host copy: sample geometry is derived from it
   size_t bytes = 0, mat_bytes = 0, cfg_bytes = 0;
   std::vector<void*> allocs, cfg_allocs;  // this handle's own arrays
@@ -623,7 +623,7 @@ int Engine::run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair) {
     AES_CK(chain(k_cand_tc<2, false>, tc_grid, TcShape<false>::THREADS, tc_smem, s, a));
   }
   AES_CK(cudaGetLastError());
-  if (prof && (rc = prof_close(s))) return rc;
+  if (prof && !use_tf && (rc = prof_close(s))) return rc;  // (a filter's time ends with its check)
   n_launch++;
   n_cand++;
   return AES_OK;
@@ -658,7 +658,7 @@ int Engine::run_check(uint32_t q0, uint32_t n, cudaStream_t s, uint32_t ctas) {
               check_smem_bytes(ld8), s>>>(c);
   AES_CK(cudaGetLastError());
   n_launch++;
-  return AES_OK;
+  return (prm.flags & AES_FLAG_PROFILE) ? prof_close(s) : AES_OK;
 }
 
 int Engine::collect_profile() {
@@ -1405,8 +1405,10 @@ int Engine::run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s) {
 int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score,
                     cudaStream_t s, bool pre, bool host_q, bool filter) {
   const bool batched = takes_blocks(nq, filter);
-  last_batched = batched;
   const bool tf = batched && filter, tc = tf || (batched && use_tc);
+  last_pass = tf ? AES_PASS_FILTER
+                 : (tc ? AES_PASS_TENSOR
+                       : (batched ? AES_PASS_DP4A : (batch_mode == 0 && nq > 1 ? AES_PASS_FOUR : AES_PASS_PLAIN)));
   last_tf = tf;
   last_pre = pre;
   // memsets first: the kernels that follow start one out of the other (chain)
@@ -1584,14 +1586,14 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
     ce = cudaGraphInstantiate(&ex, graph, 0);
     cudaGraphDestroy(graph);
     if (ce != cudaSuccess) return ::aes::fail(AES_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ce));
-    it = graphs.emplace(key, Graph{ex, n_launch - saved_launch, n_cand - saved_cand, last_batched}).first;
+    it = graphs.emplace(key, Graph{ex, n_launch - saved_launch, n_cand - saved_cand, last_pass}).first;
     n_launch = saved_launch;
     n_cand = saved_cand;
   }
   AES_CK(cudaGraphLaunch(it->second.ex, s));
   n_launch += it->second.launches;
   n_cand += it->second.cands;
-  last_batched = it->second.batched;
+  last_pass = it->second.pass;
   last_tf = filter;
   last_pre = pre;
   n_graph_launch++;
@@ -2057,6 +2059,12 @@ int aes_get_stats(aes_handle* h, aes_stats* st, int reset) {
     e.n_launch = e.n_cand = e.n_repaired = e.prof_n = 0;
     e.prof_ms = 0.0;
   }
+  return AES_OK;
+}
+
+int aes_last_pass(const aes_handle* h, uint32_t* pass) {
+  if (!h || !pass) return aes::fail(AES_ERR_INVALID, "NULL argument");
+  *pass = h->e.ran ? h->e.last_pass : AES_PASS_NONE;
   return AES_OK;
 }
 

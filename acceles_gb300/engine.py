@@ -41,7 +41,10 @@ GEN_FIXED_UNIFORM = 3
 EXPORTS = ["aes_params_default", "aes_create", "aes_create_csr", "aes_create_quantized",
            "aes_create_view", "aes_destroy", "aes_get_info", "aes_set_query", "aes_set_query_quantized", "aes_run", "aes_read_candidates", "aes_run_device", "aes_finish",
            "aes_last_error", "aes_gen_matrix", "aes_pack_host", "aes_pack_tc_host", "aes_score_all", "aes_get_stats", "aes_run_noalloc", "aes_run_exact",
-           "aes_retune", "aes_read_mtx", "aes_free", "aes_write_mtx", "aes_resparse"]
+           "aes_retune", "aes_read_mtx", "aes_free", "aes_write_mtx", "aes_resparse", "aes_last_pass"]
+
+# forms of the candidate pass (last_pass)
+PASS_NONE, PASS_PLAIN, PASS_FOUR, PASS_DP4A, PASS_TENSOR, PASS_FILTER = range(6)
 
 FLAG_PROFILE = 1
 FLAG_GRAPHS = 2
@@ -178,6 +181,8 @@ def load(build_if_missing: bool = True):
     L.aes_retune.argtypes = [ctypes.c_void_p, ctypes.POINTER(Params)]
     L.aes_get_stats.restype = ctypes.c_int
     L.aes_get_stats.argtypes = [ctypes.c_void_p, ctypes.POINTER(Stats), ctypes.c_int]
+    L.aes_last_pass.restype = ctypes.c_int
+    L.aes_last_pass.argtypes = [ctypes.c_void_p, _u32p]
     L.aes_score_all.restype = ctypes.c_int
     L.aes_score_all.argtypes = [ctypes.c_void_p, _f32p, _u32p]
     _lib = L
@@ -471,6 +476,12 @@ class SpMV:
         st = Stats()
         _check(load().aes_get_stats(self._h, ctypes.byref(st), 1 if reset else 0))
         return {f: getattr(st, f) for f, _ in st._fields_}
+
+    def last_pass(self) -> int:
+        """The form of the candidate pass that the last run took (PASS_*)."""
+        n = ctypes.c_uint32(0)
+        _check(load().aes_last_pass(self._h, ctypes.byref(n)))
+        return n.value
 
     def info(self):
         inf = Info()

@@ -588,7 +588,8 @@ def main():
                   flags=E.FLAG_GRAPHS)
 
     def cand_launch_ms(eng, B, n=3):
-        """Average candidate-pass launch time (CUDA events on the engine's stream), untimed."""
+        """Average candidate-pass launch time (CUDA events on the engine's stream), untimed; launches
+        per step; the form of the pass.  A filter's time is that of its launch and its exact check."""
         eng.retune(flags=E.FLAG_PROFILE)
         Qp = make_queries(B, seed=SEED + 99)
         dq = torch.from_numpy(Qp).cuda()
@@ -602,9 +603,9 @@ def main():
             eng.run_device(dq.data_ptr(), B, K, di.data_ptr(), ds.data_ptr(), sptr)
         torch.cuda.synchronize()
         eng.finish()
-        sp = eng.stats(reset=True)
+        sp, form = eng.stats(reset=True), eng.last_pass()
         eng.retune(flags=E.FLAG_GRAPHS)
-        return sp["cand_ms"] / max(sp["cand_timed"], 1), sp["cand_launches"] / max(n, 1)
+        return sp["cand_ms"] / max(sp["cand_timed"], 1), sp["cand_launches"] / max(n, 1), form
 
     # plain: one candidate pass per query
     Bp = args.batch
@@ -612,7 +613,7 @@ def main():
     info = eng_p.info()
     ms_p, st_p, rep_p, clk_p, Qp_pool, out_p = measure(eng_p, Bp, args.steps, args.warmup)
     plain_qps = world * args.steps * Bp / (ms_p / 1e3)
-    plain_launch_ms, _ = cand_launch_ms(eng_p, Bp)
+    plain_launch_ms, _, _ = cand_launch_ms(eng_p, Bp)
     eng_p.close()
     # batched: one candidate pass per 128 queries
     Bb = args.batch_batched
@@ -620,17 +621,29 @@ def main():
     ms, st, repaired, clk, Qh, out_b = measure(eng, Bb, args.steps, args.warmup)
     B = Bb
     qps = world * args.steps * Bb / (ms / 1e3)
-    batch_launch_ms, cand_per_step = cand_launch_ms(eng, Bb)
+    batch_launch_ms, cand_per_step, form = cand_launch_ms(eng, Bb)
     blocks = (Bb + 127) // 128
 
     # with room for its layout the batched pass is the tensor-core filter (a launch per two blocks of
     # 128 queries, then an exact check), else the dp4a pass (one launch for all blocks)
-    filtered = cand_per_step > 1
+    filtered = form == E.PASS_FILTER
     # dominant kernel of the batched path: the batched candidate pass; algorithmic bytes of one
-    # 128-query block = Ultra-CSR packets + tile row bases + the block's query table
+    # 128-query block = Ultra-CSR packets + tile row bases + the block's query table; of the filter its
+    # share of what a launch reads, the layout's entries, offsets and row sums, and its operand
     alg_bytes = info["packets"] * 64 + (info["tiles"] + 1) * 4 + COLS * 128
+    kpad, rtiles = (COLS + 31) // 32 * 32, (rows + 127) // 128
+    if filtered:
+        layout = info["nnz"] * 4 + rtiles * ((kpad + 255) // 256) * 4 + rows * 8
+        alg_bytes = int(layout * cand_per_step / blocks) + kpad * 128
     cand_ms = batch_launch_ms * cand_per_step / blocks  # device time per 128-query block
     achieved = alg_bytes / (cand_ms / 1e3) / 1e9
+    fp8 = None  # dense products of the filter, its exact check in the time
+    if filtered:
+        p = os.path.join(REPO, "MEASURED_PEAKS.json")
+        bf16 = float(json.load(open(p)).get("bf16_tflops", 1900.0)) if os.path.exists(p) else 1900.0
+        tf = 2.0 * rtiles * 128 * 128 * kpad / (cand_ms / 1e3) / 1e12
+        fp8 = {"bound": "fp8", "unit": "TFLOP/s", "achieved": tf, "peak": 2 * bf16, "frac": tf / (2 * bf16),
+               "peak_note": f"FP8 dense taken as twice bf16 {bf16:.1f} TFLOP/s"}
     plain_alg = info["packets"] * 64 + (info["tiles"] + 1) * 4 + COLS
     plain_achieved = plain_alg / (plain_launch_ms / 1e3) / 1e9
     peak, peak_kind = peaks()
@@ -751,12 +764,13 @@ def main():
                          "kernel": ("k_cand_tc (approximate FP8 scores with a bound; CTA pairs, 256 queries "
                                     "per matrix read), then k_recheck" if filtered else
                                     f"k_cand_batch<{BITS},signed,FILTER> (128 queries per matrix read)"),
-                         "limiter": ("FP8 products of the densified rows and their epilogue" if filtered else
+                         "limiter": ("FP8 products of the densified rows, their epilogue and the exact check"
+                                     if filtered else
                                      "CUDA-core integer issue (gathers, byte transposes, dp4a); "
                                      "one matrix read serves 128 queries"),
                          "alg_bytes_per_block": alg_bytes, "ms_per_block": cand_ms,
                          "launches_per_step": cand_per_step, "blocks_per_step": blocks,
-                         "issue": issue},
+                         "issue": issue, "fp8": fp8},
             "plain_roofline": {"bound": "hbm", "achieved": plain_achieved, "peak": peak,
                                "unit": "GB/s", "frac": plain_achieved / peak,
                                "traffic": plain_traffic, "kernel": f"k_cand_plain<{BITS},signed,FILTER>",

@@ -100,7 +100,8 @@ typedef struct aes_params {
 typedef struct aes_stats {
   uint64_t launches;       /* kernels launched by the engine since the last reset */
   uint64_t cand_launches;  /* full-matrix candidate-pass launches (the dominant kernel) */
-  double cand_ms;          /* device time of those launches (AES_FLAG_PROFILE only) */
+  double cand_ms;          /* device time of those launches (AES_FLAG_PROFILE only), a filter's with
+                              its exact check */
   uint64_t cand_timed;     /* launches included in cand_ms */
   uint64_t repaired;       /* queries sent down the exact slow path */
 } aes_stats;
@@ -238,6 +239,16 @@ int aes_score_all(aes_handle* h, const float* q, uint32_t* keys);
 /* Counters since the previous call (reset = 1 clears them).  Waits for the handle's pending
  * timing events. */
 int aes_get_stats(aes_handle* h, aes_stats* st, int reset);
+
+/* The form of the candidate pass that the last aes_run or aes_run_device took (where a batch was
+ * run again without the filter, the form of that run). */
+#define AES_PASS_NONE 0   /* no run yet */
+#define AES_PASS_PLAIN 1  /* one query per matrix read */
+#define AES_PASS_FOUR 2   /* four */
+#define AES_PASS_DP4A 3   /* blocks of 128 queries */
+#define AES_PASS_TENSOR 4 /* ... on the tensor cores (AES_FLAG_TENSOR) */
+#define AES_PASS_FILTER 5 /* ... as a filter of approximate scores with an exact check */
+int aes_last_pass(const aes_handle* h, uint32_t* pass);
 
 /* Text of the last error on this thread. */
 const char* aes_last_error(void);

@@ -40,3 +40,58 @@ def test_exact_pass_between_a_device_batch_and_its_finish(cols):
         assert np.array_equal(oi[i].cpu().numpy().view(np.uint32), ri), f"device {i}"
         assert np.array_equal(os_[i].cpu().numpy(), rs), f"device {i}"
     assert eng.finish() == 0
+
+
+def test_last_pass():
+    rows, cols, k = 30_000, 256, 10
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 4, 10, seed=2)
+    kw = dict(ptr=ptr, col=col, val=val, split=1, ck=64, k_max=k, max_batch=200)
+    Q = np.random.default_rng(1).random((200, cols)).astype(np.float32)
+
+    def passes(eng, *sizes):
+        out = []
+        for n in sizes:
+            eng.Q_reset(Q[:n])
+            eng(k=k)
+            out.append(eng.last_pass())
+        return out
+
+    eng = E.SpMV(rows, cols, bits=8, flags=E.FLAG_GRAPHS, **kw)
+    assert eng.last_pass() == E.PASS_NONE
+    for _ in range(2):  # captured, replayed
+        assert passes(eng, 1, 4, 32, 33, 100, 200) == [
+            E.PASS_PLAIN, E.PASS_FOUR, E.PASS_FOUR, E.PASS_FILTER, E.PASS_FILTER, E.PASS_FILTER]
+    eng.retune(batch_tile=1)
+    assert passes(eng, 4, 100) == [E.PASS_PLAIN] * 2
+    lim = E.SpMV(rows, cols, bits=8, mem_limit=1 << 40, **kw)
+    assert passes(lim, 33, 48, 49, 200) == [E.PASS_FOUR, E.PASS_FOUR, E.PASS_DP4A, E.PASS_DP4A]
+    ten = E.SpMV(rows, cols, bits=4, flags=E.FLAG_TENSOR, **kw)
+    assert passes(ten, 12, 13, 200) == [E.PASS_FOUR, E.PASS_TENSOR, E.PASS_TENSOR]
+
+
+@pytest.mark.parametrize("nq", [70, 128, 200])
+def test_profile_covers_the_exact_check(nq):
+    """The candidate pass's time of a filter launch holds its exact check: with wide bounds that check
+    scores most rows for every query and takes longer than the FP8 products."""
+    rows, cols, k = 60_000, 512, 10
+    rng = np.random.default_rng(5)
+    deg = 60
+    ptr = (np.arange(rows + 1) * deg).astype(np.uint64)
+    start = rng.integers(0, cols - deg, rows)
+    col = (start[:, None] + np.arange(deg)[None, :]).astype(np.uint32).reshape(-1)
+    val = (100 + rng.integers(-8, 9, rows * deg)).astype(np.float32)
+    val[0] = 127
+    Q = (100 + rng.integers(-8, 9, (nq, cols))).astype(np.float32)
+    Q[:, 0] = 127
+    eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=8, split=1, ck=2048, k_max=k, max_batch=nq,
+                 flags=E.FLAG_PROFILE, sample_stride=4)
+    ns, cand = [], []
+    for _ in range(4):
+        eng.Q_reset(Q)
+        eng.stats(reset=True)
+        t = eng(k=k)
+        assert eng.last_pass() == E.PASS_FILTER
+        st = eng.stats(reset=True)
+        ns.append(t)
+        cand.append(st["cand_ms"] * 1e6)
+    assert min(cand) > 0.5 * min(ns)
