@@ -10,10 +10,13 @@ batched sparse-query workload it was written for.
    CK only adds candidates: the first CK that reaches the target is the smallest.
 2. Sample stride and candidate pass: for each split's CK, every (stride, pass) of the grid is
    timed on the sample batch (wall time of aes_run, repairs included); the fastest wins.  The
-   passes are the plain one (one query per matrix read), the dp4a batched one (128 queries per
-   read) with 16 (the most that fit at 1024 columns), 12 or 8 warps per CTA and, for 4-bit
-   matrices created with AES_FLAG_TENSOR, the tensor-core batched one (FP8 tcgen05 products of
-   128-row tiles; same results).
+   passes are the plain one (one query per matrix read), blocks of 128 queries, and the four-query
+   pass where the handle's own choice (batch_tile 0) is that one.  Blocks are the dp4a pass, with 16
+   (the most that fit at 1024 columns), 12 or 8 warps per CTA, or, where the handle holds the
+   filter's layout and the sample is large enough, the filter, timed once (warps do not change
+   it); for 4-bit matrices created with AES_FLAG_TENSOR also the tensor-core pass (FP8 tcgen05
+   products of 128-row tiles; same results).  A handle holds the filter only for more than 64
+   queries, so a sample of 64 or fewer chooses for batches of that size.
 
 Every trial re-plans the handle with aes_retune; the packed matrix stays resident.
 
@@ -53,6 +56,15 @@ def _recall(idx, exact, k):
     return out
 
 
+def _pass_of(eng, queries, k):
+    """The form of the candidate pass that a run of `queries` takes; None where the engine cannot tell."""
+    if not hasattr(eng, "last_pass"):
+        return None
+    eng.Q_reset(queries)
+    eng(k=k)
+    return eng.last_pass()
+
+
 def _time_runs(eng, queries, k, reps):
     eng.Q_reset(queries)
     eng(k=k)  # warm: graphs, caches
@@ -66,8 +78,9 @@ def _time_runs(eng, queries, k, reps):
     return best, st["repaired"]
 
 
-# (batch_tile, tensor cores, warps per CTA of the dp4a batched pass; 0 = the most that fit)
-PASSES = ((1, False, 0), (128, False, 0), (128, False, 12), (128, False, 8), (128, True, 0))
+# (batch_tile, tensor cores, warps per CTA of the dp4a batched pass; 0 = the most that fit); batch_tile
+# 0 stands for the four-query pass
+PASSES = ((1, False, 0), (128, False, 0), (128, False, 12), (128, False, 8), (128, True, 0), (0, False, 0))
 
 
 def tune(eng: E.SpMV, queries, k, ck_ladder=CK_LADDER, splits=(1,), strides=(0, 16, 64, 256),
@@ -123,6 +136,11 @@ def tune(eng: E.SpMV, queries, k, ck_ladder=CK_LADDER, splits=(1,), strides=(0, 
                     break  # no tensor-core layout for this matrix or split
                 if warps and eng.info()["batch_warps"] != warps:
                     break  # fewer warps fit: the trial of the most that fit covers it
+                form = _pass_of(eng, Q, k) if (warps or tile == 0) else None
+                if tile == 0 and form != E.PASS_FOUR:
+                    break  # the handle's choice is one of the other passes
+                if warps and form == E.PASS_FILTER:
+                    break  # the filter, whatever the dp4a pass's warps
                 sec, repaired = _time_runs(eng, Q, k, reps)
                 row = {"split": split, "ck": ck, "batch_tile": tile, "tensor": tensor,
                        "batch_warps": warps, "sample_stride": stride,
@@ -230,7 +248,7 @@ def main():
         alg = info["quantized_nnz"] * 4 + (rtiles * ((kpad + 255) // 256) + 1) * 4 + q_launch * kpad
         flops = 2.0 * rtiles * 128 * q_launch * kpad
     else:
-        alg = info["packets"] * 64 + (info["tiles"] + 1) * 4 + args.cols * (128 if prm["batch_tile"] == 128 else 1)
+        alg = info["packets"] * 64 + (info["tiles"] + 1) * 4 + args.cols * {128: 128, 0: 4}.get(prm["batch_tile"], 1)
         flops = None
     gbs = alg / (launch_ms / 1e3) / 1e9
     # recall of the measured queries against the FP32-only Top-K
