@@ -142,8 +142,8 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {
 // Waits for the phase of the given parity to complete, for about a second at most, whether or
 // not another role has given up: the MMA thread's wait for its own MMAs in flight before the CTA
 // frees its tensor memory and leaves.
-// Scope: what crosses the CTAs of a pair is waited for at cluster scope, with an acquire for shared
-// memory and relaxed where a tcgen05 fence follows.
+// Scope: what crosses the CTAs of a pair is waited for at cluster scope, relaxed, behind it a fence that
+// acquires shared memory or the tcgen05 fence of the caller.
 enum TcScope { TC_CTA, TC_CLUSTER, TC_CLUSTER_RELAXED };
 template <TcScope SCOPE = TC_CTA>
 __device__ __forceinline__ uint32_t tc_try(uint32_t bar, uint32_t parity) {
@@ -153,16 +153,13 @@ __device__ __forceinline__ uint32_t tc_try(uint32_t bar, uint32_t parity) {
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
         " selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  else if constexpr (SCOPE == TC_CLUSTER)
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   else
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n"
         " selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  if constexpr (SCOPE == TC_CLUSTER)
+    if (done) asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
   return done;
 }
 template <TcScope SCOPE = TC_CTA>
@@ -203,24 +200,21 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 // A warp's arrival, once for its 32 threads.  PAIR: on the barrier at the same offset in the pair's even
-// CTA (the one whose thread issues the MMAs), through its shared::cluster address and at cluster scope.
-// RELAXED where only tensor-memory reads are handed over: tcgen05.fence orders those, the arrival gives
-// the execution order.  Operand bytes in shared memory want a release, and a release at cluster
-// scope holds the arriving warp up: from the producers it cost 256 queries of 2M rows x 1024, 64M
-// entries 14 us (435 us the whole call for 421 with arrivals at CTA scope, which order nothing
-// between CTAs).  So the odd CTA's producers arrive on their own CTA's barrier, and its MMA warp,
-// which has no MMAs to issue, passes each phase on: 428 us.
-template <bool PAIR, bool RELAXED>
+// CTA (the one whose thread issues the MMAs), through its shared::cluster address and at cluster scope,
+// relaxed.  BYTES: operand bytes in shared memory are handed over, released by a fence for shared memory
+// alone (a plain release also waits for global memory: 256 queries of 8M rows x 1024, 256M entries,
+// 1080 us a launch where this takes 1042); else only tensor-memory reads, which tcgen05.fence has ordered.
+// The odd CTA's producers arrive on their own CTA's barrier, and its MMA warp, which has no MMAs to
+// issue, passes each phase on: the fence is off the producers' path (1046 us on it).
+template <bool PAIR, bool BYTES>
 __device__ __forceinline__ void tc_arrive_warp(uint32_t bar) {
   __syncwarp();
   if ((threadIdx.x & 31u) == 0) {
     if constexpr (PAIR) {
       uint32_t ra;
       asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(ra) : "r"(bar));
-      if constexpr (RELAXED)
-        asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(ra) : "memory");
-      else
-        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(ra) : "memory");
+      if constexpr (BYTES) asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+      asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(ra) : "memory");
     } else {
       tc_arrive(bar);
     }
@@ -424,7 +418,7 @@ __device__ __forceinline__ void tc_epilogue(const TcArgs& a, uint32_t T, uint32_
     tc_ld16(tmem + dbuf * Q + col0 + ((g * 32u) << 16), v);
     if (col0 + 16u == end) {  // the last load of this unit has completed
       tc_fence_before();
-      tc_arrive_warp<PAIR, true>(empty);
+      tc_arrive_warp<PAIR, false>(empty);
     }
     float m[2];
 #pragma unroll
@@ -695,7 +689,7 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
       if (tc_group_any<G>(grp, !ok)) return false;
       cur.stage(ab, a.ent, t, false);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      tc_arrive_warp<false, false>(b_staged + 8u * grp);
+      tc_arrive_warp<false, true>(b_staged + 8u * grp);
       old.load(a.ent, pb, pe - pb, t);
       ptr_next(pb, pe);
       j++;
@@ -757,7 +751,7 @@ __global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1) k_cand_tc(TcArgs a)
       const uint32_t buf = i % NB;
       ok = tc_wait(b_staged + 8u * buf, (i / NB) & 1u, gave_up);
       if (!__all_sync(0xFFFFFFFFu, ok)) break;
-      tc_arrive_warp<true, false>(b_staged + 8u * buf);
+      tc_arrive_warp<true, true>(b_staged + 8u * buf);
     }
   } else if (warp == kTcMmaWarp && rank == 0) {
     // ---- MMA issue (one thread of the warp; PAIR: of the even CTA) -----------------------------

@@ -69,6 +69,14 @@ def test_pair_barriers_are_used_at_cluster_scope():
     for a in arrives:
         if "shared::cluster" in a:
             assert re.match(r"\.(release|relaxed)\.cluster\.", a), a
+    # relaxed ones stand behind a fence: of shared memory where bytes are handed over, else tcgen05's
+    hand = text[text.index("void tc_arrive_warp"):]
+    hand = hand[:hand.index("\n}\n")]
+    assert "if constexpr (BYTES) asm volatile(\"fence.release.sync_restrict::shared::cta.cluster;\"" in hand
+    assert hand.index("fence.release") < hand.index("mbarrier.arrive.relaxed.cluster")
+    assert re.search(r"tc_fence_before\(\);\s+tc_arrive_warp<PAIR, false>\(empty\)", text)
+    assert "tc_arrive_warp<true, true>(b_staged" in text
+    assert "if (done) asm volatile(\"fence.acquire.sync_restrict::shared::cluster.cluster;\"" in text
     body = text[text.index("k_cand_tc(TcArgs a)"):]
     waits = re.findall(r"tc_wait(?:_own)?(<\w+>)?\((b_\w+)", body)
     for scope, bar in waits:
