@@ -513,6 +513,7 @@ struct Engine {
   int run_multi(uint32_t nq, cudaStream_t s, bool sample = false, bool first = false);
   int run_threshold(const uint32_t* keys, uint32_t nq, uint32_t* thr, uint32_t* cnt, cudaStream_t s);
   int run_select(SelectArgs& sa, uint32_t nq, cudaStream_t s);
+  int run_final(const FinalArgs& fa, uint32_t per_query, uint32_t nq, cudaStream_t s);
   int run_check(uint32_t q0, uint32_t n, cudaStream_t s, uint32_t ctas);
   int run_tc(uint32_t blk, uint32_t nq_blk, cudaStream_t s, bool pair);
   int prof_open(cudaStream_t s);
@@ -1535,10 +1536,15 @@ int Engine::enqueue(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d_idx, 
   const uint32_t fg = final_grid(nq, d_sample_keys, tail_bytes, &fa);
   sa.done = fa.done;
   if ((rct = run_select(sa, nq, s))) return rct;
-  if (fg * nq <= (uint32_t)sm_count) {
-    AES_CK(chain(k_final, dim3(fg, nq), kThreadsFinal, final_smem, s, fa));
+  return run_final(fa, fg, nq, s);
+}
+
+// k_final behind a select, as its dependent where one CTA per SM holds it (chain)
+int Engine::run_final(const FinalArgs& fa, uint32_t per_query, uint32_t nq, cudaStream_t s) {
+  if (per_query * nq <= (uint32_t)sm_count) {
+    AES_CK(chain(k_final, dim3(per_query, nq), kThreadsFinal, final_smem, s, fa));
   } else {  // two CTAs per SM
-    k_final<<<dim3(fg, nq), kThreadsFinal, final_smem, s>>>(fa);
+    k_final<<<dim3(per_query, nq), kThreadsFinal, final_smem, s>>>(fa);
     AES_CK(cudaGetLastError());
   }
   return AES_OK;
@@ -2223,7 +2229,7 @@ int aes_run_exact(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score
     fa.out_score = e.h_out_score + (size_t)q0 * k;
     fa.status = d_status;
     fa.status_out = h_status + q0;
-    AES_CK(e.chain(k_final, dim3(1, n), kThreadsFinal, e.final_smem, s, fa));
+    if (int rc = e.run_final(fa, 1, n, s)) return rc;
   }
   AES_CK(cudaEventRecord(e.ev1, s));
   AES_CK(cudaStreamSynchronize(s));

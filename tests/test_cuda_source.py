@@ -84,3 +84,12 @@ def test_pair_barriers_are_used_at_cluster_scope():
             assert scope in ("<kAcq>", "<kRlx>"), (bar, scope)
     staged = [scope for scope, bar in waits if bar == "b_staged"]
     assert sorted(staged) == ["", "<kAcq>"], staged  # the odd CTA's own phases; the MMA role's
+
+
+def test_k_final_is_dependent_only_where_one_wave_holds_it():
+    """A dependent kernel of several large CTAs per SM may get one (Engine::chain): k_final is launched
+    so in one place, which looks at its size."""
+    eng = _src("aes_engine.cu")
+    at = [m.start() for m in re.finditer(r"chain\(k_final", eng)]
+    assert len(at) == 1
+    assert "<= (uint32_t)sm_count) {" in eng[at[0] - 80:at[0]]

@@ -95,3 +95,17 @@ def test_profile_covers_the_exact_check(nq):
         ns.append(t)
         cand.append(st["cand_ms"] * 1e6)
     assert min(cand) > 0.5 * min(ns)
+
+
+def test_exact_pass_of_more_queries_than_sms():
+    rows, cols, nq, k = 20_000, 128, 333, 10
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 4, 10, seed=6)
+    val = val - np.float32(0.4)
+    Q = (np.random.default_rng(3).random((nq, cols)) * 2 - 1).astype(np.float32)
+    eng = E.SpMV(rows, cols, ptr=ptr, col=col, val=val, bits=8, split=1, ck=64, k_max=k, max_batch=nq)
+    eng.Q_reset(Q)
+    idx, sc, _ = eng.run_exact(k=k)
+    allrows = np.arange(rows, dtype=np.uint32)
+    for i in range(0, nq, 37):
+        ri, rs = orc.sort_tuples_f32(allrows, orc.rescore_f32(ptr, col, val, Q[i], allrows))
+        assert np.array_equal(idx[i], ri[:k]) and np.array_equal(sc[i], rs[:k]), i
