@@ -139,9 +139,6 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(2048u >> 4) << 16) |
          ((uint64_t)(128u >> 4) << 32) | ((uint64_t)1 << 46);
 }
-// Waits for the phase of the given parity to complete, for about a second at most, whether or
-// not another role has given up: the MMA thread's wait for its own MMAs in flight before the CTA
-// frees its tensor memory and leaves.
 // Scope: what crosses the CTAs of a pair is waited for at cluster scope, relaxed, behind it a fence that
 // acquires shared memory or the tcgen05 fence of the caller.
 enum TcScope { TC_CTA, TC_CLUSTER, TC_CLUSTER_RELAXED };
@@ -162,6 +159,9 @@ __device__ __forceinline__ uint32_t tc_try(uint32_t bar, uint32_t parity) {
     if (done) asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
   return done;
 }
+// Waits for the phase of the given parity to complete, for about a second at most, whether or
+// not another role has given up: the MMA thread's wait for its own MMAs in flight before the CTA
+// frees its tensor memory and leaves.
 template <TcScope SCOPE = TC_CTA>
 __device__ __forceinline__ bool tc_wait_own(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();

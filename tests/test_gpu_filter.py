@@ -259,3 +259,35 @@ def test_full_rows_of_large_values(quant, split):
     for i in range(nq):
         for a, b in zip(eng.read_candidates(i), lim.read_candidates(i)):
             assert np.array_equal(a, b)
+
+
+def test_no_layout_where_a_row_repeats_a_column():
+    """A large value given several times in one column: the dense tile would hold one of them, and the row, a
+    candidate of every query, could be lost.  No layout is built, and blocks take the dp4a pass."""
+    rows, cols, nq, ck, k = 3000, 64, 70, 64, 10
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 3, 6, seed=2)
+    r = np.repeat(np.arange(rows, dtype=np.uint32), np.diff(ptr).astype(np.int64))
+    plain = dict(row=r, col=col, val=val, bits=8, split=1, ck=ck, k_max=k, max_batch=nq)
+    dup = dict(plain, row=np.concatenate([r, np.full(8, 9, np.uint32)]),
+               col=np.concatenate([col, np.repeat(col[int(ptr[9])], 8)]),
+               val=np.concatenate([val, np.full(8, 0.99, np.float32)]))
+    Q = (0.5 + 0.5 * np.random.default_rng(1).random((nq, cols))).astype(np.float32)
+    got = {}
+    for name, kw in (("plain", plain), ("dup", dup), ("limit", dict(dup, mem_limit=1 << 40))):
+        e = E.SpMV(rows, cols, **kw)
+        e.Q_reset(Q)
+        e(k=k)
+        got[name] = (e.last_pass(), e.info()["device_bytes"], e.read_topk()[0])
+    assert got["plain"][0] == E.PASS_FILTER and got["dup"][0] == got["limit"][0] == E.PASS_DP4A
+    assert got["dup"][1] + 8 * len(val) < got["plain"][1]
+    assert np.array_equal(got["dup"][2], got["limit"][2])
+    assert all(9 in row for row in got["dup"][2])
+
+
+def test_the_pass_that_gave_the_results():
+    """Where the lists overflowed, the results are the dp4a pass's."""
+    rows, cols, Q, kw = _wide()
+    eng = E.SpMV(rows, cols, batch_tile=128, flags=E.FLAG_GRAPHS, **kw)
+    eng.Q_reset(Q)
+    eng(k=8)
+    assert eng.last_pass() == E.PASS_DP4A
