@@ -689,11 +689,16 @@ static size_t matrix_plan(uint64_t tiles, uint32_t rows, uint64_t nnz, uint32_t 
 // of the configuration's buffers.  Needs rows, cols, tiles and h_tile_rowbase.
 int Engine::plan_config(const aes_params& p, bool lean, Config* c) const {
   // auto: every tile of a tiny matrix, else one tile in 64, or in 256 of a large matrix with one
-  // partition (a 512-query batch of 95k tiles: 1.92 ms at 256, 2.02 at 128).  Several partitions keep Top-(CK/split) each: the bound of so few candidates from a
-  // sparse sample sits far below the boundary and lets many rows through to the survivor buffers
-  // (10M x 1024, 8-bit, 32 partitions: 99 us per pass at one tile in 256, 85 us at 64), so partitions
-  // of fewer rows are sampled up to one tile in 16, for some 780 rows each (100 queries of
-  // 400k x 500, 6-bit, 32 partitions: 278 us per call at 64, 223 us at 16).
+  // partition.  There a denser sample pays for larger batches up to some 65k tiles (256 queries, 8 bits,
+  // CK 1024, at 64 and 256: 387 / 436 us with 24k tiles, 531 / 583 with 48k, 617 / 693 with 65k, 818 / 770
+  // with 96k; 8 and 40 queries within 4 % from 34k tiles on, 10 % better below); one query pays up to 6 us for it (58 / 52 with
+  // 48k).  Several partitions keep Top-(CK/split) each: the bound of so few candidates from a sparse
+  // sample sits far below the boundary and lets many rows through to the survivor buffers (10M x 1024,
+  // 8-bit, 32 partitions: 99 us per pass at one tile in 256, 85 us at 64), so partitions of fewer rows
+  // are sampled up to one tile in 16, for some 780 rows each (6 bits, 32 partitions, CK 512, 100 queries,
+  // at 16, 32 and 64: 121 / 147 / 193 us with 3125 rows per partition, 174 / 182 / 223 with 12500,
+  // 272 / 252 / 279 with 25000, 389 / 391 / 398 with 50000; 8 queries 65 / 65 / 89, 72 / 77 / 99 and
+  // 101 / 98 / 105 from 12500 on).
   // Under a memory limit, or where memory is short (admit), the sparser rule, whose buffers are smaller:
   // one in 64 and, above 16384 tiles with one partition, 256.  That rule also where the denser one takes
   // the handle past aes_run_noalloc's scratch or costs it more than kDenseBytes.
