@@ -18,6 +18,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <shared_mutex>
 #include <tuple>
 #include <string>
 #include <vector>
@@ -128,37 +129,26 @@ struct SharedAllocs {
 };
 
 // The filter's layout of one matrix (aes_tf.cuh), shared by the handle that built it and its views.
-// Optional memory: where a create, a view or a retune would not fit, the layouts of its device that no
-// batch is on are given back (give_back_layout), and their handles go on with the dp4a pass.
+// Optional memory: where a create, a view or a retune would not fit, the layouts of its device are given
+// back (give_back_layout), and their handles go on with the dp4a pass.
 struct TfLayout {
   int device = -1;
   uint32_t *q = nullptr, *ptr = nullptr, *ent = nullptr;  // quantised rows; tile offsets, entries
   uint2* rowstat = nullptr;
   size_t bytes = 0;
+  std::shared_mutex mu;            // shared: a batch is being enqueued on it
+  bool gone = false;               // given back
+  std::atomic<bool> kept{false};   // a caller's graph holds its addresses
 
   ~TfLayout() { free_arrays(); }
-  bool enter() {  // a handle puts a batch on it; false: given back
-    std::lock_guard<std::mutex> lk(mu);
-    if (gone) return false;
-    users++;
-    return true;
-  }
-  void leave() {
-    std::lock_guard<std::mutex> lk(mu);
-    users--;
-  }
-  void keep() {  // a caller's graph holds its addresses
-    std::lock_guard<std::mutex> lk(mu);
-    kept = true;
-  }
   size_t held() {
-    std::lock_guard<std::mutex> lk(mu);
+    std::shared_lock<std::shared_mutex> lk(mu);
     return gone ? 0 : bytes;
   }
   bool give_back() {
-    std::lock_guard<std::mutex> lk(mu);
-    if (gone || kept || users) return false;
-    // (a batch of aes_run_device whose handle has run another since may still be on the device)
+    std::unique_lock<std::shared_mutex> lk(mu);
+    if (gone || kept) return false;
+    // the batches enqueued on it end first; a later one finds it gone
     if (cudaSetDevice(device) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
       cudaGetLastError();
       return false;
@@ -175,15 +165,12 @@ struct TfLayout {
     q = ptr = ent = nullptr;
     rowstat = nullptr;
   }
-  std::mutex mu;
-  uint32_t users = 0;  // handles with a batch on it
-  bool kept = false, gone = false;
 };
 
 static std::mutex g_layouts_mu;
 static std::vector<std::weak_ptr<TfLayout>> g_layouts;  // of every handle of the process
 
-// Frees one idle layout of the device; false: there is none.
+// Frees one layout of the device; false: there is none to free.
 static bool give_back_layout(int device) {
   std::vector<std::shared_ptr<TfLayout>> all;
   {
@@ -246,7 +233,6 @@ struct Engine {
   // the tensor-core pass as a filter (aes_tf.cuh), or null
   std::shared_ptr<TfLayout> tf;
   bool tf_mine = false;  // built by this handle: counted in its device bytes
-  bool tf_in = false;    // this handle has a batch on it
   uint2* d_tf_list = nullptr;  // of the configuration: the filter's lists
   uint32_t* d_tf_list_n = nullptr;
   uint32_t tf_list_cap = 0;
@@ -415,7 +401,6 @@ struct Engine {
     free_config();
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
-    tf_leave();
     tf.reset();
     mat_store.reset();
     if (ev0) cudaEventDestroy(ev0);
@@ -487,19 +472,18 @@ struct Engine {
   bool takes_blocks(uint32_t nq, bool filter) const {
     return batch_mode != 1 && (batch_mode != 0 || nq > (filter ? multi_max_tf : multi_max));
   }
-  // This batch takes the filter: there is one, the batch is large enough, and it is not resting
-  bool filter_turn(uint32_t nq) {
-    if (!use_tf || !takes_blocks(nq, true)) return false;
+  // Owns its lock where this batch takes the filter: there is one, the batch is large enough, and the
+  // filter is not resting.  Held while the batch is enqueued.
+  std::shared_lock<std::shared_mutex> filter_turn(uint32_t nq) {
+    if (!use_tf || !takes_blocks(nq, true)) return {};
     if (tf_rest) {
       tf_rest--;
-      return false;
+      return {};
     }
-    if (!tf_in && !tf->enter()) return use_tf = false;
-    return tf_in = true;
-  }
-  void tf_leave() {
-    if (tf_in) tf->leave();
-    tf_in = false;
+    std::shared_lock<std::shared_mutex> lk(tf->mu);
+    if (!tf->gone) return lk;
+    use_tf = false;
+    return {};
   }
   // CTAs per query of k_final (FinalArgs::comp and done set in `scratch`, nq queries, where more
   // than one)
@@ -1211,7 +1195,6 @@ int Engine::retune(const aes_params& p) {
                 "bits, quant, pack_parts, seed and device are fixed by the packed matrix");
   AES_CK(cudaSetDevice(device));
   AES_CK(cudaDeviceSynchronize());  // runs on caller streams may still read the old buffers
-  tf_leave();
   Config c;
   // (the matrix arrays count against the limit and are there already)
   int rc = admit(p, mat_bytes, mat_bytes + cfg_bytes, "configuration", &c);
@@ -1616,7 +1599,6 @@ int Engine::enqueue_graph(const float* d_q, uint32_t nq, uint32_t k, uint32_t* d
 int Engine::repair(uint32_t nq, uint32_t k, uint32_t* d_idx, float* d_score, cudaStream_t s,
                    uint32_t* repaired) {
   AES_CK(cudaStreamSynchronize(s));  // (k_final has written the status words to h_status)
-  tf_leave();
   uint32_t nrep = 0;
   for (uint32_t q = 0; q < nq; q++) {
     if (h_status[q] & ST_QUERY) return fail(AES_ERR_QUERY, "query " + std::to_string(q) +
@@ -1981,10 +1963,12 @@ int aes_run(aes_handle* h, uint32_t k, uint32_t* out_idx, float* out_score, uint
   e.last_q32 = dq;
   e.last_int_final = e.int_final(dq);
   AES_CK(cudaEventRecord(e.ev0, e.stream));
-  const bool filter = e.filter_turn(nq);
+  auto turn = e.filter_turn(nq);
+  const bool filter = turn.owns_lock();
   int rc = (e.prm.flags & AES_FLAG_GRAPHS)
                ? e.enqueue_graph(dq, nq, k, e.h_out_idx, e.h_out_score, e.stream, e.q_pre, host_q, filter)
                : e.enqueue(dq, nq, k, e.h_out_idx, e.h_out_score, e.stream, e.q_pre, host_q, filter);
+  if (filter) turn.unlock();
   if (rc) return rc;
   AES_CK(cudaEventRecord(e.ev1, e.stream));
   uint32_t rep = 0;
@@ -2022,15 +2006,17 @@ int aes_run_device(aes_handle* h, const float* d_queries, uint32_t nq, uint32_t 
   }
   e.last_q32 = d_queries;
   e.last_int_final = e.int_final(d_queries);
-  const bool filter = e.filter_turn(nq);
+  auto turn = e.filter_turn(nq);
+  const bool filter = turn.owns_lock();
   if (filter) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     AES_CK(cudaStreamIsCapturing(s, &cap));
-    if (cap != cudaStreamCaptureStatusNone) e.tf->keep();
+    if (cap != cudaStreamCaptureStatusNone) e.tf->kept = true;
   }
   int rc = (e.prm.flags & AES_FLAG_GRAPHS)
                ? e.enqueue_graph(d_queries, nq, k, d_idx, d_score, s, false, false, filter)
                : e.enqueue(d_queries, nq, k, d_idx, d_score, s, false, false, filter);
+  if (filter) turn.unlock();
   if (rc) return rc;
   e.last_nq = nq;
   e.last_k = k;

@@ -291,3 +291,104 @@ def test_the_pass_that_gave_the_results():
     eng.Q_reset(Q)
     eng(k=8)
     assert eng.last_pass() == E.PASS_DP4A
+
+
+def test_layout_in_use_is_given_back_between_batches():
+    """Threads that keep batches on a layout do not keep its memory from a create that needs it."""
+    import threading
+    rows, cols, nq, ck, k = 3_000_000, 256, 80, 64, 20
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 15, 25, seed=8)
+    Q = np.random.default_rng(1).random((nq, cols)).astype(np.float32)
+    kw = dict(ptr=ptr, col=col, val=val, bits=8, split=1, ck=ck, k_max=k, max_batch=nq)
+    probe = E.SpMV(rows, cols, mem_limit=1 << 40, **kw)
+    alone = probe.info()["device_bytes"]
+    probe.Q_reset(Q)
+    probe(k=k)
+    want = probe.read_topk()
+    probe.close()
+    first = E.SpMV(rows, cols, **kw)
+    layout = first.info()["device_bytes"] - alone
+    handles = [first, first.view(), first.view(flags=E.FLAG_GRAPHS)]
+    seen, bad, stop = [set(), set(), set()], [], threading.Event()
+
+    def serve(i):
+        e = handles[i]
+        while not stop.is_set():
+            e.Q_reset(Q)
+            e(k=k)
+            seen[i].add(e.last_pass())
+            idx, sc = e.read_topk()
+            if not (np.array_equal(idx, want[0]) and np.array_equal(sc, want[1])):
+                bad.append(i)
+
+    threads = [threading.Thread(target=serve, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    try:
+        while not all(E.PASS_FILTER in s for s in seen):
+            assert any(t.is_alive() for t in threads)
+        with _memory_short(alone + (64 << 20) - layout // 2):
+            second = E.SpMV(rows, cols, **kw)
+            second.Q_reset(Q)
+            second(k=k)
+            assert np.array_equal(second.read_topk()[0], want[0])
+            for s in seen:
+                s.clear()
+            while not all(seen):
+                assert any(t.is_alive() for t in threads)
+    finally:
+        stop.set()
+        for t in threads:
+            t.join()
+    assert not bad
+    assert all(s == {E.PASS_DP4A} for s in seen)
+
+
+def test_layout_of_a_captured_batch_is_kept():
+    """A caller's graph holds the layout's addresses: its replays stay valid, a create that would need that
+    memory is refused."""
+    import torch
+    rows, cols, nq, ck, k = 3_000_000, 256, 80, 64, 20
+    ptr, col, val = E.gen_matrix(E.GEN_UNIFORM_DEG, rows, cols, 15, 25, seed=8)
+    rng = np.random.default_rng(1)
+    Q = rng.random((2, nq, cols)).astype(np.float32)
+    kw = dict(ptr=ptr, col=col, val=val, bits=8, split=1, ck=ck, k_max=k, max_batch=nq)
+    eng = E.SpMV(rows, cols, **kw)
+    lim = E.SpMV(rows, cols, mem_limit=1 << 40, **kw)
+    alone = lim.info()["device_bytes"]
+    layout = eng.info()["device_bytes"] - alone
+    want = []
+    for q in Q:
+        lim.Q_reset(q)
+        lim(k=k)
+        want.append(tuple(x.copy() for x in lim.read_topk()))
+    lim.close()
+    dq = torch.from_numpy(Q[0]).cuda()
+    oi = torch.zeros((nq, k), dtype=torch.int32, device="cuda")
+    os_ = torch.zeros((nq, k), dtype=torch.float32, device="cuda")
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    eng.run_device(dq.data_ptr(), nq, k, oi.data_ptr(), os_.data_ptr(), s.cuda_stream)
+    eng.finish()
+    assert eng.last_pass() == E.PASS_FILTER
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s, capture_error_mode="thread_local"):
+        eng.run_device(dq.data_ptr(), nq, k, oi.data_ptr(), os_.data_ptr(), s.cuda_stream)
+
+    def replay(i):
+        dq.copy_(torch.from_numpy(Q[i]))
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        assert eng.finish() == 0
+        assert np.array_equal(oi.cpu().numpy().view(np.uint32), want[i][0])
+        assert np.array_equal(os_.cpu().numpy(), want[i][1])
+
+    replay(0)
+    replay(1)
+    with _memory_short(alone + (64 << 20) - layout // 2):
+        with pytest.raises(E.AesError) as ei:
+            E.SpMV(rows, cols, **kw)
+        assert ei.value.code == E.AES_ERR_NOMEM
+        replay(0)
+    replay(1)
