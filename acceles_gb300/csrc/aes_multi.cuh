@@ -40,7 +40,7 @@ struct MultiArgs {
 
 __host__ inline size_t multi_smem_bytes(uint32_t cols, uint32_t split) {
   return (size_t)cols * kPlainTableBytesPerCol + (size_t)kMultiWarps * kPlainTileBuf +
-         (split > 1 && split <= kThrSmemMax ? (size_t)split * kMultiQ * 4 : 0);
+         (split <= kThrSmemMax ? (size_t)split * kMultiQ * 4 : 0);
 }
 
 // Thresholds and survivors of the CTA's four queries.  A row is compared with bounds on what the
@@ -89,13 +89,10 @@ struct MultiEmit {
     const bool hit = (x[0] >= b[0]) | (x[1] >= b[1]) | (x[2] >= b[2]) | (x[3] >= b[3]);
     if (valid && hit) {
       const uint32_t p = part_of(row, a.split, a.slice);
-      uint32_t th[kMultiQ];  // all four in flight, before the atomics
-#pragma unroll
-      for (int t = 0; t < kMultiQ; t++) th[t] = thr_key(p, t);
 #pragma unroll
       for (int t = 0; t < kMultiQ; t++) {
         const uint32_t key = SCALED ? key_f32(__uint_as_float((uint32_t)x[t])) : key_i32(x[t] >> SHIFT);
-        if (key >= th[t] && (uint32_t)t < nq) {
+        if (key >= thr_key(p, t) && (uint32_t)t < nq) {
           const size_t qp = (size_t)(q0 + t) * a.split + p;
           const uint32_t i = atomicAdd(a.cnt + qp, 1u);
           if (i < a.cap) a.surv[qp * a.cap + i] = make_uint2(key, row);
@@ -419,7 +416,9 @@ __global__ void __launch_bounds__(kMultiThreads, 1) k_cand_multi(MultiArgs a) {
     return;
   }
   grid_wait();
-  const bool in_smem = a.split > 1 && a.split <= kThrSmemMax;
+  // (one partition too: 40 queries of 2M x 1024, 8 bits, the whole call 324 us; with its four thresholds
+  // read from global memory between a hit's atomics 340, before them 335 and 24 bytes of spills)
+  const bool in_smem = a.split <= kThrSmemMax;
   if (in_smem)
     for (uint32_t i = threadIdx.x; i < a.split * kMultiQ; i += kMultiThreads) {
       const uint32_t p = i / kMultiQ, t = i % kMultiQ;
